@@ -256,6 +256,8 @@ __device__ __forceinline__ void block_sort_desc(float* key, uint32_t* id, int n)
     __syncthreads();
 }
 
+__device__ __forceinline__ int pow2_ceil_dev(int v) { return v <= 1 ? 1 : 1 << (32 - __clz(v - 1)); }
+
 // Largest-value update of a float in global memory (compare-and-swap; a few writers at most).
 __device__ __forceinline__ void atomic_max_f32(float* addr, float v) {
     int* ai = reinterpret_cast<int*>(addr);
@@ -265,6 +267,14 @@ __device__ __forceinline__ void atomic_max_f32(float* addr, float v) {
         old = atomicCAS(ai, assumed, __float_as_int(v));
         if (old == assumed) break;
     }
+}
+
+// Folds sqrt(sq) into the largest row norm (its bits, zero-initialised: norms are >= 0, so bit patterns
+// order like values).  A plain read first: all but a few dozen of a million rows find a larger norm
+// already there, and a million atomics on one address take 0.7 ms.
+__device__ __forceinline__ void max_norm_update(unsigned int* maxnorm_bits, float sq) {
+    const unsigned int v = __float_as_uint(sqrtf(sq));
+    if (*reinterpret_cast<volatile unsigned int*>(maxnorm_bits) < v) atomicMax(maxnorm_bits, v);
 }
 
 #endif  // __CUDACC__

@@ -64,7 +64,7 @@ __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
     if (lane == 0) {
         hnorm[row] = 0.5f * s;
-        atomicMax(maxnorm_bits, __float_as_uint(sqrtf(s)));
+        max_norm_update(maxnorm_bits, s);
     }
     if (lane < PLANE_AUG_COLS) {
         const float nh = -0.5f * s;
