@@ -67,6 +67,11 @@ SIGNATURES = {
     "fl_debug_tc_experiment": (c_int, [c_int, ctypes.c_uint]),
     "fl_debug_tc_prof_read": (c_int, [c_void_p, c_int]),
     "fl_knn_resolve_mode": (c_int, [c_int64, c_int64, c_int, c_int]),
+    "fl_publish_status": (c_int, [c_void_p, c_void_p, c_void_p]),
+    "fl_knn_wants_plane": (c_int, [c_int64, c_int64, c_int, c_int]),
+    "fl_knn_search": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int,
+                              c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
+                              c_void_p]),
     "fl_debug_knn_tc_scores": (c_int, [c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_void_p, c_int64,
                                        c_void_p, c_int64, c_void_p, c_void_p]),
     "fl_topk_merge_f32": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
@@ -160,8 +165,15 @@ def check(rc: int, what: str = "") -> None:
     raise FlashlibError(msg)
 
 
+_device_ok = False
+
+
 def require_device() -> None:
     """Raise unless an sm_100 device is visible; there is nothing to fall back to."""
-    if not load().fl_device_ok():
+    global _device_ok
+    if _device_ok:
+        return
+    _device_ok = bool(load().fl_device_ok())
+    if not _device_ok:
         raise RuntimeError("flashlib_b200 needs an NVIDIA B200 (sm_100) device; "
                            "no CPU or other-GPU fallback exists")

@@ -86,6 +86,9 @@ __global__ void ivf_halfnorm_kernel(const float* __restrict__ x, int64_t n, int 
     if (lane == 0) out[row] = 0.5f * s;
 }
 
+// Up to this many (query, probe) pairs the few-query scan takes the fine scan: every pair reads its list.
+constexpr int64_t IVF_DIRECT_PAIRS = 8192;
+
 struct IvfWs {
     int K1, bq;
     int64_t max_items;
@@ -115,6 +118,8 @@ static IvfWs ivf_ws_plan(int64_t nq, int nprobe, int nlist, int64_t m, int k) {
     w.off_part_id = take(cur, npairs * w.K1 * 4);
     w.off_hnorm = take(cur, m * 4);
     w.off_tau = take(cur, nq * 4);
+    const int64_t direct = direct_ivf_workspace_bytes(npairs, direct_ivf_chunks(npairs), k);
+    if (npairs <= IVF_DIRECT_PAIRS && direct > cur) cur = direct;
     w.bytes = cur;
     return w;
 }
@@ -338,6 +343,14 @@ extern "C" int fl_ivf_fine_scan_f32(const float* q, int64_t nq, int64_t ldq, con
     float* part_sc = reinterpret_cast<float*>(base + w.off_part_sc);
     uint32_t* part_id = reinterpret_cast<uint32_t*>(base + w.off_part_id);
     const int64_t npairs = nq * nprobe;
+    if (npairs <= IVF_DIRECT_PAIRS && direct_supported(nq, m, d, k)) {
+        DirectParams dp{};
+        dp.dt = DT_F32; dp.q = q; dp.ldq = ldq; dp.nq = nq; dp.db = data; dp.m = m; dp.ldb = ldd; dp.d = d;
+        dp.vec = dt_vec_ok(q, ldq, DT_F32) && dt_vec_ok(data, ldd, DT_F32) && d % 4 == 0;
+        dp.k = k; dp.probed = probed; dp.nprobe = nprobe; dp.ivf_nlist = nlist; dp.list_offsets = list_offsets;
+        dp.out_dist = out_dist; dp.out_idx = out_pos;
+        return launch_ivf_direct(dp, base, st);
+    }
 
     const float* hnorm = data_hnorm;
     if (!hnorm) {

@@ -104,7 +104,7 @@ __global__ void ivf_plane_rows_kernel(const float* __restrict__ data, int64_t ld
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
     if (lane == 0) {
         hnorm[row] = 0.5f * s;
-        atomicMax(maxnorm_bits, __float_as_uint(sqrtf(s)));
+        max_norm_update(maxnorm_bits, s);
     }
     if (lane < PLANE_AUG_COLS) {
         const float nh = -0.5f * s;
@@ -671,7 +671,7 @@ static IvfTcWs ivf_tc_plan(int64_t nq, int nprobe, int nlist, int d, int k) {
     w.off_qplane = take(cur, w.cap_rows * w.pitch * 2);
     w.off_tau = take(cur, w.cap_rows * 4);
     w.off_seed_cls = take(cur, w.cap_rows * 32 * 4);
-    w.off_pools = take(cur, w.cap_rows * tc_taus_per_range() * tc_pair_pool_cap() * 8);
+    w.off_pools = take(cur, w.cap_rows * tc_taus_per_range() * tc_pair_pool_cap(k) * 8);
     w.off_part_cnt = take(cur, w.cap_rows * tc_taus_per_range() * 4);
     w.off_part_tau = take(cur, w.cap_rows * tc_taus_per_range() * 4);
     w.off_fblist = take(cur, nq * 4);

@@ -24,7 +24,7 @@ __global__ void halfnorm_kernel(const void* __restrict__ x, int64_t n, int d, in
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
     if (lane == 0) {
         out[row] = 0.5f * s;
-        atomicMax(maxnorm_bits, __float_as_uint(sqrtf(s)));    // norms are >= 0: their bit patterns order like the values
+        max_norm_update(maxnorm_bits, s);
     }
 }
 
@@ -49,6 +49,48 @@ __global__ void query_plane_kernel(const void* __restrict__ q, int64_t nq, int64
         else if (c >= d_pad && c < d_pad + 3) v = 1.f;
     }
     out[i] = __float2bfloat16_rn(v);
+}
+
+// What a tensor-core call needs before its first scoring launch, in one pass: the bf16 query plane, the
+// starting thresholds (-inf; +inf for the rows that pad the last tile, so that nothing is ever a
+// candidate for them) and cleared counters and status words.  One warp per plane row.
+__global__ void __launch_bounds__(256) knn_prep_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
+                                                       __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt,
+                                                       float* __restrict__ tau, int* __restrict__ counters,
+                                                       int32_t* __restrict__ status) {
+    if (blockIdx.x == 0) {
+        counters[threadIdx.x] = 0;
+        if (status != nullptr && threadIdx.x < FL_STATUS_WORDS) status[threadIdx.x] = 0;
+    }
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= nq_pad) return;
+    const int pitch = d_pad + PLANE_AUG_COLS;              // (a multiple of 16 columns: rows are 32-byte aligned)
+    __nv_bfloat16* o = out + row * pitch;
+    const bool live = row < nq;
+    const void* p = row_at(q, live ? row : 0, ldq, dt);
+    for (int c = lane * 4; c < pitch; c += 128) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live) {
+            if (c < d) {
+                if (vec) v = ld_elem4(p, c, dt);
+                else {
+                    v.x = ld_elem(p, c, dt);
+                    if (c + 1 < d) v.y = ld_elem(p, c + 1, dt);
+                    if (c + 2 < d) v.z = ld_elem(p, c + 2, dt);
+                    if (c + 3 < d) v.w = ld_elem(p, c + 3, dt);
+                }
+            } else if (c == d_pad) {
+                v = make_float4(1.f, 1.f, 1.f, 0.f);
+            }
+        }
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+        uint2 w;
+        w.x = *reinterpret_cast<const uint32_t*>(&a);
+        w.y = *reinterpret_cast<const uint32_t*>(&b);
+        *reinterpret_cast<uint2*>(o + c) = w;
+    }
+    if (lane == 0) tau[row] = live ? neg_inf() : pos_inf();
 }
 
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad,
@@ -79,6 +121,20 @@ __global__ void fallback_fixup_kernel(int* fb_count, int fb_cap, int32_t* status
     if (c > fb_cap) *fb_count = fb_cap;
 }
 
+// Copies the status words to mapped host memory and marks them complete (host[FL_STATUS_WORDS] = 1): the
+// host looks at them later without a copy in the stream and without an event.
+__global__ void status_publish_kernel(const int32_t* __restrict__ status, volatile int32_t* host) {
+    if (threadIdx.x < FL_STATUS_WORDS) host[threadIdx.x] = status[threadIdx.x];
+    __threadfence_system();
+    __syncwarp();
+    if (threadIdx.x == 0) host[FL_STATUS_WORDS] = 1;
+}
+int launch_status_publish(const int32_t* status, int32_t* host, cudaStream_t st) {
+    status_publish_kernel<<<1, 32, 0, st>>>(status, host);
+    FL_CHECK_LAUNCH();
+    return FL_OK;
+}
+
 int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t st) {
     fill_f32_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(p, n, v);
     FL_CHECK_LAUNCH();
@@ -95,6 +151,8 @@ struct KnnWs {
     int mode, K1, K1f;
     int kg;                                    // k that selects the tensor-core pool geometry (see knn_geometry_k)
     int deep, plen;                            // tensor-core path: deep pools, published entries per (query, range)
+    int small;                                 // latency-bound call (tc_small): global pair pools
+    TcSeedPlan seed;                           // seeding sample (splits 0: the one-CTA sample of tc_seed_tiles, or none)
     int nsplit; int64_t rows_per_split;        // main pass (SIMT: rows; TC: tiles of 256)
     int nsplit_fb; int64_t rows_per_split_fb;  // fallback pass
     int64_t nq_pad; int d_pad; int fb_cap; int fb_bq, fb_blocks;
@@ -128,7 +186,9 @@ static int knn_stage2_rows(int64_t nq) {
 // query finalisation, the seeding rule of k = 17).
 static int knn_geometry_k(int d, int k) { return (d > 256 && k < 17) ? 17 : k; }
 
-static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int staged = 0) {
+// shared_seed: never the small-problem plan (a row-sharded caller runs the phases one by one with class maxima of its
+// own, [nq_pad][32]; that plan's sample has more classes).
+static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int staged = 0, int shared_seed = 0) {
     KnnWs w{};
     w.mode = mode;
     w.kg = k;
@@ -142,7 +202,14 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.nq_pad = tc_query_rows_padded(nq);
         w.d_pad = (int)round_up(d, 64);
         const int64_t m_pad = round_up(m, 256);
-        tc_split_plan(w.nq_pad, m_pad, k, &w.nsplit, &w.rows_per_split);
+        w.small = !shared_seed && (tc_small(w.nq_pad, m_pad) || d > 512);
+        if (w.small) {
+            w.kg = k_real;                                 // (no pool in shared memory whatever d is)
+            tc_small_split(w.nq_pad, m_pad, &w.nsplit, &w.rows_per_split);
+        } else {
+            tc_split_plan(w.nq_pad, m_pad, k, &w.nsplit, &w.rows_per_split);
+        }
+        if (!shared_seed) tc_seed_plan(w.nq_pad, m_pad, k_real, &w.seed);
         // Every query may fail its proof (near-duplicate or offset data): the list holds them all, so
         // no row is ever returned unproven.  The exact pass sizes its partial storage by blocks, not
         // by rows x ranges (simt_dyn_split), so the cost of the full list is nq pools of K1f entries.
@@ -158,14 +225,19 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.nsplit_fb = (int)ceil_div(m, w.rows_per_split_fb);
         w.off_hnorm = -1;
         w.off_qplane = take(cur, w.nq_pad * (w.d_pad + PLANE_AUG_COLS) * 2);
-        w.deep = tc_use_deep_pools(k, w.d_pad, w.nsplit, w.nq_pad);
+        w.deep = !w.small && tc_use_deep_pools(k, w.d_pad, w.nsplit, w.nq_pad);
         w.plen = w.deep ? tc_deep_partial_len() : tc_partial_len(k);
         if (w.deep) w.K1 = tc_deep_pool_size();
-        w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
-        w.off_part_id = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
+        if (w.small) {
+            w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)(tc_taus_per_range() * tc_pair_pool_cap(k_real)) * 8);
+            w.off_part_id = w.off_part_sc;
+        } else {
+            w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
+            w.off_part_id = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
+        }
         w.off_part_tau = take(cur, w.nq_pad * w.nsplit * tc_taus_per_range() * 4);
         w.off_part_cnt = take(cur, w.nq_pad * w.nsplit * tc_taus_per_range() * 4);
-        w.off_seed_cls = take(cur, w.nq_pad * 32 * 4);
+        w.off_seed_cls = take(cur, w.nq_pad * (w.seed.splits > 1 ? w.seed.splits : 1) * 32 * 4);
         w.off_tau = take(cur, w.nq_pad * 4);
         w.off_cert = take(cur, w.nq_pad * 4);
         w.off_cnt = take(cur, 1024);
@@ -211,6 +283,10 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.off_part_sc = take(cur, nq * w.nsplit * (int64_t)w.K1 * 4);
         w.off_part_id = take(cur, nq * w.nsplit * (int64_t)w.K1 * 4);
         w.off_cnt = take(cur, 1024);
+        if (direct_pick(nq, m, d, k)) {
+            const int64_t direct = direct_workspace_bytes(nq, m, d, k);
+            if (direct > cur) cur = direct;
+        }
     }
     w.bytes = cur;
     return w;
@@ -293,8 +369,24 @@ extern "C" int fl_knn_resolve_mode(int64_t nq, int64_t m, int d, int k) {
 
 extern "C" int64_t fl_knn_workspace_bytes(int64_t nq, int64_t m, int d, int k, int mode) {
     if (nq < 1 || m < 1 || d < 1 || k < 1) return 0;
+    const bool wide = mode == FL_KNN_AUTO && tc_wide_supported(nq, m, d, k);
     mode = resolve_mode(nq, m, d, k, mode);
-    return knn_ws_plan(nq, m, d, k, mode).bytes;
+    int64_t bytes = knn_ws_plan(nq, m, d, k, mode).bytes;
+    // one size for both flows: the phases of a row-sharded caller, and (more than 512 features) either kernel
+    if (mode == FL_KNN_BF16_RERANK) {
+        const int64_t b = knn_ws_plan(nq, m, d, k, mode, 0, 1).bytes;
+        if (b > bytes) bytes = b;
+    }
+    if (wide) {
+        const int64_t b = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK).bytes;
+        if (b > bytes) bytes = b;
+    }
+    return bytes;
+}
+
+extern "C" int fl_knn_wants_plane(int64_t nq, int64_t m, int d, int k) {
+    if (nq < 1 || m < 1 || d < 1 || k < 1) return 0;
+    return tc_knn_auto(nq, m, d, k) || tc_wide_supported(nq, m, d, k);
 }
 
 // Argument checks shared by the kNN entry points; resolves FL_KNN_AUTO.
@@ -339,7 +431,10 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
                          int d, int k, const void* plane, int64_t row_offset, float* seed_cls, const float* gmaxnorm,
                          float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status,
                          cudaStream_t st, const void* split_plane = nullptr, int dt = DT_F32) {
-    const KnnWs w = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, split_plane != nullptr);
+    const bool whole = phases == (TC_PREP | TC_SEED | TC_SCORE);
+    // (the timing experiments belong to the screening epilogue of the large-problem plan)
+    const KnnWs w = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, split_plane != nullptr, !whole || tc_debug_active());
+    const float eps1 = tc_eps_rel(dt, d);
     if (ws_bytes < w.bytes) {
         set_error("fl_knn: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes);
         return FL_EWORKSPACE;
@@ -351,6 +446,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     const PlaneLayout L = plane_layout(m, d);
     const char* pl = static_cast<const char*>(plane);
     int* fb_count = reinterpret_cast<int*>(base + w.off_cnt);
+    if (status == nullptr) status = fb_count + 192;        // (cleared with the counters)
     int* fb_list = reinterpret_cast<int*>(base + w.off_fblist);
     float* tau = reinterpret_cast<float*>(base + w.off_tau);
     float* cert = reinterpret_cast<float*>(base + w.off_cert);
@@ -363,6 +459,8 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     tp.nsplit = w.nsplit; tp.tiles_per_split = w.rows_per_split;
     tp.part_sc = reinterpret_cast<float*>(base + w.off_part_sc);
     tp.part_id = reinterpret_cast<uint32_t*>(base + w.off_part_id);
+    if (w.small) tp.pair_pools = base + w.off_part_sc;
+    tp.seed_tiles = w.seed.tiles; tp.seed_splits = w.seed.splits; tp.seed_rank = w.seed.rank;
     tp.tau = tau; tp.status = status;
     tp.part_tau = reinterpret_cast<float*>(base + w.off_part_tau);
     tp.part_cnt = reinterpret_cast<int*>(base + w.off_part_cnt);
@@ -371,15 +469,15 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     tp.k = w.kg;
     int rc;
 
-    if (phases & TC_SCORE) FL_CHECK_CUDA(cudaMemsetAsync(fb_count, 0, 1024, st));
     if (phases & TC_PREP) {
-        if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
-        rc = launch_fill_f32(tau, w.nq_pad, -INFINITY, st);
-        if (rc != FL_OK) return rc;
-        rc = launch_query_plane(q, nq, ldq, d, base + w.off_qplane, w.nq_pad, w.d_pad, st, dt);
-        if (rc != FL_OK) return rc;
+        knn_prep_kernel<<<(unsigned)ceil_div(w.nq_pad, 8), 256, 0, st>>>(q, nq, ldq, d, vecq && d % 4 == 0,
+            reinterpret_cast<__nv_bfloat16*>(base + w.off_qplane), w.nq_pad, w.d_pad, dt, tau, fb_count, status);
+        FL_CHECK_LAUNCH();
+    } else {
+        FL_CHECK_CUDA(cudaMemsetAsync(fb_count, 0, 1024, st));
     }
-    if (phases & TC_SEED) {
+    const bool seeded = !w.small || w.seed.splits > 1;
+    if ((phases & TC_SEED) && seeded) {
         if (phases & TC_SCORE) profile_begin(st);
         rc = launch_knn_tc_seed(tp, st);
         if (rc != FL_OK) return rc;
@@ -387,20 +485,23 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     if (!(phases & TC_SCORE)) return FL_OK;
 
     if (!(phases & TC_PREP)) {
-        rc = launch_fill_f32(tau, w.nq_pad, -INFINITY, st);
+        rc = launch_fill_f32(tau, nq, -INFINITY, st);
+        if (rc == FL_OK && w.nq_pad > nq) rc = launch_fill_f32(tau + nq, w.nq_pad - nq, INFINITY, st);
         if (rc != FL_OK) return rc;
     }
-    if (!(phases & TC_SEED)) profile_begin(st);
+    if (!(phases & TC_SEED) || !seeded) profile_begin(st);
     TcSeedMargin mg{};
     mg.dt = dt;
     if (gmaxnorm != nullptr) {
-        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.maxnorm = gmaxnorm; mg.eps_rel = 0.004f; mg.cert_out = cert;
-    } else if (tc_seed_dense(L.m_pad, w.kg)) {
-        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.eps_rel = 0.004f; mg.cert_out = nullptr;
+        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.maxnorm = gmaxnorm; mg.eps_rel = eps1; mg.cert_out = cert;
+    } else if (w.seed.splits > 1 ? w.seed.dense : tc_seed_dense(L.m_pad, w.kg)) {
+        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.eps_rel = eps1; mg.cert_out = nullptr;
         mg.maxnorm = reinterpret_cast<const float*>(pl + L.off_meta);
     }
-    rc = launch_knn_tc_seed_select(tp, mg, st);
-    if (rc != FL_OK) return rc;
+    if (seeded) {
+        rc = launch_knn_tc_seed_select(tp, mg, st);
+        if (rc != FL_OK) return rc;
+    }
     rc = launch_knn_tc_scoring(tp, st);
     profile_end(st);
     if (rc != FL_OK) return rc;
@@ -415,7 +516,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     fp.k = k; fp.rerank = fp.K1; fp.row_offset = row_offset;
     fp.part_tau = tp.part_tau; fp.ntau = w.nsplit * tc_taus_per_range();
     fp.out_dist = out_dist; fp.out_idx = out_idx;
-    fp.verify = 1; fp.eps_rel = 0.004f;  // 2^-8 operand rounding of both bf16 factors, rounded up
+    fp.verify = 1; fp.eps_rel = eps1;
     // a sharded caller's error bound must hold for rows of every shard: the largest norm of all
     fp.maxnorm = gmaxnorm != nullptr ? gmaxnorm : reinterpret_cast<const float*>(pl + L.off_meta);
     fp.cert_tau = gmaxnorm != nullptr ? cert : nullptr;
@@ -424,7 +525,19 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     int* s2_count = fb_count + 64;
     int* s2_list = w.s2 ? reinterpret_cast<int*>(base + w.off_s2_list) : nullptr;
     if (w.s2) { fp.next_count = s2_count; fp.next_list = s2_list; fp.next_cap = w.s2_cap; }
-    rc = tc_knn_big(w.kg) ? launch_knn_finalize_big(fp, nq, st) : launch_knn_finalize(fp, nq, st);
+    if (w.small) {
+        PairFinalizeParams pf{};
+        pf.dt = dt; pf.q = q; pf.ldq = ldq; pf.nq = nq; pf.db = db; pf.m = m; pf.ldb = ldb; pf.d = d; pf.vec = vec;
+        pf.pools = static_cast<const float2*>(tp.pair_pools); pf.pool_cnt = tp.part_cnt; pf.pool_tau = tp.part_tau;
+        pf.cap = tc_pair_pool_cap(k); pf.npool = w.nsplit * tc_taus_per_range();
+        pf.k = k; pf.eps_rel = eps1; pf.maxnorm = fp.maxnorm; pf.row_offset = row_offset;
+        pf.out_dist = out_dist; pf.out_idx = out_idx;
+        pf.fb_count = fb_count; pf.fb_list = fb_list; pf.fb_cap = w.fb_cap;
+        pf.next_count = fp.next_count; pf.next_list = fp.next_list; pf.next_cap = fp.next_cap;
+        rc = launch_pairs_finalize(pf, st);
+    } else {
+        rc = tc_knn_big(w.kg) ? launch_knn_finalize_big(fp, nq, st) : launch_knn_finalize(fp, nq, st);
+    }
     if (rc != FL_OK) return rc;
 
     // Second stage: the rejected rows are scored again with split (hi/lo) operands -- an error
@@ -494,6 +607,8 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
                          int d, int k, int dt, int mode, const void* plane, const void* split_plane, int64_t row_offset,
                          float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status, void* stream) {
     FL_CHECK_ARG(dt == DT_F32 || dt == DT_BF16 || dt == DT_F16, "%s: unknown dtype %d", who, dt);
+    // more than 512 features: the automatic mode takes the tensor cores when it is given an operand plane
+    const bool wide = mode == FL_KNN_AUTO && plane != nullptr && nq > 0 && tc_wide_supported(nq, m, d, k);
     int rc = knn_check_args(who, q, nq, ldq, db, m, ldb, d, k, &mode, plane, row_offset, out_dist, out_idx, ws);
     if (rc != FL_OK || nq == 0) return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -502,7 +617,7 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
         FL_CHECK_ARG(split_plane_supported(d), "%s: d=%d > 128 has no split plane", who, d);
         FL_CHECK_ARG((reinterpret_cast<uintptr_t>(split_plane) & 255) == 0, "%s: split plane must be 256-byte aligned", who);
     }
-    if (mode == FL_KNN_BF16_RERANK)
+    if (mode == FL_KNN_BF16_RERANK || wide)
         return knn_tc_phases(TC_PREP | TC_SEED | TC_SCORE, q, nq, ldq, db, m, ldb, d, k, plane, row_offset, nullptr,
                              nullptr, out_dist, out_idx, ws, ws_bytes, status, st, split_plane, dt);
 
@@ -515,6 +630,14 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
     const int vecq = dt_vec_ok(q, ldq, dt);
     const int vecd = dt_vec_ok(db, ldb, dt);
     const int vec = vecq && vecd && (d % 4 == 0);
+    if (direct_pick(nq, m, d, k)) {
+        DirectParams dp{};
+        dp.dt = dt; dp.q = q; dp.ldq = ldq; dp.nq = nq;
+        dp.db = db; dp.m = m; dp.ldb = ldb; dp.d = d; dp.vec = vec;
+        dp.k = k; dp.row_offset = row_offset;
+        dp.out_dist = out_dist; dp.out_idx = out_idx; dp.status = status;
+        return launch_knn_direct(dp, base, st);
+    }
     if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
     FL_CHECK_CUDA(cudaMemsetAsync(base + w.off_cnt, 0, 1024, st));
     const float* hnorm;
@@ -565,6 +688,24 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
         FL_CHECK_LAUNCH();
     }
     return FL_OK;
+}
+
+extern "C" int fl_publish_status(const int32_t* status, int32_t* host_status, void* stream) {
+    FL_CHECK_ARG(status && host_status, "fl_publish_status: null pointer");
+    return launch_status_publish(status, host_status, (cudaStream_t)stream);
+}
+
+// Everything fl_knn_rows and fl_knn_staged_f32 do, plus `host_status` (optional): mapped host memory of
+// FL_STATUS_WORDS + 1 words that receives the status words and then a completion mark.
+extern "C" int fl_knn_search(const void* q, int64_t nq, int64_t ldq, const void* db, int64_t m, int64_t ldb, int d, int k,
+                             int dtype, int mode, const void* plane, const void* split_plane, int64_t row_offset,
+                             float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status,
+                             int32_t* host_status, void* stream) {
+    const int rc = knn_rows_impl("fl_knn_search", q, nq, ldq, db, m, ldb, d, k, dtype, mode, plane, split_plane, row_offset,
+                                 out_dist, out_idx, ws, ws_bytes, status, stream);
+    if (rc != FL_OK || nq == 0 || host_status == nullptr) return rc;
+    FL_CHECK_ARG(status != nullptr, "fl_knn_search: host_status needs status");
+    return launch_status_publish(status, host_status, (cudaStream_t)stream);
 }
 
 extern "C" int fl_knn_f32(const float* q, int64_t nq, int64_t ldq, const float* db, int64_t m,
@@ -749,7 +890,8 @@ extern "C" int fl_knn_prepare_split_f32(const float* db, int64_t m, int d, int64
 
 extern "C" int64_t fl_knn_staged_workspace_bytes(int64_t nq, int64_t m, int d, int k) {
     if (nq < 1 || m < 1 || d < 1 || k < 1 || tc_knn_supported(nq, m, d, k) != FL_OK) return 0;
-    return knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, 1).bytes;
+    const int64_t a = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, 1).bytes, b = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, 1, 1).bytes;
+    return a > b ? a : b;
 }
 
 extern "C" int fl_knn_staged_f32(const float* q, int64_t nq, int64_t ldq, const float* db, int64_t m, int64_t ldb, int d,

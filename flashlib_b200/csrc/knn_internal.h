@@ -68,6 +68,31 @@ void simt_split_plan(int64_t slots, int64_t m, int K1, int d, int* nsplit, int64
 // Queries per block the CUDA-core pass uses for a pool of K1 entries (0: does not fit).
 int simt_block_queries(int K1);
 
+// Exact scan for few queries (knn_direct.cu): fp32 sum (q - x)^2 of every (query, row) pair from the stored
+// values, in two launches (scan, merge).
+struct DirectParams {
+    int dt;                  // element type of the q and db rows (DT_*; leading dimensions in elements)
+    const void* q; int64_t ldq; int64_t nq;
+    const void* db; int64_t m; int64_t ldb; int d; int vec;   // vec: as FinalizeParams::vec
+    int k; int64_t row_offset;
+    // inverted-file scan (probed != nullptr): pair i = (query i / nprobe, list probed[i])
+    const int32_t* probed; int nprobe; int ivf_nlist; const int64_t* list_offsets;
+    float* out_dist; int32_t* out_idx;       // out_idx (rows) and out_ids (id_map64[row]) are each optional
+    int64_t* out_ids; const int64_t* id_map64;
+    int32_t* status;         // optional
+    // filled in by the launch functions
+    int npl, nchunk, lists_per_query; int64_t rows_per_chunk;
+    float* part_key; uint32_t* part_id;
+};
+int direct_supported(int64_t nq, int64_t m, int d, int k);
+int direct_pick(int64_t nq, int64_t m, int d, int k);      // 1: the exact mode takes this scan for the shape
+double direct_estimate_us(int64_t nq, int64_t m, int d);
+int64_t direct_workspace_bytes(int64_t nq, int64_t m, int d, int k);
+int launch_knn_direct(DirectParams p, void* ws, cudaStream_t st);
+int direct_ivf_chunks(int64_t npairs);
+int64_t direct_ivf_workspace_bytes(int64_t npairs, int nchunk, int k);
+int launch_ivf_direct(DirectParams p, void* ws, cudaStream_t st);
+
 // Merge of the per-split pools, exact fp32 re-rank, top-k selection and (optionally)
 // verification of the candidate pool against the scoring error bound.
 struct FinalizeParams {
@@ -101,6 +126,21 @@ struct FinalizeParams {
     // pools and its outputs follow those of problem b - 1.
     int batch; int64_t q_bstride, db_bstride;
 };
+// Finalisation of the global pair pools (one block per query): see knn_pairs.cu.
+struct PairFinalizeParams {
+    int dt; const void* q; int64_t ldq; int64_t nq;
+    const void* db; int64_t m; int64_t ldb; int d; int vec;
+    const float2* pools; const int* pool_cnt; const float* pool_tau;
+    int cap;                 // slots per pool
+    int npool;               // pools per query: pool i of query q is number q * npool + i, or, with pair_row,
+    const int* pair_row;     //   2 * pair_row[q * npool / 2 + i / 2] + i % 2 (pair_row < 0: none)
+    const int* row_map; int64_t rows_max;    // optional: published id -> row (< 0: padding)
+    int k; float eps_rel; const float* maxnorm; int64_t row_offset;
+    float* out_dist; int32_t* out_idx;
+    int* fb_count; int* fb_list; int fb_cap;
+    int* next_count; int* next_list; int next_cap;
+};
+int launch_pairs_finalize(const PairFinalizeParams& p, cudaStream_t st);
 // Finalisation of the large-k tensor-core pools (one block per query).
 int launch_knn_finalize_big(const FinalizeParams& p, int64_t max_slots, cudaStream_t st);
 int launch_knn_finalize(const FinalizeParams& p, int64_t max_slots, cudaStream_t st);
@@ -118,7 +158,8 @@ struct TcKnnParams {
     float* tau;              // f32 [nq_pad], running per-query thresholds, -inf initialised
     float* part_tau;         // f32 [nq_pad][nsplit][tc_taus_per_range]: thresholds each (query, range) ended with
     int* part_cnt;           // large-k pools only: i32 [nq_pad][nsplit][tc_taus_per_range] entries per pool
-    float* seed_cls;         // f32 [nq_pad][32] scratch of the threshold-seeding pass (nullptr: no seeding)
+    float* seed_cls;         // f32 [nq_pad][max(1, seed_splits)][32] scratch of the threshold-seeding pass (nullptr: no seeding)
+    int seed_tiles, seed_splits, seed_rank;   // > 0: sample and rank of tc_seed_plan
     int deep_pools;          // 1: pools keep tc_deep_pool_size() entries and publish tc_deep_partial_len() per
                              //    (query, range) (k <= 16): for queries with only a few pools each
     const int* nq_dev;       // optional: live query rows (device); query tiles beyond them are skipped
@@ -128,8 +169,8 @@ struct TcKnnParams {
     const int* item_t1;      //   query tile t instead of one uniform range (inverted-file scan)
     int item_tile_cap;       // seeding pass over item tables: tiles of every item's range it samples
     const int* item_order;   // optional, with item tables: order in which the items are dealt to the CTAs
-    void* pair_pools;        // optional (k <= 16): pools kept in global memory as (score f32, row u32) pairs,
-                             //   [nq_pad][nsplit][tc_taus_per_range][tc_pair_pool_cap]; entry counts go to
+    void* pair_pools;        // optional: pools kept in global memory as (score f32, row u32) pairs,
+                             //   [nq_pad][nsplit][tc_taus_per_range][tc_pair_pool_cap(k)]; entry counts go to
                              //   part_cnt, thresholds to part_tau, part_sc / part_id are not used
     int k;                   // neighbours wanted: selects the pool geometry (tc_knn_big)
     int big_pools;           // 1: the large global-memory pools whatever k is (no pool in shared memory:
@@ -148,8 +189,19 @@ int tc_use_deep_pools(int k, int d_pad, int nsplit, int64_t nq_pad);
 int tc_deep_partial_len();
 // Thresholds the tensor-core pass publishes per (query, range).
 int tc_taus_per_range();
-// Slots of a (query row, warpgroup) pool in the global pair-pool mode.
-int tc_pair_pool_cap();
+// Slots of a (query row, warpgroup) pool in the global pair-pool modes.
+int tc_pair_pool_cap(int k);
+// Calls bound by latencies rather than by the tensor pipe, their row ranges, and the seeding sample of any
+// call that is not part of a row-sharded search (splits 0: none).
+struct TcSeedPlan { int tiles, splits, rank, dense; };
+int tc_small(int64_t nq_pad, int64_t m_pad);
+void tc_small_split(int64_t nq_pad, int64_t m_pad, int* nsplit, int64_t* tiles_per_split);
+void tc_seed_plan(int64_t nq_pad, int64_t m_pad, int k, TcSeedPlan* w);
+// Relative bound (of ||q|| max||x||) on the error of the tensor-core scores: 2^-8 for operands rounded to bf16
+// (2 * 2^-9 + 2^-18, plus the accumulation, which is what is left where both sides are stored as bf16).
+float tc_eps_rel(int dt, int d);
+// 1 when rows of this shape (more than 512 features) take the tensor-core path with a streamed query tile.
+int tc_wide_supported(int64_t nq, int64_t m, int d, int k);
 // 1 when FL_KNN_AUTO should take the tensor-core path for this shape.
 int tc_knn_auto(int64_t nq, int64_t m, int d, int k);
 // Margin applied by the threshold selection when the class maxima cover more than this shard's rows
@@ -169,6 +221,7 @@ int launch_knn_tc_scoring(const TcKnnParams& p, cudaStream_t st);
 int tc_seed_dense(int64_t m_pad, int k);
 // Experiment flags of the scoring kernel and the limit of its barrier waits (0: default).
 void tc_debug_set(int flags, unsigned wait_us);
+int tc_debug_active();       // 1 while experiment flags are set
 // Same as launch_knn_tc, additionally dumping the scores of query tile 0 to dbg[128][dbg_ld].
 int tc_prof_read(unsigned long long* host_out, int words);
 int launch_knn_tc_debug(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cudaStream_t st);
@@ -202,6 +255,7 @@ int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qpla
 
 // Small helpers shared by the entry points.
 int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt = DT_F32);
+int launch_status_publish(const int32_t* status, int32_t* host, cudaStream_t st);
 int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t st);
 int launch_ivf_group(const int32_t* probed, int64_t npairs, int nlist, int bq, const int64_t* list_offsets, int* cnt,
                      int* pair_off, int* item_off, int* cursor, int* sorted_pair, cudaStream_t st);

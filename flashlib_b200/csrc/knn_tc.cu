@@ -47,6 +47,9 @@ constexpr int TC_B_CHUNK = TC_BN * 128;   // bytes of one K-chunk of a database 
 constexpr int TC_B_AUG = TC_BN * 32;      // bytes of a database tile's 16 norm columns
 constexpr int TC_B_STAGE = TC_B_CHUNK + TC_B_AUG;   // ring slot: a K-chunk, plus the norm
                                                     // columns when it is the tile's last chunk
+// Streamed query tile (more than 512 features): a slot also holds the query tile's chunk and, for the
+// tile's last chunk, its norm columns.
+constexpr int TC_STREAM_STAGE = TC_B_STAGE + TC_A_CHUNK + TC_A_AUG;
 constexpr int TC_MAX_STAGES = 6;
 constexpr uint64_t TC_WAIT_DEFAULT_NS = 2000000000ull;   // 2 s per wait unless the launch says otherwise
 
@@ -94,6 +97,7 @@ __device__ unsigned long long g_tc_prof[160 * TC_PROF_WORDS];
 struct TcKernelParams {
     int n_qtiles, n_tiles, nsplit, tiles_per_split, nkc, nstage;
     int nabuf;               // query-tile buffers in shared memory (1 or 2)
+    int stream_a;            // 1: the query tile is not resident; its chunk travels with every database chunk
     int off_b, off_pool_sc, off_pool_id, off_bar;
     int64_t nq_pad;
     float* part_sc; uint32_t* part_id;
@@ -108,8 +112,8 @@ struct TcKernelParams {
     int item_tile_cap;       // > 0: at most this many tiles of every table range (seeding over item tables)
     const int* item_order;   // optional, with item tables: the CTAs walk item item_order[i] in place of item i
                              //   (longest ranges first, so that the round-robin deal comes out even)
-    float* seed_cls;         // seeding output: [nq_pad][TC_NWG][16] class maxima
-    float2* gpool;           // global-pool mode: (score, row) pairs, [nq_pad][nsplit][TC_NWG][TC_GP_CAP]
+    float* seed_cls;         // seeding output: [nq_pad][nsplit][TC_NWG][16] class maxima
+    float2* gpool;           // global-pool modes: (score, row) pairs, [nq_pad][nsplit][TC_NWG][CAP]
     float* asg_sc; uint32_t* asg_id;   // assignment mode outputs: [rows][TC_NWG] x (best, second) / centroid
     int32_t* status;
     uint32_t wait_hint_ns;   // suspend-time hint of the barrier waits
@@ -232,8 +236,10 @@ static __device__ __noinline__ float2 tc_compact_rows_pairs(unsigned need, float
 // query row and launch), so their stores and the compactions' reads can afford the L2, and the
 // 67 KB of shared memory the pools took go to the TMA ring (four slots instead of three at 128
 // features, four instead of two at 256).
+//
+// MODE 7 (TC_MODE_KNN_GPOOL_BIG) is MODE 5 with 256 slots, 128 kept, for 16 < k <= 112.
 constexpr int TC_MODE_KNN = 0, TC_MODE_SEED = 1, TC_MODE_ASSIGN = 2, TC_MODE_KNN_BIG = 3, TC_MODE_KNN_MID = 4,
-              TC_MODE_KNN_GPOOL = 5, TC_MODE_KNN_GS = 6;
+              TC_MODE_KNN_GPOOL = 5, TC_MODE_KNN_GS = 6, TC_MODE_KNN_GPOOL_BIG = 7;
 constexpr int TC_GP_K1 = 24, TC_GP_CAP = 64;
 //
 // PAIR: two CTAs of a cluster work as one (tcgen05 cta_group::2).  CTA r of the pair owns query
@@ -284,7 +290,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const bool leader = cta_rank == 0;
     // geometry of one ring slot and of the work split
     constexpr int B_ROWS = PAIR ? TC_BN / 2 : TC_BN;          // database rows this CTA loads per tile
-    constexpr int SLOT_CHUNK = B_ROWS * 128, SLOT_BYTES = B_ROWS * 128 + B_ROWS * 32;
+    constexpr int SLOT_CHUNK = B_ROWS * 128, SLOT_B_BYTES = B_ROWS * 128 + B_ROWS * 32;
+    constexpr bool CAN_STREAM = MODE == TC_MODE_KNN_GPOOL || MODE == TC_MODE_KNN_GPOOL_BIG || MODE == TC_MODE_SEED;
+    const bool stream_a = CAN_STREAM && p.stream_a != 0;
+    const uint32_t slot_bytes = stream_a ? (uint32_t)TC_STREAM_STAGE : (uint32_t)SLOT_B_BYTES;
     constexpr uint32_t OPERAND_CTAS = PAIR ? 2u : 1u;         // CTAs whose loads one operand barrier counts
 
     if (tid == 0) {
@@ -344,13 +353,15 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 int t0, t1;
                 tc_item_range(p, itp, split, t0, t1);
                 const uint32_t ab = a_buf(item_no), a_off = ab * a_stride;
-                if (!mbar_wait(a_empty_bar(ab), a_phase(item_no) ^ 1u, abort_flag, 2 * p.wait_ns, p.wait_hint_ns)) {
-                    tc_report_timeout(p.status, 4, ab ? 19 : B_AEMPTY); ok = false; break;
+                if (!stream_a) {
+                    if (!mbar_wait(a_empty_bar(ab), a_phase(item_no) ^ 1u, abort_flag, 2 * p.wait_ns, p.wait_hint_ns)) {
+                        tc_report_timeout(p.status, 4, ab ? 19 : B_AEMPTY); ok = false; break;
+                    }
+                    if (leader) mbar_expect_tx(a_full_bar(ab), (p.nkc * TC_A_CHUNK + TC_A_AUG) * OPERAND_CTAS);
+                    for (int kc = 0; kc < p.nkc; ++kc)
+                        load(a_addr + a_off + kc * TC_A_CHUNK, &map_q, kc * TC_BK, qt * TC_BM, a_full_bar(ab));
+                    load(a_aug_addr + a_off, &map_q_aug, d_pad, qt * TC_BM, a_full_bar(ab));
                 }
-                if (leader) mbar_expect_tx(a_full_bar(ab), (p.nkc * TC_A_CHUNK + TC_A_AUG) * OPERAND_CTAS);
-                for (int kc = 0; kc < p.nkc; ++kc)
-                    load(a_addr + a_off + kc * TC_A_CHUNK, &map_q, kc * TC_BK, qt * TC_BM, a_full_bar(ab));
-                load(a_aug_addr + a_off, &map_q_aug, d_pad, qt * TC_BM, a_full_bar(ab));
                 const int nt = t1 - t0;
                 const int rot = (int)(((int64_t)unit * nt) / n_units);
                 for (int i = 0; i < nt && ok; ++i) {
@@ -368,9 +379,18 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                         const bool last = (kc == p.nkc - 1);
                         const int row0 = t * p.tile_stride * TC_BN + (int)cta_rank * B_ROWS;
                         if (DBG && (p.dbg_flags & 32) && fill == 3) continue;   // this slot never fills
-                        if (leader) mbar_expect_tx(BAR(B_FULL + s), (last ? SLOT_BYTES : SLOT_CHUNK) * OPERAND_CTAS);
-                        load(b_addr + s * SLOT_BYTES, &map_db, kc * TC_BK, row0, BAR(B_FULL + s));
-                        if (last) load(b_addr + s * SLOT_BYTES + SLOT_CHUNK, &map_db_aug, d_pad, row0, BAR(B_FULL + s));
+                        const uint32_t slot = b_addr + s * slot_bytes;
+                        if (leader) {
+                            uint32_t bytes = (last ? SLOT_B_BYTES : SLOT_CHUNK) * OPERAND_CTAS;
+                            if (stream_a) bytes += TC_A_CHUNK + (last ? TC_A_AUG : 0);
+                            mbar_expect_tx(BAR(B_FULL + s), bytes);
+                        }
+                        load(slot, &map_db, kc * TC_BK, row0, BAR(B_FULL + s));
+                        if (last) load(slot + SLOT_CHUNK, &map_db_aug, d_pad, row0, BAR(B_FULL + s));
+                        if (stream_a) {
+                            load(slot + SLOT_B_BYTES, &map_q, kc * TC_BK, qt * TC_BM, BAR(B_FULL + s));
+                            if (last) load(slot + SLOT_B_BYTES + TC_A_CHUNK, &map_q_aug, d_pad, qt * TC_BM, BAR(B_FULL + s));
+                        }
                     }
                 }
             }
@@ -401,7 +421,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 int t0, t1;
                 tc_item_range(p, itp, split, t0, t1);
                 const uint32_t ab = a_buf(item_no), a_off = ab * a_stride;
-                if (!mbar_wait(a_full_bar(ab), a_phase(item_no), abort_flag, p.wait_ns, p.wait_hint_ns)) {
+                if (!stream_a && !mbar_wait(a_full_bar(ab), a_phase(item_no), abort_flag, p.wait_ns, p.wait_hint_ns)) {
                     tc_report_timeout(p.status, 5, ab ? 18 : B_AFULL); ok = false; break;
                 }
                 for (int t = t0; t < t1 && ok; ++t, ++tile_no) {
@@ -422,22 +442,25 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                         }
                         TC_PROF(prof_full += clock64() - c1;)
                         tc_fence_after_sync();
-                        const uint64_t da = umma_desc(a_addr + a_off + kc * TC_A_CHUNK);
-                        const uint64_t db = umma_desc(b_addr + s * SLOT_BYTES);
+                        const uint32_t slot = b_addr + s * slot_bytes;
+                        const bool last = kc == p.nkc - 1;
+                        const uint64_t da = umma_desc(stream_a ? slot + SLOT_B_BYTES : a_addr + a_off + kc * TC_A_CHUNK);
+                        const uint64_t db = umma_desc(slot);
 #pragma unroll
                         for (int k4 = 0; k4 < TC_BK / 16; ++k4) {
                             // +32 bytes per 16-feature step inside the 128-byte swizzled row
                             mma(d_tmem, da + 2 * k4, db + 2 * k4, (kc | k4) != 0 ? 1u : 0u);
                         }
-                        if (kc == p.nkc - 1 && !(DBG && (p.dbg_flags & 8))) {
+                        if (last && !(DBG && (p.dbg_flags & 8))) {
                             // norm columns: ones x split(-||x||^2/2), 32-byte rows, 32-byte swizzle
-                            mma(d_tmem, umma_desc_sw32(a_aug_addr + a_off), umma_desc_sw32(b_addr + s * SLOT_BYTES + SLOT_CHUNK), 1u);
+                            const uint32_t a_aug = stream_a ? slot + SLOT_B_BYTES + TC_A_CHUNK : a_aug_addr + a_off;
+                            mma(d_tmem, umma_desc_sw32(a_aug), umma_desc_sw32(slot + SLOT_CHUNK), 1u);
                         }
                         commit(BAR(B_EMPTY + s));   // slot reusable once these MMAs retire
                     }
                     if (ok) commit(BAR(B_TFULL + b));
                 }
-                if (ok) commit(a_empty_bar(ab));     // query tile buffer reusable
+                if (ok && !stream_a) commit(a_empty_bar(ab));     // query tile buffer reusable
             }
             TC_PROF(if (blockIdx.x < 160) {
                 g_tc_prof[blockIdx.x * TC_PROF_WORDS + 1] = prof_full;
@@ -453,9 +476,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         constexpr bool GS = (MODE == TC_MODE_KNN_GS);
         constexpr bool GLOB = BIG || GS;                 // pools addressed in global memory
         constexpr bool MID = (MODE == TC_MODE_KNN_MID);
-        constexpr bool GP = (MODE == TC_MODE_KNN_GPOOL);
-        constexpr int CAP = BIG ? TC_BIG_CAP : MID ? TC_MID_CAP : GP ? TC_GP_CAP : TC_CAP;
-        constexpr int K1 = BIG ? TC_BIG_K1 : MID ? TC_MID_K1 : GP ? TC_GP_K1 : TC_K1;
+        constexpr bool GPB = (MODE == TC_MODE_KNN_GPOOL_BIG);
+        constexpr bool GP = (MODE == TC_MODE_KNN_GPOOL) || GPB;
+        constexpr int CAP = (BIG || GPB) ? TC_BIG_CAP : MID ? TC_MID_CAP : GP ? TC_GP_CAP : TC_CAP;
+        constexpr int K1 = (BIG || GPB) ? TC_BIG_K1 : MID ? TC_MID_K1 : GP ? TC_GP_K1 : TC_K1;
         constexpr int PSTR = CAP + 1;                    // shared pools: padded stride, slot CAP is scratch
         constexpr int PUB = BIG ? TC_BIG_CAP : MID ? TC_MID_PUB : TC_CAP;   // published entries per pool
         // pool of lane 0's row and distance (elements) between the pools of consecutive rows
@@ -594,13 +618,14 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                     fold(vd);
                     continue;
                 }
-                if (GP) {
-                    // this row's pool in global memory and the address of its next free slot
-                    float2* warp_pool = p.gpool + (((int64_t)(qt * TC_BM + quarter * 32) * p.nsplit + split) * TC_NWG + wg) * CAP;
-                    const int gstride = p.nsplit * TC_NWG * CAP;      // pairs between the pools of consecutive rows
+                if (GP || MID) {
+                    // This row's pool of (score, row) pairs -- in global memory (GP) or shared memory (MID) --
+                    // and the address of its next free slot.
+                    float2* warp_pool = GP ? p.gpool + (((int64_t)(qt * TC_BM + quarter * 32) * p.nsplit + split) * TC_NWG + wg) * CAP
+                                           : reinterpret_cast<float2*>(pool_sc) + warp * 32 * PSTR;
+                    const int gstride = GP ? p.nsplit * TC_NWG * CAP : PSTR;      // pairs between the pools of consecutive rows
                     const uint64_t my_addr = reinterpret_cast<uint64_t>(warp_pool + (int64_t)lane * gstride);
-                    uint64_t waddr = my_addr + 8ull * (uint64_t)cnt;
-                    const uint64_t lim = my_addr + 8ull * (uint64_t)(CAP - 8);
+                    const uint32_t my_saddr = MID ? smem_u32(warp_pool + lane * gstride) : 0u;
                     tmem_ld_32x32b_x32(tile_taddr, va);
                     tmem_ld_32x32b_x32(tile_taddr + 32, vb);
                     tmem_ld_32x32b_x32(tile_taddr + 64, vc);
@@ -613,112 +638,75 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0) release_acc(b);
-                    auto dense = [&](uint32_t (&v)[32], int slice) {
+                    // Which groups of 8 columns hold a score above the threshold of any row of the warp:
+                    // branch-free maxima, one vote for the tile.  Only those are compared score by score --
+                    // appending every group costs a chain of 128 address increments, 2.6 us per tile.
+                    unsigned wm = 0;
+                    auto screen = [&](uint32_t (&v)[32], int slice) {
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
-                            if (__any_sync(FULL_MASK, waddr > lim)) {
-                                cnt = (int)((waddr - my_addr) >> 3);
-                                const unsigned need = __ballot_sync(FULL_MASK, cnt > CAP - 8);
-                                TC_PROF(prof_compact += __popc(need);)
-                                const float2 cr = tc_compact_rows_pairs<CAP, K1>(need, warp_pool, gstride, cnt, tau);
-                                cnt = __float_as_int(cr.x);
-                                tau = cr.y;
-                                waddr = my_addr + 8ull * (uint64_t)cnt;
-                            }
-                            // the 8 comparisons first (independent), then the predicated stores: only
-                            // the address increments form a chain
-                            const uint32_t col0 = row_base + slice * 32 + g * 8;
-                            const uint32_t* x = v + g * 8;
-                            asm volatile(
-                                "{\n\t.reg .pred p0, p1, p2, p3, p4, p5, p6, p7;\n\t.reg .b32 c;\n\t"
-                                "setp.gt.f32 p0, %3, %1;\n\tsetp.gt.f32 p1, %4, %1;\n\tsetp.gt.f32 p2, %5, %1;\n\tsetp.gt.f32 p3, %6, %1;\n\t"
-                                "setp.gt.f32 p4, %7, %1;\n\tsetp.gt.f32 p5, %8, %1;\n\tsetp.gt.f32 p6, %9, %1;\n\tsetp.gt.f32 p7, %10, %1;\n\t"
-                                "@p0 st.global.v2.b32 [%0], {%11, %2};\n\t@p0 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 1;\n\t"
-                                "@p1 st.global.v2.b32 [%0], {%12, c};\n\t@p1 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 2;\n\t"
-                                "@p2 st.global.v2.b32 [%0], {%13, c};\n\t@p2 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 3;\n\t"
-                                "@p3 st.global.v2.b32 [%0], {%14, c};\n\t@p3 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 4;\n\t"
-                                "@p4 st.global.v2.b32 [%0], {%15, c};\n\t@p4 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 5;\n\t"
-                                "@p5 st.global.v2.b32 [%0], {%16, c};\n\t@p5 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 6;\n\t"
-                                "@p6 st.global.v2.b32 [%0], {%17, c};\n\t@p6 add.u64 %0, %0, 8;\n\tadd.u32 c, %2, 7;\n\t"
-                                "@p7 st.global.v2.b32 [%0], {%18, c};\n\t@p7 add.u64 %0, %0, 8;\n\t}"
-                                : "+l"(waddr)
-                                : "f"(tau), "r"(col0),
-                                  "f"(__uint_as_float(x[0])), "f"(__uint_as_float(x[1])), "f"(__uint_as_float(x[2])),
-                                  "f"(__uint_as_float(x[3])), "f"(__uint_as_float(x[4])), "f"(__uint_as_float(x[5])),
-                                  "f"(__uint_as_float(x[6])), "f"(__uint_as_float(x[7])),
-                                  "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7])
-                                : "memory");
+                            const float x = fmax3(__uint_as_float(v[g * 8 + 0]), __uint_as_float(v[g * 8 + 1]), __uint_as_float(v[g * 8 + 2]));
+                            const float y = fmax3(__uint_as_float(v[g * 8 + 3]), __uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
+                            const float z = fmax3(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]), x);
+                            wm |= (fmaxf(y, z) > tau) ? (1u << (slice * 4 + g)) : 0u;
                         }
                     };
-                    dense(va, 0);
-                    dense(vb, 1);
-                    dense(vc, 2);
-                    dense(vd, 3);
-                    TC_PROF(prof_append += (int)((waddr - my_addr) >> 3) - cnt;)
-                    cnt = (int)((waddr - my_addr) >> 3);
-                    continue;
-                }
-                if (MID) {
-                    // pools of this mode hold (score, row) pairs; `waddr` is the shared-memory address
-                    // of this row's next free slot
-                    float2* warp_pool = reinterpret_cast<float2*>(pool_sc) + warp * 32 * PSTR;
-                    const uint32_t my_addr = smem_u32(warp_pool + lane * PSTR);
-                    uint32_t waddr = my_addr + 8u * (uint32_t)cnt;
-                    const uint32_t lim = my_addr + 8u * (uint32_t)(CAP - 8);
-                    tmem_ld_32x32b_x32(tile_taddr, va);
-                    tmem_ld_32x32b_x32(tile_taddr + 32, vb);
-                    tmem_ld_32x32b_x32(tile_taddr + 64, vc);
-                    tmem_ld_32x32b_x32(tile_taddr + 96, vd);
-                    tmem_ld_wait();
-                    reg_fence32(va);
-                    reg_fence32(vb);
-                    reg_fence32(vc);
-                    reg_fence32(vd);
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) release_acc(b);
-                    auto dense = [&](uint32_t (&v)[32], int slice) {
+                    screen(va, 0);
+                    screen(vb, 1);
+                    screen(vc, 2);
+                    screen(vd, 3);
+                    wm = __reduce_or_sync(FULL_MASK, wm);
+                    if (wm) {
+                        uint64_t waddr = my_addr + 8ull * (uint64_t)cnt;
+                        uint32_t saddr = my_saddr + 8u * (uint32_t)cnt;
+                        auto append = [&](uint32_t (&v)[32], int slice) {
 #pragma unroll
-                        for (int g = 0; g < 4; ++g) {
-                            // every lane's pool has room for the 8 scores of the group
-                            if (__any_sync(FULL_MASK, waddr > lim)) {
-                                cnt = (int)((waddr - my_addr) >> 3);
-                                const unsigned need = __ballot_sync(FULL_MASK, cnt > CAP - 8);
-                                TC_PROF(prof_compact += __popc(need);)
-                                const float2 cr = tc_compact_rows_pairs<CAP, K1>(need, warp_pool, PSTR, cnt, tau);
-                                cnt = __float_as_int(cr.x);
-                                tau = cr.y;
-                                waddr = my_addr + 8u * (uint32_t)cnt;
+                            for (int g = 0; g < 4; ++g) {
+                                if (!((wm >> (slice * 4 + g)) & 1u)) continue;
+                                // every lane's pool has room for the 8 scores of the group
+                                const int now = MID ? (int)((saddr - my_saddr) >> 3) : (int)((waddr - my_addr) >> 3);
+                                const unsigned need = __ballot_sync(FULL_MASK, now > CAP - 8);
+                                if (need) {
+                                    TC_PROF(prof_compact += __popc(need);)
+                                    const float2 cr = tc_compact_rows_pairs<CAP, K1>(need, warp_pool, gstride, now, tau);
+                                    tau = cr.y;
+                                    waddr = my_addr + 8ull * (uint64_t)__float_as_int(cr.x);
+                                    saddr = my_saddr + 8u * (uint32_t)__float_as_int(cr.x);
+                                }
+                                // the 8 comparisons first (independent), then the predicated stores: only
+                                // the address increments form a chain
+                                const uint32_t col0 = row_base + slice * 32 + g * 8;
+                                const uint32_t* x = v + g * 8;
+#define FL_APPEND(ST, ADD, C, ADDR)                                                                                    \
+    asm volatile(                                                                                                      \
+        "{\n\t.reg .pred p0, p1, p2, p3, p4, p5, p6, p7;\n\t.reg .b32 c;\n\t"                                         \
+        "setp.gt.f32 p0, %3, %1;\n\tsetp.gt.f32 p1, %4, %1;\n\tsetp.gt.f32 p2, %5, %1;\n\tsetp.gt.f32 p3, %6, %1;\n\t" \
+        "setp.gt.f32 p4, %7, %1;\n\tsetp.gt.f32 p5, %8, %1;\n\tsetp.gt.f32 p6, %9, %1;\n\tsetp.gt.f32 p7, %10, %1;\n\t" \
+        "@p0 " ST " [%0], {%3, %2};\n\t@p0 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 1;\n\t"                              \
+        "@p1 " ST " [%0], {%4, c};\n\t@p1 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 2;\n\t"                               \
+        "@p2 " ST " [%0], {%5, c};\n\t@p2 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 3;\n\t"                               \
+        "@p3 " ST " [%0], {%6, c};\n\t@p3 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 4;\n\t"                               \
+        "@p4 " ST " [%0], {%7, c};\n\t@p4 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 5;\n\t"                               \
+        "@p5 " ST " [%0], {%8, c};\n\t@p5 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 6;\n\t"                               \
+        "@p6 " ST " [%0], {%9, c};\n\t@p6 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 7;\n\t"                               \
+        "@p7 " ST " [%0], {%10, c};\n\t@p7 " ADD " %0, %0, 8;\n\t}"                                                  \
+        : "+" C(ADDR)                                                                                                  \
+        : "r"(__float_as_uint(tau)), "r"(col0), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]),      \
+          "r"(x[6]), "r"(x[7])                                                                                         \
+        : "memory")
+                                if (MID) FL_APPEND("st.shared.v2.b32", "add.u32", "r", saddr);
+                                else FL_APPEND("st.global.v2.b32", "add.u64", "l", waddr);
+#undef FL_APPEND
                             }
-                            const uint32_t col0 = row_base + slice * 32 + g * 8;
-                            const uint32_t* x = v + g * 8;
-                            asm volatile(
-                                "{\n\t.reg .pred p0, p1, p2, p3, p4, p5, p6, p7;\n\t.reg .b32 c;\n\t"
-                                "setp.gt.f32 p0, %3, %1;\n\tsetp.gt.f32 p1, %4, %1;\n\tsetp.gt.f32 p2, %5, %1;\n\tsetp.gt.f32 p3, %6, %1;\n\t"
-                                "setp.gt.f32 p4, %7, %1;\n\tsetp.gt.f32 p5, %8, %1;\n\tsetp.gt.f32 p6, %9, %1;\n\tsetp.gt.f32 p7, %10, %1;\n\t"
-                                "@p0 st.shared.v2.b32 [%0], {%11, %2};\n\t@p0 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 1;\n\t"
-                                "@p1 st.shared.v2.b32 [%0], {%12, c};\n\t@p1 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 2;\n\t"
-                                "@p2 st.shared.v2.b32 [%0], {%13, c};\n\t@p2 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 3;\n\t"
-                                "@p3 st.shared.v2.b32 [%0], {%14, c};\n\t@p3 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 4;\n\t"
-                                "@p4 st.shared.v2.b32 [%0], {%15, c};\n\t@p4 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 5;\n\t"
-                                "@p5 st.shared.v2.b32 [%0], {%16, c};\n\t@p5 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 6;\n\t"
-                                "@p6 st.shared.v2.b32 [%0], {%17, c};\n\t@p6 add.u32 %0, %0, 8;\n\tadd.u32 c, %2, 7;\n\t"
-                                "@p7 st.shared.v2.b32 [%0], {%18, c};\n\t@p7 add.u32 %0, %0, 8;\n\t}"
-                                : "+r"(waddr)
-                                : "f"(tau), "r"(col0),
-                                  "f"(__uint_as_float(x[0])), "f"(__uint_as_float(x[1])), "f"(__uint_as_float(x[2])),
-                                  "f"(__uint_as_float(x[3])), "f"(__uint_as_float(x[4])), "f"(__uint_as_float(x[5])),
-                                  "f"(__uint_as_float(x[6])), "f"(__uint_as_float(x[7])),
-                                  "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7])
-                                : "memory");
-                        }
-                    };
-                    dense(va, 0);
-                    dense(vb, 1);
-                    dense(vc, 2);
-                    dense(vd, 3);
-                    TC_PROF(prof_append += ((waddr - my_addr) >> 3) - cnt;)
-                    cnt = (int)((waddr - my_addr) >> 3);
+                        };
+                        append(va, 0);
+                        append(vb, 1);
+                        append(vc, 2);
+                        append(vd, 3);
+                        const int now = MID ? (int)((saddr - my_saddr) >> 3) : (int)((waddr - my_addr) >> 3);
+                        TC_PROF(prof_append += now - cnt;)
+                        cnt = now;
+                    }
                     continue;
                 }
                 unsigned hits = 0;
@@ -892,7 +880,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 continue;
             }
             if (MODE == TC_MODE_SEED) {
-                float4* o = reinterpret_cast<float4*>(p.seed_cls + (qrow * TC_NWG + wg) * 16);
+                float4* o = reinterpret_cast<float4*>(p.seed_cls + ((qrow * p.nsplit + split) * TC_NWG + wg) * 16);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) o[c] = make_float4(cls[4 * c], cls[4 * c + 1], cls[4 * c + 2], cls[4 * c + 3]);
                 continue;
@@ -993,10 +981,10 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 // so a shard that re-scores every row above `cert` cannot miss a global neighbour.  `cert` is
 // also written to mg.cert_out, where the finalisation reads it.
 __global__ void __launch_bounds__(256) tc_seed_select_kernel(const float* __restrict__ seed_cls, float* __restrict__ tau,
-                                                             int64_t nq_pad, int rank, const TcSeedMargin mg) {
+                                                             int64_t nq, int rank, const TcSeedMargin mg) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= nq_pad) return;
+    if (row >= nq) return;                                 // padding rows keep their +inf
     const float v = __ldg(seed_cls + row * (TC_NWG * 16) + lane);
     // rank of each value among the 32 (ties broken by position): a permutation
     int r = 0;
@@ -1009,10 +997,8 @@ __global__ void __launch_bounds__(256) tc_seed_select_kernel(const float* __rest
     float pick = __shfl_sync(FULL_MASK, v, __ffs(sel) - 1);
     if (mg.q != nullptr) {
         float qsq = 0.f;
-        if (row < mg.nq) {
-            const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
-            for (int c = lane; c < mg.d; c += 32) { const float x = ld_elem(qp, c, mg.dt); qsq += x * x; }
-        }
+        const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
+        for (int c = lane; c < mg.d; c += 32) { const float x = ld_elem(qp, c, mg.dt); qsq += x * x; }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
         const float mn = __ldg(mg.maxnorm);
@@ -1020,6 +1006,60 @@ __global__ void __launch_bounds__(256) tc_seed_select_kernel(const float* __rest
         if (lane == 0 && mg.cert_out != nullptr) mg.cert_out[row] = pick;
     }
     if (lane == 0 && pick > neg_inf()) tau[row] = pick;
+}
+
+// The same from a sample whose tiles were dealt to several CTAs: every row has nsplit x 32 class maxima of
+// disjoint sets of rows, folded to at most 512 (the maximum of several disjoint classes is the maximum
+// of their union), and the threshold is a value that at least `rank` of them reach, close to the
+// largest such -- so `rank` may go beyond 32, where the one-CTA form above has to make do with 32
+// classes.  One warp per query row; rows without a query keep their +inf.
+__global__ void __launch_bounds__(256) tc_seed_select_split_kernel(const float* __restrict__ seed_cls, float* __restrict__ tau,
+                                                                   int64_t nq, int nsplit, int rank, const TcSeedMargin mg) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= nq) return;
+    constexpr int R = 16;
+    float v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = neg_inf();
+    const float* base = seed_cls + row * (int64_t)nsplit * (TC_NWG * 16) + lane;
+    for (int s0 = 0; s0 < nsplit; s0 += R) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (s0 + r < nsplit) v[r] = fmaxf(v[r], __ldg(base + (int64_t)(s0 + r) * (TC_NWG * 16)));
+    }
+    int b[R], lo = 0x7fffffff, hi = (int)0x80000000, have = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int x = __float_as_int(v[r]);
+        b[r] = x >= 0 ? x : (x ^ 0x7fffffff);              // orders like the float
+        const bool real = v[r] > -1e37f;                   // neither empty nor padding rows
+        have += __popc(__ballot_sync(FULL_MASK, real));
+        if (real) { lo = min(lo, b[r]); hi = max(hi, b[r]); }
+    }
+    if (have < rank) return;
+    lo = __reduce_min_sync(FULL_MASK, lo);
+    hi = __reduce_max_sync(FULL_MASK, hi);
+    for (int it = 0; it < 32 && lo < hi; ++it) {
+        const int mid = (int)(((long long)lo + hi + 1) >> 1);
+        int c = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) c += __popc(__ballot_sync(FULL_MASK, b[r] >= mid));
+        if (c >= rank) lo = mid; else hi = mid - 1;
+        if (c >= rank && c <= rank + (rank >> 3) + 1) break;
+    }
+    float pick = __int_as_float(lo >= 0 ? lo : (lo ^ 0x7fffffff));
+    if (mg.q != nullptr) {
+        const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
+        float qsq = 0.f;
+        for (int c = lane; c < mg.d; c += 32) { const float x = ld_elem(qp, c, mg.dt); qsq += x * x; }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+        const float mn = __ldg(mg.maxnorm);
+        pick -= 2.f * mg.eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
+    }
+    // a score equal to the threshold is not kept: one step below it, so that the `rank` rows are
+    if (lane == 0) tau[row] = pick - fabsf(pick) * 1.2e-7f;
 }
 
 // ---- host side ---------------------------------------------------------------------------
@@ -1072,7 +1112,7 @@ int tc_use_deep_pools(int k, int d_pad, int nsplit, int64_t nq_pad) {
 int tc_deep_pool_size() { return TC_MID_K1; }
 int tc_deep_partial_len() { return TC_NWG * TC_MID_PUB; }
 int tc_taus_per_range() { return TC_NWG; }
-int tc_pair_pool_cap() { return TC_GP_CAP; }
+int tc_pair_pool_cap(int k) { return tc_knn_big(k) ? TC_BIG_CAP : TC_GP_CAP; }
 
 int tc_knn_supported(int64_t nq, int64_t m, int d, int k) {
     if (nq < 1 || m < 1) return FL_EUNSUPPORTED;
@@ -1083,10 +1123,27 @@ int tc_knn_supported(int64_t nq, int64_t m, int d, int k) {
     return FL_OK;
 }
 
-// Auto mode takes the tensor-core path once the problem is large enough to amortise it.
+float tc_eps_rel(int dt, int d) {
+    const float acc = 1.2e-7f * (float)(d + 16);           // fp32 accumulation of d + 16 products, 2^-23 each
+    if (dt == DT_BF16) return 2.f * acc;                   // operands are exact
+    return 0.00391f + acc > 0.004f ? 0.00391f + acc : 0.004f;
+}
+// (the streamed query tile has no limit of its own; 8 192 features keep the error bound near 2^-8)
+int tc_wide_supported(int64_t nq, int64_t m, int d, int k) {
+    if (d <= 512 || d > 8192 || nq < 1 || k > 112) return 0;
+    if (m < 512 || round_up(m, 256) / 256 > (1 << 23)) return 0;
+    if (!direct_pick(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
+    return direct_estimate_us(nq, m, d) > 60.0 + (double)m * (double)(round_up(d, 64) + PLANE_AUG_COLS) * 2.0 / 5.5e6;
+}
+
+// Auto mode takes the tensor-core path where it is the faster one.  Its dozen launches cost about 60 us
+// whatever the size, then a few queries stream the bf16 plane from HBM; the CUDA-core scan for few
+// queries has two launches and reads the stored rows once per four queries.
 int tc_knn_auto(int64_t nq, int64_t m, int d, int k) {
-    if (tc_knn_supported(nq, m, d, k) != FL_OK) return 0;
-    return (m >= 2048 && nq * m >= (int64_t(1) << 24)) ? 1 : 0;
+    if (tc_knn_supported(nq, m, d, k) != FL_OK || m < 512) return 0;
+    if (!direct_pick(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
+    const double tc = 60.0 + (double)m * (double)(round_up(d, 64) + PLANE_AUG_COLS) * 2.0 / 5.5e6;
+    return direct_estimate_us(nq, m, d) > tc;
 }
 
 // CTA pairs (cta_group::2) for plain k <= 16 scoring.  Measured on the 1M x 128 benchmark they are
@@ -1153,10 +1210,75 @@ static TcExperiment& tc_experiment() {
     }();
     return e;
 }
+int tc_debug_active() { return tc_experiment().flags != 0; }
 void tc_debug_set(int flags, unsigned wait_us) {
     TcExperiment& e = tc_experiment();
     e.flags = flags;
     e.wait_ns = wait_us ? (uint64_t)wait_us * 1000ull : TC_WAIT_DEFAULT_NS;
+}
+
+// Few query tiles or a small database: such calls are bound by latencies and by the fixed cost of their
+// launches, not by the tensor pipe.  They keep their pools in global memory as pairs (mode KNN_GPOOL: no
+// pool in shared memory, four ring slots, nothing published at the end of an item), cut the database
+// into row ranges so that every SM has one, and finalise with a block per query.  The line, measured
+// with k = 10: up to eight query tiles whatever the database (300 queries x 1M rows 402 -> 241 us,
+// 1 000 554 -> 460; 3 000 1 240 -> 1 265), beyond that up to 64 tiles of work per SM (10 000 x 100 000
+// x 64, 208 tiles per SM: 507 -> 771).
+int tc_small(int64_t nq_pad, int64_t m_pad) {
+    if (tc_pair_requested()) return 0;
+    const int64_t n_qtiles = nq_pad / TC_BM;
+    return n_qtiles <= 8 || n_qtiles * (m_pad / TC_BN) <= 64 * (int64_t)sm_count();
+}
+
+// Row ranges of such a call: every item costs about four tiles of latency on top of its own.
+void tc_small_split(int64_t nq_pad, int64_t m_pad, int* nsplit, int64_t* tiles_per_split) {
+    const int64_t n_qtiles = nq_pad / TC_BM, n_tiles = m_pad / TC_BN;
+    const int sms = sm_count();
+    int64_t max_s = n_tiles / 2;
+    if (max_s > sms) max_s = sms;
+    if (max_s < 1) max_s = 1;
+    int64_t best_cost = -1, best_s = 1;
+    for (int64_t s = 1; s <= max_s; ++s) {
+        const int64_t tps = ceil_div(n_tiles, s), se = ceil_div(n_tiles, tps);
+        const int64_t cost = ceil_div(n_qtiles * se, sms) * (tps + 4);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_s = se; }
+    }
+    *tiles_per_split = ceil_div(n_tiles, best_s);
+    *nsplit = (int)ceil_div(n_tiles, *tiles_per_split);
+}
+
+// Seeding sample of a call that is not part of a row-sharded search: `tiles` tiles dealt to `splits` CTAs per
+// query tile (32 class maxima each), and the threshold is a value that `rank` sampled rows reach -- about
+// rank n_tiles / tiles rows of the whole database.  The aim is 10 k + 200 of them (k > 16: 6 k + 50): enough that
+// the k-th neighbour's error band stays inside, few enough that the pools hardly ever fill.  Rank 24
+// holds that figure within a fifth; k + 6 rows are enough for small k.
+// `dense`: the sample is an eighth of the database or more, so the threshold cuts close to the k-th
+// neighbour: k + 6 rows must reach it, and it is lowered by twice the scoring error bound
+// (tc_seed_select_split_kernel).
+void tc_seed_plan(int64_t nq_pad, int64_t m_pad, int k, TcSeedPlan* w) {
+    const int64_t n_qtiles = nq_pad / TC_BM, n_tiles = m_pad / TC_BN;
+    const int sms = sm_count();
+    *w = TcSeedPlan{};
+    if (tc_experiment().noseed || tc_experiment().seed_tiles >= 0 || tc_experiment().seed_rank >= 0) return;
+    w->rank = k + 6 < 24 ? k + 6 : 24;
+    const int64_t aim = k <= 16 ? 10 * k + 200 : 6 * k + 50 > 250 ? 6 * k + 50 : 250;
+    int64_t tiles = ceil_div(w->rank * n_tiles, aim);
+    if (tiles < 16) tiles = 16;
+    if (n_qtiles > 8 && k <= 16 && tiles > 96) tiles = 96;       // (the scoring pass of many query tiles tightens them itself)
+    if (tiles > n_tiles) tiles = n_tiles;
+    w->dense = tiles * 8 >= n_tiles;
+    if (w->dense) w->rank = k + 6;
+    const int64_t need = ceil_div(w->rank, 2 * 16);              // classes enough for the rank
+    int64_t best = -1, best_s = 0;
+    for (int64_t s = need > 2 ? need : 2; s <= tiles && s <= sms; ++s) {
+        const int64_t per = ceil_div(tiles, s), se = ceil_div(tiles, per);
+        if (se < need || se < 2) continue;
+        const int64_t cost = ceil_div(n_qtiles * se, sms) * (per + 4);
+        if (best < 0 || cost < best) { best = cost; best_s = se; }
+    }
+    if (best_s == 0) return;                                     // a database of one tile: no seeding
+    w->tiles = (int)tiles;
+    w->splits = (int)best_s;
 }
 
 // Tensor maps are encoded once per (buffer, shape, box) and kept in a small per-thread cache:
@@ -1183,13 +1305,12 @@ static int cached_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int
 }
 
 int tc_seed_tiles(int64_t m_pad, int k);
-
 struct TcLaunch {
     CUtensorMap map_q, map_q_aug, map_db, map_db_aug;
     TcSmemPlan sp;
     TcKernelParams kp;
     int seed_tiles, seed_rank;
-    bool big, mid, gs;
+    bool big, mid, gs, gpb;
 };
 
 // Plain k <= 16 scoring with the small pools in global memory (mode KNN_GS) instead of shared memory.
@@ -1207,7 +1328,8 @@ static int tc_gs_requested(int d_pad) {
 // the seeding sample.
 static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch* L) {
     FL_CHECK_ARG(p.qplane && p.dbrows && p.tau, "tensor-core kNN launch with a null buffer");
-    L->big = tc_knn_big(p.k) != 0 || p.big_pools != 0;
+    L->big = (tc_knn_big(p.k) != 0 || p.big_pools != 0) && p.pair_pools == nullptr;
+    L->gpb = p.pair_pools != nullptr && tc_knn_big(p.k) != 0;
     L->mid = p.deep_pools != 0;
     const TcExperiment& ex0 = tc_experiment();
     L->gs = !L->big && !L->mid && p.pair_pools == nullptr && dbg == nullptr && ex0.flags == 0 && p.row_query == nullptr &&
@@ -1219,7 +1341,11 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     if (rc == FL_OK) rc = cached_map_bf16(&L->map_db_aug, p.dbrows, p.m_pad, pitch, PLANE_AUG_COLS, TC_BN);
     if (rc != FL_OK) return rc;
     FL_CHECK_ARG(!(L->mid && (L->big || dbg)), "tensor-core kNN launch: deep pools go with k <= 16");
-    L->sp = tc_smem_plan(p.d_pad, smem_optin_bytes(), (L->big || L->gs || p.pair_pools != nullptr) ? 0 : L->mid ? TC_MID_CAP + 1 : TC_PSTR);
+    // a query tile of more than 512 features is streamed with the database chunks
+    const bool stream = p.d_pad > 512;
+    FL_CHECK_ARG(!stream || p.pair_pools != nullptr, "tensor-core kNN launch: more than 512 features go with pair pools");
+    L->sp = tc_smem_plan(p.d_pad, smem_optin_bytes(), (L->big || L->gs || p.pair_pools != nullptr) ? 0 : L->mid ? TC_MID_CAP + 1 : TC_PSTR,
+                         stream ? TC_STREAM_STAGE : TC_B_STAGE, stream ? 0 : 1);
     if (L->sp.nstage < 2) { set_error("tensor-core kNN: feature dimension %d leaves no room for the TMA ring", p.d_pad); return FL_EUNSUPPORTED; }
     const TcExperiment& ex = tc_experiment();
     TcKernelParams& kp = L->kp;
@@ -1229,6 +1355,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     kp.nsplit = p.nsplit;
     kp.tiles_per_split = (int)p.tiles_per_split;
     kp.nkc = L->sp.nkc; kp.nstage = L->sp.nstage;
+    kp.stream_a = stream ? 1 : 0;
     kp.off_b = L->sp.off_b; kp.off_pool_sc = L->sp.off_pool_sc; kp.off_pool_id = L->sp.off_pool_id;
     kp.off_bar = L->sp.off_bar;
     kp.nq_pad = p.nq_pad; kp.part_sc = p.part_sc; kp.part_id = p.part_id;
@@ -1310,16 +1437,18 @@ int launch_knn_tc_seed(const TcKnnParams& p, cudaStream_t st) {
         FL_CHECK_ARG(p.item_tile_cap > 0 && p.nsplit == 1, "tensor-core seeding over item tables needs a tile cap");
         sk.item_tile_cap = p.item_tile_cap;
     } else {
-        if (L.seed_tiles == 0) return launch_fill_f32(p.seed_cls, p.nq_pad * (TC_NWG * 16), -INFINITY, st);
-        sk.nsplit = 1;
-        sk.tiles_per_split = L.seed_tiles;
-        sk.tile_stride = L.kp.n_tiles / L.seed_tiles;
-        sk.n_tiles = L.seed_tiles;
+        const int tiles = p.seed_tiles > 0 ? p.seed_tiles : L.seed_tiles;
+        if (tiles == 0) return launch_fill_f32(p.seed_cls, p.nq_pad * (TC_NWG * 16), -INFINITY, st);
+        sk.nsplit = p.seed_splits > 1 ? p.seed_splits : 1;
+        sk.tiles_per_split = (int)ceil_div(tiles, sk.nsplit);
+        sk.tile_stride = L.kp.n_tiles / tiles;
+        sk.n_tiles = tiles;
         sk.nq_dev = nullptr;
     }
     // the seeding kernel keeps no pools: the ring gets the shared memory the pools would take
     const TcSmemPlan sp = L.sp;
-    const int sgrid = sk.n_qtiles < sm_count() ? sk.n_qtiles : sm_count();
+    const int sitems = sk.n_qtiles * sk.nsplit;
+    const int sgrid = sitems < sm_count() ? sitems : sm_count();
     FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_SEED>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
     knn_tc_kernel<false, TC_MODE_SEED><<<sgrid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, sk);
     FL_CHECK_LAUNCH();
@@ -1330,10 +1459,15 @@ int launch_knn_tc_seed(const TcKnnParams& p, cudaStream_t st) {
 // shards of a sharded database): see tc_seed_select_kernel.
 int launch_knn_tc_seed_select(const TcKnnParams& p, const TcSeedMargin& mg, cudaStream_t st) {
     FL_CHECK_ARG(p.seed_cls != nullptr && p.tau != nullptr, "tensor-core threshold selection without buffers");
+    if (p.seed_splits > 1) {
+        tc_seed_select_split_kernel<<<(unsigned)ceil_div(p.nq, 8), 256, 0, st>>>(p.seed_cls, p.tau, p.nq, p.seed_splits, p.seed_rank, mg);
+        FL_CHECK_LAUNCH();
+        return FL_OK;
+    }
     TcLaunch L;
     int rc = tc_prepare(p, nullptr, 0, &L);
     if (rc != FL_OK) return rc;
-    tc_seed_select_kernel<<<(unsigned)ceil_div(p.nq_pad, 8), 256, 0, st>>>(p.seed_cls, p.tau, p.nq_pad, L.seed_rank, mg);
+    tc_seed_select_kernel<<<(unsigned)ceil_div(p.nq, 8), 256, 0, st>>>(p.seed_cls, p.tau, p.nq, L.seed_rank, mg);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
@@ -1346,7 +1480,7 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
     int rc = tc_prepare(p, dbg, dbg_ld, &L);
     if (rc != FL_OK) return rc;
     const bool big = L.big, mid = L.mid;
-    FL_CHECK_ARG(!gp || (!big && !dbg && p.k <= 16), "tensor-core kNN launch: global pair pools go with k <= 16");
+    FL_CHECK_ARG(!gp || !dbg, "tensor-core kNN launch: no score dump with global pair pools");
     FL_CHECK_ARG(!big || (p.part_cnt && !dbg), "tensor-core kNN launch (large k) without a count buffer");
     FL_CHECK_ARG((p.row_query == nullptr) == (p.tau_q == nullptr), "tensor-core kNN launch: row_query and tau_q go together");
     FL_CHECK_ARG((p.item_t0 == nullptr) == (p.item_t1 == nullptr) && (p.item_t0 == nullptr || (p.nsplit == 1 && !big)),
@@ -1360,7 +1494,10 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
     // tiles, at least one pair-item per cluster of a full grid.  FLASHLIB_B200_TC_PAIR=0/1 overrides.
     const bool pair = !gp && !mid && dbg == nullptr && p.item_t0 == nullptr && p.nq_dev == nullptr &&
                       tc_pair_enabled(p.nq_pad, p.k);
-    if (gp) {
+    if (L.gpb) {
+        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
+        knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
+    } else if (gp) {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
         knn_tc_kernel<false, TC_MODE_KNN_GPOOL><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     } else if (pair) {

@@ -8,6 +8,7 @@ rejected because this library has no CPU path.
 """
 from __future__ import annotations
 
+import ctypes
 import os
 import weakref
 from collections import OrderedDict, deque
@@ -23,8 +24,31 @@ _MODES = {None: _lib.FL_KNN_AUTO, "auto": _lib.FL_KNN_AUTO, "exact": _lib.FL_KNN
           "tc": _lib.FL_KNN_BF16_RERANK}
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(device: torch.device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)       # the handle alone, without building a Stream object
     return torch.cuda.current_stream(device).cuda_stream
+
+
+class _OnDevice:
+    """``torch.cuda.device`` for the (usual) case that the tensor's device is current already: no
+    context is entered then."""
+
+    __slots__ = ("_ctx",)
+
+    def __init__(self, device: torch.device):
+        self._ctx = None if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self._ctx is not None:
+            self._ctx.__enter__()
+
+    def __exit__(self, *exc):
+        if self._ctx is not None:
+            self._ctx.__exit__(*exc)
 
 
 def _as_f32_rows(t: torch.Tensor) -> torch.Tensor:
@@ -173,11 +197,49 @@ def clear_plane_cache() -> None:
     _PLANE_CACHE.clear()
 
 
-# Status words of calls whose check was deferred: (pinned host copy, event of the copy).  The
-# tensor-core kernel reports a timed-out wait there; reading it right after the call would
-# serialise host and device once per call, so the public entry points look at the words of
-# EARLIER calls instead (and ``check_pending()`` looks at all of them).
+# Status words of calls whose check was deferred.  The tensor-core kernels report a timed-out wait
+# there; reading them right after the call would serialise host and device once per call, so the
+# public entry points look at the words of EARLIER calls instead (and ``check_pending()`` looks at
+# all of them).  A slot is a few words of pinned host memory that the last kernel of a call fills in,
+# completion mark last: neither a copy nor an event enters the stream.
+class _StatusSlot:
+    __slots__ = ("buf", "words", "ptr", "device")
+
+    def __init__(self, device: torch.device):
+        self.buf = torch.zeros(_lib.FL_STATUS_WORDS + 1, dtype=torch.int32).pin_memory()
+        self.ptr = self.buf.data_ptr()
+        self.words = (ctypes.c_int32 * (_lib.FL_STATUS_WORDS + 1)).from_address(self.ptr)
+        self.device = device
+
+
 _PENDING_STATUS: deque = deque()
+_FREE_SLOTS: deque = deque()               # at most as many as calls were pending at once (64)
+
+
+def _take_status_slot(device: torch.device) -> _StatusSlot:
+    check_pending(block=False)
+    while len(_PENDING_STATUS) >= 64:      # bounded: the oldest calls have long finished
+        _finish_slot(_PENDING_STATUS.popleft(), wait=True)
+    try:
+        slot = _FREE_SLOTS.popleft()
+    except IndexError:
+        slot = _StatusSlot(device)
+    slot.device = device
+    slot.words[_lib.FL_STATUS_WORDS] = 0
+    return slot
+
+
+def _finish_slot(slot: _StatusSlot, wait: bool) -> bool:
+    """Looks at a slot's words (waiting for its call first when asked to) and gives the slot back;
+    ``False`` when the call is still running."""
+    if slot.words[_lib.FL_STATUS_WORDS] == 0:
+        if not wait:
+            return False
+        torch.cuda.synchronize(slot.device)
+    st = list(slot.words)[:_lib.FL_STATUS_WORDS]
+    _FREE_SLOTS.append(slot)
+    _raise_on_status(st)
+    return True
 
 
 _STATUS_TEXT = {_lib.FL_ETIMEOUT: "a bounded device-side wait ran out",
@@ -197,33 +259,52 @@ def check_pending(block: bool = True) -> None:
     """Raises if an earlier call whose status check was deferred reported an error.  With
     ``block=False`` only calls that have already finished on the device are looked at."""
     while _PENDING_STATUS:
-        host, ev = _PENDING_STATUS[0]
-        if not block and not ev.query():
+        try:
+            slot = _PENDING_STATUS.popleft()
+        except IndexError:                 # another thread took it
             return
-        ev.synchronize()
-        _PENDING_STATUS.popleft()
-        _raise_on_status(host.tolist())
+        if not block and slot.words[_lib.FL_STATUS_WORDS] == 0:
+            _PENDING_STATUS.appendleft(slot)
+            return
+        _finish_slot(slot, wait=True)
 
 
 def _defer_status_check(status: torch.Tensor) -> None:
-    check_pending(block=False)
-    host = torch.empty(_lib.FL_STATUS_WORDS, dtype=torch.int32).pin_memory()
-    host.copy_(status, non_blocking=True)
-    ev = torch.cuda.Event()
-    ev.record(torch.cuda.current_stream(status.device))
-    _PENDING_STATUS.append((host, ev))
-    while len(_PENDING_STATUS) > 64:              # bounded: the oldest calls have long finished
-        check_pending_one = _PENDING_STATUS[0]
-        check_pending_one[1].synchronize()
-        _PENDING_STATUS.popleft()
-        _raise_on_status(check_pending_one[0].tolist())
+    """Queues the status words of a call that has just been launched on the current stream."""
+    slot = _take_status_slot(status.device)
+    _lib.check(_lib.load().fl_publish_status(status.data_ptr(), slot.ptr, _stream_ptr(status.device)))
+    _PENDING_STATUS.append(slot)
+
+
+# Which kernel a shape takes and the workspace it needs: asked from the library once per shape.
+_PLANS: dict = {}
+
+
+def _knn_plan(lib, nq: int, m: int, d: int, k: int, mode: int):
+    """``(resolved mode, mode to pass on, wants an operand plane, workspace bytes, staged workspace bytes)``."""
+    key = (nq, m, d, k, mode)
+    hit = _PLANS.get(key)
+    if hit is not None:
+        return hit
+    resolved = lib.fl_knn_resolve_mode(nq, m, d, k) if mode == _lib.FL_KNN_AUTO else mode
+    wants = resolved == _lib.FL_KNN_BF16_RERANK
+    passed = resolved
+    if not wants and mode == _lib.FL_KNN_AUTO and nq > 0 and lib.fl_knn_wants_plane(nq, m, d, k):
+        # more than 512 features: automatic mode with a plane takes the streamed tensor-core kernel
+        resolved, passed, wants = _lib.FL_KNN_BF16_RERANK, _lib.FL_KNN_AUTO, True
+    ws = lib.fl_knn_workspace_bytes(max(nq, 1), m, d, k, passed)
+    staged = lib.fl_knn_staged_workspace_bytes(nq, m, d, k) if passed == _lib.FL_KNN_BF16_RERANK else 0
+    if len(_PLANS) >= 512:
+        _PLANS.clear()
+    plan = _PLANS[key] = (resolved, passed, wants, ws, staged)
+    return plan
 
 
 def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KNN_AUTO,
             row_offset: int = 0, plane: Optional[DbPlane] = None, check_status=True,
-            second_stage: Optional[bool] = None):
-    """One 2-D problem through ``fl_knn_f32`` / ``fl_knn_staged_f32`` (fp32 rows) or ``fl_knn_rows``
-    (bf16 / fp16 rows, read as stored): returns ``(dist fp32 (nq,k), idx int32 (nq,k), info)``.
+            second_stage: Optional[bool] = None, out=None):
+    """One 2-D problem through ``fl_knn_search`` (fp32, or bf16 / fp16 rows read as stored): returns
+    ``(dist fp32 (nq,k), idx int32 (nq,k), info)``, in ``out = (dist, idx)`` when given.
     ``check_status=True`` reads the kernel's status words before returning (one host/device
     round trip; ``info["fallback_rows"]`` and ``info["stage2_rows"]`` are filled), ``"deferred"``
     leaves that to a later call or to ``check_pending()``, ``False`` skips it.
@@ -237,36 +318,36 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
     dev = q.device
     if q.dtype != db.dtype or db.dtype not in _DTYPE_CODES:
         raise TypeError(f"knn_f32 takes q and db of one dtype out of fp32 / bf16 / fp16, got {q.dtype} and {db.dtype}")
-    resolved = lib.fl_knn_resolve_mode(nq, m, d, k) if mode == _lib.FL_KNN_AUTO else mode
-    if resolved == _lib.FL_KNN_BF16_RERANK and plane is None:
+    resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, nq, m, d, k, mode)
+    if wants_plane and plane is None:
         plane = get_plane(db)
-    out_d = torch.empty((nq, k), dtype=torch.float32, device=dev)
-    out_i = torch.empty((nq, k), dtype=torch.int32, device=dev)
+    if out is not None:
+        out_d, out_i = out
+    else:
+        out_d = torch.empty((nq, k), dtype=torch.float32, device=dev)
+        out_i = torch.empty((nq, k), dtype=torch.int32, device=dev)
     split = None
-    if resolved == _lib.FL_KNN_BF16_RERANK and nq > 0:
+    if wants_plane and staged_bytes and nq > 0:
         if second_stage is None:
             second_stage = _second_stage_default()
         if second_stage:
             split = plane.split_ptr(db)
-    status = torch.zeros(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=dev)
-    if split is not None:
-        ws_bytes = lib.fl_knn_staged_workspace_bytes(nq, m, d, k)
-        ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-        rc = lib.fl_knn_staged_f32(q.data_ptr(), nq, q.stride(0), db.data_ptr(), m, db.stride(0), d, k,
-                                   plane.ptr, split, row_offset, out_d.data_ptr(), out_i.data_ptr(),
-                                   ws.data_ptr(), ws_bytes, status.data_ptr(), _stream_ptr(dev))
-    else:
-        ws_bytes = lib.fl_knn_workspace_bytes(max(nq, 1), m, d, k, resolved)
-        ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-        rc = lib.fl_knn_rows(q.data_ptr(), nq, q.stride(0) if nq else d, db.data_ptr(), m, db.stride(0), d, k,
-                             _DTYPE_CODES[db.dtype], resolved, plane.ptr if plane is not None else None, row_offset,
-                             out_d.data_ptr(), out_i.data_ptr(), ws.data_ptr(), ws_bytes,
-                             status.data_ptr(), _stream_ptr(dev))
-    _lib.check(rc)
+            if split is not None:
+                ws_bytes = staged_bytes
+    # (the kernels clear the status words themselves)
+    status = torch.empty(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=dev) if nq else torch.zeros(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=dev)
+    ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
+    slot = _take_status_slot(dev) if check_status == "deferred" and wants_plane and nq else None
+    rc = lib.fl_knn_search(q.data_ptr(), nq, q.stride(0) if nq else d, db.data_ptr(), m, db.stride(0), d, k,
+                           _DTYPE_CODES[db.dtype], passed, plane.ptr if plane is not None else None, split, row_offset,
+                           out_d.data_ptr(), out_i.data_ptr(), ws.data_ptr(), ws_bytes, status.data_ptr(),
+                           slot.ptr if slot is not None else None, _stream_ptr(dev))
+    if rc != _lib.FL_OK:
+        _lib.check(rc)
+    if slot is not None:
+        _PENDING_STATUS.append(slot)
     info = {"mode": resolved, "status": status, "second_stage": split is not None}
-    if check_status == "deferred" and resolved == _lib.FL_KNN_BF16_RERANK:
-        _defer_status_check(status)
-    elif check_status and resolved == _lib.FL_KNN_BF16_RERANK:
+    if check_status and check_status != "deferred" and wants_plane:
         st = status.tolist()
         info["fallback_rows"] = st[_lib.FL_STATUS_FALLBACK]
         info["stage2_rows"] = st[_lib.FL_STATUS_STAGE2]
@@ -315,6 +396,15 @@ def flash_knn_dispatch(x: torch.Tensor, c: torch.Tensor, k: int, *, tol: Optiona
     idxs = torch.empty((B, N, k), dtype=torch.int32, device=x.device)
     target = storage_dtype_for(tol)
     lib = _lib.load()
+    if B == 1:
+        with _OnDevice(x.device):
+            qb, cb = x[0], c[0]
+            if target is not None and qb.dtype != target:
+                qb, cb = qb.to(target), _cast_rows_cached(cb, target)
+            knn_f32(_as_rows(qb), _as_rows(cb), k, mode=m, check_status="deferred", out=(vals[0], idxs[0]))
+        if not return_distances:
+            return idxs[0] if squeeze else idxs
+        return (vals[0], idxs[0]) if squeeze else (vals, idxs)
     batched = (B > 1 and N > 0 and target is None and x.dtype == torch.float32 and m != _lib.FL_KNN_BF16_RERANK
                and lib.fl_knn_resolve_mode(N, M, D, k) == _lib.FL_KNN_EXACT_SIMT
                and x.stride(2) == 1 and c.stride(2) == 1 and x.stride(1) >= D and c.stride(1) >= D)
@@ -336,13 +426,9 @@ def flash_knn_dispatch(x: torch.Tensor, c: torch.Tensor, k: int, *, tol: Optiona
             if target is not None and qb.dtype != target:
                 qb, cb = qb.to(target), _cast_rows_cached(cb, target)
             qb, cb = _as_rows(qb), _as_rows(cb)
-            d_b, i_b, _ = knn_f32(qb, cb, k, mode=m, check_status="deferred")
-            vals[b] = d_b
-            idxs[b] = i_b
+            knn_f32(qb, cb, k, mode=m, check_status="deferred", out=(vals[b], idxs[b]))
     if not return_distances:
-        return idxs[0] if squeeze else idxs
-    if squeeze:
-        return vals[0], idxs[0]
+        return idxs
     return vals, idxs
 
 

@@ -215,6 +215,20 @@ int     fl_debug_tc_prof_read(unsigned long long* host_out, int words);
 
 /* Which mode FL_KNN_AUTO resolves to for a shape (no device work). */
 int     fl_knn_resolve_mode(int64_t nq, int64_t m, int d, int k);
+/* 1 when FL_KNN_AUTO can use an operand plane (fl_knn_prepare_db_rows) for the shape: the shapes that
+ * resolve to FL_KNN_BF16_RERANK, and rows of more than 512 features, which fl_knn_search and fl_knn_rows
+ * score on the tensor cores in automatic mode when they are given a plane. */
+int     fl_knn_wants_plane(int64_t nq, int64_t m, int d, int k);
+/* Copies FL_STATUS_WORDS status words from device memory to mapped (pinned) host memory of
+ * FL_STATUS_WORDS + 1 words in stream order, followed by a non-zero completion mark in the last word. */
+int     fl_publish_status(const int32_t* status, int32_t* host_status, void* stream);
+/* fl_knn_rows / fl_knn_staged_f32 in one entry (split_plane: optional, as in the latter).  host_status:
+ * optional mapped (pinned) host memory of FL_STATUS_WORDS + 1 words; when the call's kernels are through,
+ * it holds the status words, followed by a non-zero completion mark. */
+int     fl_knn_search(const void* q, int64_t nq, int64_t ldq, const void* db, int64_t m, int64_t ldb, int d, int k,
+                      int dtype, int mode, const void* plane, const void* split_plane, int64_t row_offset,
+                      float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status,
+                      int32_t* host_status, void* stream);
 
 /* ---------------------------------------------------------------------------------- */
 /* k-way merge of per-shard candidates (the reference has no sharded kNN; within one    */
