@@ -93,6 +93,11 @@ int direct_ivf_chunks(int64_t npairs);
 int64_t direct_ivf_workspace_bytes(int64_t npairs, int nchunk, int k);
 int launch_ivf_direct(DirectParams p, void* ws, cudaStream_t st);
 
+// Batches of small problems with few features (knn_clouds.cu): one launch, no workspace.
+int clouds_pick(int64_t nq, int64_t m, int d, int k);      // 1: the batch entry point takes it for the shape
+int launch_knn_clouds(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride, const float* db, int64_t m,
+                      int64_t ldb, int64_t db_bstride, int d, int k, float* out_dist, int32_t* out_idx, cudaStream_t st);
+
 // Merge of the per-split pools, exact fp32 re-rank, top-k selection and (optionally)
 // verification of the candidate pool against the scoring error bound.
 struct FinalizeParams {

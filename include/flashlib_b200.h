@@ -117,7 +117,9 @@ int     fl_knn_f32(const float* q, int64_t nq, int64_t ldq,
 /* the batch on a grid axis, knn/triton/insert.py:49; its callers are many small problems, */
 /* where a launch per problem is the whole cost).  Problem b reads q + b * q_bstride and    */
 /* db + b * db_bstride (elements) and writes out_dist / out_idx [batch][nq][k].  Exact      */
-/* CUDA-core path; large problems are better served by one fl_knn_f32 call each.            */
+/* CUDA-core path; large problems are better served by one fl_knn_f32 call each             */
+/* (fl_knn_batch_pick: 1 where the batch is the better way).                                */
+int     fl_knn_batch_pick(int64_t nq, int64_t m, int d, int k);
 int64_t fl_knn_batch_workspace_bytes(int batch, int64_t nq, int64_t m, int d, int k);
 int     fl_knn_batch_f32(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride,
                          const float* db, int64_t m, int64_t ldb, int64_t db_bstride, int d, int k,
