@@ -2,6 +2,7 @@
 // centroid finalisation with per-centroid shift.
 #include "common.cuh"
 #include "simt_tile.cuh"
+#include "kmeans_rows.h"
 
 namespace fl {
 
@@ -324,6 +325,12 @@ extern "C" int fl_kmeans_assign_f32(const float* x, int64_t n, int64_t ldx, cons
         return FL_EWORKSPACE;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    if (kmeans_rows_pick(n, K, d)) {
+        profile_begin(st);
+        const int rc = launch_kmeans_rows(x, 1, n, ldx, 0, c, K, ldc, 0, d, labels, st);
+        profile_end(st);
+        return rc;
+    }
     float* hnorm = static_cast<float*>(ws);
     kmeans_halfnorm_kernel<<<(unsigned)ceil_div(K, 8), 256, 0, st>>>(c, K, d, ldc, hnorm);
     FL_CHECK_LAUNCH();
@@ -488,6 +495,8 @@ extern "C" int fl_kmeans_assign_batch_f32(const float* x, int batch, int64_t n, 
         return FL_EWORKSPACE;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    if (kmeans_rows_pick((int64_t)batch * n, K, d))
+        return launch_kmeans_rows(x, batch, n, ldx, x_batch_stride, c, K, ldc, c_batch_stride, d, labels, st);
     float* hnorm = static_cast<float*>(ws);
     // the centroid sets are contiguous: one pass gives the half norms of all batch items
     kmeans_halfnorm_kernel<<<(unsigned)ceil_div((int64_t)batch * K, 8), 256, 0, st>>>(c, batch * K, d, ldc, hnorm);

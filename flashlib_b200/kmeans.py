@@ -8,6 +8,7 @@ imports; all of them run the sm_100a kernels behind the C ABI.
 """
 from __future__ import annotations
 
+import ctypes
 import os
 from typing import Optional
 
@@ -41,7 +42,7 @@ def _x_plane(x: torch.Tensor) -> torch.Tensor:
     return buf
 
 
-def _use_tensor_cores(n: int, K: int, d: int, mode: Optional[str]) -> bool:
+def _use_tensor_cores(n: int, K: int, d: int, mode: Optional[str], batch: int = 1) -> bool:
     if mode in ("exact", "simt"):
         return False
     if d > 256:
@@ -50,7 +51,7 @@ def _use_tensor_cores(n: int, K: int, d: int, mode: Optional[str]) -> bool:
         return False
     if mode in ("bf16", "tc"):
         return True
-    return n * K >= (1 << 24) and K >= 64
+    return n * K >= (1 << 24) and K >= 64 and not _lib.load().fl_kmeans_assign_pick(batch, n, K, d)
 
 
 def _assign_2d(x: torch.Tensor, c: torch.Tensor, out: torch.Tensor, mode: Optional[str] = None) -> None:
@@ -100,7 +101,7 @@ def euclid_assign_triton(x: torch.Tensor, centroids: torch.Tensor, out: Optional
     if mode is None:
         mode = os.environ.get("FLASHLIB_B200_ASSIGN_MODE") or None
     with torch.cuda.device(x.device):
-        if B > 1 and not _use_tensor_cores(N, K, D, mode):
+        if B > 1 and not _use_tensor_cores(N, K, D, mode, B):
             # many small problems (IVF-PQ's sub-quantisers: a few features, 256 centroids each):
             # one launch with the batch on a grid axis instead of 2 B launches
             lib = _lib.load()
@@ -237,6 +238,22 @@ def triton_lloyd_centroid_step_euclid(x: torch.Tensor, cluster_ids: torch.Tensor
     return new_centroids, cluster_ids, max_shift
 
 
+def _lloyd_rows(x: torch.Tensor, K: int, cur, nxt, sums, cnts, labels, iters: int, tol: float, refresh: int) -> int:
+    """The whole Lloyd loop in one library call (two launches an iteration); returns the iterations run."""
+    lib = _lib.load()
+    _lib.require_device()
+    B, N, D = x.shape
+    ctl = torch.empty(lib.fl_kmeans_lloyd_words(), dtype=torch.int32, device=x.device)
+    host = torch.empty(1, dtype=torch.int32, pin_memory=True) if tol > 0.0 else None
+    n_iter = ctypes.c_int(0)
+    with torch.cuda.device(x.device):
+        _lib.check(lib.fl_kmeans_lloyd_f32(x.data_ptr(), B, N, x.stride(1), x.stride(0), D, K, cur.data_ptr(), nxt.data_ptr(),
+                                           sums.data_ptr(), cnts.data_ptr(), labels.data_ptr(), iters, max(tol, 0.0), refresh,
+                                           ctl.data_ptr(), host.data_ptr() if host is not None else None,
+                                           ctypes.addressof(n_iter), _stream_ptr(x.device)))
+    return n_iter.value
+
+
 def batch_kmeans_Euclid(x: torch.Tensor, n_clusters: int, max_iters: int = 100, tol: float = 0.0,
                         init_centroids: Optional[torch.Tensor] = None, verbose: bool = False, **_ignored):
     """Batched Lloyd k-means, ``x`` ``(B, N, D)`` on CUDA.
@@ -268,6 +285,14 @@ def batch_kmeans_Euclid(x: torch.Tensor, n_clusters: int, max_iters: int = 100, 
     # DELTA_REFRESH-th iteration recomputes them from all rows
     incremental = B == 1 and x32.stride(2) == 1 and os.environ.get("FLASHLIB_B200_KMEANS_DELTA", "1") != "0"
     prev_ids = torch.empty((B, N), device=x.device, dtype=torch.int32) if incremental else None
+    assign_mode = os.environ.get("FLASHLIB_B200_ASSIGN_MODE") or None
+    if (max_iters >= 1 and N >= 1 and not verbose and not _use_tensor_cores(N, K, D, assign_mode, B)
+            and _lib.load().fl_kmeans_lloyd_pick(B, N, K, D)):
+        if x32.stride(2) != 1 or x32.stride(1) < D:
+            x32 = x32.contiguous()
+        n_iter = _lloyd_rows(x32, K, cur, nxt, sums_buf, cnts_buf, cluster_ids, max_iters, tol,
+                             DELTA_REFRESH if incremental else 1)
+        return cluster_ids, (nxt if n_iter % 2 else cur).to(x.dtype), n_iter
     it = 0
     for it in range(max_iters):
         euclid_assign_triton(x32, cur, out=cluster_ids)

@@ -338,6 +338,22 @@ int     fl_kmeans_update_batch_f32(const float* x, int batch, int64_t n, int64_t
 /* new_c = cnt ? sums/cnt : old_c ; shift[j] = ||new_c[j] - old_c[j]||_2.               */
 int     fl_kmeans_finalize_f32(const float* sums, const int32_t* cnts, const float* old_c,
                                float* new_c, float* shift, int K, int d, void* stream);
+/* Lloyd iterations of `batch` independent problems on the CUDA cores (d <= 128), two launches each:  */
+/* x [batch][n][ldx], centroids [batch][K][d] starting in cents_a, sums / cnts scratch of that        */
+/* shape, labels [batch][n].  Every `refresh`-th iteration sums all rows, the ones between move the    */
+/* rows whose label changed.  tol > 0: ends after the iteration whose largest centroid shift is below  */
+/* tol; `host` (an int of pinned memory) then tells the host how far the loop is, the call returns     */
+/* when the loop has ended, and the stream must not be captured.  tol <= 0: only launches (host may be */
+/* null).  *n_iter iterations ran: the centroids are in cents_b when that is odd, else in cents_a.     */
+/* ctl: fl_kmeans_lloyd_words() ints of device scratch.                                                */
+int     fl_kmeans_lloyd_words(void);
+int     fl_kmeans_lloyd_f32(const float* x, int batch, int64_t n, int64_t ldx, int64_t x_batch_stride, int d, int K,
+                            float* cents_a, float* cents_b, float* sums, int32_t* cnts, int32_t* labels, int iters,
+                            float tol, int refresh, int32_t* ctl, int32_t* host, int* n_iter, void* stream);
+/* 1 where that loop beats single steps with the tile kernel; 1 where an assignment is faster on the   */
+/* CUDA cores than on the tensor cores (fl_kmeans_assign_tc_f32).                                      */
+int     fl_kmeans_lloyd_pick(int batch, int64_t n, int K, int d);
+int     fl_kmeans_assign_pick(int batch, int64_t n, int K, int d);
 
 /* ---------------------------------------------------------------------------------- */
 /* IVF-Flat fine scan.  Replaces ivf_fine_scan_gemm + _ivf_fine_gemm_kernel             */
