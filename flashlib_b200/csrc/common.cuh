@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
+#include <cuda_bf16.h>
 #include <stdint.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -92,6 +93,25 @@ __device__ __forceinline__ float4 ld_elem4(const void* base, int64_t i, int dt) 
                            __uint_as_float(w.y & 0xffff0000u));
     return make_float4(f16_bits_to_f32((unsigned short)(w.x & 0xffffu)), f16_bits_to_f32((unsigned short)(w.x >> 16)),
                        f16_bits_to_f32((unsigned short)(w.y & 0xffffu)), f16_bits_to_f32((unsigned short)(w.y >> 16)));
+}
+// Four values as bf16 (round to nearest even), for one 8-byte store.
+__device__ __forceinline__ uint2 bf16x4_bits(float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    uint2 w;
+    w.x = *reinterpret_cast<const uint32_t*>(&a);
+    w.y = *reinterpret_cast<const uint32_t*>(&b);
+    return w;
+}
+// Elements c .. c + 3 of a row of d (zero beyond it); vec: the row allows one wide read and d is a multiple of 4.
+__device__ __forceinline__ float4 ld_row4(const void* p, int c, int d, int vec, int dt) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= d) return v;
+    if (vec) return ld_elem4(p, c, dt);
+    v.x = ld_elem(p, c, dt);
+    if (c + 1 < d) v.y = ld_elem(p, c + 1, dt);
+    if (c + 2 < d) v.z = ld_elem(p, c + 2, dt);
+    if (c + 3 < d) v.w = ld_elem(p, c + 3, dt);
+    return v;
 }
 __device__ __forceinline__ int dt_size_dev(int dt) { return dt == DT_F32 ? 4 : 2; }
 // Address of row r (ld in elements).

@@ -19,11 +19,24 @@ __device__ __forceinline__ void bf16_split(float v, __nv_bfloat16& hi, __nv_bflo
     lo = __float2bfloat16_rn(v - __bfloat162float(hi));
 }
 
-// Centroid side, one warp per row: [m_pad][3 d_pad + 16] rows, ||c||^2/2 per row and the
+__device__ __forceinline__ void bf16_split4(float4 v, uint2& hi, uint2& lo) {
+    __nv_bfloat16 h[4], l[4];
+    bf16_split(v.x, h[0], l[0]);
+    bf16_split(v.y, h[1], l[1]);
+    bf16_split(v.z, h[2], l[2]);
+    bf16_split(v.w, h[3], l[3]);
+    auto bits = [](__nv_bfloat16 a, __nv_bfloat16 b) {
+        return (uint32_t)__bfloat16_as_ushort(a) | (uint32_t)__bfloat16_as_ushort(b) << 16;
+    };
+    hi = make_uint2(bits(h[0], h[1]), bits(h[2], h[3]));
+    lo = make_uint2(bits(l[0], l[1]), bits(l[2], l[3]));
+}
+
+// Centroid side, one warp per row (four columns a lane: wide reads where `vec` allows, 8-byte writes): [m_pad][3 d_pad + 16] rows, ||c||^2/2 per row and the
 // largest row norm.  Padding rows score -3e38.
 __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int d, int64_t ld,
                                      __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                     unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad) {
+                                     unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= m_pad) return;
@@ -36,14 +49,14 @@ __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int
     }
     const float* p = c + row * ld;
     float s = 0.f;
-    for (int t = lane; t < d_pad; t += 32) {
-        const float v = (t < d) ? __ldg(p + t) : 0.f;
-        s += v * v;
-        __nv_bfloat16 hi, lo;
-        bf16_split(v, hi, lo);
-        o[t] = hi;
-        o[d_pad + t] = hi;
-        o[2 * d_pad + t] = lo;
+    for (int t = lane * 4; t < d_pad; t += 128) {
+        const float4 v = ld_row4(p, t, d, vec, DT_F32);
+        s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        uint2 hi, lo;
+        bf16_split4(v, hi, lo);
+        *reinterpret_cast<uint2*>(o + t) = hi;
+        *reinterpret_cast<uint2*>(o + d_pad + t) = hi;
+        *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = lo;
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
@@ -72,7 +85,7 @@ __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int
 __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, int d, const int* __restrict__ rows,
                                       const int* __restrict__ rows_count, int cap, __nv_bfloat16* __restrict__ out,
                                       int d_pad, const float* __restrict__ prev_dist, int k,
-                                      const float* __restrict__ maxnorm, float eps_rel, float* __restrict__ tau_out) {
+                                      const float* __restrict__ maxnorm, float eps_rel, float* __restrict__ tau_out, int vec) {
     const int lane = threadIdx.x & 31;
     const int pitch = 3 * d_pad + PLANE_AUG_COLS;
     int count = *rows_count;
@@ -88,14 +101,14 @@ __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, 
         const float* src = x + pt * ldx;
         __nv_bfloat16* o = out + (int64_t)r * pitch;
         float qsq = 0.f;
-        for (int t = lane; t < d_pad; t += 32) {
-            __nv_bfloat16 hi, lo;
-            const float v = t < d ? __ldg(src + t) : 0.f;
-            qsq += v * v;
-            bf16_split(v, hi, lo);
-            o[t] = hi;
-            o[d_pad + t] = lo;
-            o[2 * d_pad + t] = hi;
+        for (int t = lane * 4; t < d_pad; t += 128) {
+            uint2 hi, lo;
+            const float4 v = ld_row4(src, t, d, vec, DT_F32);
+            qsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            bf16_split4(v, hi, lo);
+            *reinterpret_cast<uint2*>(o + t) = hi;
+            *reinterpret_cast<uint2*>(o + d_pad + t) = lo;
+            *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = hi;
         }
         if (lane < PLANE_AUG_COLS) o[3 * d_pad + lane] = __float2bfloat16_rn(lane < 3 ? 1.f : 0.f);
         if (tau_out != nullptr) {
@@ -202,19 +215,6 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
             }
         }
     }
-}
-
-// ||x||^2 of every sample row (one warp per row); the scoring error bound of a point needs it.
-__global__ void rowsq_kernel(const float* __restrict__ x, int64_t n, int d, int64_t ld, float* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= n) return;
-    const float* p = x + row * ld;
-    float s = 0.f;
-    for (int c = lane; c < d; c += 32) { const float v = __ldg(p + c); s += v * v; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
-    if (lane == 0) out[row] = s;
 }
 
 // First-stage proof from the scores alone, one thread per point: the best-scoring centroid is the
@@ -331,7 +331,7 @@ int launch_split_db_plane(const float* c, int64_t m, int d, int64_t ldc, void* p
     const int wpb = 8;
     split_c_plane_kernel<<<(unsigned)ceil_div(L.m_pad, wpb), wpb * 32, 0, st>>>(
         c, m, d, ldc, reinterpret_cast<__nv_bfloat16*>(pl + L.off_rows), reinterpret_cast<float*>(pl + L.off_hnorm),
-        reinterpret_cast<unsigned int*>(pl + L.off_meta), L.m_pad, d_pad);
+        reinterpret_cast<unsigned int*>(pl + L.off_meta), L.m_pad, d_pad, dt_vec_ok(c, ldc, DT_F32) && d % 4 == 0);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
@@ -341,7 +341,8 @@ int launch_split_query_gather(const float* x, int64_t ldx, int d, const int* row
                               float* tau_out, cudaStream_t st) {
     split_x_gather_kernel<<<(unsigned)(8 * sm_count()), 256, 0, st>>>(x, ldx, d, rows, rows_count, cap,
                                                                      static_cast<__nv_bfloat16*>(out), d_pad, prev_dist, k,
-                                                                     maxnorm, eps_rel, tau_out);
+                                                                     maxnorm, eps_rel, tau_out,
+                                                                     dt_vec_ok(x, ldx, DT_F32) && d % 4 == 0);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
@@ -366,12 +367,9 @@ extern "C" int fl_kmeans_prepare_x_f32(const float* x, int64_t n, int d, int64_t
     FL_CHECK_ARG(x && xplane && n >= 1 && d >= 1 && ldx >= d, "fl_kmeans_prepare_x_f32: bad arguments");
     if (xplane_bytes < fl_kmeans_xplane_bytes(n, d)) { set_error("fl_kmeans_prepare_x_f32: plane buffer too small"); return FL_EWORKSPACE; }
     const int64_t n_pad = round_up(n, 128);
-    const int rc = launch_query_plane(x, n, ldx, d, xplane, n_pad, (int)round_up(d, 64), (cudaStream_t)stream);
-    if (rc != FL_OK) return rc;
+    // the rows' norms (the scoring error bound of a point needs its own) come from the same read
     float* xsq = reinterpret_cast<float*>(static_cast<char*>(xplane) + round_up(n_pad * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024));
-    rowsq_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, (cudaStream_t)stream>>>(x, n, d, ldx, xsq);
-    FL_CHECK_LAUNCH();
-    return FL_OK;
+    return launch_query_plane(x, n, ldx, d, xplane, n_pad, (int)round_up(d, 64), (cudaStream_t)stream, DT_F32, xsq);
 }
 
 extern "C" int64_t fl_kmeans_assign_tc_workspace_bytes(int64_t n, int K, int d, int have_xplane) {
@@ -412,12 +410,10 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     const char* xpl = static_cast<const char*>(xplane);
     const float* xsq;
     if (!xpl) {
-        rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st);
+        float* xs = reinterpret_cast<float*>(base + w.off_xsq);
+        rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs);
         if (rc != FL_OK) return rc;
         xpl = base + w.off_xplane;
-        float* xs = reinterpret_cast<float*>(base + w.off_xsq);
-        rowsq_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(x, n, d, ldx, xs);
-        FL_CHECK_LAUNCH();
         xsq = xs;
     } else {
         xsq = reinterpret_cast<const float*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
@@ -475,7 +471,7 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     if (w.split) {
         __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(base + w.off_xsplit);
         split_x_gather_kernel<<<(unsigned)(8 * sm_count()), 256, 0, st>>>(x, ldx, d, l1_list, l1_count, w.l1_cap, xs, w.d_pad,
-                                                                         nullptr, 0, nullptr, 0.f, nullptr);
+                                                                         nullptr, 0, nullptr, 0.f, nullptr, vecx && d % 4 == 0);
         FL_CHECK_LAUNCH();
         TcKnnParams tp{};
         tp.qplane = xs; tp.nq = w.l1_cap; tp.nq_pad = w.l1_pad;

@@ -33,22 +33,42 @@ __global__ void halfnorm_kernel(const void* __restrict__ x, int64_t n, int d, in
 // still change the answer.
 constexpr float SIMT_EPS_REL = 4e-6f;
 
-// bf16 query plane [nq_pad][d_pad + 16]: the features, zero padding, and ones in the three
-// columns that meet the database plane's split -||x||^2/2 terms.
-__global__ void query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d,
-                                   __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt) {
-    const int pitch = d_pad + PLANE_AUG_COLS;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t total = nq_pad * pitch;
-    if (i >= total) return;
-    const int64_t r = i / pitch;
-    const int c = (int)(i - r * pitch);
-    float v = 0.f;
-    if (r < nq) {
-        if (c < d) v = ld_elem(row_at(q, r, ldq, dt), c, dt);
-        else if (c >= d_pad && c < d_pad + 3) v = 1.f;
+// One row of a bf16 query plane by a warp: the features, zero padding, and ones in the three columns that meet
+// the database plane's split -||x||^2/2 terms (all zero for rows that pad the last tile).  Four columns a
+// lane: 16-byte reads where `vec` says that the rows allow them, 8-byte writes (plane rows are 32-byte
+// aligned: their pitch is a multiple of 16 columns).  Returns the lane's share of ||q||^2.
+__device__ __forceinline__ float query_plane_row(const void* p, bool live, int d, int vec, __nv_bfloat16* o, int d_pad, int dt) {
+    const int lane = threadIdx.x & 31;
+    float sq = 0.f;
+    for (int c = lane * 4; c < d_pad + PLANE_AUG_COLS; c += 128) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live) {
+            if (c < d) {
+                v = ld_row4(p, c, d, vec, dt);
+                sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            } else if (c == d_pad) {
+                v = make_float4(1.f, 1.f, 1.f, 0.f);
+            }
+        }
+        *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
     }
-    out[i] = __float2bfloat16_rn(v);
+    return sq;
+}
+
+// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row from the same read.
+// Bound by HBM: 250 001 x 96 rows take 43 us (96 MB in, 72 MB out).  One thread per plane element and a second
+// pass over the rows for the norms took some 180.
+__global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
+                                                          __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt,
+                                                          float* __restrict__ sq_out) {
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= nq_pad) return;
+    const bool live = row < nq;
+    float s = query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
+    if (sq_out == nullptr || !live) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+    if ((threadIdx.x & 31) == 0) sq_out[row] = s;
 }
 
 // What a tensor-core call needs before its first scoring launch, in one pass: the bf16 query plane, the
@@ -62,42 +82,17 @@ __global__ void __launch_bounds__(256) knn_prep_kernel(const void* __restrict__ 
         counters[threadIdx.x] = 0;
         if (status != nullptr && threadIdx.x < FL_STATUS_WORDS) status[threadIdx.x] = 0;
     }
-    const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= nq_pad) return;
-    const int pitch = d_pad + PLANE_AUG_COLS;              // (a multiple of 16 columns: rows are 32-byte aligned)
-    __nv_bfloat16* o = out + row * pitch;
     const bool live = row < nq;
-    const void* p = row_at(q, live ? row : 0, ldq, dt);
-    for (int c = lane * 4; c < pitch; c += 128) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
-            if (c < d) {
-                if (vec) v = ld_elem4(p, c, dt);
-                else {
-                    v.x = ld_elem(p, c, dt);
-                    if (c + 1 < d) v.y = ld_elem(p, c + 1, dt);
-                    if (c + 2 < d) v.z = ld_elem(p, c + 2, dt);
-                    if (c + 3 < d) v.w = ld_elem(p, c + 3, dt);
-                }
-            } else if (c == d_pad) {
-                v = make_float4(1.f, 1.f, 1.f, 0.f);
-            }
-        }
-        const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-        uint2 w;
-        w.x = *reinterpret_cast<const uint32_t*>(&a);
-        w.y = *reinterpret_cast<const uint32_t*>(&b);
-        *reinterpret_cast<uint2*>(o + c) = w;
-    }
-    if (lane == 0) tau[row] = live ? neg_inf() : pos_inf();
+    query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
+    if ((threadIdx.x & 31) == 0) tau[row] = live ? neg_inf() : pos_inf();
 }
 
-int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad,
-                       int d_pad, cudaStream_t st, int dt) {
-    const int64_t total = nq_pad * (d_pad + PLANE_AUG_COLS);
-    query_plane_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, st>>>(
-        q, nq, ldq, d, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt);
+int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad, int d_pad,
+                       cudaStream_t st, int dt, float* sq_out) {
+    query_plane_kernel<<<(unsigned)ceil_div(nq_pad, 8), 256, 0, st>>>(
+        q, nq, ldq, d, dt_vec_ok(q, ldq, dt) && d % 4 == 0, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt, sq_out);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }

@@ -39,10 +39,11 @@ __global__ void rownorm_kernel(const float* __restrict__ x, int64_t n, int d, in
 // make the tensor-core product come out as <q,x> - ||x||^2/2.  Padding rows carry a huge
 // negative value there so they can never rank.
 // Rows of 16-bit storage (dt): bf16 values enter the plane as they are, fp16 values are rounded to
-// bf16 like fp32 ones; the norms are those of the stored values.
+// bf16 like fp32 ones; the norms are those of the stored values.  Four columns a lane: 16-byte reads where the
+// rows allow them (vec) and 8-byte writes.
 __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d, int64_t ld,
                                    __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                   unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad, int dt) {
+                                   unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad, int dt, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= m_pad) return;
@@ -55,10 +56,10 @@ __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d
     }
     const void* p = row_at(db, row, ld, dt);
     float s = 0.f;
-    for (int c = lane; c < d_pad; c += 32) {
-        const float v = (c < d) ? ld_elem(p, c, dt) : 0.f;
-        s += v * v;
-        o[c] = __float2bfloat16_rn(v);
+    for (int c = lane * 4; c < d_pad; c += 128) {
+        const float4 v = ld_row4(p, c, d, vec, dt);
+        s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
@@ -98,7 +99,7 @@ int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane
     plane_build_kernel<<<(unsigned)ceil_div(L.m_pad, wpb), wpb * 32, 0, st>>>(
         db, m, d, ld, reinterpret_cast<__nv_bfloat16*>(base + L.off_rows),
         reinterpret_cast<float*>(base + L.off_hnorm), reinterpret_cast<unsigned int*>(base + L.off_meta),
-        L.m_pad, L.d_pad, dt);
+        L.m_pad, L.d_pad, dt, dt_vec_ok(db, ld, dt) && d % 4 == 0);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
