@@ -260,6 +260,82 @@ __global__ void __launch_bounds__(256) assign_by_lead_kernel(
     }
 }
 
+// Points whose label could not be proven, when they are few: one block per listed point, eight lanes per centroid,
+// the fp32 sum (x - c)^2 to every centroid; the lowest index wins exact ties.  Left to the tile pass (`rest`,
+// whose counter starts at zero): longer lists as a whole, where the tiles' reuse of the centroids pays, and
+// points without a finite distance.  Bound by latency -- a block walks K / 64 dependent loads: for the few dozen points
+// of the 1M x 128, K = 1 024 loop 24 us (and 7 for the empty tile pass) where the tile pass and its finalisation took 78 + 20.
+constexpr int ASSIGN_DIRECT_MAX = 2048, ASSIGN_DIRECT_MAX_K = 4096;
+__global__ void __launch_bounds__(256) assign_direct_kernel(
+    const float* __restrict__ x, int64_t ldx, const float* __restrict__ c, int K, int64_t ldc, int d, int vec,
+    const int* __restrict__ list, const int* __restrict__ list_count, int32_t* __restrict__ labels,
+    int* __restrict__ rest_list, int* __restrict__ rest_count) {
+    __shared__ __align__(16) float xs[256];
+    __shared__ float s_best[8];
+    __shared__ int s_idx[8];
+    const int tid = threadIdx.x, lane = tid & 31, sl = tid & 7, g = tid >> 3;
+    const int count = *list_count;
+    if (count > ASSIGN_DIRECT_MAX) {
+        for (int i = blockIdx.x * 256 + tid; i < count; i += gridDim.x * 256) rest_list[i] = list[i];
+        if (blockIdx.x == 0 && tid == 0) *rest_count = count;
+        return;
+    }
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int pt = list[i];
+        if (tid < d) xs[tid] = __ldg(x + (int64_t)pt * ldx + tid);
+        __syncthreads();
+        float best = pos_inf();
+        int bi = 0x7fffffff;
+        for (int base = 0; base < K; base += 64) {
+            const int j0 = base + g, j1 = base + 32 + g;
+            const float* c0 = c + (int64_t)(j0 < K ? j0 : K - 1) * ldc;
+            const float* c1 = c + (int64_t)(j1 < K ? j1 : K - 1) * ldc;
+            float a0 = 0.f, a1 = 0.f;
+            if (vec) {
+#pragma unroll 4
+                for (int t = sl * 4; t < d; t += 32) {
+                    const float4 xv = *reinterpret_cast<const float4*>(xs + t);
+                    const float4 p0 = __ldg(reinterpret_cast<const float4*>(c0 + t));
+                    const float4 p1 = __ldg(reinterpret_cast<const float4*>(c1 + t));
+                    float e0 = xv.x - p0.x, e1 = xv.y - p0.y, e2 = xv.z - p0.z, e3 = xv.w - p0.w;
+                    a0 += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
+                    e0 = xv.x - p1.x; e1 = xv.y - p1.y; e2 = xv.z - p1.z; e3 = xv.w - p1.w;
+                    a1 += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
+                }
+            } else {
+#pragma unroll 4
+                for (int t = sl; t < d; t += 8) {
+                    const float e0 = xs[t] - __ldg(c0 + t), e1 = xs[t] - __ldg(c1 + t);
+                    a0 += e0 * e0;
+                    a1 += e1 * e1;
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                a0 += __shfl_xor_sync(FULL_MASK, a0, o);
+                a1 += __shfl_xor_sync(FULL_MASK, a1, o);
+            }
+            if (j0 < K && a0 < best) { best = a0; bi = j0; }       // ascending: the lower index stays on ties
+            if (j1 < K && a1 < best) { best = a1; bi = j1; }
+        }
+#pragma unroll
+        for (int o = 16; o >= 8; o >>= 1) {
+            const float ob = __shfl_xor_sync(FULL_MASK, best, o);
+            const int oi = __shfl_xor_sync(FULL_MASK, bi, o);
+            if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+        }
+        if (lane == 0) { s_best[tid >> 5] = best; s_idx[tid >> 5] = bi; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < 8; ++w)
+                if (s_best[w] < best || (s_best[w] == best && s_idx[w] < bi)) { best = s_best[w]; bi = s_idx[w]; }
+            if (bi != 0x7fffffff) labels[pt] = bi;
+            else rest_list[atomicAdd(rest_count, 1)] = pt;
+        }
+        __syncthreads();
+    }
+}
+
 struct AssignTcWs {
     int64_t n_pad; int d_pad, pitch; int fb_cap;
     int split;          // 1: a second stage with split (hi/lo) operand planes of 3 d_pad columns
@@ -267,7 +343,7 @@ struct AssignTcWs {
     int nsplit_fb; int64_t rows_per_split_fb; int fb_bq, fb_blocks;
     PlaneLayout cl, cl3;
     int64_t off_cplane, off_cplane3, off_xplane, off_xsq, off_xsplit, off_asg_sc, off_asg_id, off_tau, off_cnt, off_l0list, off_l1list,
-        off_fblist, off_fbpart_sc, off_fbpart_id, off_fbdist, bytes;
+        off_fblist, off_fblist2, off_fbpart_sc, off_fbpart_id, off_fbdist, bytes;
 };
 
 // Split planes need the 128-row sample tile of 3 d_pad columns resident in shared memory
@@ -313,6 +389,7 @@ static AssignTcWs assign_tc_plan(int64_t n, int K, int d, int have_xplane) {
     w.off_l0list = take(cur, (w.split ? n : 1) * 4);
     w.off_l1list = take(cur, (int64_t)(w.l1_cap > 0 ? w.l1_cap : 1) * 4);
     w.off_fblist = take(cur, (int64_t)w.fb_cap * 4);
+    w.off_fblist2 = take(cur, (int64_t)w.fb_cap * 4);
     w.off_fbpart_sc = take(cur, fb_pools * 32 * 4);
     w.off_fbpart_id = take(cur, fb_pools * 32 * 4);
     w.off_fbdist = take(cur, n * 4);
@@ -489,7 +566,16 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     rc = launch_fallback_fixup(fb_count, w.fb_cap, status, tc_pool_size(1), st);
     if (rc != FL_OK) return rc;
 
-    // points whose label could not be proven: exact CUDA-core scoring + exact re-rank, k = 1
+    // points whose label could not be proven: a few directly, otherwise exact CUDA-core scoring + exact re-rank, k = 1
+    if (K <= ASSIGN_DIRECT_MAX_K) {
+        int* rest_count = counters + 192;                          // (cleared with the others)
+        int* rest_list = reinterpret_cast<int*>(base + w.off_fblist2);
+        assign_direct_kernel<<<(unsigned)(4 * sm_count()), 256, 0, st>>>(x, ldx, c, K, ldc, d, vec, fb_list, fb_count, labels,
+                                                                        rest_list, rest_count);
+        FL_CHECK_LAUNCH();
+        fb_list = rest_list;
+        fb_count = rest_count;
+    }
     SimtKnnParams sp{};
     sp.q = x; sp.ldq = ldx; sp.qlist = fb_list; sp.count_dev = fb_count; sp.count = 0;
     sp.db = c; sp.m = K; sp.ldb = ldc; sp.d = d;

@@ -92,3 +92,20 @@ def test_lloyd_loop_keeps_empty_clusters():
     init[0, 5] = 1e6
     _, cents, _ = km.batch_kmeans_Euclid(x, 6, max_iters=4, init_centroids=init)
     assert torch.equal(cents[0, 5], init[0, 5])
+
+
+@pytest.mark.parametrize("n,d,K,dup", [(3000, 128, 200, 0), (3000, 33, 70, 0), (5000, 64, 130, 8), (1500, 250, 65, 1500)])
+def test_tensor_core_assignment_of_unprovable_points(n, d, K, dup):
+    # centroids in near-equal and equal pairs: no scoring bound decides between the two; with `dup` points (a few, or
+    # more than the direct pass takes) on the bisector of two equal centroids the lower index wins
+    x, c = _problem(1, n, d, K, seed=11)
+    c[0, K // 2:2 * (K // 2)] = c[0, :K // 2] * (1 + 1e-6)
+    c[0, K - 1] = c[0, 0]
+    if dup:
+        x[0, :dup] = c[0, 0]
+    lab = fl.euclid_assign_triton(x, c, mode="bf16")
+    _check_labels(x, c, lab)
+    assert (lab[0, :dup] == 0).all()
+    x[0, 7, 0] = float("nan")
+    lab = fl.euclid_assign_triton(x, c, mode="bf16")
+    _check_labels(x[:, 8:], c, lab[:, 8:])
