@@ -6,65 +6,65 @@
 // sorts each query's list.  A list that overflows -- many equal distances, or an order of the rows that
 // resonates with the groups -- is answered by a warp that scans the rows with a sorted pool.
 //
-// Bound: issue slots and the FP32 pipe (about 10 instructions a pair and pass).  The tile kernel
-// (knn_simt.cu) pads 3 features to 32 and keeps a pool per query in shared memory: 32 problems of
-// 2 048 x 2 048 x 3, k = 16, took it 1 700 us; here 317.
+// The rows lie feature by feature in shared memory and a thread takes four at a time in packed pairs: a
+// shared-memory read returns 128 bytes a cycle and SM however many lanes want the same word, so rows padded
+// to four features, one at a time, cost 16 such cycles a warp and row of the four sub-cores (317 us for
+// the batch below), three features of four rows 12, and no sum has to be folded.
+//
+// Bound: shared-memory return bandwidth and the FP32 pipe.  The tile kernel (knn_simt.cu) pads 3 features to 32 and
+// keeps a pool per query in shared memory: 32 problems of 2 048 x 2 048 x 3, k = 16, took it 1 710 us; here 232.
 #include "knn_internal.h"
 #include "packed.cuh"
 
 namespace fl {
 
 constexpr int CLOUD_THREADS = 128, CLOUD_WARPS = CLOUD_THREADS / 32;
-constexpr int CLOUD_CHUNK_BYTES = 16 * 1024;
 constexpr int CLOUD_LIST = 32;                    // entries a thread keeps
 
-template <int DP>
-__device__ __forceinline__ float cloud_dist(const unsigned long long (&q)[DP / 2], const ulonglong2* row) {
-    unsigned long long s0 = 0ull, s1 = 0ull;
+// Squared distances of four consecutive rows, two packed pairs of rows at a time: the rows lie feature by feature
+// (negated) in shared memory, CP floats apart, so nothing is padded but the features to DP and no sum
+// has to be folded.
+template <int DP, int CP>
+__device__ __forceinline__ void cloud_dist4(const unsigned long long (&q)[DP], const float* rows, float (&s)[4]) {
+    unsigned long long s01 = 0ull, s23 = 0ull;
 #pragma unroll
-    for (int i = 0; i < DP / 4; ++i) {
-        const ulonglong2 v = row[i];
-        s0 = sqadd2(add2(q[2 * i], v.x), s0);
-        s1 = sqadd2(add2(q[2 * i + 1], v.y), s1);
+    for (int f = 0; f < DP; ++f) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(rows + f * CP);
+        s01 = sqadd2(add2(q[f], v.x), s01);
+        s23 = sqadd2(add2(q[f], v.y), s23);
     }
-    return fold2(add2(s0, s1));
+    unpk2(s01, s[0], s[1]);
+    unpk2(s23, s[2], s[3]);
 }
 
-// Rows [c0, c0 + kc) of the problem, negated and zero padded to DP features.
-template <int DP>
+// Rows [c0, c0 + kc) of the problem, and NaN up to a multiple of four rows: no comparison lets those pass.
+template <int DP, int CP>
 __device__ __forceinline__ void cloud_stage(float* rows, const float* db, int64_t ldb, int d, int c0, int kc) {
-    for (int e = threadIdx.x; e < kc * DP; e += CLOUD_THREADS) {
+    const int kp = (kc + 3) & ~3;
+    for (int e = threadIdx.x; e < kp * DP; e += CLOUD_THREADS) {
         const int j = e / DP, f = e - j * DP;
-        rows[e] = f < d ? -__ldg(db + (int64_t)(c0 + j) * ldb + f) : 0.f;
+        rows[f * CP + j] = j >= kc ? __int_as_float(0x7fc00000) : f < d ? -__ldg(db + (int64_t)(c0 + j) * ldb + f) : 0.f;
     }
 }
 
 // One query's answer by a warp: 32 rows at a time, sorted and merged into the pool when one of them
 // belongs there.  Out of line: rare.
-template <int DP, int NPL>
+template <int NPL>
 static __device__ __noinline__ void cloud_scan_query(const float* q, const float* db, int m, int64_t ldb, int d, int k,
                                                      float (&ka)[NPL], uint32_t (&ia)[NPL]) {
     const int lane = threadIdx.x & 31;
-    unsigned long long xr[DP / 2];
-#pragma unroll
-    for (int i = 0; i < DP / 2; ++i) xr[i] = pk2(2 * i < d ? __ldg(q + 2 * i) : 0.f, 2 * i + 1 < d ? __ldg(q + 2 * i + 1) : 0.f);
 #pragma unroll
     for (int r = 0; r < NPL; ++r) { ka[r] = neg_inf(); ia[r] = INVALID_ID; }
     float kth = neg_inf();
     int have = 0;
     for (int base = 0; base < m; base += 32) {
         const int row = base + lane;
-        ulonglong2 v[DP / 4];
-#pragma unroll
-        for (int i = 0; i < DP / 4; ++i) {
-            const float* p = db + (int64_t)row * ldb + 4 * i;
-            float f[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) f[e] = (row < m && 4 * i + e < d) ? -__ldg(p + e) : 0.f;
-            v[i].x = pk2(f[0], f[1]);
-            v[i].y = pk2(f[2], f[3]);
+        const float* p = db + (int64_t)(row < m ? row : m - 1) * ldb;
+        float s = 0.f;
+        for (int f = 0; f < d; ++f) {
+            const float df = __ldg(q + f) - __ldg(p + f);
+            s = fmaf(df, df, s);
         }
-        const float s = cloud_dist<DP>(xr, v);
         const bool real = row < m && s == s;
         float kb[NPL];
         uint32_t ib[NPL];
@@ -92,19 +92,19 @@ struct CloudParams {
 };
 
 // G groups; answers of up to 32 NPL entries are sorted.  Every thread lists what it meets on its own --
-// no counter is shared and nothing branches in the second pass.
+// no counter is shared and only a row group with a candidate branches in the second pass.
 template <int DP, int G, int NPL>
 __global__ void __launch_bounds__(CLOUD_THREADS) knn_clouds_kernel(const CloudParams p) {
     extern __shared__ __align__(16) float cloud_smem[];
-    constexpr int CH = CLOUD_CHUNK_BYTES / (DP * 4), LP = CLOUD_LIST + 1;
+    constexpr int CH = DP <= 4 ? 1024 : DP <= 8 ? 512 : 256, CP = CH + 4, LP = CLOUD_LIST + 1;
     static_assert(CH % G == 0, "a chunk holds whole rounds of the groups");
     __shared__ int s_cnt[CLOUD_THREADS];
     __shared__ float s_thr[CLOUD_THREADS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Q = CLOUD_THREADS / p.splits;        // queries of this block
     const int ql = tid % Q, split = tid / Q;
-    float* rows = cloud_smem;                      // [CH][DP]
-    float* mins = rows + CH * DP;                  // [G][Q], then the lists [thread][LP]
+    float* rows = cloud_smem;                      // [DP][CP]
+    float* mins = rows + DP * CP;                  // [G][Q], then the lists [thread][LP]
     float* l_key = mins;
     uint32_t* l_id = reinterpret_cast<uint32_t*>(l_key + CLOUD_THREADS * LP);
     const float* q = p.q + blockIdx.y * p.q_bstride;
@@ -113,24 +113,30 @@ __global__ void __launch_bounds__(CLOUD_THREADS) knn_clouds_kernel(const CloudPa
     const int64_t qi = q0 + ql;
     const int m = p.m, k = p.k;
 
-    unsigned long long xr[DP / 2];
+    unsigned long long xr[DP];                     // every feature twice
 #pragma unroll
-    for (int i = 0; i < DP / 2; ++i) {
-        const float a = (qi < p.nq && 2 * i < p.d) ? __ldg(q + qi * p.ldq + 2 * i) : 0.f;
-        const float b = (qi < p.nq && 2 * i + 1 < p.d) ? __ldg(q + qi * p.ldq + 2 * i + 1) : 0.f;
-        xr[i] = pk2(a, b);
+    for (int f = 0; f < DP; ++f) {
+        const float v = (qi < p.nq && f < p.d) ? __ldg(q + qi * p.ldq + f) : 0.f;
+        xr[f] = pk2(v, v);
     }
     for (int c0 = 0; c0 < m; c0 += CH) {
         const int kc = min(CH, m - c0);
         if (c0 > 0) __syncthreads();
-        cloud_stage<DP>(rows, db, p.ldb, p.d, c0, kc);
+        cloud_stage<DP, CP>(rows, db, p.ldb, p.d, c0, kc);
         __syncthreads();
-        for (int g = split; g < G; g += p.splits) {
-            float mn = c0 > 0 ? mins[g * Q + ql] : pos_inf();
-#pragma unroll 4
-            for (int j = g; j < kc; j += G)        // (fminf takes the number where the other is NaN)
-                mn = fminf(mn, cloud_dist<DP>(xr, reinterpret_cast<const ulonglong2*>(rows + j * DP)));
-            mins[g * Q + ql] = mn;
+        for (int g = split * 4; g < G; g += p.splits * 4) {
+            float mn[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mn[i] = c0 > 0 ? mins[(g + i) * Q + ql] : pos_inf();
+#pragma unroll 2
+            for (int j = g; j < kc; j += G) {      // (fminf takes the number where the other is NaN)
+                float s[4];
+                cloud_dist4<DP, CP>(xr, rows + j, s);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mn[i] = fminf(mn[i], s[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mins[(g + i) * Q + ql] = mn[i];
         }
     }
     __syncthreads();
@@ -164,15 +170,21 @@ __global__ void __launch_bounds__(CLOUD_THREADS) knn_clouds_kernel(const CloudPa
         const int kc = min(CH, m - c0);
         if (m > CH) {
             if (c0 > 0) __syncthreads();
-            cloud_stage<DP>(rows, db, p.ldb, p.d, c0, kc);
+            cloud_stage<DP, CP>(rows, db, p.ldb, p.d, c0, kc);
             __syncthreads();
         }
-#pragma unroll 4
-        for (int j = split; j < kc; j += p.splits) {
-            const float s = cloud_dist<DP>(xr, reinterpret_cast<const ulonglong2*>(rows + j * DP));
-            const bool in = s <= thr;
-            if (in && cnt < CLOUD_LIST) { my_key[cnt] = -s; my_id[cnt] = (uint32_t)(c0 + j); }
-            cnt += in ? 1 : 0;
+#pragma unroll 2
+        for (int j = split * 4; j < kc; j += p.splits * 4) {
+            float s[4];
+            cloud_dist4<DP, CP>(xr, rows + j, s);
+            if (fminf(fminf(s[0], s[1]), fminf(s[2], s[3])) <= thr) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool in = s[i] <= thr;
+                    if (in && cnt < CLOUD_LIST) { my_key[cnt] = -s[i]; my_id[cnt] = (uint32_t)(c0 + j + i); }
+                    cnt += in ? 1 : 0;
+                }
+            }
         }
     }
     s_cnt[tid] = cnt;
@@ -198,7 +210,7 @@ __global__ void __launch_bounds__(CLOUD_THREADS) knn_clouds_kernel(const CloudPa
             }
             warp_sort_desc<NPL, true>(ka, ia);
         } else {
-            cloud_scan_query<DP, NPL>(q + (q0 + t) * p.ldq, db, m, p.ldb, p.d, k, ka, ia);
+            cloud_scan_query<NPL>(q + (q0 + t) * p.ldq, db, m, p.ldb, p.d, k, ka, ia);
         }
         const int64_t o = (blockIdx.y * p.nq + q0 + t) * k;
 #pragma unroll
@@ -221,7 +233,7 @@ static int clouds_launch(CloudParams p, int batch, cudaStream_t st) {
     while (p.splits < 4 && batch * ceil_div(p.nq, CLOUD_THREADS / p.splits) < 4 * (int64_t)sm_count()) p.splits *= 2;
     const int Q = CLOUD_THREADS / p.splits;
     const size_t lists = (size_t)CLOUD_THREADS * (CLOUD_LIST + 1) * 2, mins = (size_t)G * Q;
-    const size_t smem = CLOUD_CHUNK_BYTES + sizeof(float) * (lists > mins ? lists : mins);
+    const size_t smem = sizeof(float) * (DP * ((DP <= 4 ? 1024 : DP <= 8 ? 512 : 256) + 4) + (lists > mins ? lists : mins));
     FL_CHECK_CUDA(cudaFuncSetAttribute(knn_clouds_kernel<DP, G, NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     knn_clouds_kernel<DP, G, NPL><<<dim3((unsigned)ceil_div(p.nq, Q), (unsigned)batch), CLOUD_THREADS, smem, st>>>(p);
     FL_CHECK_LAUNCH();
@@ -238,8 +250,9 @@ static int clouds_dispatch(const CloudParams& p, int batch, cudaStream_t st) {
 }
 
 // The time of a problem pair grows with the padded features and the number of neighbours; one problem after
-// the other on the tensor cores costs 100 us or more each.  Measured, batch against one by one: 2 x 4 000^2 x 6,
-// k = 40: 259 and 289 us; 4 x 8 192^2 x 3, k = 16: 551 and 853; 4 x 8 192^2 x 16, k = 40: 1 618 and 996.
+// the other on the tensor cores costs 100 us or more each.  Measured, batch against one by one: 2 x 4 000^2 x 16,
+// k = 40: 276 and 286 us; 2 x 8 192^2 x 8, k = 32: 377 and 483; 4 x 8 192^2 x 3, k = 16: 387 and 831; with 16
+// features and k = 40 at 8 192^2 the batch lost (1 618 and 996 for four problems).
 int clouds_pick(int64_t nq, int64_t m, int d, int k) {
     return nq >= 1 && d <= 16 && k <= 40 && nq * m <= ((int64_t)1 << (d <= 8 && k <= 32 ? 26 : 24));
 }
@@ -250,7 +263,8 @@ int launch_knn_clouds(const float* q, int batch, int64_t nq, int64_t ldq, int64_
     p.q = q; p.nq = nq; p.ldq = ldq; p.q_bstride = q_bstride;
     p.db = db; p.m = (int)m; p.ldb = ldb; p.db_bstride = db_bstride;
     p.d = d; p.k = k; p.out_dist = out_dist; p.out_idx = out_idx;
-    if (d <= 4) return clouds_dispatch<4>(p, batch, st);
+    if (d <= 3) return clouds_dispatch<3>(p, batch, st);
+    if (d == 4) return clouds_dispatch<4>(p, batch, st);
     if (d <= 8) return clouds_dispatch<8>(p, batch, st);
     return clouds_dispatch<16>(p, batch, st);
 }
