@@ -11,7 +11,7 @@
 // to four features, one at a time, cost 16 such cycles a warp and row of the four sub-cores (317 us for
 // the batch below), three features of four rows 12, and no sum has to be folded.
 //
-// Bound: shared-memory return bandwidth and the FP32 pipe.  The tile kernel (knn_simt.cu) pads 3 features to 32 and
+// Bound: dependent instructions with few warps to hide them (3.5 a scheduler; issue slots 53 % busy).  The tile kernel (knn_simt.cu) pads 3 features to 32 and
 // keeps a pool per query in shared memory: 32 problems of 2 048 x 2 048 x 3, k = 16, took it 1 710 us; here 232.
 #include "knn_internal.h"
 #include "packed.cuh"
