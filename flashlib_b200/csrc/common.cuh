@@ -289,6 +289,16 @@ __device__ __forceinline__ void atomic_max_f32(float* addr, float v) {
     }
 }
 
+// The proof that a candidate list is complete: every row outside it has a score (half of qsq minus its distance) of at
+// most bound + eps, so none of them comes closer than the k-th distance dk on it.  A bound of -inf says that no row
+// was left out at all, which a score of NaN -- infinite or NaN operands, a norm that overflows -- does
+// not obey: such a row passes no comparison and raises no threshold.  Where one can exist, `slack` (a
+// multiple of ||q||^2 plus the square of the largest row norm) is not finite and nothing is proven.
+__device__ __forceinline__ bool list_proven(float dk, float qsq, float bound, float eps, float slack) {
+    if (bound == neg_inf()) return slack < pos_inf();
+    return dk < qsq - 2.f * (bound + eps) - slack;
+}
+
 // Folds sqrt(sq) into the largest row norm (its bits, zero-initialised: norms are >= 0, so bit patterns
 // order like values).  A plain read first: all but a few dozen of a million rows find a larger norm
 // already there, and a million atomics on one address take 0.7 ms.

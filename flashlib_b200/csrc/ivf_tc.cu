@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(128) ivf_tc_seed_select_kernel(const float* __
     for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
     const float mn = __ldg(maxnorm);
     if (pick > neg_inf()) pick -= 2.f * eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
-    if (lane == 0) tau_q[qi] = pick;
+    // (NaN where a row's norm or the query is not finite: no score would exceed it)
+    if (lane == 0) tau_q[qi] = pick > neg_inf() ? pick : neg_inf();
 }
 
 // Finalisation of the inverted-file scan: one warp per query.
@@ -368,7 +369,7 @@ __device__ __forceinline__ void ivf_rerank(const float* __restrict__ s_sc, const
         }
     }
     // every row that was not re-scored has a score <= bound: its distance is at least qsq - 2 (bound + eps)
-    proven = bound == neg_inf() || dk < qsq - 2.f * (bound + eps) - slack;
+    proven = list_proven(dk, qsq, bound, eps, slack);
 #pragma unroll
     for (int r = 0; r < NPL; ++r) {
         const int e = (r << 5) | lane;

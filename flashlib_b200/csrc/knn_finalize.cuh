@@ -261,7 +261,7 @@ __device__ __forceinline__ void finalize_slot(const FinalizeParams& p, const int
         // Verification: every row that was not re-scored has a score <= bound, so its exact
         // distance is at least qsq - 2 (bound + eps).
         bool proven = true;
-        if (p.verify && bound > neg_inf()) proven = dk < qsq - 2.f * (bound + eps) - slack;
+        if (p.verify) proven = list_proven(dk, qsq, bound, eps, slack);
         if (!proven && p.cert_tau != nullptr) proven = bound <= __ldg(p.cert_tau + qi);
         if (!proven && attempt == 0) continue;
 #pragma unroll

@@ -253,17 +253,13 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
     }
     block_sort_desc<PF_THREADS>(s_key, s_id, P2);
     for (int e = tid; e < p.k; e += PF_THREADS) {
-        const bool ok = s_id[e] != INVALID_ID;
+        const bool ok = s_id[e] != INVALID_ID && s_key[e] > neg_inf();
         p.out_dist[qi * p.k + e] = ok ? -s_key[e] : pos_inf();
         p.out_idx[qi * p.k + e] = ok ? (int32_t)((int64_t)s_id[e] + p.row_offset) : -1;
     }
     if (tid == 0) {
-        bool proven = !overflow && fits;
-        if (proven && bound > neg_inf()) {
-            const float dk = s_id[p.k - 1] != INVALID_ID ? -s_key[p.k - 1] : pos_inf();
-            proven = dk < qsq - 2.f * (bound + eps) - slack;
-        }
-        if (!proven) {
+        const float dk = s_id[p.k - 1] != INVALID_ID ? -s_key[p.k - 1] : pos_inf();
+        if (overflow || !fits || !list_proven(dk, qsq, bound, eps, slack)) {
             bool queued = false;
             if (p.next_count != nullptr) {
                 const int i = atomicAdd(p.next_count, 1);

@@ -1058,8 +1058,11 @@ __global__ void __launch_bounds__(256) tc_seed_select_split_kernel(const float* 
         const float mn = __ldg(mg.maxnorm);
         pick -= 2.f * mg.eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
     }
-    // a score equal to the threshold is not kept: one step below it, so that the `rank` rows are
-    if (lane == 0) tau[row] = pick - fabsf(pick) * 1.2e-7f;
+    // A score equal to the threshold is not kept: one step below it, so that the `rank` rows are.  A norm of NaN or
+    // infinity among the rows makes the margin, and an infinite score the step, NaN: no score exceeds that, so
+    // the row keeps its -inf.
+    pick -= fabsf(pick) * 1.2e-7f;
+    if (lane == 0 && pick > neg_inf()) tau[row] = pick;
 }
 
 // ---- host side ---------------------------------------------------------------------------
