@@ -130,7 +130,7 @@ static __device__ __noinline__ void dir_collect(float* key, uint32_t* id, int st
 
 // A key that at least k of the up to 256 keys (eight per lane, -inf where there is none) reach, close
 // to the largest such: bisection over the keys' order-preserving integer image.  -inf when fewer
-// than k keys exist.
+// than k keys exist.  Keys of -inf and NaN do not count.
 static __device__ __noinline__ float dir_first_threshold(const float* keys, int k) {
     const int lane = threadIdx.x & 31;
     int v[8], lo = 0x7fffffff, hi = (int)0x80000000, have = 0;
@@ -138,8 +138,8 @@ static __device__ __noinline__ float dir_first_threshold(const float* keys, int 
     for (int r = 0; r < 8; ++r) {
         const float x = keys[r * 32 + lane];
         const int b = __float_as_int(x);
-        v[r] = b >= 0 ? b : (b ^ 0x7fffffff);             // orders like the float
-        const bool real = x > neg_inf();
+        const bool real = x > neg_inf();                  // (a NaN would order by its sign: not counted below either)
+        v[r] = real ? (b >= 0 ? b : (b ^ 0x7fffffff)) : (int)0x80000000;      // orders like the float
         have += __popc(__ballot_sync(FULL_MASK, real));
         if (real) { lo = min(lo, v[r]); hi = max(hi, v[r]); }
     }

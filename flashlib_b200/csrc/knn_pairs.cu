@@ -22,8 +22,8 @@ __device__ __forceinline__ float pf_kth_reached(const float (&key)[R], int k) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int b = __float_as_int(key[r]);
-        v[r] = b >= 0 ? b : (b ^ 0x7fffffff);             // orders like the float
         const bool real = key[r] > neg_inf();
+        v[r] = real ? (b >= 0 ? b : (b ^ 0x7fffffff)) : (int)0x80000000;      // orders like the float
         have += __popc(__ballot_sync(FULL_MASK, real));
         if (real) { lo = min(lo, v[r]); hi = max(hi, v[r]); }
     }
