@@ -61,7 +61,11 @@ SIGNATURES = {
     "fl_knn_seed_f32": (c_int, [c_void_p, c_int64, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p,
                                 c_void_p, c_int64, c_void_p, c_void_p]),
     "fl_knn_plane_maxnorm_offset": (c_int64, [c_int64, c_int]),
+    "fl_knn_plane_norm_floats": (c_int, []),
     "fl_knn_seeded_f32": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int,
+                                  c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                  c_void_p, c_void_p]),
+    "fl_knn_seeded_norms_f32": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int,
                                   c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                   c_void_p, c_void_p]),
     "fl_debug_tc_experiment": (c_int, [c_int, ctypes.c_uint]),

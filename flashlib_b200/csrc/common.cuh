@@ -72,6 +72,13 @@ static inline bool dt_vec_ok(const void* p, int64_t ld, int dt) {
     return (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(p) & (dt == DT_F32 ? 15 : 7)) == 0);
 }
 
+// fp32 accumulation of `terms` products in a tensor-core score, relative to ||q|| ||x||: one rounding of 2^-23 each
+// (truncation; the products themselves are exact), raised by the 2^-7 by which rounded operands may be longer.
+// Measured with operands of one sign: at most 0.016 of it (64 to 256 features).
+static inline float score_acc(int terms) { return 1.25e-7f * (float)terms; }
+// Split planes of d features: the 2 d products with a low half come first, while the sum is 2^-7 of ||q|| ||x|| at most.
+static inline float score_acc_split(int d) { return score_acc(d + 16 + d / 64 + 1); }
+
 #if defined(__CUDACC__)
 
 __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); }
@@ -289,6 +296,43 @@ __device__ __forceinline__ void atomic_max_f32(float* addr, float v) {
     }
 }
 
+// What rounding a value to bf16 takes from it (exact in fp32; NaN for infinities).
+__device__ __forceinline__ float bf16_lost(float v) { return v - __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ float sq4(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
+__device__ __forceinline__ float4 bf16_lost4(float4 v) {
+    return make_float4(bf16_lost(v.x), bf16_lost(v.y), bf16_lost(v.z), bf16_lost(v.w));
+}
+
+// Largest norms over the rows of a database, left by the passes that write its operand planes: of the rows x, of what
+// one rounding to bf16 takes from them (x - hi) and of what the second half of a split plane still misses
+// (x - hi - lo).
+enum { NORM_ROW = 0, NORM_LOST = 1, NORM_LOST2 = 2, NORM_WORDS = 4 };
+
+// Bound on |score - (<q,x> - ||x||^2/2)| over the rows behind `norms`, from the rounding that happened to this query
+// (sums of squares: qsq of its values, lost of q - hi, lost2 of q - hi - lo) and to those rows.  With
+// q' = q - dq, x' = x - dx the product errs by <dq, x> + <q', dx>; the split planes leave out <lo, lo> besides.
+// Whatever the values, no constant is assumed: a bf16 rounding may move a value by 2^-8 of itself, and where
+// all roundings go one way the product is off by nearly 2^-7 ||q|| ||x||; on ordinary data the norms give
+// half of that.  Nothing is lost where the rows are stored as bf16.  `acc`: see score_acc().
+constexpr int OPERANDS_F32 = 0, OPERANDS_BF16 = 1, OPERANDS_SPLIT = 2;
+__device__ __forceinline__ float score_eps(int operands, float qsq, float lost, float lost2, const float* __restrict__ norms, float acc) {
+    const float qn = sqrtf(qsq), xn = __ldg(norms + NORM_ROW);
+    float eps = acc * qn * xn;
+    if (operands == OPERANDS_BF16) {
+        const float l = sqrtf(lost);
+        eps += l * xn + (qn + l) * __ldg(norms + NORM_LOST);
+    } else if (operands == OPERANDS_SPLIT) {
+        const float l = sqrtf(lost), l2 = sqrtf(lost2), xl = __ldg(norms + NORM_LOST), xl2 = __ldg(norms + NORM_LOST2);
+        eps += l2 * xn + (qn + l2) * xl2 + (l + l2) * (xl + xl2);
+    }
+    return eps;
+}
+// What the fp32 sums beside the product -- ||q||^2, ||x||^2, the exact distances, the norm columns -- may be off by
+// together, in squared distance: chains of d / 32 + 10 roundings of 2^-24 at most.
+__device__ __forceinline__ float proof_slack(float qsq, float xn, int d) {
+    return fmaxf(1e-5f, 1e-8f * (float)d) * (qsq + xn * xn);
+}
+
 // The proof that a candidate list is complete: every row outside it has a score (half of qsq minus its distance) of at
 // most bound + eps, so none of them comes closer than the k-th distance dk on it.  A bound of -inf says that no row
 // was left out at all, which a score of NaN -- infinite or NaN operands, a norm that overflows -- does
@@ -303,7 +347,7 @@ __device__ __forceinline__ bool list_proven(float dk, float qsq, float bound, fl
 // order like values).  A plain read first: all but a few dozen of a million rows find a larger norm
 // already there, and a million atomics on one address take 0.7 ms.
 __device__ __forceinline__ void max_norm_update(unsigned int* maxnorm_bits, float sq) {
-    const unsigned int v = __float_as_uint(sqrtf(sq));
+    const unsigned int v = __float_as_uint(sqrtf(sq));           // (NaN orders above infinity)
     if (*reinterpret_cast<volatile unsigned int*>(maxnorm_bits) < v) atomicMax(maxnorm_bits, v);
 }
 

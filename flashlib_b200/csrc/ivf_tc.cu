@@ -78,10 +78,10 @@ __global__ void ivf_row_map_kernel(const int64_t* __restrict__ list_offsets, con
     for (int r = threadIdx.x; r < len; r += blockDim.x) row_map[p0 + r] = (int)(r0 + r);
 }
 
-// One warp per plane row: bf16 features, the split -||x||^2/2 columns, half norm, max norm.
+// One warp per plane row: bf16 features, the split -||x||^2/2 columns, half norm, largest norms.
 __global__ void ivf_plane_rows_kernel(const float* __restrict__ data, int64_t ld, int d, const int* __restrict__ row_map,
                                       int64_t rows_max, __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                      unsigned int* __restrict__ maxnorm_bits, int d_pad) {
+                                      unsigned int* __restrict__ norm_bits, int d_pad) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows_max) return;
@@ -94,17 +94,22 @@ __global__ void ivf_plane_rows_kernel(const float* __restrict__ data, int64_t ld
         return;
     }
     const float* p = data + (int64_t)src * ld;
-    float s = 0.f;
+    float s = 0.f, lost = 0.f;
     for (int c = lane; c < d_pad; c += 32) {
-        const float v = (c < d) ? __ldg(p + c) : 0.f;
+        const float v = (c < d) ? __ldg(p + c) : 0.f, l = bf16_lost(v);
         s += v * v;
+        lost += l * l;
         o[c] = __float2bfloat16_rn(v);
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
+    for (int off = 16; off > 0; off >>= 1) {
+        s += __shfl_xor_sync(FULL_MASK, s, off);
+        lost += __shfl_xor_sync(FULL_MASK, lost, off);
+    }
     if (lane == 0) {
         hnorm[row] = 0.5f * s;
-        max_norm_update(maxnorm_bits, s);
+        max_norm_update(norm_bits + NORM_ROW, s);
+        max_norm_update(norm_bits + NORM_LOST, lost);
     }
     if (lane < PLANE_AUG_COLS) {
         const float nh = -0.5f * s;
@@ -197,6 +202,21 @@ __global__ void ivf_tc_gather_kernel(const float* __restrict__ q, int64_t ldq, i
     }
 }
 
+// ||q||^2 and the square of what rounding q to bf16 takes from it (all lanes of a warp).
+__device__ __forceinline__ void ivf_query_norms(const float* __restrict__ qp, int d, float& qsq, float& lost) {
+    qsq = lost = 0.f;
+    for (int c = threadIdx.x & 31; c < d; c += 32) {
+        const float v = __ldg(qp + c), l = bf16_lost(v);
+        qsq += v * v;
+        lost += l * l;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+        lost += __shfl_xor_sync(FULL_MASK, lost, o);
+    }
+}
+
 // Starting threshold of every query from the seeding pass.  The pass left, for every gathered row
 // (= one (query, probed list) pair), the 32 class maxima of the first tiles of that list: disjoint
 // sets of rows, and the lists of one query are disjoint too.  One warp per query folds its pairs'
@@ -208,7 +228,7 @@ __global__ void ivf_tc_gather_kernel(const float* __restrict__ q, int64_t ldq, i
 __global__ void __launch_bounds__(128) ivf_tc_seed_select_kernel(const float* __restrict__ seed_cls,
                                                                  const int* __restrict__ pair_row, int64_t nq, int nprobe,
                                                                  int rank, const float* __restrict__ q, int64_t ldq, int d,
-                                                                 const float* __restrict__ maxnorm, float eps_rel,
+                                                                 const float* __restrict__ norms, float acc,
                                                                  float* __restrict__ tau_q) {
     const int lane = threadIdx.x & 31;
     const int64_t qi = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -257,12 +277,10 @@ __global__ void __launch_bounds__(128) ivf_tc_seed_select_kernel(const float* __
         }
         pick = __shfl_sync(FULL_MASK, key[0], rank - 1);     // -inf while fewer than `rank` rows were sampled
     }
-    float qsq = 0.f;
-    for (int c = lane; c < d; c += 32) { const float v = __ldg(q + qi * ldq + c); qsq += v * v; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
-    const float mn = __ldg(maxnorm);
-    if (pick > neg_inf()) pick -= 2.f * eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
+    float qsq, lost;
+    ivf_query_norms(q + qi * ldq, d, qsq, lost);
+    if (pick > neg_inf())
+        pick -= 2.f * score_eps(OPERANDS_BF16, qsq, lost, 0.f, norms, acc) + proof_slack(qsq, __ldg(norms + NORM_ROW), d);
     // (NaN where a row's norm or the query is not finite: no score would exceed it)
     if (lane == 0) tau_q[qi] = pick > neg_inf() ? pick : neg_inf();
 }
@@ -384,8 +402,8 @@ __device__ __forceinline__ void ivf_rerank(const float* __restrict__ s_sc, const
 __global__ void __launch_bounds__(128) ivf_tc_finalize_kernel(
     const float* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec, const float* __restrict__ data, int64_t ldd,
     const int* __restrict__ pair_row, int nprobe, const float2* __restrict__ pools, const int* __restrict__ pool_cnt,
-    const float* __restrict__ pool_tau, const int* __restrict__ row_map, int64_t rows_max, int k, float eps_rel,
-    const float* __restrict__ maxnorm, float* __restrict__ out_dist, int32_t* __restrict__ out_pos, int* fb_count,
+    const float* __restrict__ pool_tau, const int* __restrict__ row_map, int64_t rows_max, int k, float acc,
+    const float* __restrict__ norms, float* __restrict__ out_dist, int32_t* __restrict__ out_pos, int* fb_count,
     int* fb_list) {
     __shared__ float s_sc[4][IVF_GATHER];
     __shared__ uint32_t s_id[4][IVF_GATHER];
@@ -395,13 +413,10 @@ __global__ void __launch_bounds__(128) ivf_tc_finalize_kernel(
     const int64_t qi = (int64_t)blockIdx.x * 4 + w;
     if (qi >= nq) return;
     const float* qp = q + qi * ldq;
-    float qsq = 0.f;
-    for (int c = lane; c < d; c += 32) { const float v = __ldg(qp + c); qsq += v * v; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
-    const float mn = __ldg(maxnorm);
-    const float eps = eps_rel * sqrtf(qsq) * mn;
-    const float slack = 1e-5f * (qsq + mn * mn);
+    float qsq, lost;
+    ivf_query_norms(qp, d, qsq, lost);
+    const float eps = score_eps(OPERANDS_BF16, qsq, lost, 0.f, norms, acc);
+    const float slack = proof_slack(qsq, __ldg(norms + NORM_ROW), d);
 
     // Gather: 32 pools at a time, one pool per lane for the bookkeeping (gathered row, entry count,
     // threshold: independent loads), then the pools' entries are copied to the warp's list at
@@ -755,6 +770,7 @@ extern "C" int fl_ivf_fine_scan_tc_f32(const float* q, int64_t nq, int64_t ldq, 
     const char* pl = static_cast<const char*>(ivf_plane);
     const int* tile_off = reinterpret_cast<const int*>(pl + L.off_tile_off);
     const int* row_map = reinterpret_cast<const int*>(pl + L.off_row_map);
+    const float* norms = reinterpret_cast<const float*>(pl + L.pl.off_meta);
     int* cnt = reinterpret_cast<int*>(base + w.off_cnt);
     int* pair_off = reinterpret_cast<int*>(base + w.off_pair_off);
     int* item_off = reinterpret_cast<int*>(base + w.off_item_off);
@@ -824,7 +840,7 @@ extern "C" int fl_ivf_fine_scan_tc_f32(const float* q, int64_t nq, int64_t ldq, 
         const int rank = k + 6 < 32 ? k + 6 : 32;
         profile_mark(st);  // 4: threshold selection
         ivf_tc_seed_select_kernel<<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(
-            sd.seed_cls, pair_row, nq, nprobe, rank, q, ldq, d, reinterpret_cast<const float*>(pl + L.pl.off_meta), 0.004f, tau_q);
+            sd.seed_cls, pair_row, nq, nprobe, rank, q, ldq, d, norms, score_acc(d + PLANE_AUG_COLS), tau_q);
         FL_CHECK_LAUNCH();
     }
     profile_mark(st);      // 5: scoring pass
@@ -840,7 +856,7 @@ extern "C" int fl_ivf_fine_scan_tc_f32(const float* q, int64_t nq, int64_t ldq, 
     const int vec = vecq && vecd && (d % 4 == 0);
     ivf_tc_finalize_kernel<<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(
         q, nq, ldq, d, vec, data, ldd, pair_row, nprobe, reinterpret_cast<const float2*>(base + w.off_pools), tp.part_cnt,
-        tp.part_tau, row_map, L.rows_max, k, 0.004f, reinterpret_cast<const float*>(pl + L.pl.off_meta), out_dist, out_pos,
+        tp.part_tau, row_map, L.rows_max, k, score_acc(d + PLANE_AUG_COLS), norms, out_dist, out_pos,
         fb_count, fb_list);
     FL_CHECK_LAUNCH();
     profile_mark(st);      // 7: exact pass for unproven queries

@@ -9,17 +9,22 @@
 namespace fl {
 
 // Split operand planes.  An fp32 value v is carried as hi = bf16(v) and lo = bf16(v - hi); the
-// plane rows hold [hi | lo | hi | ones] (samples) and [hi | hi | lo | norm terms] (centroids), so one bf16 product
-// over 3 d_pad columns yields  hi.hi + lo.hi + hi.lo,  i.e. the fp32 inner product up to the
-// dropped lo.lo term and the second-order residuals: a relative error of about 3 * 2^-18 of
-// ||x|| ||c|| instead of 2^-8.  Used when 3 d_pad columns of a 128-row tile fit in shared
+// plane rows hold [hi | lo | hi | ones] (samples) and [lo | hi | hi | norm terms] (centroids), so one bf16 product
+// over 3 d_pad columns yields  hi.lo + lo.hi + hi.hi,  i.e. the fp32 inner product up to the
+// dropped lo.lo term and the second-order residuals: an error of about 10^-5 ||x|| ||c|| on ordinary data, at
+// most 2^-15, where one rounding errs by 0.0037 and at most 2^-7.  (The large term comes last: fp32 roundings of the
+// small ones do not count, see score_acc_split.)  Used when 3 d_pad columns of a 128-row tile fit in shared
 // memory (d <= 128).
 __device__ __forceinline__ void bf16_split(float v, __nv_bfloat16& hi, __nv_bfloat16& lo) {
     hi = __float2bfloat16_rn(v);
     lo = __float2bfloat16_rn(v - __bfloat162float(hi));
 }
 
-__device__ __forceinline__ void bf16_split4(float4 v, uint2& hi, uint2& lo) {
+// The two halves of four values, and the squares of what the first and both of them miss added to lost and lost2.
+__device__ __forceinline__ void bf16_split4(float4 v, uint2& hi, uint2& lo, float& lost, float& lost2) {
+    const float4 rest = bf16_lost4(v);
+    lost += sq4(rest);
+    lost2 += sq4(bf16_lost4(rest));
     __nv_bfloat16 h[4], l[4];
     bf16_split(v.x, h[0], l[0]);
     bf16_split(v.y, h[1], l[1]);
@@ -33,10 +38,10 @@ __device__ __forceinline__ void bf16_split4(float4 v, uint2& hi, uint2& lo) {
 }
 
 // Centroid side, one warp per row (four columns a lane: wide reads where `vec` allows, 8-byte writes): [m_pad][3 d_pad + 16] rows, ||c||^2/2 per row and the
-// largest row norm.  Padding rows score -3e38.
+// largest norms (of the rows, of what hi and hi + lo miss of them).  Padding rows score -3e38.
 __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int d, int64_t ld,
                                      __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                     unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad, int vec) {
+                                     unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= m_pad) return;
@@ -48,21 +53,27 @@ __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int
         return;
     }
     const float* p = c + row * ld;
-    float s = 0.f;
+    float s = 0.f, lost = 0.f, lost2 = 0.f;
     for (int t = lane * 4; t < d_pad; t += 128) {
         const float4 v = ld_row4(p, t, d, vec, DT_F32);
-        s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        s += sq4(v);
         uint2 hi, lo;
-        bf16_split4(v, hi, lo);
-        *reinterpret_cast<uint2*>(o + t) = hi;
+        bf16_split4(v, hi, lo, lost, lost2);
+        *reinterpret_cast<uint2*>(o + t) = lo;
         *reinterpret_cast<uint2*>(o + d_pad + t) = hi;
-        *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = lo;
+        *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = hi;
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
+    for (int off = 16; off > 0; off >>= 1) {
+        s += __shfl_xor_sync(FULL_MASK, s, off);
+        lost += __shfl_xor_sync(FULL_MASK, lost, off);
+        lost2 += __shfl_xor_sync(FULL_MASK, lost2, off);
+    }
     if (lane == 0) {
         hnorm[row] = 0.5f * s;
-        max_norm_update(maxnorm_bits, s);
+        max_norm_update(norm_bits + NORM_ROW, s);
+        max_norm_update(norm_bits + NORM_LOST, lost);
+        max_norm_update(norm_bits + NORM_LOST2, lost2);
     }
     if (lane < PLANE_AUG_COLS) {
         const float nh = -0.5f * s;
@@ -79,13 +90,13 @@ __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int
 // `cap`), one warp per row in a grid-stride loop, written as split rows [hi | lo | hi | ones].
 // With `tau_out` (kNN second stage) row r also gets its starting threshold: the exact k-th distance
 // d_k found so far (prev_dist [point][k]) bounds the true one from above, so every true neighbour
-// scores at least (||x||^2 - d_k) / 2 exactly and at most eps = eps_rel ||x|| *maxnorm less in
+// scores at least (||x||^2 - d_k) / 2 exactly and at most eps (score_eps of split operands) less in
 // this stage; the threshold sits 2 eps and the proof's slack below that, so that a pool that never
 // overflowed proves its row.
 __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, int d, const int* __restrict__ rows,
                                       const int* __restrict__ rows_count, int cap, __nv_bfloat16* __restrict__ out,
                                       int d_pad, const float* __restrict__ prev_dist, int k,
-                                      const float* __restrict__ maxnorm, float eps_rel, float* __restrict__ tau_out, int vec) {
+                                      const float* __restrict__ norms, float acc, float* __restrict__ tau_out, int vec) {
     const int lane = threadIdx.x & 31;
     const int pitch = 3 * d_pad + PLANE_AUG_COLS;
     int count = *rows_count;
@@ -100,12 +111,12 @@ __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, 
         const int64_t pt = rows[r];
         const float* src = x + pt * ldx;
         __nv_bfloat16* o = out + (int64_t)r * pitch;
-        float qsq = 0.f;
+        float qsq = 0.f, lost = 0.f, lost2 = 0.f;
         for (int t = lane * 4; t < d_pad; t += 128) {
             uint2 hi, lo;
             const float4 v = ld_row4(src, t, d, vec, DT_F32);
-            qsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            bf16_split4(v, hi, lo);
+            qsq += sq4(v);
+            bf16_split4(v, hi, lo, lost, lost2);
             *reinterpret_cast<uint2*>(o + t) = hi;
             *reinterpret_cast<uint2*>(o + d_pad + t) = lo;
             *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = hi;
@@ -113,14 +124,18 @@ __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, 
         if (lane < PLANE_AUG_COLS) o[3 * d_pad + lane] = __float2bfloat16_rn(lane < 3 ? 1.f : 0.f);
         if (tau_out != nullptr) {
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, off);
+            for (int off = 16; off > 0; off >>= 1) {
+                qsq += __shfl_xor_sync(FULL_MASK, qsq, off);
+                lost += __shfl_xor_sync(FULL_MASK, lost, off);
+                lost2 += __shfl_xor_sync(FULL_MASK, lost2, off);
+            }
             if (lane == 0) {
                 const float dk = prev_dist[pt * k + (k - 1)];
-                const float mn = __ldg(maxnorm);
                 float tau = neg_inf();
                 if (dk < pos_inf())
-                    tau = 0.5f * (qsq - dk) - 2.f * eps_rel * sqrtf(qsq) * mn - 1e-5f * (qsq + mn * mn);
-                tau_out[r] = tau;
+                    tau = 0.5f * (qsq - dk) - 2.f * score_eps(OPERANDS_SPLIT, qsq, lost, lost2, norms, acc) -
+                          proof_slack(qsq, __ldg(norms + NORM_ROW), d);
+                tau_out[r] = tau > neg_inf() ? tau : neg_inf();
             }
         }
     }
@@ -137,8 +152,8 @@ __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, 
 // stage) or, when that is absent or full, to the exact-path list.
 __global__ void __launch_bounds__(128) assign_finalize_kernel(
     const float* __restrict__ x, int64_t n, int64_t ldx, const float* __restrict__ c, int K, int64_t ldc, int d,
-    int vec, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, float eps_rel,
-    const float* __restrict__ maxnorm, int32_t* __restrict__ labels, const int* __restrict__ rows,
+    int vec, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, int operands, float acc,
+    const float* __restrict__ norms, int32_t* __restrict__ labels, const int* __restrict__ rows,
     const int* __restrict__ rows_count, int* __restrict__ next_count, int* __restrict__ next_list, int next_cap,
     int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap, int scores_by_point) {
     const int sl = threadIdx.x & 7;
@@ -161,14 +176,17 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
         const float* xp = x + pt * ldx;
         const float* c0 = c + (int64_t)(v0 ? ids.x : 0u) * ldc;
         const float* c1 = c + (int64_t)(v1 ? ids.y : 0u) * ldc;
-        float qsq = 0.f, a0 = 0.f, a1 = 0.f;
+        float qsq = 0.f, lost = 0.f, lost2 = 0.f, a0 = 0.f, a1 = 0.f;
         if (vec) {
 #pragma unroll 4
             for (int t = sl * 4; t < d; t += 32) {
                 const float4 xv = __ldg(reinterpret_cast<const float4*>(xp + t));
                 const float4 p0 = __ldg(reinterpret_cast<const float4*>(c0 + t));
                 const float4 p1 = __ldg(reinterpret_cast<const float4*>(c1 + t));
-                qsq += xv.x * xv.x + xv.y * xv.y + xv.z * xv.z + xv.w * xv.w;
+                qsq += sq4(xv);
+                const float4 l = bf16_lost4(xv);
+                lost += sq4(l);
+                lost2 += sq4(bf16_lost4(l));
                 float e0 = xv.x - p0.x, e1 = xv.y - p0.y, e2 = xv.z - p0.z, e3 = xv.w - p0.w;
                 a0 += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
                 e0 = xv.x - p1.x; e1 = xv.y - p1.y; e2 = xv.z - p1.z; e3 = xv.w - p1.w;
@@ -178,12 +196,15 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
             for (int t = sl; t < d; t += 8) {
                 const float xv = __ldg(xp + t);
                 const float e0 = xv - __ldg(c0 + t), e1 = xv - __ldg(c1 + t);
-                qsq += xv * xv; a0 += e0 * e0; a1 += e1 * e1;
+                const float l = bf16_lost(xv), l2 = bf16_lost(l);
+                qsq += xv * xv; lost += l * l; lost2 += l2 * l2; a0 += e0 * e0; a1 += e1 * e1;
             }
         }
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) {
             qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+            lost += __shfl_xor_sync(FULL_MASK, lost, o);
+            lost2 += __shfl_xor_sync(FULL_MASK, lost2, o);
             a0 += __shfl_xor_sync(FULL_MASK, a0, o);
             a1 += __shfl_xor_sync(FULL_MASK, a1, o);
         }
@@ -196,11 +217,8 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
         bool ok = best_i != INVALID_ID;
         if (ok && bound > -1e37f) {
             bound += fabsf(bound) * 3.1e-5f;                       // index bits in the mantissa: 2^-15 relative
-            const float mn = __ldg(maxnorm);
-            const float eps = eps_rel * sqrtf(qsq) * mn;
-            const float lb = qsq - 2.f * (bound + eps);
-            const float slack = 1e-5f * (qsq + mn * mn);
-            ok = best_d < lb - slack;
+            ok = list_proven(best_d, qsq, bound, score_eps(operands, qsq, lost, lost2, norms, acc),
+                             proof_slack(qsq, __ldg(norms + NORM_ROW), d));
         }
         labels[pt] = ok ? (int32_t)best_i : 0;
         if (!ok) {
@@ -220,12 +238,12 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
 // First-stage proof from the scores alone, one thread per point: the best-scoring centroid is the
 // nearest one if its score leads the runner-up's by more than twice the scoring error bound (every
 // score is within eps of the exact <x,c> - ||c||^2/2, so the exact scores keep that order).  No
-// sample row and no centroid is read -- 28 bytes per point instead of its 4 d -- at the price of a
+// sample row and no centroid is read -- 32 bytes per point instead of its 4 d -- at the price of a
 // lead of 2 eps where the exact re-scoring of assign_finalize_kernel needs eps; what the lead does
 // not decide goes to the `next` list (the second stage, whose bound is a hundred times smaller).
 __global__ void __launch_bounds__(256) assign_by_lead_kernel(
-    int64_t n, int K, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float* __restrict__ xsq,
-    float eps_rel, const float* __restrict__ maxnorm, int32_t* __restrict__ labels, int* __restrict__ next_count,
+    int64_t n, int K, int d, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float* __restrict__ xsq,
+    const float* __restrict__ xlost, float acc, const float* __restrict__ norms, int32_t* __restrict__ labels, int* __restrict__ next_count,
     int* __restrict__ next_list, int next_cap, int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap) {
     const int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pt >= n) return;
@@ -240,11 +258,11 @@ __global__ void __launch_bounds__(256) assign_by_lead_kernel(
     if (v0 && v1) second = fmaxf(second, first ? sc.z : sc.x);   // ... or the other half's best
     bool ok = v0 || v1;
     if (ok && second > -1e37f) {
-        const float q2 = __ldg(xsq + pt), mn = __ldg(maxnorm);
-        const float eps = eps_rel * sqrtf(q2) * mn;
+        const float q2 = __ldg(xsq + pt), l = __ldg(xlost + pt);
+        const float eps = score_eps(OPERANDS_BF16, q2, l * l, 0.f, norms, acc);
         // the column index rides in the low mantissa bits of both scores: 2^-15 relative each
         const float lead = (best - fabsf(best) * 3.1e-5f) - (second + fabsf(second) * 3.1e-5f);
-        ok = lead > 2.f * eps + 1e-5f * (q2 + mn * mn);
+        ok = lead > 2.f * eps + proof_slack(q2, __ldg(norms + NORM_ROW), d);
     }
     labels[pt] = ok ? (int32_t)best_i : 0;
     if (!ok) {
@@ -380,7 +398,7 @@ static AssignTcWs assign_tc_plan(int64_t n, int K, int d, int have_xplane) {
     w.off_cplane = take(cur, w.cl.bytes);
     w.off_cplane3 = w.split ? take(cur, w.cl3.bytes) : -1;
     w.off_xplane = have_xplane ? -1 : take(cur, w.n_pad * w.pitch * 2);
-    w.off_xsq = have_xplane ? -1 : take(cur, w.n_pad * 4);
+    w.off_xsq = have_xplane ? -1 : take(cur, w.n_pad * 8);
     w.off_xsplit = w.split ? take(cur, w.l1_pad * w.pitch3 * 2) : -1;
     w.off_asg_sc = take(cur, w.n_pad * 4 * 4);
     w.off_asg_id = take(cur, w.n_pad * 2 * 4);
@@ -399,7 +417,7 @@ static AssignTcWs assign_tc_plan(int64_t n, int K, int d, int have_xplane) {
 
 int split_plane_supported(int d) { return assign_tc_split(d); }
 
-// Split database plane [hi | hi | lo | norm terms] in the layout plane_layout(m, 3 d_pad).
+// Split database plane [lo | hi | hi | norm terms] in the layout plane_layout(m, 3 d_pad).
 int launch_split_db_plane(const float* c, int64_t m, int d, int64_t ldc, void* plane, cudaStream_t st) {
     const int d_pad = (int)round_up(d, 64);
     const PlaneLayout L = plane_layout(m, 3 * d_pad);
@@ -414,11 +432,11 @@ int launch_split_db_plane(const float* c, int64_t m, int d, int64_t ldc, void* p
 }
 
 int launch_split_query_gather(const float* x, int64_t ldx, int d, const int* rows, const int* rows_count, int cap,
-                              void* out, int d_pad, const float* prev_dist, int k, const float* maxnorm, float eps_rel,
+                              void* out, int d_pad, const float* prev_dist, int k, const float* norms, float acc,
                               float* tau_out, cudaStream_t st) {
     split_x_gather_kernel<<<(unsigned)(8 * sm_count()), 256, 0, st>>>(x, ldx, d, rows, rows_count, cap,
                                                                      static_cast<__nv_bfloat16*>(out), d_pad, prev_dist, k,
-                                                                     maxnorm, eps_rel, tau_out,
+                                                                     norms, acc, tau_out,
                                                                      dt_vec_ok(x, ldx, DT_F32) && d % 4 == 0);
     FL_CHECK_LAUNCH();
     return FL_OK;
@@ -435,8 +453,8 @@ using namespace fl;
 
 extern "C" int64_t fl_kmeans_xplane_bytes(int64_t n, int d) {
     if (n < 1 || d < 1) return 0;
-    // the bf16 rows, then ||x||^2 of every row (f32 [n_pad])
-    return round_up(round_up(n, 128) * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024) + round_up(n, 128) * 4;
+    // the bf16 rows, then ||x||^2 of every row and the norm of what rounding it took (f32 [2][n_pad])
+    return round_up(round_up(n, 128) * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024) + round_up(n, 128) * 8;
 }
 
 extern "C" int fl_kmeans_prepare_x_f32(const float* x, int64_t n, int d, int64_t ldx, void* xplane,
@@ -455,8 +473,8 @@ extern "C" int64_t fl_kmeans_assign_tc_workspace_bytes(int64_t n, int K, int d, 
 }
 
 // Two stages.  (1) plain bf16 planes: every point is scored against every centroid; labels the
-// proof accepts (scoring error 2^-8 ||x|| max||c||) are final.  (2) d <= 128: the unproven points
-// (a device-side list) are gathered into split planes and scored again, error 4e-5: nearly all of
+// proof accepts (scoring error about 0.0037 ||x|| max||c||) are final.  (2) d <= 128: the unproven points
+// (a device-side list) are gathered into split planes and scored again, error about 6e-5: nearly all of
 // the rest is proven.  What is left takes the exact CUDA-core path.
 extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, const float* c,
                                        int K, int64_t ldc, int d, int32_t* labels, void* ws, int64_t ws_bytes,
@@ -510,7 +528,8 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     float* asg_sc = reinterpret_cast<float*>(base + w.off_asg_sc);
     uint32_t* asg_id = reinterpret_cast<uint32_t*>(base + w.off_asg_id);
     const unsigned fin_grid = (unsigned)(4 * sm_count());      // grid-stride finalisation
-    const float* maxnorm = reinterpret_cast<const float*>(cpl + w.cl.off_meta);
+    const float* norms = reinterpret_cast<const float*>(cpl + w.cl.off_meta);
+    const float acc1 = score_acc(d + PLANE_AUG_COLS);
 
     // ---- stage 1: plain bf16 ---------------------------------------------------------------
     {
@@ -525,21 +544,20 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         rc = launch_assign_tc(tp, asg_sc, asg_id, nullptr, st);
         profile_end(st);
         if (rc != FL_OK) return rc;
-        // scoring error relative to ||x|| max||c||: 2^-8 for plain bf16 operands, rounded up
         if (w.split) {
             // a second, far more precise stage follows: decide what the scores' lead decides
             // without touching the rows
             assign_by_lead_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(
-                n, K, asg_sc, asg_id, xsq, 0.004f, maxnorm, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap);
+                n, K, d, asg_sc, asg_id, xsq, xsq + w.n_pad, acc1, norms, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap);
             FL_CHECK_LAUNCH();
             // ... then, for the undecided ones only, the exact distances to the two half-winners, which
             // need half the lead; what is still open goes to the second stage
             assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, 0.004f, maxnorm, labels, l0_list, l0_count,
+                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_BF16, acc1, norms, labels, l0_list, l0_count,
                 l1_count, l1_list, w.l1_cap, fb_count, fb_list, w.fb_cap, 1);
         } else {
             assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, 0.004f, maxnorm, labels, nullptr, nullptr,
+                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_BF16, acc1, norms, labels, nullptr, nullptr,
                 nullptr, l1_list, w.l1_cap, fb_count, fb_list, w.fb_cap, 0);
         }
         FL_CHECK_LAUNCH();
@@ -557,9 +575,9 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         tp.tau = tau; tp.status = status;
         rc = launch_assign_tc(tp, asg_sc, asg_id, l1_count, st);
         if (rc != FL_OK) return rc;
-        // split operands: 3 * 2^-18 from the dropped terms plus the fp32 accumulation of 400 products
         assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-            x, w.l1_cap, ldx, c, K, ldc, d, vec, asg_sc, asg_id, 4e-5f, maxnorm, labels, l1_list, l1_count,
+            x, w.l1_cap, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_SPLIT, score_acc_split(d),
+            reinterpret_cast<const float*>(cpl3 + w.cl3.off_meta), labels, l1_list, l1_count,
             nullptr, nullptr, 0, fb_count, fb_list, w.fb_cap, 0);
         FL_CHECK_LAUNCH();
     }

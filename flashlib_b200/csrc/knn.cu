@@ -36,26 +36,29 @@ constexpr float SIMT_EPS_REL = 4e-6f;
 // One row of a bf16 query plane by a warp: the features, zero padding, and ones in the three columns that meet
 // the database plane's split -||x||^2/2 terms (all zero for rows that pad the last tile).  Four columns a
 // lane: 16-byte reads where `vec` says that the rows allow them, 8-byte writes (plane rows are 32-byte
-// aligned: their pitch is a multiple of 16 columns).  Returns the lane's share of ||q||^2.
-__device__ __forceinline__ float query_plane_row(const void* p, bool live, int d, int vec, __nv_bfloat16* o, int d_pad, int dt) {
+// aligned: their pitch is a multiple of 16 columns).  Returns the lane's share of ||q||^2 and of the square of what
+// the rounding took.
+__device__ __forceinline__ float2 query_plane_row(const void* p, bool live, int d, int vec, __nv_bfloat16* o, int d_pad, int dt) {
     const int lane = threadIdx.x & 31;
-    float sq = 0.f;
+    float sq = 0.f, lost = 0.f;
     for (int c = lane * 4; c < d_pad + PLANE_AUG_COLS; c += 128) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (live) {
             if (c < d) {
                 v = ld_row4(p, c, d, vec, dt);
-                sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                sq += sq4(v);
+                lost += sq4(bf16_lost4(v));
             } else if (c == d_pad) {
                 v = make_float4(1.f, 1.f, 1.f, 0.f);
             }
         }
         *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
     }
-    return sq;
+    return make_float2(sq, lost);
 }
 
-// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row from the same read.
+// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row, and nq_pad words further the
+// norm of what its rounding took, from the same read.
 // Bound by HBM: 250 001 x 96 rows take 43 us (96 MB in, 72 MB out).  One thread per plane element and a second
 // pass over the rows for the norms took some 180.
 __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
@@ -64,11 +67,17 @@ __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= nq_pad) return;
     const bool live = row < nq;
-    float s = query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
+    float2 s = query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
     if (sq_out == nullptr || !live) return;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
-    if ((threadIdx.x & 31) == 0) sq_out[row] = s;
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(FULL_MASK, s.x, o);
+        s.y += __shfl_xor_sync(FULL_MASK, s.y, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sq_out[row] = s.x;
+        sq_out[nq_pad + row] = sqrtf(s.y);
+    }
 }
 
 // What a tensor-core call needs before its first scoring launch, in one pass: the bf16 query plane, the
@@ -104,6 +113,11 @@ __global__ void fill_f32_kernel(float* p, int64_t n, float v) {
 
 // Clamps the fallback count to the list capacity and publishes it (and the number of rows the
 // split-plane stage took) in the status words.
+__global__ void norms_from_row_norm_kernel(const float* __restrict__ row_norm, float* __restrict__ norms) {
+    norms[NORM_ROW] = *row_norm;
+    norms[NORM_LOST] = *row_norm * 0.00390625f;
+}
+
 __global__ void fallback_fixup_kernel(int* fb_count, int fb_cap, int32_t* status, int K1, const int* s2_count = nullptr,
                                       int s2_cap = 0) {
     int c = *fb_count;
@@ -151,7 +165,7 @@ struct KnnWs {
     int nsplit; int64_t rows_per_split;        // main pass (SIMT: rows; TC: tiles of 256)
     int nsplit_fb; int64_t rows_per_split_fb;  // fallback pass
     int64_t nq_pad; int d_pad; int fb_cap; int fb_bq, fb_blocks;
-    int64_t off_hnorm, off_qplane, off_part_sc, off_part_id, off_part_tau, off_part_cnt, off_seed_cls, off_tau, off_cert, off_cnt, off_fblist,
+    int64_t off_hnorm, off_qplane, off_part_sc, off_part_id, off_part_tau, off_part_cnt, off_seed_cls, off_tau, off_cert, off_norms, off_cnt, off_fblist,
         off_fbpart_sc, off_fbpart_id, bytes;
     // second stage (split hi/lo planes) for the rows the first proof rejects
     int s2;                                    // 1: planned
@@ -235,6 +249,7 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.off_seed_cls = take(cur, w.nq_pad * (w.seed.splits > 1 ? w.seed.splits : 1) * 32 * 4);
         w.off_tau = take(cur, w.nq_pad * 4);
         w.off_cert = take(cur, w.nq_pad * 4);
+        w.off_norms = take(cur, NORM_WORDS * 4);
         w.off_cnt = take(cur, 1024);
         w.off_fblist = take(cur, (int64_t)w.fb_cap * 4);
         // the fallback scan spreads its blocks over the live slots (simt_dyn_split): at most
@@ -418,18 +433,18 @@ static int knn_check_args(const char* who, const void* q, int64_t nq, int64_t ld
 // results between the first and the second:
 //   TC_PREP    status / counters cleared, thresholds -inf, bf16 query plane built in the workspace
 //   TC_SEED    class maxima of the seeding sample into `seed_cls`
-//   TC_SCORE   thresholds from `seed_cls` (lowered by the cross-shard margin when `gmaxnorm` is
+//   TC_SCORE   thresholds from `seed_cls` (lowered by the cross-shard margin when `gnorms` is
 //              given), scoring pass, finalisation, exact pass for what could not be proven
 enum { TC_PREP = 1, TC_SEED = 2, TC_SCORE = 4 };
 
 static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, const void* db, int64_t m, int64_t ldb,
-                         int d, int k, const void* plane, int64_t row_offset, float* seed_cls, const float* gmaxnorm,
+                         int d, int k, const void* plane, int64_t row_offset, float* seed_cls, const float* gnorms,
                          float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status,
                          cudaStream_t st, const void* split_plane = nullptr, int dt = DT_F32) {
     const bool whole = phases == (TC_PREP | TC_SEED | TC_SCORE);
     // (the timing experiments belong to the screening epilogue of the large-problem plan)
     const KnnWs w = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, split_plane != nullptr, !whole || tc_debug_active());
-    const float eps1 = tc_eps_rel(dt, d);
+    const float acc1 = score_acc(d + PLANE_AUG_COLS);
     if (ws_bytes < w.bytes) {
         set_error("fl_knn: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes);
         return FL_EWORKSPACE;
@@ -487,11 +502,12 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     if (!(phases & TC_SEED) || !seeded) profile_begin(st);
     TcSeedMargin mg{};
     mg.dt = dt;
-    if (gmaxnorm != nullptr) {
-        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.maxnorm = gmaxnorm; mg.eps_rel = eps1; mg.cert_out = cert;
+    // a sharded caller's error bound must hold for rows of every shard: the largest norms of all
+    const float* norms = gnorms != nullptr ? gnorms : reinterpret_cast<const float*>(pl + L.off_meta);
+    if (gnorms != nullptr) {
+        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.norms = norms; mg.acc = acc1; mg.cert_out = cert;
     } else if (w.seed.splits > 1 ? w.seed.dense : tc_seed_dense(L.m_pad, w.kg)) {
-        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.eps_rel = eps1; mg.cert_out = nullptr;
-        mg.maxnorm = reinterpret_cast<const float*>(pl + L.off_meta);
+        mg.q = q; mg.ldq = ldq; mg.d = d; mg.nq = nq; mg.norms = norms; mg.acc = acc1; mg.cert_out = nullptr;
     }
     if (seeded) {
         rc = launch_knn_tc_seed_select(tp, mg, st);
@@ -511,10 +527,8 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     fp.k = k; fp.rerank = fp.K1; fp.row_offset = row_offset;
     fp.part_tau = tp.part_tau; fp.ntau = w.nsplit * tc_taus_per_range();
     fp.out_dist = out_dist; fp.out_idx = out_idx;
-    fp.verify = 1; fp.eps_rel = eps1;
-    // a sharded caller's error bound must hold for rows of every shard: the largest norm of all
-    fp.maxnorm = gmaxnorm != nullptr ? gmaxnorm : reinterpret_cast<const float*>(pl + L.off_meta);
-    fp.cert_tau = gmaxnorm != nullptr ? cert : nullptr;
+    fp.verify = 1; fp.operands = OPERANDS_BF16; fp.acc = acc1; fp.norms = norms;
+    fp.cert_tau = gnorms != nullptr ? cert : nullptr;
     fp.fb_count = fb_count; fp.fb_list = fb_list; fp.fb_cap = w.fb_cap;
     fp.part_cnt = tp.part_cnt;
     int* s2_count = fb_count + 64;
@@ -525,7 +539,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
         pf.dt = dt; pf.q = q; pf.ldq = ldq; pf.nq = nq; pf.db = db; pf.m = m; pf.ldb = ldb; pf.d = d; pf.vec = vec;
         pf.pools = static_cast<const float2*>(tp.pair_pools); pf.pool_cnt = tp.part_cnt; pf.pool_tau = tp.part_tau;
         pf.cap = tc_pair_pool_cap(k); pf.npool = w.nsplit * tc_taus_per_range();
-        pf.k = k; pf.eps_rel = eps1; pf.maxnorm = fp.maxnorm; pf.row_offset = row_offset;
+        pf.k = k; pf.acc = acc1; pf.norms = norms; pf.row_offset = row_offset;
         pf.out_dist = out_dist; pf.out_idx = out_idx;
         pf.fb_count = fb_count; pf.fb_list = fb_list; pf.fb_cap = w.fb_cap;
         pf.next_count = fp.next_count; pf.next_list = fp.next_list; pf.next_cap = fp.next_cap;
@@ -541,11 +555,11 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     if (w.s2) {
         const PlaneLayout L3 = plane_layout(m, 3 * w.d_pad);
         const char* pl3 = static_cast<const char*>(split_plane);
-        const float* maxnorm3 = reinterpret_cast<const float*>(pl3 + L3.off_meta);
-        const float eps2 = 4e-5f;   // 3 * 2^-18 from the dropped lo.lo and rounded lo terms, plus fp32 accumulation
+        const float* norms3 = reinterpret_cast<const float*>(pl3 + L3.off_meta);
+        const float acc2 = score_acc_split(d);
         float* tau2 = reinterpret_cast<float*>(base + w.off_s2_tau);
         rc = launch_split_query_gather(static_cast<const float*>(q), ldq, d, s2_list, s2_count, w.s2_cap, base + w.off_s2_qplane, w.d_pad, out_dist, k,
-                                       maxnorm3, eps2, tau2, st);
+                                       norms3, acc2, tau2, st);
         if (rc != FL_OK) return rc;
         TcKnnParams t2{};
         t2.qplane = base + w.off_s2_qplane; t2.nq = w.s2_cap; t2.nq_pad = w.s2_pad;
@@ -563,7 +577,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
         f2.qlist = s2_list; f2.count_dev = s2_count; f2.count = w.s2_cap;
         f2.part_sc = t2.part_sc; f2.part_id = t2.part_id; f2.nsplit = w.s2_nsplit; f2.K1 = w.s2_plen;
         f2.rerank = f2.K1; f2.part_tau = t2.part_tau; f2.ntau = w.s2_nsplit * tc_taus_per_range();
-        f2.part_cnt = t2.part_cnt; f2.eps_rel = eps2; f2.maxnorm = maxnorm3; f2.cert_tau = nullptr;
+        f2.part_cnt = t2.part_cnt; f2.operands = OPERANDS_SPLIT; f2.acc = acc2; f2.norms = norms3; f2.cert_tau = nullptr;
         f2.next_count = nullptr; f2.next_list = nullptr; f2.next_cap = 0;
         rc = launch_knn_finalize_big(f2, w.s2_cap, st);
         if (rc != FL_OK) return rc;
@@ -589,7 +603,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     ff.qlist = fb_list; ff.count_dev = fb_count; ff.count = 0;
     ff.part_sc = sp.part_sc; ff.part_id = sp.part_id; ff.nsplit = w.nsplit_fb; ff.K1 = w.K1f;
     // as in the exact mode: walk until k distances are safe against the fp32 scoring error; last pass
-    ff.rerank = simt_pool_keep(w.K1f, k); ff.verify = 1; ff.eps_rel = SIMT_EPS_REL; ff.part_tau = nullptr; ff.ntau = 0;
+    ff.rerank = simt_pool_keep(w.K1f, k); ff.verify = 1; ff.operands = OPERANDS_F32; ff.acc = SIMT_EPS_REL; ff.part_tau = nullptr; ff.ntau = 0;
     ff.fb_count = nullptr; ff.fb_list = nullptr; ff.fb_cap = 0;
     ff.cert_tau = nullptr;
     ff.next_count = nullptr; ff.next_list = nullptr; ff.next_cap = 0;
@@ -636,18 +650,18 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
     if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
     FL_CHECK_CUDA(cudaMemsetAsync(base + w.off_cnt, 0, 1024, st));
     const float* hnorm;
-    const float* maxnorm;
+    const float* norms;
     if (plane) {
         const PlaneLayout L = plane_layout(m, d);
         hnorm = reinterpret_cast<const float*>(static_cast<const char*>(plane) + L.off_hnorm);
-        maxnorm = reinterpret_cast<const float*>(static_cast<const char*>(plane) + L.off_meta);
+        norms = reinterpret_cast<const float*>(static_cast<const char*>(plane) + L.off_meta);
     } else {
         float* h = reinterpret_cast<float*>(base + w.off_hnorm);
         unsigned int* mx = reinterpret_cast<unsigned int*>(base + w.off_cnt) + 128;    // cleared above
         halfnorm_kernel<<<(unsigned)ceil_div(m, 8), 256, 0, st>>>(db, m, d, ldb, h, mx, dt);
         FL_CHECK_LAUNCH();
         hnorm = h;
-        maxnorm = reinterpret_cast<const float*>(mx);
+        norms = reinterpret_cast<const float*>(mx);
     }
     SimtKnnParams sp{};
     sp.dt = dt;
@@ -674,7 +688,7 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
     // (The scan's compactions keep simt_pool_keep entries per pool: down to that depth the merged list
     // misses no row that scored above its entries, so that is how far the walk may go.)
     fp.k = k; fp.rerank = simt_pool_keep(w.K1, k); fp.row_offset = row_offset;
-    fp.out_dist = out_dist; fp.out_idx = out_idx; fp.verify = 1; fp.eps_rel = SIMT_EPS_REL; fp.maxnorm = maxnorm;
+    fp.out_dist = out_dist; fp.out_idx = out_idx; fp.verify = 1; fp.operands = OPERANDS_F32; fp.acc = SIMT_EPS_REL; fp.norms = norms;
     rc = launch_knn_finalize(fp, nq, st);
     if (rc != FL_OK) return rc;
     if (status) {
@@ -788,8 +802,8 @@ extern "C" int fl_knn_batch_f32(const float* q, int batch, int64_t nq, int64_t l
     fp.q = q; fp.ldq = ldq; fp.count = nq; fp.db = db; fp.m = m; fp.ldb = ldb; fp.d = d; fp.vec = vec;
     fp.part_sc = sp.part_sc; fp.part_id = sp.part_id; fp.nsplit = w.nsplit; fp.K1 = w.K1;
     fp.k = k; fp.rerank = simt_pool_keep(w.K1, k); fp.row_offset = 0;
-    fp.out_dist = out_dist; fp.out_idx = out_idx; fp.verify = 1; fp.eps_rel = SIMT_EPS_REL;
-    fp.maxnorm = reinterpret_cast<const float*>(mx);
+    fp.out_dist = out_dist; fp.out_idx = out_idx; fp.verify = 1; fp.operands = OPERANDS_F32; fp.acc = SIMT_EPS_REL;
+    fp.norms = reinterpret_cast<const float*>(mx);
     fp.batch = batch; fp.q_bstride = q_bstride; fp.db_bstride = db_bstride;
     return launch_knn_finalize(fp, nq, st);
 }
@@ -815,17 +829,44 @@ extern "C" int fl_knn_seed_f32(const float* q, int64_t nq, int64_t ldq, int d, i
                          nullptr, ws, ws_bytes, status, (cudaStream_t)stream);
 }
 
+static int knn_seeded(const char* who, bool one_norm, const float* q, int64_t nq, int64_t ldq, const float* db, int64_t m,
+                      int64_t ldb, int d, int k, const void* plane, int64_t row_offset, const float* seed_cls,
+                      const float* norms, float* out_dist, int32_t* out_idx, void* ws, int64_t ws_bytes, int32_t* status,
+                      cudaStream_t st) {
+    int mode = FL_KNN_BF16_RERANK;
+    int rc = knn_check_args(who, q, nq, ldq, db, m, ldb, d, k, &mode, plane, row_offset, out_dist, out_idx, ws);
+    if (rc != FL_OK || nq == 0) return rc;
+    FL_CHECK_ARG(seed_cls != nullptr && norms != nullptr, "%s: null pointer", who);
+    if (one_norm) {
+        // the caller knows the largest row norm alone: a rounding takes at most 2^-8 of it
+        const KnnWs w = knn_ws_plan(nq, m, d, k, FL_KNN_BF16_RERANK, 0, 1);
+        if (ws_bytes < w.bytes) { set_error("%s: workspace %lld < %lld bytes", who, (long long)ws_bytes, (long long)w.bytes); return FL_EWORKSPACE; }
+        float* both = reinterpret_cast<float*>(static_cast<char*>(ws) + w.off_norms);
+        norms_from_row_norm_kernel<<<1, 1, 0, st>>>(norms, both);
+        FL_CHECK_LAUNCH();
+        norms = both;
+    }
+    return knn_tc_phases(TC_SCORE, q, nq, ldq, db, m, ldb, d, k, plane, row_offset, const_cast<float*>(seed_cls),
+                         norms, out_dist, out_idx, ws, ws_bytes, status, st);
+}
+
 extern "C" int fl_knn_seeded_f32(const float* q, int64_t nq, int64_t ldq, const float* db, int64_t m, int64_t ldb,
                                  int d, int k, const void* plane, int64_t row_offset, const float* seed_cls,
                                  const float* global_maxnorm, float* out_dist, int32_t* out_idx, void* ws,
                                  int64_t ws_bytes, int32_t* status, void* stream) {
-    int mode = FL_KNN_BF16_RERANK;
-    int rc = knn_check_args("fl_knn_seeded_f32", q, nq, ldq, db, m, ldb, d, k, &mode, plane, row_offset, out_dist, out_idx, ws);
-    if (rc != FL_OK || nq == 0) return rc;
-    FL_CHECK_ARG(seed_cls != nullptr && global_maxnorm != nullptr, "fl_knn_seeded_f32: null pointer");
-    return knn_tc_phases(TC_SCORE, q, nq, ldq, db, m, ldb, d, k, plane, row_offset, const_cast<float*>(seed_cls),
-                         global_maxnorm, out_dist, out_idx, ws, ws_bytes, status, (cudaStream_t)stream);
+    return knn_seeded("fl_knn_seeded_f32", true, q, nq, ldq, db, m, ldb, d, k, plane, row_offset, seed_cls, global_maxnorm,
+                      out_dist, out_idx, ws, ws_bytes, status, (cudaStream_t)stream);
 }
+
+extern "C" int fl_knn_seeded_norms_f32(const float* q, int64_t nq, int64_t ldq, const float* db, int64_t m, int64_t ldb,
+                                       int d, int k, const void* plane, int64_t row_offset, const float* seed_cls,
+                                       const float* global_norms, float* out_dist, int32_t* out_idx, void* ws,
+                                       int64_t ws_bytes, int32_t* status, void* stream) {
+    return knn_seeded("fl_knn_seeded_norms_f32", false, q, nq, ldq, db, m, ldb, d, k, plane, row_offset, seed_cls, global_norms,
+                      out_dist, out_idx, ws, ws_bytes, status, (cudaStream_t)stream);
+}
+
+extern "C" int fl_knn_plane_norm_floats(void) { return NORM_LOST + 1; }
 
 extern "C" int64_t fl_knn_plane_maxnorm_offset(int64_t m, int d) {
     if (m < 1 || d < 1) return -1;

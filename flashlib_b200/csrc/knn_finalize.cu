@@ -48,33 +48,40 @@ static __device__ __forceinline__ void finalize_big_slot(const FinalizeParams& p
     __shared__ float s_key[BIG_CAND];
     __shared__ uint32_t s_id[BIG_CAND];
     __shared__ float s_q[512];
-    __shared__ float s_red[BIG_THREADS / 32];
+    __shared__ float4 s_red[BIG_THREADS / 32];
     __shared__ int s_n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t qi = p.qlist != nullptr ? (int64_t)p.qlist[slot] : slot;
     const void* qp = row_at(p.q, qi, p.ldq, p.dt);
 
-    // u and ||q||^2
-    float u = neg_inf(), qs = 0.f;
+    // u, ||q||^2 and what rounding q once and twice takes from it
+    float u = neg_inf(), qs = 0.f, ls = 0.f, ls2 = 0.f;
     for (int i = tid; i < p.ntau; i += BIG_THREADS) u = fmaxf(u, p.part_tau[slot * p.ntau + i]);
-    for (int c = tid; c < p.d; c += BIG_THREADS) { const float v = ld_elem(qp, c, p.dt); s_q[c] = v; qs += v * v; }
+    for (int c = tid; c < p.d; c += BIG_THREADS) {
+        const float v = ld_elem(qp, c, p.dt), l = bf16_lost(v), l2 = bf16_lost(l);
+        s_q[c] = v;
+        qs += v * v;
+        ls += l * l;
+        ls2 += l2 * l2;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         u = fmaxf(u, __shfl_xor_sync(FULL_MASK, u, o));
         qs += __shfl_xor_sync(FULL_MASK, qs, o);
+        ls += __shfl_xor_sync(FULL_MASK, ls, o);
+        ls2 += __shfl_xor_sync(FULL_MASK, ls2, o);
     }
-    if (lane == 0) s_red[warp] = u;
+    if (lane == 0) s_red[warp] = make_float4(u, qs, ls, ls2);
     if (tid == 0) s_n = 0;
     __syncthreads();
-    u = s_red[0];
+    float qsq = 0.f, lost = 0.f, lost2 = 0.f;
 #pragma unroll
-    for (int w = 1; w < BIG_THREADS / 32; ++w) u = fmaxf(u, s_red[w]);
-    __syncthreads();
-    if (lane == 0) s_red[warp] = qs;
-    __syncthreads();
-    float qsq = 0.f;
-#pragma unroll
-    for (int w = 0; w < BIG_THREADS / 32; ++w) qsq += s_red[w];
+    for (int w = 0; w < BIG_THREADS / 32; ++w) {
+        u = fmaxf(u, s_red[w].x);
+        qsq += s_red[w].y;
+        lost += s_red[w].z;
+        lost2 += s_red[w].w;
+    }
 
     // Gather the survivors (score above `cut`), one pool per warp at a time.  If more than
     // BIG_CAND survive (a loose starting threshold), the BIG_CAND that were stored -- an
@@ -124,9 +131,8 @@ static __device__ __forceinline__ void finalize_big_slot(const FinalizeParams& p
     // when k of the exact distances seen so far lie below the lower bound that the next
     // candidate's score (and the cut) puts on every row not yet re-scored; at most BIG_RERANK.
     __shared__ float s_dist[BIG_RERANK];
-    const float mn = __ldg(p.maxnorm);
-    const float eps = p.eps_rel * sqrtf(qsq) * mn;
-    const float slack = 1e-5f * (qsq + mn * mn);
+    const float eps = score_eps(p.operands, qsq, lost, lost2, p.norms, p.acc);
+    const float slack = proof_slack(qsq, __ldg(p.norms + NORM_ROW), p.d);
     const int n_rr = n < BIG_RERANK ? n : BIG_RERANK;
     float bound = cut;
     int done = 0;

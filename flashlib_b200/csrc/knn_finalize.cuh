@@ -63,22 +63,29 @@ __device__ __forceinline__ void finalize_slot(const FinalizeParams& p, const int
     }
 
     const void* qp = row_at(p.q, qi, p.ldq, dt);
-    float qsq = 0.f;
+    float qsq = 0.f, lost = 0.f;
     if (p.vec) {
         for (int c = lane * 4; c < p.d; c += 128) {
             const float4 v = ld_elem4(qp, c, dt);
-            qsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            qsq += sq4(v);
+            lost += sq4(bf16_lost4(v));
         }
     } else {
-        for (int c = lane; c < p.d; c += 32) { const float v = ld_elem(qp, c, dt); qsq += v * v; }
+        for (int c = lane; c < p.d; c += 32) {
+            const float v = ld_elem(qp, c, dt), l = bf16_lost(v);
+            qsq += v * v;
+            lost += l * l;
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+        lost += __shfl_xor_sync(FULL_MASK, lost, o);
+    }
     float eps = 0.f, slack = 0.f;
     if (p.verify) {
-        const float mn = __ldg(p.maxnorm);
-        eps = p.eps_rel * sqrtf(qsq) * mn;
-        slack = 1e-5f * (qsq + mn * mn);
+        eps = score_eps(p.operands, qsq, lost, 0.f, p.norms, p.acc);
+        slack = proof_slack(qsq, __ldg(p.norms + NORM_ROW), p.d);
     }
 
     constexpr bool HAS_FILTER = NPL1 <= 4;

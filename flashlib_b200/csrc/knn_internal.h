@@ -108,7 +108,8 @@ struct FinalizeParams {
     const float* part_sc; const uint32_t* part_id; int nsplit; int K1;
     int k; int rerank; int64_t row_offset;
     float* out_dist; int32_t* out_idx;
-    int verify; float eps_rel; const float* maxnorm;
+    // scoring error: operands (OPERANDS_*) as they were rounded, fp32 accumulation relative to ||q|| ||x||, largest norms
+    int verify; int operands; float acc; const float* norms;
     // thresholds the scoring pass published per (slot, range): every row it left out of its
     // published pool scored at most this much (nullptr: none were left out below the pool)
     const float* part_tau; int ntau;
@@ -140,7 +141,7 @@ struct PairFinalizeParams {
     int npool;               // pools per query: pool i of query q is number q * npool + i, or, with pair_row,
     const int* pair_row;     //   2 * pair_row[q * npool / 2 + i / 2] + i % 2 (pair_row < 0: none)
     const int* row_map; int64_t rows_max;    // optional: published id -> row (< 0: padding)
-    int k; float eps_rel; const float* maxnorm; int64_t row_offset;
+    int k; float acc; const float* norms; int64_t row_offset;   // scoring error of bf16 operands: as FinalizeParams
     float* out_dist; int32_t* out_idx;
     int* fb_count; int* fb_list; int fb_cap;
     int* next_count; int* next_list; int next_cap;
@@ -202,19 +203,16 @@ struct TcSeedPlan { int tiles, splits, rank, dense; };
 int tc_small(int64_t nq_pad, int64_t m_pad);
 void tc_small_split(int64_t nq_pad, int64_t m_pad, int* nsplit, int64_t* tiles_per_split);
 void tc_seed_plan(int64_t nq_pad, int64_t m_pad, int k, TcSeedPlan* w);
-// Relative bound (of ||q|| max||x||) on the error of the tensor-core scores: 2^-8 for operands rounded to bf16
-// (2 * 2^-9 + 2^-18, plus the accumulation, which is what is left where both sides are stored as bf16).
-float tc_eps_rel(int dt, int d);
 // 1 when rows of this shape (more than 512 features) take the tensor-core path with a streamed query tile.
 int tc_wide_supported(int64_t nq, int64_t m, int d, int k);
 // 1 when FL_KNN_AUTO should take the tensor-core path for this shape.
 int tc_knn_auto(int64_t nq, int64_t m, int d, int k);
 // Margin applied by the threshold selection when the class maxima cover more than this shard's rows
-// (q == nullptr: none): the threshold is lowered by 2 eps_rel ||q|| *maxnorm + slack and copied to
+// (q == nullptr: none): the threshold is lowered by twice the scoring error bound (score_eps) + slack and copied to
 // cert_out (f32 [nq_pad], may be null).
 struct TcSeedMargin {
     const void* q; int dt; int64_t ldq; int d; int64_t nq;
-    const float* maxnorm; float eps_rel;
+    const float* norms; float acc;
     float* cert_out;
 };
 // Seeding pass alone (class maxima into p.seed_cls, -inf when the database is too small to sample),
@@ -243,19 +241,19 @@ int launch_knn_tc(const TcKnnParams& p, cudaStream_t st);
 int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, const int* nq_dev, cudaStream_t st);
 
 // Split (hi/lo) operand planes of the second, more precise tensor-core stage (kmeans_tc.cu).
-// Database side: rows [m_pad][3 d_pad + 16] = [hi | hi | lo | norm terms] laid out by
+// Database side: rows [m_pad][3 d_pad + 16] = [lo | hi | hi | norm terms] laid out by
 // plane_layout(m, 3 d_pad).  Query side: the rows listed in `rows` (live count on the device, at
 // most `cap`) as [hi | lo | hi | ones]; with `tau_out` the kernel also derives each listed row's
 // starting threshold from the k-th distance found so far (`prev_dist` [nq][k]):
-// (||q||^2 - d_k) / 2 lowered by 2 eps_rel ||q|| *maxnorm and the proof's slack.
+// (||q||^2 - d_k) / 2 lowered by twice this stage's error bound and the proof's slack.
 int split_plane_supported(int d);
 int launch_split_db_plane(const float* c, int64_t m, int d, int64_t ldc, void* plane, cudaStream_t st);
 int launch_split_query_gather(const float* x, int64_t ldx, int d, const int* rows, const int* rows_count, int cap,
-                              void* out, int d_pad, const float* prev_dist, int k, const float* maxnorm, float eps_rel,
+                              void* out, int d_pad, const float* prev_dist, int k, const float* norms, float acc,
                               float* tau_out, cudaStream_t st);
 
 // bf16 query plane [nq_pad][d_pad + 16] (features zero padded, ones in the norm columns) from fp32 queries;
-// sq_out (optional): ||q||^2 of every query.
+// sq_out (optional): f32 [2][nq_pad], ||q||^2 of every query and the norm of what its rounding took.
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad,
                        int d_pad, cudaStream_t st, int dt = DT_F32, float* sq_out = nullptr);
 

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
     __shared__ float s_max[PF_THREADS];
     __shared__ int s_off[PF_THREADS + 1];
     __shared__ int s_pool[PF_THREADS];
-    __shared__ float s_f[2 * PF_WARPS];
+    __shared__ float s_f[3 * PF_WARPS];
     __shared__ int s_w[PF_WARPS];
     __shared__ int s_n, s_m;
     __shared__ float s_pick;
@@ -64,25 +64,30 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
     };
 
     // u = the largest final threshold: every row in no pool scored at most that much
-    float u = neg_inf(), qs = 0.f;
+    float u = neg_inf(), qs = 0.f, ls = 0.f;
     for (int i = tid; i < p.npool; i += PF_THREADS) {
         const int64_t pl = pool_of(i);
         if (pl >= 0) u = fmaxf(u, __ldg(p.pool_tau + pl));
     }
-    for (int c = tid; c < p.d; c += PF_THREADS) { const float v = ld_elem(qp, c, p.dt); qs += v * v; }
+    for (int c = tid; c < p.d; c += PF_THREADS) {
+        const float v = ld_elem(qp, c, p.dt), l = bf16_lost(v);
+        qs += v * v;
+        ls += l * l;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         u = fmaxf(u, __shfl_xor_sync(FULL_MASK, u, o));
         qs += __shfl_xor_sync(FULL_MASK, qs, o);
+        ls += __shfl_xor_sync(FULL_MASK, ls, o);
     }
-    if (lane == 0) { s_f[warp] = u; s_f[PF_WARPS + warp] = qs; }
+    if (lane == 0) { s_f[warp] = u; s_f[PF_WARPS + warp] = qs; s_f[2 * PF_WARPS + warp] = ls; }
     __syncthreads();
-    float qsq = 0.f;
+    float qsq = 0.f, lost = 0.f;
 #pragma unroll
-    for (int w = 0; w < PF_WARPS; ++w) { u = fmaxf(u, s_f[w]); qsq += s_f[PF_WARPS + w]; }
-    const float mn = __ldg(p.maxnorm);
-    const float eps = p.eps_rel * sqrtf(qsq) * mn;
-    const float slack = 1e-5f * (qsq + mn * mn);
+    for (int w = 0; w < PF_WARPS; ++w) { u = fmaxf(u, s_f[w]); qsq += s_f[PF_WARPS + w]; lost += s_f[2 * PF_WARPS + w]; }
+    const float mn = __ldg(p.norms + NORM_ROW);
+    const float eps = score_eps(OPERANDS_BF16, qsq, lost, 0.f, p.norms, p.acc);
+    const float slack = proof_slack(qsq, mn, p.d);
 
     // Gather what scored above `cut`.  More than fit: the cut rises to the score at the first quarter of
     // those stored (an arbitrary subset) and the gather starts over; everything below is covered by `bound`.
@@ -275,7 +280,7 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
 
 int launch_pairs_finalize(const PairFinalizeParams& p, cudaStream_t st) {
     if (p.nq <= 0) return FL_OK;
-    FL_CHECK_ARG(p.pools && p.pool_cnt && p.pool_tau && p.maxnorm && p.fb_count && p.k >= 1 && p.k <= PF_RERANK && p.npool >= 1,
+    FL_CHECK_ARG(p.pools && p.pool_cnt && p.pool_tau && p.norms && p.fb_count && p.k >= 1 && p.k <= PF_RERANK && p.npool >= 1,
                  "pair-pool finalisation: bad parameters");
     pairs_finalize_kernel<<<(unsigned)p.nq, PF_THREADS, 0, st>>>(p);
     FL_CHECK_LAUNCH();

@@ -968,6 +968,23 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
 }
 
+// What a seeded threshold is lowered by (all lanes of a warp): twice the scoring error bound plus the proof's slack.
+__device__ __forceinline__ float tc_seed_margin(const TcSeedMargin& mg, int64_t row) {
+    float qsq = 0.f, lost = 0.f;
+    const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
+    for (int c = threadIdx.x & 31; c < mg.d; c += 32) {
+        const float x = ld_elem(qp, c, mg.dt), l = bf16_lost(x);
+        qsq += x * x;
+        lost += l * l;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+        lost += __shfl_xor_sync(FULL_MASK, lost, o);
+    }
+    return 2.f * score_eps(OPERANDS_BF16, qsq, lost, 0.f, mg.norms, mg.acc) + proof_slack(qsq, __ldg(mg.norms + NORM_ROW), mg.d);
+}
+
 // Starting threshold of every query row from the seeding pass: the `rank`-th largest of the
 // row's 32 class maxima (16 column classes x 2 warpgroups, disjoint sets of database rows).  At
 // least `rank` distinct rows reach it, and being an order statistic of many classes it scatters
@@ -976,7 +993,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 // With a margin (row-sharded databases: the class maxima are the element-wise maximum over all
 // shards, so the `rank` rows may live on other shards) the threshold is lowered by twice the
 // scoring error bound plus the fp32 slack: a row whose score stays at or below
-//     cert = pick - 2 eps_rel ||q|| maxnorm - slack
+//     cert = pick - 2 score_eps - slack
 // is at least as far from the query as each of those `rank` rows, whichever shard holds them,
 // so a shard that re-scores every row above `cert` cannot miss a global neighbour.  `cert` is
 // also written to mg.cert_out, where the finalisation reads it.
@@ -996,13 +1013,8 @@ __global__ void __launch_bounds__(256) tc_seed_select_kernel(const float* __rest
     const unsigned sel = __ballot_sync(FULL_MASK, r == rank - 1);
     float pick = __shfl_sync(FULL_MASK, v, __ffs(sel) - 1);
     if (mg.q != nullptr) {
-        float qsq = 0.f;
-        const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
-        for (int c = lane; c < mg.d; c += 32) { const float x = ld_elem(qp, c, mg.dt); qsq += x * x; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
-        const float mn = __ldg(mg.maxnorm);
-        if (pick > neg_inf()) pick -= 2.f * mg.eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
+        const float margin = tc_seed_margin(mg, row);
+        if (pick > neg_inf()) pick -= margin;
         if (lane == 0 && mg.cert_out != nullptr) mg.cert_out[row] = pick;
     }
     if (lane == 0 && pick > neg_inf()) tau[row] = pick;
@@ -1049,15 +1061,7 @@ __global__ void __launch_bounds__(256) tc_seed_select_split_kernel(const float* 
         if (c >= rank && c <= rank + (rank >> 3) + 1) break;
     }
     float pick = __int_as_float(lo >= 0 ? lo : (lo ^ 0x7fffffff));
-    if (mg.q != nullptr) {
-        const void* qp = row_at(mg.q, row, mg.ldq, mg.dt);
-        float qsq = 0.f;
-        for (int c = lane; c < mg.d; c += 32) { const float x = ld_elem(qp, c, mg.dt); qsq += x * x; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
-        const float mn = __ldg(mg.maxnorm);
-        pick -= 2.f * mg.eps_rel * sqrtf(qsq) * mn + 1e-5f * (qsq + mn * mn);
-    }
+    if (mg.q != nullptr) pick -= tc_seed_margin(mg, row);
     // A score equal to the threshold is not kept: one step below it, so that the `rank` rows are.  A norm of NaN or
     // infinity among the rows makes the margin, and an infinite score the step, NaN: no score exceeds that, so
     // the row keeps its -inf.
@@ -1126,12 +1130,7 @@ int tc_knn_supported(int64_t nq, int64_t m, int d, int k) {
     return FL_OK;
 }
 
-float tc_eps_rel(int dt, int d) {
-    const float acc = 1.2e-7f * (float)(d + 16);           // fp32 accumulation of d + 16 products, 2^-23 each
-    if (dt == DT_BF16) return 2.f * acc;                   // operands are exact
-    return 0.00391f + acc > 0.004f ? 0.00391f + acc : 0.004f;
-}
-// (the streamed query tile has no limit of its own; 8 192 features keep the error bound near 2^-8)
+// (the streamed query tile has no limit of its own; 8 192 features keep the accumulation's part of the error bound at 2^-10)
 int tc_wide_supported(int64_t nq, int64_t m, int d, int k) {
     if (d <= 512 || d > 8192 || nq < 1 || k > 112) return 0;
     if (m < 512 || round_up(m, 256) / 256 > (1 << 23)) return 0;

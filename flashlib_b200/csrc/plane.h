@@ -10,7 +10,7 @@ struct PlaneLayout {
     int pitch;          // bf16 elements per plane row: d_pad features + 16 norm columns
     int64_t off_rows;   // bf16 [m_pad][pitch]
     int64_t off_hnorm;  // f32 [m_pad], ||x||^2 / 2, +inf for padding rows
-    int64_t off_meta;   // f32 [4]: [0] = max row norm
+    int64_t off_meta;   // f32 [4]: largest norms over the rows (NORM_* of common.cuh)
     int64_t bytes;
 };
 

@@ -43,7 +43,7 @@ __global__ void rownorm_kernel(const float* __restrict__ x, int64_t n, int d, in
 // rows allow them (vec) and 8-byte writes.
 __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d, int64_t ld,
                                    __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                   unsigned int* __restrict__ maxnorm_bits, int64_t m_pad, int d_pad, int dt, int vec) {
+                                   unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int dt, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= m_pad) return;
@@ -55,17 +55,22 @@ __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d
         return;
     }
     const void* p = row_at(db, row, ld, dt);
-    float s = 0.f;
+    float s = 0.f, lost = 0.f;
     for (int c = lane * 4; c < d_pad; c += 128) {
         const float4 v = ld_row4(p, c, d, vec, dt);
-        s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        s += sq4(v);
+        lost += sq4(bf16_lost4(v));
         *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL_MASK, s, off);
+    for (int off = 16; off > 0; off >>= 1) {
+        s += __shfl_xor_sync(FULL_MASK, s, off);
+        lost += __shfl_xor_sync(FULL_MASK, lost, off);
+    }
     if (lane == 0) {
         hnorm[row] = 0.5f * s;
-        max_norm_update(maxnorm_bits, s);
+        max_norm_update(norm_bits + NORM_ROW, s);
+        max_norm_update(norm_bits + NORM_LOST, lost);
     }
     if (lane < PLANE_AUG_COLS) {
         const float nh = -0.5f * s;

@@ -88,10 +88,18 @@ class DeviceKnnKernels:
         return get_plane(db)
 
     def max_norm(self, db: torch.Tensor, plane) -> torch.Tensor:
-        """Largest row norm of this shard as a 1-element fp32 device tensor."""
+        """What the scoring error bound needs of this shard's rows, as fp32 device words whose element-wise
+        maximum over the shards holds for all of them: the largest row norm and the largest norm of what
+        the bf16 rounding took of a row."""
         from . import _lib
-        off = _lib.load().fl_knn_plane_maxnorm_offset(db.shape[0], db.shape[1])
-        return plane.buf[off:off + 4].view(torch.float32).clone()
+        lib = _lib.load()
+        off = lib.fl_knn_plane_maxnorm_offset(db.shape[0], db.shape[1])
+        return plane.buf[off:off + 4 * self.norm_words].view(torch.float32).clone()
+
+    @property
+    def norm_words(self) -> int:
+        from . import _lib
+        return _lib.load().fl_knn_plane_norm_floats()
 
     def local(self, q, db, k, row_offset, mode, plane):
         from .knn import _mode_from, knn_f32
@@ -134,10 +142,10 @@ class DeviceKnnKernels:
         nq, d = q.shape
         out_d = torch.empty((nq, k), dtype=torch.float32, device=q.device)
         out_i = torch.empty((nq, k), dtype=torch.int32, device=q.device)
-        _lib.check(lib.fl_knn_seeded_f32(q.data_ptr(), nq, q.stride(0), db.data_ptr(), db.shape[0], db.stride(0), d, k,
-                                         plane.ptr, row_offset, cls.data_ptr(), gmax.data_ptr(), out_d.data_ptr(),
-                                         out_i.data_ptr(), ws.data_ptr(), ws_bytes, status.data_ptr(),
-                                         _stream_ptr(q.device)))
+        _lib.check(lib.fl_knn_seeded_norms_f32(q.data_ptr(), nq, q.stride(0), db.data_ptr(), db.shape[0], db.stride(0), d, k,
+                                               plane.ptr, row_offset, cls.data_ptr(), gmax.data_ptr(), out_d.data_ptr(),
+                                               out_i.data_ptr(), ws.data_ptr(), ws_bytes, status.data_ptr(),
+                                               _stream_ptr(q.device)))
         return out_d, out_i, status
 
     def pack(self, d_, i_, status, world: int, owner: bool) -> torch.Tensor:
@@ -171,8 +179,8 @@ class DeviceKnnKernels:
 class ShardedKnnIndex:
     """One rank's shard of a row-sharded database together with the facts that need a collective
     to establish: the smallest shard's row count, whether every shard can take the tensor-core
-    path, and the largest row norm over all shards (the scoring error bound of
-    ``fl_knn_seeded_f32`` must hold for rows of every shard).
+    path, and the largest norms over the rows of all shards (the scoring error bound of
+    ``fl_knn_seeded_norms_f32`` must hold for rows of every shard).
 
     Constructing it is a COLLECTIVE call: every rank of ``group`` must do so at the same point of
     its program.  It is the ``fit`` step of the sharded search; :func:`sharded_knn` uses it to share
@@ -186,7 +194,8 @@ class ShardedKnnIndex:
         m, d = db_shard.shape
         can_tc = m > 0 and kern.tensor_core(1 << 20, m, d, min(10, m), "bf16")
         self.plane = plane if plane is not None else (kern.plane_of(db_shard) if can_tc else None)
-        gmax = kern.max_norm(db_shard, self.plane) if self.plane is not None else torch.zeros(1, device=db_shard.device)
+        gmax = (kern.max_norm(db_shard, self.plane) if self.plane is not None
+                else torch.zeros(getattr(kern, "norm_words", 1), device=db_shard.device))
         facts = torch.tensor([m, 1 if self.plane is not None else 0], dtype=torch.int64, device=db_shard.device)
         if dist.is_initialized() and dist.get_world_size(group) > 1:
             dist.all_reduce(gmax, op=dist.ReduceOp.MAX, group=group)

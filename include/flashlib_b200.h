@@ -145,12 +145,12 @@ int     fl_knn_rows(const void* q, int64_t nq, int64_t ldq,
 /* fl_knn_f32 (tensor-core mode) with a second tensor-core stage between the bf16 pass and  */
 /* the exact CUDA-core pass.  Rows whose bf16 candidate pool cannot be proven complete are  */
 /* scored again with every fp32 operand carried as two bf16 values (hi = bf16(v),           */
-/* lo = bf16(v - hi); one product over [hi|lo|hi] x [hi|hi|lo] columns gives                */
-/* hi.hi + lo.hi + hi.lo), the error-compensated split the reference uses for fp32-exact    */
+/* lo = bf16(v - hi); one product over [hi|lo|hi] x [lo|hi|hi] columns gives                */
+/* hi.lo + lo.hi + hi.hi), the error-compensated split the reference uses for fp32-exact    */
 /* ranking on tensor cores (linalg/gemm/bf16_x3.py:1-22 with bf16 halves, the lo.lo product  */
 /* dropped and one fp32 accumulator across the three products; linalg/gemm/tf32_x3.py:9-31, */
-/* linalg/gemm/triton/fused_kernels.py:222-294 with TF32 halves).  The scoring error drops from 2^-8 to about 2^-16 of          */
-/* ||q|| max||x||, so the same proof accepts nearly every row; what is left takes the exact  */
+/* linalg/gemm/triton/fused_kernels.py:222-294 with TF32 halves).  The scoring error drops a hundredfold (its bound from        */
+/* about 0.0037 to about 3e-5 of ||q|| max||x||), so the same proof accepts nearly every row; what is left takes the exact  */
 /* pass as before (status[FL_STATUS_STAGE2] / [FL_STATUS_FALLBACK] count the two).  d <= 128.*/
 /* `split_plane` is filled once per database by fl_knn_prepare_split_f32                    */
 /* (fl_knn_split_plane_bytes = 0: no split plane for this d); NULL = no second stage.       */
@@ -173,21 +173,30 @@ int     fl_knn_staged_f32(const float* q, int64_t nq, int64_t ldq,
 /*     (f32 [fl_knn_seed_floats(nq)], 32 per padded query row; -inf when the shard is too    */
 /*     small to sample).  It clears `status`.                                                */
 /*  2. The caller takes the element-wise maximum of seed_cls over all shards (an all-reduce  */
-/*     with MAX) and, once per database, the maximum over all shards of the f32 at byte       */
-/*     offset fl_knn_plane_maxnorm_offset(m, d) of each shard's plane (largest row norm).     */
-/*  3. fl_knn_seeded_f32, with the SAME ws (untouched in between), q, nq, d, k and plane,     */
+/*     with MAX) and, once per database, the element-wise maximum over all shards of the       */
+/*     fl_knn_plane_norm_floats() f32 words at byte offset fl_knn_plane_maxnorm_offset(m, d)   */
+/*     of each shard's plane (largest row norm; largest norm of what rounding took of a row).  */
+/*  3. fl_knn_seeded_norms_f32, with the SAME ws (untouched in between), q, nq, d, k and plane,     */
 /*     scores this shard from thresholds derived from the combined maxima: k + 6 rows of the  */
 /*     whole database are known to reach them, and they are lowered by twice the scoring     */
 /*     error bound, so a row this shard leaves out cannot be one of the database's k         */
 /*     nearest.  A shard may therefore return fewer than k rows (padded +inf / -1); merging  */
 /*     all shards' lists with fl_topk_merge_f32 gives the exact result.  Rows that can be     */
 /*     neither proven nor ruled out are recomputed exactly, as in fl_knn_f32; status is not   */
-/*     cleared, so an error of step 1 stays visible.                                          */
+/*     cleared, so an error of step 1 stays visible.  fl_knn_seeded_f32 takes the first of the */
+/*     words alone and a bound that holds for any rows of that norm (a wider band).           */
 int64_t fl_knn_seed_floats(int64_t nq);
 int     fl_knn_seed_f32(const float* q, int64_t nq, int64_t ldq, int d, int k,
                         const void* plane, int64_t m, float* seed_cls,
                         void* ws, int64_t ws_bytes, int32_t* status, void* stream);
 int64_t fl_knn_plane_maxnorm_offset(int64_t m, int d);
+int     fl_knn_plane_norm_floats(void);
+int     fl_knn_seeded_norms_f32(const float* q, int64_t nq, int64_t ldq,
+                                const float* db, int64_t m, int64_t ldb, int d, int k,
+                                const void* plane, int64_t row_offset,
+                                const float* seed_cls, const float* global_norms,
+                                float* out_dist, int32_t* out_idx,
+                                void* ws, int64_t ws_bytes, int32_t* status, void* stream);
 int     fl_knn_seeded_f32(const float* q, int64_t nq, int64_t ldq,
                           const float* db, int64_t m, int64_t ldb, int d, int k,
                           const void* plane, int64_t row_offset,

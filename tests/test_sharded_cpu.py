@@ -23,7 +23,7 @@ def _free_port():
 
 
 STATUS_WORDS = 8
-EPS_REL = 0.004          # the scoring error bound of the tensor-core kernels, relative to ||q|| max||x||
+EPS_REL = 0.0079         # the largest scoring error of the tensor-core kernels, relative to ||q|| max||x|| (2^-7 and a little)
 
 
 class OracleKnnKernels:
