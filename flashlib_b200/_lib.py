@@ -73,6 +73,7 @@ SIGNATURES = {
     "fl_knn_resolve_mode": (c_int, [c_int64, c_int64, c_int, c_int]),
     "fl_publish_status": (c_int, [c_void_p, c_void_p, c_void_p]),
     "fl_knn_wants_plane": (c_int, [c_int64, c_int64, c_int, c_int]),
+    "fl_knn_batch_route": (c_int, [c_int, c_int64, c_int64, c_int, c_int]),
     "fl_knn_batch_pick": (c_int, [c_int64, c_int64, c_int, c_int]),
     "fl_knn_search": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int,
                               c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,

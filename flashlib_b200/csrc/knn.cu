@@ -751,18 +751,21 @@ static KnnBatchWs knn_batch_plan(int batch, int64_t nq, int64_t m, int d, int k)
 
 extern "C" int64_t fl_knn_batch_workspace_bytes(int batch, int64_t nq, int64_t m, int d, int k) {
     if (batch < 1 || nq < 1 || m < 1 || d < 1 || k < 1 || k > 512) return 0;
-    if (clouds_pick(nq, m, d, k)) return 1024;
+    if (clouds_pick(batch, nq, m, d, k)) return 1024;
     return knn_batch_plan(batch, nq, m, d, k).bytes;
 }
 
 // 1: a batch of problems of this shape goes through fl_knn_batch_f32 at once; 0: problem by problem through
 // the tensor-core kernel, whose launches cost more than its scoring saves below 2^24 pairs (32 problems of
 // 2 048 x 2 048: 3.2 ms one by one, 1.7 ms in the CUDA-core batch).
-extern "C" int fl_knn_batch_pick(int64_t nq, int64_t m, int d, int k) {
-    if (nq < 1 || m < 1 || d < 1 || k < 1) return 0;
-    if (clouds_pick(nq, m, d, k)) return 1;
-    return tc_knn_supported(nq, m, d, k) != FL_OK || m < 2048 || nq * m < (int64_t(1) << 24);
+extern "C" int fl_knn_batch_route(int batch, int64_t nq, int64_t m, int d, int k) {
+    if (batch < 1 || nq < 1 || m < 1 || d < 1 || k < 1) return 0;
+    if (tc_knn_supported(nq, m, d, k) != FL_OK || m < 2048 || nq * m < (int64_t(1) << 24)) return 1;
+    return clouds_beat_single(batch, nq, m, d, k);
 }
+
+// (a batch of unknown size: two problems, of which one by one asks the least)
+extern "C" int fl_knn_batch_pick(int64_t nq, int64_t m, int d, int k) { return fl_knn_batch_route(2, nq, m, d, k); }
 
 extern "C" int fl_knn_batch_f32(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride, const float* db,
                                 int64_t m, int64_t ldb, int64_t db_bstride, int d, int k, float* out_dist, int32_t* out_idx,
@@ -772,7 +775,7 @@ extern "C" int fl_knn_batch_f32(const float* q, int batch, int64_t nq, int64_t l
     int rc = knn_check_args("fl_knn_batch_f32", q, nq, ldq, db, m, ldb, d, k, &mode, nullptr, 0, out_dist, out_idx, ws);
     if (rc != FL_OK || nq == 0) return rc;
     FL_CHECK_ARG(q_bstride >= 0 && db_bstride >= 0, "fl_knn_batch_f32: negative batch stride");
-    if (clouds_pick(nq, m, d, k))
+    if (clouds_pick(batch, nq, m, d, k))
         return launch_knn_clouds(q, batch, nq, ldq, q_bstride, db, m, ldb, db_bstride, d, k, out_dist, out_idx, (cudaStream_t)stream);
     const KnnBatchWs w = knn_batch_plan(batch, nq, m, d, k);
     if (ws_bytes < w.bytes) { set_error("fl_knn_batch_f32: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes); return FL_EWORKSPACE; }

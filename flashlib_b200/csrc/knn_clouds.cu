@@ -249,12 +249,36 @@ static int clouds_dispatch(const CloudParams& p, int batch, cudaStream_t st) {
     return clouds_launch<DP, 256, 2>(p, batch, st);
 }
 
-// The time of a problem pair grows with the padded features and the number of neighbours; one problem after
-// the other on the tensor cores costs 100 us or more each.  Measured, batch against one by one: 2 x 4 000^2 x 16,
-// k = 40: 276 and 286 us; 2 x 8 192^2 x 8, k = 32: 377 and 483; 4 x 8 192^2 x 3, k = 16: 387 and 831; with 16
-// features and k = 40 at 8 192^2 the batch lost (1 618 and 996 for four problems).
-int clouds_pick(int64_t nq, int64_t m, int d, int k) {
+// Estimated us of a batch by this kernel and by the tile kernel (knn_simt.cu), fitted to 900 shapes (2 to 64
+// problems, 1 to 4 096 queries, 512 to 1M rows, 3 to 16 features, k = 16 to 40).  A block here walks every row of its
+// problem twice and no other block helps it: 16 ns a row with 3 features, 24 with 8, 40 with 16, 1.6 times that once
+// the problems outgrow the L2, whatever the number of queries -- then the pairs.  The tile kernel deals the rows of a
+// problem to up to 64 blocks of 64 queries.
+static double clouds_estimate_us(int batch, int64_t nq, int64_t m, int d, int k) {
+    const double dp = d <= 3 ? 3 : d <= 4 ? 4 : d <= 8 ? 8 : 16;
+    const double walk = (double)m * (1.02e-2 + 2.0e-3 * dp) * ((double)batch * m * d * 4 > 90e6 ? 1.6 : 1.0);
+    const double pairs = (double)batch * nq * m * (0.3e-6 + 0.17e-6 * dp) * (k > 16 ? 1.25 : 1.0);
+    return 12 + (k <= 16 ? (nq < 2 ? 6 : 10) : (nq < 2 ? 14 : 32)) + (walk > pairs ? walk : pairs);
+}
+static double tile_batch_estimate_us(int batch, int64_t nq, int64_t m, int k) {
+    const double per_row = nq <= 16 ? 1.0e-3 : nq <= 64 ? 1.25e-3 : 0.9e-3;
+    return (nq < 8 ? 46 : 95) + (k > 16 ? (nq < 8 ? 12 : 36) : 0) + (m < 16384 ? 2.9e-3 * m : 31.0 + 1e-3 * m) +
+           (double)(batch - 1) * ceil_div(nq, 64) * m * per_row;
+}
+static int clouds_supported(int64_t nq, int64_t m, int d, int k) {
     return nq >= 1 && d <= 16 && k <= 40 && nq * m <= ((int64_t)1 << (d <= 8 && k <= 32 ? 26 : 24));
+}
+// Measured, this against the tile kernel: 32 x 2 048^2 x 3, k = 16: 232 and 1 704 us; 64 x 64 x 4 096 x 3: 87 and 564;
+// 2 x 16 x 65 536 x 3: 1 050 and 308; 8 x 16 x 1 000 000 x 3: 24 600 and 9 100; 2 x 64 x 8 192 x 16: 367 and 156.
+int clouds_pick(int batch, int64_t nq, int64_t m, int d, int k) {
+    return clouds_supported(nq, m, d, k) && clouds_estimate_us(batch, nq, m, d, k) <= tile_batch_estimate_us(batch, nq, m, k);
+}
+
+// One problem after the other on the tensor cores costs 130 us and its scoring, and for more problems than operand planes
+// are kept (four) the building of its planes (2 x 8 192^2 x 8, k = 32: 377 us in the batch and 483 one by one; 4 x
+// 8 192^2 x 3, k = 16: 387 and 831; 4 x 8 192^2 x 16, k = 40: 1 618 and 996; 32 x 64 x 262 144 x 3: 5.8 and 17.9 ms).
+int clouds_beat_single(int batch, int64_t nq, int64_t m, int d, int k) {
+    return clouds_supported(nq, m, d, k) && clouds_estimate_us(batch, nq, m, d, k) <= batch * (130 + (double)nq * m * 1e-6 + (batch > 4 ? 8e-4 * m : 0.0));
 }
 
 int launch_knn_clouds(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride, const float* db, int64_t m,

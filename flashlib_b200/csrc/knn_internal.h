@@ -94,7 +94,8 @@ int64_t direct_ivf_workspace_bytes(int64_t npairs, int nchunk, int k);
 int launch_ivf_direct(DirectParams p, void* ws, cudaStream_t st);
 
 // Batches of small problems with few features (knn_clouds.cu): one launch, no workspace.
-int clouds_pick(int64_t nq, int64_t m, int d, int k);      // 1: the batch entry point takes it for the shape
+int clouds_pick(int batch, int64_t nq, int64_t m, int d, int k);         // 1: the batch entry point takes it for the shape
+int clouds_beat_single(int batch, int64_t nq, int64_t m, int d, int k);  // 1: it beats one tensor-core call per problem
 int launch_knn_clouds(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride, const float* db, int64_t m,
                       int64_t ldb, int64_t db_bstride, int d, int k, float* out_dist, int32_t* out_idx, cudaStream_t st);
 

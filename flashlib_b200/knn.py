@@ -406,7 +406,7 @@ def flash_knn_dispatch(x: torch.Tensor, c: torch.Tensor, k: int, *, tol: Optiona
             return idxs[0] if squeeze else idxs
         return (vals[0], idxs[0]) if squeeze else (vals, idxs)
     batched = (B > 1 and N > 0 and target is None and x.dtype == torch.float32 and m != _lib.FL_KNN_BF16_RERANK
-               and lib.fl_knn_batch_pick(N, M, D, k)
+               and lib.fl_knn_batch_route(B, N, M, D, k)
                and x.stride(2) == 1 and c.stride(2) == 1 and x.stride(1) >= D and c.stride(1) >= D)
     if batched:
         # many small problems: one launch sequence for the whole batch

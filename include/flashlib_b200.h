@@ -118,7 +118,9 @@ int     fl_knn_f32(const float* q, int64_t nq, int64_t ldq,
 /* where a launch per problem is the whole cost).  Problem b reads q + b * q_bstride and    */
 /* db + b * db_bstride (elements) and writes out_dist / out_idx [batch][nq][k].  Exact      */
 /* CUDA-core path; large problems are better served by one fl_knn_f32 call each             */
-/* (fl_knn_batch_pick: 1 where the batch is the better way).                                */
+/* (fl_knn_batch_route: 1 where the batch is the better way; fl_knn_batch_pick: the same      */
+/* for two problems).                                                                       */
+int     fl_knn_batch_route(int batch, int64_t nq, int64_t m, int d, int k);
 int     fl_knn_batch_pick(int64_t nq, int64_t m, int d, int k);
 int64_t fl_knn_batch_workspace_bytes(int batch, int64_t nq, int64_t m, int d, int k);
 int     fl_knn_batch_f32(const float* q, int batch, int64_t nq, int64_t ldq, int64_t q_bstride,

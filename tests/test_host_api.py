@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import flashlib_b200 as fl
-from flashlib_b200 import synthetic
+from flashlib_b200 import _lib, synthetic
 
 
 def test_lazy_names_resolve():
@@ -141,3 +141,14 @@ def test_tol_to_storage_dtype_follows_the_reference_rule():
                 (4e-4, torch.float16), (1e-3, torch.float16), (3e-3, torch.float16), (1e-2, torch.float16), (1.0, torch.float16)]
     for tol, want in recorded:
         assert storage_dtype_for(tol) is want, (tol, want)
+
+
+@pytest.mark.parametrize("B,nq,m,d,k,clouds", [(32, 2_048, 2_048, 3, 16, True), (64, 64, 4_096, 3, 16, True), (4, 8_192, 8_192, 3, 16, True),
+                                               (8, 16, 1_000_000, 3, 16, False), (2, 16, 65_536, 3, 16, False),
+                                               (2, 64, 8_192, 16, 16, False), (2, 1, 1_000_000, 16, 40, False)])
+def test_batch_kernel_by_walk_and_blocks(B, nq, m, d, k, clouds):
+    """The kernel whose blocks walk every row of a problem (its workspace is a token 1 024 bytes) is for problems with
+    queries enough; few queries against many rows go to the kernel that deals the rows to many blocks."""
+    lib = _lib.load()
+    assert (lib.fl_knn_batch_workspace_bytes(B, nq, m, d, k) == 1024) == clouds
+    assert lib.fl_knn_batch_route(B, nq, m, d, k) == 1 or nq * m >= 1 << 24

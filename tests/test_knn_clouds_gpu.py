@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import flashlib_b200 as fl
+from flashlib_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,17 @@ def test_rows_without_a_finite_distance():
     assert torch.isfinite(vals[..., :finite]).all() and torch.isinf(vals[..., finite:]).all()
     assert (idxs != 10).all()
     assert (idxs[..., finite:] == torch.tensor([20, 30], device="cuda")).all()
+
+
+@pytest.mark.parametrize("B,nq,m,d,k", [(2, 16, 65_536, 3, 16), (3, 1, 20_001, 16, 40), (2, 300, 40_000, 8, 10), (2, 1, 300_000, 3, 5)])
+def test_few_queries_of_large_problems(B, nq, m, d, k):
+    """Shapes that go to the tile kernel, which deals a problem's rows to many blocks."""
+    assert _lib.load().fl_knn_batch_workspace_bytes(B, nq, m, d, k) > 1024
+    g = torch.Generator().manual_seed(m)
+    q, x = torch.randn(B, nq, d, generator=g).cuda(), torch.randn(B, m, d, generator=g).cuda()
+    vals, idxs = fl.flash_knn(q, x, k)
+    want = torch.cat([((q[:, i:i + 1].double() - x.double()) ** 2).sum(-1)[:, None].topk(k, dim=2, largest=False).values
+                      for i in range(nq)], 1)
+    own = ((q.double()[:, :, None] - x.double()[torch.arange(B, device="cuda")[:, None, None], idxs.long()]) ** 2).sum(-1)
+    eps = (d + 2) * 2.0 ** -24
+    assert ((vals - own).abs() <= eps * own).all() and ((own - want).abs() <= 2 * eps * want).all()
