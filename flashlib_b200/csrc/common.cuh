@@ -302,6 +302,11 @@ __device__ __forceinline__ float sq4(float4 v) { return v.x * v.x + v.y * v.y + 
 __device__ __forceinline__ float4 bf16_lost4(float4 v) {
     return make_float4(bf16_lost(v.x), bf16_lost(v.y), bf16_lost(v.z), bf16_lost(v.w));
 }
+// The same from the rounded values (bf16x4_bits(v)).
+__device__ __forceinline__ float4 bf16_lost4(float4 v, uint2 w) {
+    return make_float4(v.x - __uint_as_float(w.x << 16), v.y - __uint_as_float(w.x & 0xffff0000u),
+                       v.z - __uint_as_float(w.y << 16), v.w - __uint_as_float(w.y & 0xffff0000u));
+}
 
 // Largest norms over the rows of a database, left by the passes that write its operand planes: of the rows x, of what
 // one rounding to bf16 takes from them (x - hi) and of what the second half of a split plane still misses
@@ -341,6 +346,38 @@ __device__ __forceinline__ float proof_slack(float qsq, float xn, int d) {
 __device__ __forceinline__ bool list_proven(float dk, float qsq, float bound, float eps, float slack) {
     if (bound == neg_inf()) return slack < pos_inf();
     return dk < qsq - 2.f * (bound + eps) - slack;
+}
+
+// The split -||x||^2 / 2 columns of a plane row (lanes below PLANE_AUG_COLS write them): three bf16 terms that sum to it.
+__device__ __forceinline__ void write_norm_columns(__nv_bfloat16* o, float sq, int cols) {
+    const int lane = threadIdx.x & 31;
+    if (lane >= cols) return;
+    const float nh = -0.5f * sq;
+    const __nv_bfloat16 h1 = __float2bfloat16_rn(nh);
+    const float r1 = nh - __bfloat162float(h1);
+    const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
+    const float r2 = r1 - __bfloat162float(h2);
+    const __nv_bfloat16 h3 = __float2bfloat16_rn(r2);
+    o[lane] = lane == 0 ? h1 : lane == 1 ? h2 : lane == 2 ? h3 : __float2bfloat16_rn(0.f);
+}
+
+// Folds the squares that lane 0 of every warp holds (0 where its row is none) into the largest norms; all threads of
+// a block call it.  A maximum per block in shared memory first: one read of the global words per warp and norm
+// made the planes of 262 144 x 16 rows 200 us slower, so many reads of one address they are.
+template <int N>
+__device__ __forceinline__ void block_norms_update(unsigned int* norm_bits, const float (&sq)[N]) {
+    __shared__ unsigned int s_norm[N];
+    if (threadIdx.x < N) s_norm[threadIdx.x] = 0u;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) atomicMax(s_norm + i, __float_as_uint(sqrtf(sq[i])));      // (NaN orders above infinity)
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        const unsigned int v = s_norm[threadIdx.x];
+        if (*reinterpret_cast<volatile unsigned int*>(norm_bits + threadIdx.x) < v) atomicMax(norm_bits + threadIdx.x, v);
+    }
 }
 
 // Folds sqrt(sq) into the largest row norm (its bits, zero-initialised: norms are >= 0, so bit patterns

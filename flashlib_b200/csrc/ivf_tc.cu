@@ -78,48 +78,36 @@ __global__ void ivf_row_map_kernel(const int64_t* __restrict__ list_offsets, con
     for (int r = threadIdx.x; r < len; r += blockDim.x) row_map[p0 + r] = (int)(r0 + r);
 }
 
-// One warp per plane row: bf16 features, the split -||x||^2/2 columns, half norm, largest norms.
+// One warp per plane row: bf16 features, the split -||x||^2/2 columns, half norm, largest norms.  rows_max is a multiple of the block's rows.
 __global__ void ivf_plane_rows_kernel(const float* __restrict__ data, int64_t ld, int d, const int* __restrict__ row_map,
                                       int64_t rows_max, __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
                                       unsigned int* __restrict__ norm_bits, int d_pad) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= rows_max) return;
     const int pitch = d_pad + PLANE_AUG_COLS;
     __nv_bfloat16* o = rows + row * pitch;
     const int src = __ldg(row_map + row);
+    float sq[2] = {0.f, 0.f};                   // NORM_ROW, NORM_LOST
     if (src < 0) {
         for (int c = lane; c < pitch; c += 32) o[c] = __float2bfloat16_rn(c == d_pad ? -3.0e38f : 0.f);
         if (lane == 0) hnorm[row] = pos_inf();
-        return;
-    }
-    const float* p = data + (int64_t)src * ld;
-    float s = 0.f, lost = 0.f;
-    for (int c = lane; c < d_pad; c += 32) {
-        const float v = (c < d) ? __ldg(p + c) : 0.f, l = bf16_lost(v);
-        s += v * v;
-        lost += l * l;
-        o[c] = __float2bfloat16_rn(v);
-    }
+    } else {
+        const float* p = data + (int64_t)src * ld;
+        for (int c = lane; c < d_pad; c += 32) {
+            const float v = (c < d) ? __ldg(p + c) : 0.f, l = bf16_lost(v);
+            sq[0] += v * v;
+            sq[1] += l * l;
+            o[c] = __float2bfloat16_rn(v);
+        }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        s += __shfl_xor_sync(FULL_MASK, s, off);
-        lost += __shfl_xor_sync(FULL_MASK, lost, off);
+        for (int off = 16; off > 0; off >>= 1) {
+            sq[0] += __shfl_xor_sync(FULL_MASK, sq[0], off);
+            sq[1] += __shfl_xor_sync(FULL_MASK, sq[1], off);
+        }
+        if (lane == 0) hnorm[row] = 0.5f * sq[0];
+        write_norm_columns(o + d_pad, sq[0], PLANE_AUG_COLS);
     }
-    if (lane == 0) {
-        hnorm[row] = 0.5f * s;
-        max_norm_update(norm_bits + NORM_ROW, s);
-        max_norm_update(norm_bits + NORM_LOST, lost);
-    }
-    if (lane < PLANE_AUG_COLS) {
-        const float nh = -0.5f * s;
-        const __nv_bfloat16 h1 = __float2bfloat16_rn(nh);
-        const float r1 = nh - __bfloat162float(h1);
-        const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(h2);
-        const __nv_bfloat16 h3 = __float2bfloat16_rn(r2);
-        o[d_pad + lane] = lane == 0 ? h1 : lane == 1 ? h2 : lane == 2 ? h3 : __float2bfloat16_rn(0.f);
-    }
+    block_norms_update(norm_bits, sq);
 }
 
 // One block per list: the work items of the list (groups of IVF_TC_BQ of its pairs), the pair

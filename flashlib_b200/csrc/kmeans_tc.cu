@@ -44,46 +44,32 @@ __global__ void split_c_plane_kernel(const float* __restrict__ c, int64_t m, int
                                      unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= m_pad) return;
     const int pitch = 3 * d_pad + PLANE_AUG_COLS;
     __nv_bfloat16* o = rows + row * pitch;
+    float sq[3] = {0.f, 0.f, 0.f};              // NORM_ROW, NORM_LOST, NORM_LOST2
     if (row >= m) {
         for (int t = lane; t < pitch; t += 32) o[t] = __float2bfloat16_rn(t == 3 * d_pad ? -3.0e38f : 0.f);
         if (lane == 0) hnorm[row] = pos_inf();
-        return;
-    }
-    const float* p = c + row * ld;
-    float s = 0.f, lost = 0.f, lost2 = 0.f;
-    for (int t = lane * 4; t < d_pad; t += 128) {
-        const float4 v = ld_row4(p, t, d, vec, DT_F32);
-        s += sq4(v);
-        uint2 hi, lo;
-        bf16_split4(v, hi, lo, lost, lost2);
-        *reinterpret_cast<uint2*>(o + t) = lo;
-        *reinterpret_cast<uint2*>(o + d_pad + t) = hi;
-        *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = hi;
-    }
+    } else {
+        const float* p = c + row * ld;
+        for (int t = lane * 4; t < d_pad; t += 128) {
+            const float4 v = ld_row4(p, t, d, vec, DT_F32);
+            sq[0] += sq4(v);
+            uint2 hi, lo;
+            bf16_split4(v, hi, lo, sq[1], sq[2]);
+            *reinterpret_cast<uint2*>(o + t) = lo;
+            *reinterpret_cast<uint2*>(o + d_pad + t) = hi;
+            *reinterpret_cast<uint2*>(o + 2 * d_pad + t) = hi;
+        }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        s += __shfl_xor_sync(FULL_MASK, s, off);
-        lost += __shfl_xor_sync(FULL_MASK, lost, off);
-        lost2 += __shfl_xor_sync(FULL_MASK, lost2, off);
+        for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) sq[i] += __shfl_xor_sync(FULL_MASK, sq[i], off);
+        }
+        if (lane == 0) hnorm[row] = 0.5f * sq[0];
+        write_norm_columns(o + 3 * d_pad, sq[0], PLANE_AUG_COLS);
     }
-    if (lane == 0) {
-        hnorm[row] = 0.5f * s;
-        max_norm_update(norm_bits + NORM_ROW, s);
-        max_norm_update(norm_bits + NORM_LOST, lost);
-        max_norm_update(norm_bits + NORM_LOST2, lost2);
-    }
-    if (lane < PLANE_AUG_COLS) {
-        const float nh = -0.5f * s;
-        const __nv_bfloat16 h1 = __float2bfloat16_rn(nh);
-        const float r1 = nh - __bfloat162float(h1);
-        const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(h2);
-        const __nv_bfloat16 h3 = __float2bfloat16_rn(r2);
-        o[3 * d_pad + lane] = lane == 0 ? h1 : lane == 1 ? h2 : lane == 2 ? h3 : __float2bfloat16_rn(0.f);
-    }
+    block_norms_update(norm_bits, sq);
 }
 
 // Sample side of the second stage: the points listed in `rows` (live count on the device, at most
@@ -242,8 +228,8 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
 // lead of 2 eps where the exact re-scoring of assign_finalize_kernel needs eps; what the lead does
 // not decide goes to the `next` list (the second stage, whose bound is a hundred times smaller).
 __global__ void __launch_bounds__(256) assign_by_lead_kernel(
-    int64_t n, int K, int d, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float* __restrict__ xsq,
-    const float* __restrict__ xlost, float acc, const float* __restrict__ norms, int32_t* __restrict__ labels, int* __restrict__ next_count,
+    int64_t n, int K, int d, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float2* __restrict__ xsq,
+    float acc, const float* __restrict__ norms, int32_t* __restrict__ labels, int* __restrict__ next_count,
     int* __restrict__ next_list, int next_cap, int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap) {
     const int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pt >= n) return;
@@ -258,8 +244,8 @@ __global__ void __launch_bounds__(256) assign_by_lead_kernel(
     if (v0 && v1) second = fmaxf(second, first ? sc.z : sc.x);   // ... or the other half's best
     bool ok = v0 || v1;
     if (ok && second > -1e37f) {
-        const float q2 = __ldg(xsq + pt), l = __ldg(xlost + pt);
-        const float eps = score_eps(OPERANDS_BF16, q2, l * l, 0.f, norms, acc);
+        const float2 x2 = __ldg(xsq + pt);
+        const float q2 = x2.x, eps = score_eps(OPERANDS_BF16, q2, x2.y, 0.f, norms, acc);
         // the column index rides in the low mantissa bits of both scores: 2^-15 relative each
         const float lead = (best - fabsf(best) * 3.1e-5f) - (second + fabsf(second) * 3.1e-5f);
         ok = lead > 2.f * eps + proof_slack(q2, __ldg(norms + NORM_ROW), d);
@@ -453,7 +439,7 @@ using namespace fl;
 
 extern "C" int64_t fl_kmeans_xplane_bytes(int64_t n, int d) {
     if (n < 1 || d < 1) return 0;
-    // the bf16 rows, then ||x||^2 of every row and the norm of what rounding it took (f32 [2][n_pad])
+    // the bf16 rows, then ||x||^2 of every row and the square of the norm of what rounding took of it (f32 [n_pad][2])
     return round_up(round_up(n, 128) * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024) + round_up(n, 128) * 8;
 }
 
@@ -463,7 +449,7 @@ extern "C" int fl_kmeans_prepare_x_f32(const float* x, int64_t n, int d, int64_t
     if (xplane_bytes < fl_kmeans_xplane_bytes(n, d)) { set_error("fl_kmeans_prepare_x_f32: plane buffer too small"); return FL_EWORKSPACE; }
     const int64_t n_pad = round_up(n, 128);
     // the rows' norms (the scoring error bound of a point needs its own) come from the same read
-    float* xsq = reinterpret_cast<float*>(static_cast<char*>(xplane) + round_up(n_pad * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024));
+    float2* xsq = reinterpret_cast<float2*>(static_cast<char*>(xplane) + round_up(n_pad * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024));
     return launch_query_plane(x, n, ldx, d, xplane, n_pad, (int)round_up(d, 64), (cudaStream_t)stream, DT_F32, xsq);
 }
 
@@ -503,15 +489,15 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     }
     // sample plane (query side)
     const char* xpl = static_cast<const char*>(xplane);
-    const float* xsq;
+    const float2* xsq;
     if (!xpl) {
-        float* xs = reinterpret_cast<float*>(base + w.off_xsq);
+        float2* xs = reinterpret_cast<float2*>(base + w.off_xsq);
         rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs);
         if (rc != FL_OK) return rc;
         xpl = base + w.off_xplane;
         xsq = xs;
     } else {
-        xsq = reinterpret_cast<const float*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
+        xsq = reinterpret_cast<const float2*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
     }
     int* counters = reinterpret_cast<int*>(base + w.off_cnt);
     int* fb_count = counters;          // points for the exact path
@@ -548,7 +534,7 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
             // a second, far more precise stage follows: decide what the scores' lead decides
             // without touching the rows
             assign_by_lead_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(
-                n, K, d, asg_sc, asg_id, xsq, xsq + w.n_pad, acc1, norms, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap);
+                n, K, d, asg_sc, asg_id, xsq, acc1, norms, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap);
             FL_CHECK_LAUNCH();
             // ... then, for the undecided ones only, the exact distances to the two half-winners, which
             // need half the lead; what is still open goes to the second stage

@@ -46,24 +46,24 @@ __device__ __forceinline__ float2 query_plane_row(const void* p, bool live, int 
         if (live) {
             if (c < d) {
                 v = ld_row4(p, c, d, vec, dt);
-                sq += sq4(v);
-                lost += sq4(bf16_lost4(v));
             } else if (c == d_pad) {
                 v = make_float4(1.f, 1.f, 1.f, 0.f);
             }
         }
-        *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
+        const uint2 w = bf16x4_bits(v);
+        *reinterpret_cast<uint2*>(o + c) = w;
+        if (c < d) { sq += sq4(v); lost += sq4(bf16_lost4(v, w)); }
     }
     return make_float2(sq, lost);
 }
 
-// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row, and nq_pad words further the
-// norm of what its rounding took, from the same read.
+// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row and the square of the norm of what
+// its rounding took, from the same read.
 // Bound by HBM: 250 001 x 96 rows take 43 us (96 MB in, 72 MB out).  One thread per plane element and a second
 // pass over the rows for the norms took some 180.
 __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
                                                           __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt,
-                                                          float* __restrict__ sq_out) {
+                                                          float2* __restrict__ sq_out) {
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= nq_pad) return;
     const bool live = row < nq;
@@ -74,10 +74,7 @@ __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict
         s.x += __shfl_xor_sync(FULL_MASK, s.x, o);
         s.y += __shfl_xor_sync(FULL_MASK, s.y, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sq_out[row] = s.x;
-        sq_out[nq_pad + row] = sqrtf(s.y);
-    }
+    if ((threadIdx.x & 31) == 0) sq_out[row] = s;
 }
 
 // What a tensor-core call needs before its first scoring launch, in one pass: the bf16 query plane, the
@@ -99,7 +96,7 @@ __global__ void __launch_bounds__(256) knn_prep_kernel(const void* __restrict__ 
 }
 
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad, int d_pad,
-                       cudaStream_t st, int dt, float* sq_out) {
+                       cudaStream_t st, int dt, float2* sq_out) {
     query_plane_kernel<<<(unsigned)ceil_div(nq_pad, 8), 256, 0, st>>>(
         q, nq, ldq, d, dt_vec_ok(q, ldq, dt) && d % 4 == 0, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt, sq_out);
     FL_CHECK_LAUNCH();

@@ -254,9 +254,9 @@ int launch_split_query_gather(const float* x, int64_t ldx, int d, const int* row
                               float* tau_out, cudaStream_t st);
 
 // bf16 query plane [nq_pad][d_pad + 16] (features zero padded, ones in the norm columns) from fp32 queries;
-// sq_out (optional): f32 [2][nq_pad], ||q||^2 of every query and the norm of what its rounding took.
+// sq_out (optional): ||q||^2 of every query and the square of the norm of what its rounding took.
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad,
-                       int d_pad, cudaStream_t st, int dt = DT_F32, float* sq_out = nullptr);
+                       int d_pad, cudaStream_t st, int dt = DT_F32, float2* sq_out = nullptr);
 
 // Small helpers shared by the entry points.
 int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt = DT_F32);

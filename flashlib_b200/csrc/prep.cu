@@ -39,48 +39,37 @@ __global__ void rownorm_kernel(const float* __restrict__ x, int64_t n, int d, in
 // make the tensor-core product come out as <q,x> - ||x||^2/2.  Padding rows carry a huge
 // negative value there so they can never rank.
 // Rows of 16-bit storage (dt): bf16 values enter the plane as they are, fp16 values are rounded to
-// bf16 like fp32 ones; the norms are those of the stored values.  Four columns a lane: 16-byte reads where the
+// bf16 like fp32 ones; the norms are those of the stored values.  m_pad is a multiple of the block's rows.  Four columns a lane: 16-byte reads where the
 // rows allow them (vec) and 8-byte writes.
 __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d, int64_t ld,
                                    __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
                                    unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int dt, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= m_pad) return;
     const int pitch = d_pad + PLANE_AUG_COLS;
     __nv_bfloat16* o = rows + row * pitch;
+    float sq[2] = {0.f, 0.f};                   // NORM_ROW, NORM_LOST
     if (row >= m) {
         for (int c = lane; c < pitch; c += 32) o[c] = __float2bfloat16_rn(c == d_pad ? -3.0e38f : 0.f);
         if (lane == 0) hnorm[row] = pos_inf();
-        return;
-    }
-    const void* p = row_at(db, row, ld, dt);
-    float s = 0.f, lost = 0.f;
-    for (int c = lane * 4; c < d_pad; c += 128) {
-        const float4 v = ld_row4(p, c, d, vec, dt);
-        s += sq4(v);
-        lost += sq4(bf16_lost4(v));
-        *reinterpret_cast<uint2*>(o + c) = bf16x4_bits(v);
-    }
+    } else {
+        const void* p = row_at(db, row, ld, dt);
+        for (int c = lane * 4; c < d_pad; c += 128) {
+            const float4 v = ld_row4(p, c, d, vec, dt);
+            const uint2 w = bf16x4_bits(v);
+            sq[0] += sq4(v);
+            sq[1] += sq4(bf16_lost4(v, w));
+            *reinterpret_cast<uint2*>(o + c) = w;
+        }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        s += __shfl_xor_sync(FULL_MASK, s, off);
-        lost += __shfl_xor_sync(FULL_MASK, lost, off);
+        for (int off = 16; off > 0; off >>= 1) {
+            sq[0] += __shfl_xor_sync(FULL_MASK, sq[0], off);
+            sq[1] += __shfl_xor_sync(FULL_MASK, sq[1], off);
+        }
+        if (lane == 0) hnorm[row] = 0.5f * sq[0];
+        write_norm_columns(o + d_pad, sq[0], PLANE_AUG_COLS);
     }
-    if (lane == 0) {
-        hnorm[row] = 0.5f * s;
-        max_norm_update(norm_bits + NORM_ROW, s);
-        max_norm_update(norm_bits + NORM_LOST, lost);
-    }
-    if (lane < PLANE_AUG_COLS) {
-        const float nh = -0.5f * s;
-        const __nv_bfloat16 h1 = __float2bfloat16_rn(nh);
-        const float r1 = nh - __bfloat162float(h1);
-        const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(h2);
-        const __nv_bfloat16 h3 = __float2bfloat16_rn(r2);
-        o[d_pad + lane] = lane == 0 ? h1 : lane == 1 ? h2 : lane == 2 ? h3 : __float2bfloat16_rn(0.f);
-    }
+    block_norms_update(norm_bits, sq);
 }
 
 PlaneLayout plane_layout(int64_t m, int d) {
