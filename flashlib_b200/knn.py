@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import time
 import weakref
 from collections import OrderedDict, deque
 from typing import Optional
@@ -201,7 +202,8 @@ def clear_plane_cache() -> None:
 # there; reading them right after the call would serialise host and device once per call, so the
 # public entry points look at the words of EARLIER calls instead (and ``check_pending()`` looks at
 # all of them).  A slot is a few words of pinned host memory that the last kernel of a call fills in,
-# completion mark last: neither a copy nor an event enters the stream.
+# completion mark last: neither a copy nor an event enters the stream.  A call that is captured into a graph
+# takes none: every replay would write to the slot, whosever it is by then.
 class _StatusSlot:
     __slots__ = ("buf", "words", "ptr", "device")
 
@@ -235,11 +237,21 @@ def _finish_slot(slot: _StatusSlot, wait: bool) -> bool:
     if slot.words[_lib.FL_STATUS_WORDS] == 0:
         if not wait:
             return False
-        torch.cuda.synchronize(slot.device)
+        _await_mark(slot)
     st = list(slot.words)[:_lib.FL_STATUS_WORDS]
     _FREE_SLOTS.append(slot)
     _raise_on_status(st)
     return True
+
+
+def _await_mark(slot: _StatusSlot) -> None:
+    """Waits for this slot's own call and for nothing else on the device."""
+    look = time.monotonic() + 1.0
+    while slot.words[_lib.FL_STATUS_WORDS] == 0:
+        time.sleep(2e-5)
+        if time.monotonic() >= look:       # a device that has failed writes no mark: the query raises then
+            torch.cuda.current_stream(slot.device).query()
+            look += 1.0
 
 
 _STATUS_TEXT = {_lib.FL_ETIMEOUT: "a bounded device-side wait ran out",
@@ -271,6 +283,8 @@ def check_pending(block: bool = True) -> None:
 
 def _defer_status_check(status: torch.Tensor) -> None:
     """Queues the status words of a call that has just been launched on the current stream."""
+    if torch.cuda.is_current_stream_capturing():
+        return
     slot = _take_status_slot(status.device)
     _lib.check(_lib.load().fl_publish_status(status.data_ptr(), slot.ptr, _stream_ptr(status.device)))
     _PENDING_STATUS.append(slot)
@@ -307,7 +321,8 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
     ``(dist fp32 (nq,k), idx int32 (nq,k), info)``, in ``out = (dist, idx)`` when given.
     ``check_status=True`` reads the kernel's status words before returning (one host/device
     round trip; ``info["fallback_rows"]`` and ``info["stage2_rows"]`` are filled), ``"deferred"``
-    leaves that to a later call or to ``check_pending()``, ``False`` skips it.
+    leaves that to a later call or to ``check_pending()``, ``False`` skips it (so does ``"deferred"`` while
+    the stream is captured: nobody reads the words of a replay).
     ``second_stage`` (tensor-core mode): rows the bf16 proof rejects are scored again on the
     tensor cores with split hi/lo operands before anything takes the exact CUDA-core pass;
     ``None`` = when the database's split plane exists or is small enough to build."""
@@ -337,7 +352,9 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
     # (the kernels clear the status words themselves)
     status = torch.empty(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=dev) if nq else torch.zeros(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=dev)
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
-    slot = _take_status_slot(dev) if check_status == "deferred" and wants_plane and nq else None
+    slot = None
+    if check_status == "deferred" and wants_plane and nq and not torch.cuda.is_current_stream_capturing():
+        slot = _take_status_slot(dev)
     rc = lib.fl_knn_search(q.data_ptr(), nq, q.stride(0) if nq else d, db.data_ptr(), m, db.stride(0), d, k,
                            _DTYPE_CODES[db.dtype], passed, plane.ptr if plane is not None else None, split, row_offset,
                            out_d.data_ptr(), out_i.data_ptr(), ws.data_ptr(), ws_bytes, status.data_ptr(),
