@@ -36,6 +36,7 @@ SIGNATURES = {
     "fl_version": (c_int, []),
     "fl_last_error": (c_char_p, []),
     "fl_device_ok": (c_int, []),
+    "fl_stream_capture_id": (ctypes.c_ulonglong, [c_void_p]),
     "fl_launch_count": (ctypes.c_ulonglong, []),
     "fl_profile_enable": (c_int, [c_int]),
     "fl_profile_count": (c_int, []),

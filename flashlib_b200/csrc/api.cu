@@ -88,6 +88,13 @@ extern "C" int fl_device_ok(void) {
     return major == 10 ? 1 : 0;
 }
 
+extern "C" unsigned long long fl_stream_capture_id(void* stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 extern "C" unsigned long long fl_launch_count(void) { return __atomic_load_n(&fl::g_launches, __ATOMIC_RELAXED); }
 
 extern "C" int fl_profile_enable(int on) {

@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 from .kmeans import euclid_assign_triton, flash_kmeans
-from .knn import _as_f32_rows, _defer_status_check, _stream_ptr, knn_f32, row_sqnorm
+from .knn import _Built, _as_f32_rows, _defer_status_check, _stream_ptr, knn_f32, row_sqnorm
 
 
 @dataclass
@@ -39,6 +39,9 @@ class IvfFlatIndex:
     max_list_len: int = 0      # may be given as a 1-element device tensor: read back (one sync) on first use
     _hnorm: Optional[torch.Tensor] = field(default=None, repr=False, compare=False)
     _tc_plane: Optional[torch.Tensor] = field(default=None, repr=False, compare=False)
+    # where the two were filled: a search on another stream waits for that
+    _hnorm_built: Optional[_Built] = field(default=None, repr=False, compare=False)
+    _tc_built: Optional[_Built] = field(default=None, repr=False, compare=False)
     _last_status: Optional[torch.Tensor] = field(default=None, repr=False, compare=False)
 
     @property
@@ -58,8 +61,13 @@ class IvfFlatIndex:
 
     def half_norms(self) -> torch.Tensor:
         """fp32 ``||row||^2 / 2`` of the stored rows, computed once per index."""
-        if self._hnorm is None or self._hnorm.device != self.data.device:
-            self._hnorm = row_sqnorm(self.data).mul_(0.5)
+        built = self._hnorm_built
+        if self._hnorm is None or self._hnorm.device != self.data.device or (built is not None and not built.usable()):
+            hnorm = row_sqnorm(self.data).mul_(0.5)
+            self._hnorm_built = _Built(self.data.device)
+            self._hnorm = hnorm
+        elif built is not None:
+            built.join(self._hnorm)
         return self._hnorm
 
 
@@ -185,7 +193,10 @@ def index_from_centroids(Xp: torch.Tensor, centroids: torch.Tensor, *, D: int, n
 
 def _tc_plane(index: IvfFlatIndex, data: torch.Tensor, offs: torch.Tensor) -> torch.Tensor:
     """bf16 operand plane of the stored rows for the tensor-core fine scan, built on first use."""
-    if index._tc_plane is None or index._tc_plane.device != data.device:
+    built = index._tc_built
+    if index._tc_plane is not None and index._tc_plane.device == data.device and built is not None and built.usable():
+        built.join(index._tc_plane)
+    else:
         lib = _lib.load()
         m, d = data.shape
         nbytes = lib.fl_ivf_plane_bytes(m, index.nlist, d)
@@ -193,6 +204,7 @@ def _tc_plane(index: IvfFlatIndex, data: torch.Tensor, offs: torch.Tensor) -> to
         with torch.cuda.device(data.device):
             _lib.check(lib.fl_ivf_prepare_f32(data.data_ptr(), m, data.stride(0), d, offs.data_ptr(), index.nlist,
                                               buf.data_ptr(), nbytes, _stream_ptr(data.device)))
+            index._tc_built = _Built(data.device)
         index._tc_plane = buf
     return index._tc_plane
 

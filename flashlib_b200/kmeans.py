@@ -15,10 +15,10 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .knn import _as_f32_rows, _defer_status_check, _evict_when_freed, _stream_ptr
+from .knn import _Built, _as_f32_rows, _defer_status_check, _evict_when_freed, _keep_for_graph, _stream_ptr
 
 
-_XPLANE_CACHE = {}
+_XPLANE_CACHE = {}         # key -> (plane, where it was filled)
 
 
 def _x_plane(x: torch.Tensor) -> torch.Tensor:
@@ -27,8 +27,10 @@ def _x_plane(x: torch.Tensor) -> torch.Tensor:
     ``flashlib/primitives/knn/triton/_row_norm.py:82-93``)."""
     key = (x.data_ptr(), tuple(x.shape), x.stride(0), x._version, x.device.index)
     hit = _XPLANE_CACHE.get(key)
-    if hit is not None:
-        return hit
+    if hit is not None and hit[1].usable():
+        hit[1].join(hit[0])
+        _keep_for_graph(key, hit, x)
+        return hit[0]
     lib = _lib.load()
     n, d = x.shape
     nbytes = lib.fl_kmeans_xplane_bytes(n, d)
@@ -36,9 +38,10 @@ def _x_plane(x: torch.Tensor) -> torch.Tensor:
     _lib.check(lib.fl_kmeans_prepare_x_f32(x.data_ptr(), n, d, x.stride(0), buf.data_ptr(), nbytes,
                                            _stream_ptr(x.device)))
     if len(_XPLANE_CACHE) >= 2:
-        _XPLANE_CACHE.pop(next(iter(_XPLANE_CACHE)))
-    _XPLANE_CACHE[key] = buf
+        _XPLANE_CACHE.pop(next(iter(_XPLANE_CACHE)), None)
+    entry = _XPLANE_CACHE[key] = (buf, _Built(x.device))
     _evict_when_freed(_XPLANE_CACHE, key, x)
+    _keep_for_graph(key, entry, x)
     return buf
 
 

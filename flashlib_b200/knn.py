@@ -52,6 +52,57 @@ class _OnDevice:
             self._ctx.__exit__(*exc)
 
 
+def _capture_id(device: torch.device) -> int:
+    """Number of the graph capture the current stream takes part in (0: none)."""
+    return _lib.load().fl_stream_capture_id(_stream_ptr(device)) if torch.cuda.is_current_stream_capturing() else 0
+
+
+def _nothing():
+    return None
+
+
+class _Built:
+    """Where a kept buffer was filled.  Work on another stream is not ordered behind that: ``join`` makes the current
+    stream wait for it and tells the allocator that this stream reads the buffer, which may leave its cache
+    meanwhile.  A buffer filled under capture holds nothing until the graph runs, and only that graph may use it."""
+
+    __slots__ = ("device", "stream", "capture", "event")
+
+    def __init__(self, device: torch.device):
+        self.device = device
+        self.stream = _stream_ptr(device)
+        self.capture = _capture_id(device)
+        self.event = torch.cuda.Event()
+        self.event.record(torch.cuda.current_stream(device))
+
+    def __reduce__(self):
+        return _nothing, ()            # a copy of an index or its pickle carries no event
+
+    def usable(self) -> bool:
+        return self.capture == 0 or self.capture == _capture_id(self.device)
+
+    def join(self, buf: torch.Tensor) -> None:
+        if _stream_ptr(self.device) == self.stream:
+            return
+        if _capture_id(self.device) != self.capture:
+            return           # a capture may not wait for work outside it; torch.cuda.graph waits for the device first
+        cur = torch.cuda.current_stream(self.device)
+        cur.wait_event(self.event)
+        buf.record_stream(cur)
+
+
+# Entries that a graph was captured with: their addresses are in it, so they stay although their cache
+# drops them, until the rows they stand for are freed.
+_IN_GRAPHS: dict = {}
+
+
+def _keep_for_graph(key, entry, t: torch.Tensor) -> None:
+    if torch.cuda.is_current_stream_capturing() and _IN_GRAPHS.get(key) is not entry:
+        if key not in _IN_GRAPHS:
+            _evict_when_freed(_IN_GRAPHS, key, t)
+        _IN_GRAPHS[key] = entry
+
+
 def _as_f32_rows(t: torch.Tensor) -> torch.Tensor:
     """fp32 tensor whose last dimension is contiguous (rows may be strided)."""
     if t.dtype != torch.float32:
@@ -91,7 +142,7 @@ def storage_dtype_for(tol: Optional[float]):
     return max(ok, key=lambda v: v[2])[3]
 
 
-_CAST_CACHE: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
+_CAST_CACHE: "OrderedDict[tuple, tuple]" = OrderedDict()       # key -> (16-bit rows, where they were written)
 
 
 def _cast_rows_cached(c: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -99,12 +150,16 @@ def _cast_rows_cached(c: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     and its operand plane is found again on the next call."""
     key = _plane_key(c) + (dtype,)
     hit = _CAST_CACHE.get(key)
-    if hit is not None:
+    if hit is not None and hit[1].usable():
+        _CAST_CACHE[key] = hit
         _CAST_CACHE.move_to_end(key)
-        return hit
+        hit[1].join(hit[0])
+        _keep_for_graph(key, hit, c)
+        return hit[0]
     out = c.to(dtype)
-    _CAST_CACHE[key] = out
+    entry = _CAST_CACHE[key] = (out, _Built(c.device))
     _evict_when_freed(_CAST_CACHE, key, c)
+    _keep_for_graph(key, entry, c)
     while len(_CAST_CACHE) > _PLANE_CACHE_SIZE:
         _CAST_CACHE.popitem(last=False)
     return out
@@ -133,26 +188,35 @@ class DbPlane:
         _lib.check(lib.fl_knn_prepare_db_rows(db.data_ptr(), _DTYPE_CODES[db.dtype], m, d, db.stride(0),
                                               self.buf.data_ptr(), nbytes, _stream_ptr(db.device)))
         self.key = _plane_key(db)
-        self.split_buf = None
+        self.built = _Built(db.device)
+        self.split = None              # (buffer, where it was filled); False: none for this database
 
     @property
     def ptr(self) -> int:
+        """Address of the plane, for a call on the current stream."""
+        self.built.join(self.buf)
         return self.buf.data_ptr()
 
     def split_ptr(self, db: torch.Tensor):
         """Address of the split (hi/lo bf16) plane of the same database, built on first use; ``None``
         when the shape has none (d > 128) or it would exceed the size limit."""
-        if self.split_buf is None:
+        split = self.split
+        if split is None or (split is not False and not split[1].usable()):
             lib = _lib.load()
             m, d = db.shape
             nbytes = lib.fl_knn_split_plane_bytes(m, d) if db.dtype == torch.float32 else 0
             if nbytes == 0 or nbytes > _split_plane_limit():
-                self.split_buf = False
+                split = False
             else:
-                self.split_buf = torch.empty(nbytes, dtype=torch.uint8, device=db.device)
-                _lib.check(lib.fl_knn_prepare_split_f32(db.data_ptr(), m, d, db.stride(0), self.split_buf.data_ptr(),
+                buf = torch.empty(nbytes, dtype=torch.uint8, device=db.device)
+                _lib.check(lib.fl_knn_prepare_split_f32(db.data_ptr(), m, d, db.stride(0), buf.data_ptr(),
                                                         nbytes, _stream_ptr(db.device)))
-        return self.split_buf.data_ptr() if self.split_buf is not False else None
+                split = (buf, _Built(db.device))
+            self.split = split             # (only now: another thread must not meet a plane nobody has enqueued yet)
+        if split is False:
+            return None
+        split[1].join(split[0])
+        return split[0].data_ptr()
 
 
 def _split_plane_limit() -> int:
@@ -183,12 +247,15 @@ _PLANE_CACHE_SIZE = 4
 def get_plane(db: torch.Tensor) -> DbPlane:
     key = _plane_key(db)
     hit = _PLANE_CACHE.get(key)
-    if hit is not None:
+    if hit is not None and hit.built.usable():
+        _PLANE_CACHE[key] = hit            # (another thread may have dropped it since)
         _PLANE_CACHE.move_to_end(key)
+        _keep_for_graph(key, hit, db)
         return hit
     plane = DbPlane(db)
     _PLANE_CACHE[key] = plane
     _evict_when_freed(_PLANE_CACHE, key, db)
+    _keep_for_graph(key, plane, db)
     while len(_PLANE_CACHE) > _PLANE_CACHE_SIZE:
         _PLANE_CACHE.popitem(last=False)
     return plane

@@ -94,6 +94,7 @@ class DeviceKnnKernels:
         from . import _lib
         lib = _lib.load()
         off = lib.fl_knn_plane_maxnorm_offset(db.shape[0], db.shape[1])
+        plane.built.join(plane.buf)
         return plane.buf[off:off + 4 * self.norm_words].view(torch.float32).clone()
 
     @property

@@ -60,6 +60,8 @@ const char* fl_last_error(void);
 
 /* 1 when the running process can see an sm_100 device, 0 otherwise (never fails). */
 int         fl_device_ok(void);
+/* Number of the graph capture that `stream` takes part in, 0 when it is not being captured. */
+unsigned long long fl_stream_capture_id(void* stream);
 
 /* Measurement hooks; they have no counterpart in the reference (it times from Python,   */
 /* knn/triton/_common.py:32-44).  fl_launch_count: kernels launched by this library since */
