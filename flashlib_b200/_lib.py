@@ -10,6 +10,8 @@ import ctypes
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_void_p
 from pathlib import Path
 
+import torch
+
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libflashlib_b200.so"
 
 FL_OK = 0
@@ -177,15 +179,17 @@ def check(rc: int, what: str = "") -> None:
     raise FlashlibError(msg)
 
 
-_device_ok = False
+_devices_ok: set = set()       # devices found to be sm_100 (a process may see others beside them)
 
 
 def require_device() -> None:
-    """Raise unless an sm_100 device is visible; there is nothing to fall back to."""
-    global _device_ok
-    if _device_ok:
+    """Raise unless the current device is an sm_100 one; there is nothing to fall back to."""
+    dev = torch.cuda.current_device() if torch.cuda.is_initialized() else None
+    if dev in _devices_ok:
         return
-    _device_ok = bool(load().fl_device_ok())
-    if not _device_ok:
+    ok = bool(load().fl_device_ok())
+    if ok and dev is not None:
+        _devices_ok.add(dev)
+    if not ok:
         raise RuntimeError("flashlib_b200 needs an NVIDIA B200 (sm_100) device; "
                            "no CPU or other-GPU fallback exists")

@@ -357,13 +357,13 @@ def _defer_status_check(status: torch.Tensor) -> None:
     _PENDING_STATUS.append(slot)
 
 
-# Which kernel a shape takes and the workspace it needs: asked from the library once per shape.
+# Which kernel a shape takes and the workspace it needs: asked from the library once per device and shape.
 _PLANS: dict = {}
 
 
-def _knn_plan(lib, nq: int, m: int, d: int, k: int, mode: int):
+def _knn_plan(lib, dev: Optional[int], nq: int, m: int, d: int, k: int, mode: int):
     """``(resolved mode, mode to pass on, wants an operand plane, workspace bytes, staged workspace bytes)``."""
-    key = (nq, m, d, k, mode)
+    key = (dev, nq, m, d, k, mode)
     hit = _PLANS.get(key)
     if hit is not None:
         return hit
@@ -400,7 +400,7 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
     dev = q.device
     if q.dtype != db.dtype or db.dtype not in _DTYPE_CODES:
         raise TypeError(f"knn_f32 takes q and db of one dtype out of fp32 / bf16 / fp16, got {q.dtype} and {db.dtype}")
-    resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, nq, m, d, k, mode)
+    resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, dev.index, nq, m, d, k, mode)
     if wants_plane and plane is None:
         plane = get_plane(db)
     if out is not None:

@@ -152,3 +152,43 @@ def test_batch_kernel_by_walk_and_blocks(B, nq, m, d, k, clouds):
     lib = _lib.load()
     assert (lib.fl_knn_batch_workspace_bytes(B, nq, m, d, k) == 1024) == clouds
     assert lib.fl_knn_batch_route(B, nq, m, d, k) == 1 or nq * m >= 1 << 24
+
+
+def test_every_device_is_looked_at(monkeypatch):
+    """One sm_100 device found does not vouch for the others, and a plan is the device's own."""
+    current, asked = [0], []
+
+    class Lib:
+        def fl_device_ok(self):
+            asked.append(current[0])
+            return 1 if current[0] == 0 else 0
+
+    monkeypatch.setattr(_lib, "load", lambda: Lib())
+    monkeypatch.setattr(_lib, "_devices_ok", set())
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    _lib.require_device()
+    _lib.require_device()
+    assert asked == [0]
+    current[0] = 1
+    with pytest.raises(RuntimeError):
+        _lib.require_device()
+
+
+def test_search_plans_are_kept_by_device(monkeypatch):
+    from flashlib_b200 import knn as knn_mod
+    monkeypatch.setattr(knn_mod, "_PLANS", {})
+    sizes = iter((1_000, 2_000))
+
+    class Lib:
+        def fl_knn_resolve_mode(self, *a):
+            return _lib.FL_KNN_EXACT_SIMT
+
+        def fl_knn_wants_plane(self, *a):
+            return 0
+
+        def fl_knn_workspace_bytes(self, *a):
+            return next(sizes)
+
+    got = [knn_mod._knn_plan(Lib(), dev, 10, 1_000, 64, 5, _lib.FL_KNN_AUTO)[3] for dev in (0, 1, 0, 1)]
+    assert got == [1_000, 2_000, 1_000, 2_000]
