@@ -3,6 +3,7 @@
 // kernel and merges each query's per-probe pools with an exact fp32 re-rank.
 #include "knn_internal.h"
 #include "pool.cuh"
+#include <math.h>
 
 namespace fl {
 
@@ -86,8 +87,38 @@ __global__ void ivf_halfnorm_kernel(const float* __restrict__ x, int64_t n, int 
     if (lane == 0) out[row] = 0.5f * s;
 }
 
-// Up to this many (query, probe) pairs the few-query scan takes the fine scan: every pair reads its list.
+// Up to this many (query, probe) pairs the few-query scan may take the fine scan: every pair reads its list.
 constexpr int64_t IVF_DIRECT_PAIRS = 8192;
+
+// Estimated us of the fine scan by the few-query scan (a block per pair, or several with its share of the list) and by
+// the grouped one (an item per list and 64 of its pairs), fitted to 1 000 shapes (64 to 8 192 pairs, lists of 780
+// to 15 600 rows, 32 to 256 features, k = 10 to 100).  The first grows with the pairs, and faster with k: what passes
+// a block's first threshold, k of 256 rows, no longer fits one sort.  The second walks each list once per 64 pairs.
+static double ivf_direct_estimate_us(int64_t pairs, int nlist, int64_t m, int d, int k) {
+    const int chunks = direct_ivf_chunks(pairs);
+    const double rows = (double)m / nlist / chunks, blocks = (double)pairs * chunks, slots = 2.0 * sm_count();
+    const double waves = blocks < 8 * slots ? (double)ceil_div((int64_t)blocks, (int64_t)slots) : blocks / slots;
+    const bool hbm = (double)m * d * 4 > 1.2e8;            // the rows do not stay in the L2
+    const double full = (k * rows / (k <= 32 ? 16384.0 : 65536.0) - 0.65) / 0.6;
+    const double over = full < 0 ? 0 : full > 1 ? 1 : full;
+    const double block = k <= 32 ? 7.5 + rows * (3e-3 + (hbm ? 1.2e-4 : 6e-5) * d) + 16 * over
+                                 : (rows < 500 ? 14 : 18) + rows * (7.5e-3 + (hbm ? 1.9e-4 : 8e-5) * d) + 165 * over;
+    return 20 + waves * block;
+}
+static double ivf_grouped_estimate_us(int64_t pairs, int nprobe, int nlist, int64_t m, int d, int k) {
+    const double walk = (double)m / nlist * (0.042 + 5.6e-4 * d) * (k <= 32 ? 1.0 : 1.05);
+    const double hit = nlist * (1.0 - pow(1.0 - 1.0 / nlist, (double)pairs)), share = (double)pairs / nlist / 64;
+    const double many = share > 1 ? pow(share, 0.85) : 1.0, wide = hit / sm_count();
+    return (k <= 32 ? 75 : 105) + pairs * (0.012 + 1.5e-4 * k) + nprobe * (0.8 + 0.01 * k) + walk * (many > wide ? many : wide);
+}
+// Measured, few-query scan against grouped: 16 x 16 of 1 024 lists, 1M x 128, k = 10: 65 and 281 us; 125 x 16, k = 50: 652
+// and 808; 500 x 16, k = 50: 1 783 and 1 140; 170 x 48 of 64 lists, k = 50: 13 500 and 3 800; 2 000 x 4 of 128 lists,
+// 100 000 x 64, k = 20: 616 and 308.
+static bool ivf_direct_pick(int64_t nq, int nprobe, int nlist, int64_t m, int d, int k) {
+    const int64_t pairs = nq * nprobe;
+    return pairs <= IVF_DIRECT_PAIRS && direct_supported(nq, m, d, k) &&
+           ivf_direct_estimate_us(pairs, nlist, m, d, k) <= ivf_grouped_estimate_us(pairs, nprobe, nlist, m, d, k);
+}
 
 struct IvfWs {
     int K1, bq;
@@ -343,7 +374,7 @@ extern "C" int fl_ivf_fine_scan_f32(const float* q, int64_t nq, int64_t ldq, con
     float* part_sc = reinterpret_cast<float*>(base + w.off_part_sc);
     uint32_t* part_id = reinterpret_cast<uint32_t*>(base + w.off_part_id);
     const int64_t npairs = nq * nprobe;
-    if (npairs <= IVF_DIRECT_PAIRS && direct_supported(nq, m, d, k)) {
+    if (ivf_direct_pick(nq, nprobe, nlist, m, d, k)) {
         DirectParams dp{};
         dp.dt = DT_F32; dp.q = q; dp.ldq = ldq; dp.nq = nq; dp.db = data; dp.m = m; dp.ldb = ldd; dp.d = d;
         dp.vec = dt_vec_ok(q, ldq, DT_F32) && dt_vec_ok(data, ldd, DT_F32) && d % 4 == 0;

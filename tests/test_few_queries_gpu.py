@@ -117,3 +117,27 @@ def test_deferred_status_of_many_calls():
     assert len(knn_mod._PENDING_STATUS) <= 64
     fl.check_pending()
     assert len(knn_mod._PENDING_STATUS) == 0
+
+
+# few pairs: two launches, a block per pair; many that share their lists: grouped by list (lists of 1 562 rows)
+@pytest.mark.parametrize("nq,nprobe,k,few", [(8, 4, 10, True), (4, 16, 50, True), (400, 16, 50, False), (120, 60, 10, False),
+                                             (500, 16, 100, False)])
+def test_inverted_list_scan_by_pairs_and_sharing(nq, nprobe, k, few):
+    g = torch.Generator().manual_seed(nq)
+    X = torch.randn(100_000, 32, generator=g).cuda()
+    Q = torch.randn(nq, 32, generator=g).cuda()
+    from flashlib_b200.ivf_flat import index_from_centroids
+    index = index_from_centroids(X, X[:64].clone(), D=32, nprobe=nprobe)
+    probed = torch.rand(nq, 64, generator=g).argsort(1)[:, :nprobe].int().cuda()
+    index.half_norms()
+    before = _lib.load().fl_launch_count()
+    vals, pos = ivf_fine_scan(Q, index, probed, k, mode="exact")
+    assert (_lib.load().fl_launch_count() - before == 2) == few
+    offs = index.list_offsets.cpu()
+    for qi in range(0, nq, max(1, nq // 8)):
+        rows = torch.cat([torch.arange(offs[c], offs[c + 1]) for c in probed[qi].tolist()])
+        d64 = ((index.data[rows.cuda()].double() - Q[qi].double()) ** 2).sum(-1)
+        ref = rows[d64.topk(k, largest=False).indices.cpu()]
+        res = parity.knn_parity(Q[qi:qi + 1].cpu().numpy(), index.data.cpu().numpy(), vals[qi:qi + 1].cpu().numpy(),
+                                pos[qi:qi + 1].cpu().numpy(), ref[None].numpy())
+        assert res["ok"], (qi, res)
