@@ -290,7 +290,7 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.off_part_sc = take(cur, nq * w.nsplit * (int64_t)w.K1 * 4);
         w.off_part_id = take(cur, nq * w.nsplit * (int64_t)w.K1 * 4);
         w.off_cnt = take(cur, 1024);
-        if (direct_pick(nq, m, d, k)) {
+        if (direct_possible(nq, m, d, k)) {                 // (the element type decides at the call)
             const int64_t direct = direct_workspace_bytes(nq, m, d, k);
             if (direct > cur) cur = direct;
         }
@@ -636,7 +636,7 @@ static int knn_rows_impl(const char* who, const void* q, int64_t nq, int64_t ldq
     const int vecq = dt_vec_ok(q, ldq, dt);
     const int vecd = dt_vec_ok(db, ldb, dt);
     const int vec = vecq && vecd && (d % 4 == 0);
-    if (direct_pick(nq, m, d, k)) {
+    if (direct_pick(nq, m, d, k, dt, direct_wide(db, ldb, d, dt))) {
         DirectParams dp{};
         dp.dt = dt; dp.q = q; dp.ldq = ldq; dp.nq = nq;
         dp.db = db; dp.m = m; dp.ldb = ldb; dp.d = d; dp.vec = vec;

@@ -9,6 +9,7 @@
 // 64, and its row ranges stop at 64 blocks.
 #include "knn_internal.h"
 #include "pool.cuh"
+#include <math.h>
 
 namespace fl {
 
@@ -529,10 +530,55 @@ double direct_estimate_us(int64_t nq, int64_t m, int d) {
     return 14.0 + (double)ceil_div(nq, DIR_MAX_QUERIES) * (double)m * row;
 }
 
-// 1: the exact mode takes this scan.  Up to 512 queries it beats the tile kernel at every measured size
-// (1 x 1M x 128: 132 against 1 844 us, 300 x 20 000 x 64: 147 against 322); at 1 000 x 100 000 x 128 the
-// two meet (2 033 and 1 795).
-int direct_pick(int64_t nq, int64_t m, int d, int k) { return nq <= 512 && direct_supported(nq, m, d, k); }
+int direct_possible(int64_t nq, int64_t m, int d, int k) { return nq <= 512 && direct_supported(nq, m, d, k); }
+
+int direct_wide(const void* db, int64_t ldb, int d, int dt) {
+    const int v = dt == DT_F32 ? 4 : 8;
+    return d % v == 0 && ldb % v == 0 && (reinterpret_cast<uintptr_t>(db) & 15) == 0;
+}
+
+// Estimated us of this scan and of the tile kernel (knn_simt.cu) for one element type, fitted to 1 260 shapes (1 to 512
+// queries, 1 000 to 200 000 rows, 16 to 1 024 features, k = 10, 40 and 100, fp32 and bf16).  Here four queries
+// share a read, features are padded to the stretch of eight lanes, rows that 16-byte reads do not fit cost twice
+// (fp32) to five times (16 bits) as much, and from k = 33 on a range's pool is sorted several times.  The tile kernel takes
+// 64 queries at once in up to 64 row ranges: a walk over the tiles of one range, or all tiles over the SMs.
+static double direct_scan_us(int64_t nq, int64_t m, int d, int k, int dt, int wide) {
+    const bool f32 = dt == DT_F32;
+    double row;
+    if (f32) row = 1.6e-5 + (wide ? 5.5e-7 * (double)round_up(d, 32) * (d > 512 ? 1.15 : 1.0) : (d <= 64 ? 6.5e-7 : 1e-6) * (double)round_up(d, 8));
+    else if (wide) row = 1.5e-5 + 7.2e-7 * (double)round_up(d, 64) * (d > 512 ? 1.5 : 1.0);
+    else row = 4e-6 * d - 3e-5 > 6e-5 ? 4e-6 * d - 3e-5 : 6e-5;
+    const double groups = (double)ceil_div(nq, DIR_MAX_QUERIES);
+    double ranges = 2.0 * sm_count() / groups;
+    if (ranges > m / 256.0) ranges = m / 256.0;
+    if (ranges < 1) ranges = 1;
+    const double least = 256.0 * sm_count(), rows = groups * (double)m;
+    double t = 18 + (rows > least ? rows : least) * row + 0.04 * (double)nq;
+    if (k > 32) t += 4.6 * pow(k / 100.0, 0.6) * pow((double)m / ranges, 0.52) * (nq > 8 ? 1.0 : 0.9) * (f32 || nq < 32 ? 1.0 : 1.5);
+    return t;
+}
+static double tile_scan_us(int64_t nq, int64_t m, int d, int k, int dt) {
+    const int c = k <= 24 ? 0 : k <= 56 ? 1 : 2;           // pools of 32, 64, 128 entries
+    const double alone[3] = {112, 160, 243}, shared[3] = {88, 100, 175}, walk[3] = {0, 4, 12}, work[3] = {0, 2, 9.7};
+    const double sms = sm_count(), groups = (double)ceil_div(nq, 64), tiles = (double)ceil_div(m, 128);
+    double ranges = (double)ceil_div(2 * (int64_t)sms, (int64_t)groups);
+    if (ranges > tiles / 4) ranges = tiles / 4;
+    if (ranges > 64) ranges = 64;
+    if (ranges < 1) ranges = 1;
+    const double dp = (double)round_up(d, 32) * (dt == DT_F32 || d <= 128 ? 1.0 : 1.65);
+    const double blocks = groups * ranges, per = tiles / ranges;
+    const double one = ceil(per) * (14 + 0.089 * dp + walk[c]);
+    if (blocks <= sms) return alone[c] + one * (nq < 8 ? 0.85 : 1.0);
+    const double both = (blocks <= 2 * sms ? 2 * per : tiles * groups / sms) * (8 + 0.08 * dp + work[c]);
+    const double second = blocks >= 2 * sms ? 1.0 : (blocks - sms) / sms;
+    return alone[c] + shared[c] * second + (one > both ? one : both);
+}
+// 1: the exact mode takes this scan.  Measured, this and the tile kernel: 1 x 1M x 128: 132 and 1 844 us; 300 x 20 000 x 64:
+// 147 and 322; 512 x 200 000 x 128: 2 329 and 1 687; 256 x 20 000 x 64, k = 100: 664 and 408; 512 x 20 000 x 100 in
+// bf16 (no 16-byte reads): 936 and 405; 512 x 200 000 x 333 in bf16: 38 600 and 6 350.
+int direct_pick(int64_t nq, int64_t m, int d, int k, int dt, int wide) {
+    return direct_possible(nq, m, d, k) && direct_scan_us(nq, m, d, k, dt, wide) <= tile_scan_us(nq, m, d, k, dt);
+}
 
 int64_t direct_workspace_bytes(int64_t nq, int64_t m, int d, int k) {
     int nqb, nchunk;
@@ -581,14 +627,12 @@ static int dir_launch(DirectParams& p, int nqb, int64_t grid, void* ws, cudaStre
     p.part_key = static_cast<float*>(ws);
     p.part_id = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + round_up(nlists * p.k * 4, 1024));
     FL_CHECK_ARG(grid < (1ll << 31) && p.nq < (1ll << 31), "few-query scan: too many blocks");
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p.db);
+    const int wide = direct_wide(p.db, p.ldb, p.d, p.dt);
     int rc;
     if (p.dt == DT_F32)
-        rc = (p.d % 4 == 0 && p.ldb % 4 == 0 && (a & 15) == 0) ? dir_launch_nq<true, 4>(p, nqb, (unsigned)grid, st)
-                                                               : dir_launch_nq<true, 1>(p, nqb, (unsigned)grid, st);
+        rc = wide ? dir_launch_nq<true, 4>(p, nqb, (unsigned)grid, st) : dir_launch_nq<true, 1>(p, nqb, (unsigned)grid, st);
     else
-        rc = (p.d % 8 == 0 && p.ldb % 8 == 0 && (a & 15) == 0) ? dir_launch_nq<false, 8>(p, nqb, (unsigned)grid, st)
-                                                               : dir_launch_nq<false, 1>(p, nqb, (unsigned)grid, st);
+        rc = wide ? dir_launch_nq<false, 8>(p, nqb, (unsigned)grid, st) : dir_launch_nq<false, 1>(p, nqb, (unsigned)grid, st);
     if (rc != FL_OK) return rc;
     const int mn = pow2_ceil((p.k + 31) / 32);
     switch (mn) {

@@ -85,7 +85,9 @@ struct DirectParams {
     float* part_key; uint32_t* part_id;
 };
 int direct_supported(int64_t nq, int64_t m, int d, int k);
-int direct_pick(int64_t nq, int64_t m, int d, int k);      // 1: the exact mode takes this scan for the shape
+int direct_possible(int64_t nq, int64_t m, int d, int k);  // 1: the exact mode may take this scan
+int direct_wide(const void* db, int64_t ldb, int d, int dt);                    // 1: 16-byte reads fit the rows
+int direct_pick(int64_t nq, int64_t m, int d, int k, int dt, int wide);         // 1: it does, for rows of this type
 double direct_estimate_us(int64_t nq, int64_t m, int d);
 int64_t direct_workspace_bytes(int64_t nq, int64_t m, int d, int k);
 int launch_knn_direct(DirectParams p, void* ws, cudaStream_t st);

@@ -1134,7 +1134,7 @@ int tc_knn_supported(int64_t nq, int64_t m, int d, int k) {
 int tc_wide_supported(int64_t nq, int64_t m, int d, int k) {
     if (d <= 512 || d > 8192 || nq < 1 || k > 112) return 0;
     if (m < 512 || round_up(m, 256) / 256 > (1 << 23)) return 0;
-    if (!direct_pick(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
+    if (!direct_possible(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
     return direct_estimate_us(nq, m, d) > 60.0 + (double)m * (double)(round_up(d, 64) + PLANE_AUG_COLS) * 2.0 / 5.5e6;
 }
 
@@ -1143,7 +1143,7 @@ int tc_wide_supported(int64_t nq, int64_t m, int d, int k) {
 // queries has two launches and reads the stored rows once per four queries.
 int tc_knn_auto(int64_t nq, int64_t m, int d, int k) {
     if (tc_knn_supported(nq, m, d, k) != FL_OK || m < 512) return 0;
-    if (!direct_pick(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
+    if (!direct_possible(nq, m, d, k)) return nq * m >= (int64_t(1) << 20);
     const double tc = 60.0 + (double)m * (double)(round_up(d, 64) + PLANE_AUG_COLS) * 2.0 / 5.5e6;
     return direct_estimate_us(nq, m, d) > tc;
 }

@@ -141,3 +141,17 @@ def test_inverted_list_scan_by_pairs_and_sharing(nq, nprobe, k, few):
         res = parity.knn_parity(Q[qi:qi + 1].cpu().numpy(), index.data.cpu().numpy(), vals[qi:qi + 1].cpu().numpy(),
                                 pos[qi:qi + 1].cpu().numpy(), ref[None].numpy())
         assert res["ok"], (qi, res)
+
+
+# sizes on both sides of the rule: two launches are the scan, the tile kernel takes more
+@pytest.mark.parametrize("nq,m,d,k,dtype,few", [(300, 20_000, 64, 10, torch.float32, True), (512, 60_000, 1024, 10, torch.float32, False),
+                                                (256, 20_000, 64, 100, torch.float32, False), (32, 20_000, 64, 100, torch.float32, True),
+                                                (512, 20_000, 100, 10, torch.bfloat16, False), (512, 20_000, 128, 10, torch.bfloat16, True),
+                                                (8, 20_000, 333, 10, torch.float16, True)])
+def test_exact_mode_by_queries_k_and_row_reads(nq, m, d, k, dtype, few):
+    g = torch.Generator().manual_seed(nq + d)
+    db, q = torch.randn(m, d, generator=g).to(dtype).cuda(), torch.randn(nq, d, generator=g).to(dtype).cuda()
+    before = _lib.load().fl_launch_count()
+    d_, i_, _ = knn_f32(q, db, k, mode=_lib.FL_KNN_EXACT_SIMT)
+    assert (_lib.load().fl_launch_count() - before == 2) == few
+    _check(q, db, k, d_, i_)
