@@ -109,3 +109,26 @@ def test_tensor_core_assignment_of_unprovable_points(n, d, K, dup):
     x[0, 7, 0] = float("nan")
     lab = fl.euclid_assign_triton(x, c, mode="bf16")
     _check_labels(x[:, 8:], c, lab[:, 8:])
+
+
+# clusters around the number of labels a warp folds (16); rows in the order of their clusters, in runs that
+# end inside a warp, or in none; features that fill their block or not, staged rows (d > 16) among them
+@pytest.mark.parametrize("order", ["sorted", "runs", "random"])
+@pytest.mark.parametrize("K", [1, 2, 16, 17, 40])
+@pytest.mark.parametrize("B,n,d", [(1, 1_001, 1), (2, 5_003, 3), (3, 2_000, 4), (1, 9_999, 8), (2, 4_100, 13), (4, 3_333, 16),
+                                   (2, 310_000, 16), (1, 4_097, 17), (2, 3_000, 33), (1, 5_000, 128)])
+def test_sums_of_rows_that_share_a_cluster(B, n, d, K, order):
+    x, _ = _problem(B, n, d, K, seed=K)
+    c0 = x[:, torch.linspace(0, n - 1, K).long()].contiguous()
+    lab = fl.euclid_assign_triton(x, c0, mode="exact")
+    if order != "random":
+        key = lab if order == "sorted" else (torch.arange(n, device="cuda") // 37) % 7 * K + lab
+        at = key.long().argsort(dim=1, stable=True)
+        x = torch.gather(x, 1, at[..., None].expand(-1, -1, d)).contiguous()
+    lab, cent, _ = fl.flash_kmeans(x, K, max_iters=1, init_centroids=c0)
+    one = torch.nn.functional.one_hot(lab.long(), K).double()
+    cnt = one.sum(1)
+    want = torch.where(cnt[..., None] > 0, one.transpose(1, 2) @ x.double() / cnt.clamp_min(1)[..., None], c0.double())
+    size = one.transpose(1, 2) @ x.double().abs() / cnt.clamp_min(1)[..., None]
+    # a sum of n fp32 terms in any order: within n 2^-24 of the sum of their sizes; one more rounding for the division
+    assert ((cent.double() - want).abs() <= (cnt[..., None] + 2) * 2.0 ** -24 * (size + c0.abs())).all()
