@@ -174,7 +174,8 @@ def _mode_from(mode: Optional[str]) -> int:
 
 
 class DbPlane:
-    """The bf16 operand plane (+ half norms) of one fp32 database, built once per database.
+    """The bf16 operand plane (+ half norms) of one database, built once per database and kept for the four last used
+    (``clear_plane_cache`` gives them back): 2 bytes per feature, padded to 64, and 36 per row.
 
     The reference caches ``||c||^2`` per ``data_ptr`` in the same spirit
     (``flashlib/primitives/knn/triton/_row_norm.py:82-93``).
@@ -402,7 +403,13 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
         raise TypeError(f"knn_f32 takes q and db of one dtype out of fp32 / bf16 / fp16, got {q.dtype} and {db.dtype}")
     resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, dev.index, nq, m, d, k, mode)
     if wants_plane and plane is None:
-        plane = get_plane(db)
+        try:
+            plane = get_plane(db)
+        except torch.OutOfMemoryError:
+            if mode != _lib.FL_KNN_AUTO:
+                raise
+            # the plane takes half the memory of the fp32 rows again: without room for it, the exact mode
+            resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, dev.index, nq, m, d, k, _lib.FL_KNN_EXACT_SIMT)
     if out is not None:
         out_d, out_i = out
     else:
@@ -413,7 +420,10 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
         if second_stage is None:
             second_stage = _second_stage_default()
         if second_stage:
-            split = plane.split_ptr(db)
+            try:
+                split = plane.split_ptr(db)
+            except torch.OutOfMemoryError:
+                pass               # rows the first proof rejects take the exact pass at once
             if split is not None:
                 ws_bytes = staged_bytes
     # (the kernels clear the status words themselves)

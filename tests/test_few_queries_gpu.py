@@ -155,3 +155,34 @@ def test_exact_mode_by_queries_k_and_row_reads(nq, m, d, k, dtype, few):
     d_, i_, _ = knn_f32(q, db, k, mode=_lib.FL_KNN_EXACT_SIMT)
     assert (_lib.load().fl_launch_count() - before == 2) == few
     _check(q, db, k, d_, i_)
+
+
+@pytest.mark.parametrize("nq,m,d", [(600, 3_000, 700), (1_000, 20_000, 64)])
+def test_automatic_mode_without_room_for_a_plane(monkeypatch, nq, m, d):
+    from flashlib_b200 import knn as knn_mod
+    g = torch.Generator().manual_seed(d)
+    db, q = torch.randn(m, d, generator=g).cuda(), torch.randn(nq, d, generator=g).cuda()
+
+    def full(self, db):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(knn_mod.DbPlane, "__init__", full)
+    d_, i_, info = knn_f32(q, db, 10)
+    assert info["mode"] == _lib.FL_KNN_EXACT_SIMT
+    _check(q, db, 10, d_, i_)
+    with pytest.raises(torch.OutOfMemoryError):
+        knn_f32(q, db, 10, mode=_lib.FL_KNN_BF16_RERANK)
+
+
+def test_no_second_stage_without_room_for_its_plane(monkeypatch):
+    from flashlib_b200 import knn as knn_mod
+    g = torch.Generator().manual_seed(1)
+    db, q = torch.randn(20_000, 64, generator=g).cuda(), torch.randn(1_000, 64, generator=g).cuda()
+
+    def full(self, db):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(knn_mod.DbPlane, "split_ptr", full)
+    d_, i_, info = knn_f32(q, db, 10)
+    assert info["mode"] == _lib.FL_KNN_BF16_RERANK and not info["second_stage"]
+    _check(q, db, 10, d_, i_)
