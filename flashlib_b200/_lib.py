@@ -182,8 +182,11 @@ def check(rc: int, what: str = "") -> None:
 _devices_ok: set = set()       # devices found to be sm_100 (a process may see others beside them)
 
 
-def require_device() -> None:
-    """Raise unless the current device is an sm_100 one; there is nothing to fall back to."""
+def require_device(index=None) -> None:
+    """Raise unless the current device (``index``, where the caller knows it) is an sm_100 one; there is nothing to
+    fall back to."""
+    if index is not None and index in _devices_ok:
+        return
     dev = torch.cuda.current_device() if torch.cuda.is_initialized() else None
     if dev in _devices_ok:
         return

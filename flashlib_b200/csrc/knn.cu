@@ -33,48 +33,64 @@ __global__ void halfnorm_kernel(const void* __restrict__ x, int64_t n, int d, in
 // still change the answer.
 constexpr float SIMT_EPS_REL = 4e-6f;
 
-// One row of a bf16 query plane by a warp: the features, zero padding, and ones in the three columns that meet
-// the database plane's split -||x||^2/2 terms (all zero for rows that pad the last tile).  Four columns a
+// N rows of a bf16 query plane by a warp, from `row` on: the features, zero padding, and ones in the three columns that
+// meet the database plane's split -||x||^2/2 terms (all zero for rows that pad the last tile).  Four columns a
 // lane: 16-byte reads where `vec` says that the rows allow them, 8-byte writes (plane rows are 32-byte
-// aligned: their pitch is a multiple of 16 columns).  Returns the lane's share of ||q||^2 and of the square of what
-// the rounding took.
-__device__ __forceinline__ float2 query_plane_row(const void* p, bool live, int d, int vec, __nv_bfloat16* o, int d_pad, int dt) {
-    const int lane = threadIdx.x & 31;
-    float sq = 0.f, lost = 0.f;
-    for (int c = lane * 4; c < d_pad + PLANE_AUG_COLS; c += 128) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
-            if (c < d) {
-                v = ld_row4(p, c, d, vec, dt);
-            } else if (c == d_pad) {
-                v = make_float4(1.f, 1.f, 1.f, 0.f);
-            }
-        }
-        const uint2 w = bf16x4_bits(v);
-        *reinterpret_cast<uint2*>(o + c) = w;
-        if (c < d) { sq += sq4(v); lost += sq4(bf16_lost4(v, w)); }
+// aligned: their pitch is a multiple of 16 columns).  s: the lane's share of ||q||^2 and of the square of what the
+// rounding took.
+template <int N>
+__device__ __forceinline__ void query_plane_rows(const void* q, int64_t row, int64_t nq, int64_t ldq, int d, int vec,
+                                                 __nv_bfloat16* out, int d_pad, int dt, float2 (&s)[N]) {
+    const int lane = threadIdx.x & 31, pitch = d_pad + PLANE_AUG_COLS;
+    const void* p[N];
+    bool live[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        live[i] = row + i < nq;
+        p[i] = row_at(q, live[i] ? row + i : 0, ldq, dt);
+        s[i] = make_float2(0.f, 0.f);
     }
-    return make_float2(sq, lost);
+    __nv_bfloat16* o = out + row * pitch;
+    for (int c = lane * 4; c < pitch; c += 128) {
+        float4 v[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live[i] && c < d) v[i] = ld_row4(p[i], c, d, vec, dt);
+            else if (live[i] && c == d_pad) v[i] = make_float4(1.f, 1.f, 1.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const uint2 w = bf16x4_bits(v[i]);
+            *reinterpret_cast<uint2*>(o + i * pitch + c) = w;
+            if (c < d) { s[i].x += sq4(v[i]); s[i].y += sq4(bf16_lost4(v[i], w)); }
+        }
+    }
 }
 
-// Whole query plane, one warp per row; with sq_out also ||q||^2 of every live row and the square of the norm of what
-// its rounding took, from the same read.
-// Bound by HBM: 250 001 x 96 rows take 43 us (96 MB in, 72 MB out).  One thread per plane element and a second
-// pass over the rows for the norms took some 180.
+// Whole query plane, QP_ROWS rows a warp (nq_pad is a multiple of 128); with sq_out also ||q||^2 of every live row and the
+// square of the norm of what its rounding took, from the same read.
+// Bound by HBM latency: 250 001 x 96 rows (96 MB in, 72 MB out) take 43 us; one row a warp 47.
+constexpr int QP_ROWS = 2;
 __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
                                                           __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt,
                                                           float2* __restrict__ sq_out) {
-    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int64_t row = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * QP_ROWS;
     if (row >= nq_pad) return;
-    const bool live = row < nq;
-    float2 s = query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
-    if (sq_out == nullptr || !live) return;
+    float2 s[QP_ROWS];
+    query_plane_rows<QP_ROWS>(q, row, nq, ldq, d, vec, out, d_pad, dt, s);
+    if (sq_out == nullptr) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        s.x += __shfl_xor_sync(FULL_MASK, s.x, o);
-        s.y += __shfl_xor_sync(FULL_MASK, s.y, o);
+#pragma unroll
+        for (int i = 0; i < QP_ROWS; ++i) {
+            s[i].x += __shfl_xor_sync(FULL_MASK, s[i].x, o);
+            s[i].y += __shfl_xor_sync(FULL_MASK, s[i].y, o);
+        }
     }
-    if ((threadIdx.x & 31) == 0) sq_out[row] = s;
+#pragma unroll
+    for (int i = 0; i < QP_ROWS; ++i)
+        if ((threadIdx.x & 31) == 0 && row + i < nq) sq_out[row + i] = s[i];
 }
 
 // What a tensor-core call needs before its first scoring launch, in one pass: the bf16 query plane, the
@@ -91,13 +107,14 @@ __global__ void __launch_bounds__(256) knn_prep_kernel(const void* __restrict__ 
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= nq_pad) return;
     const bool live = row < nq;
-    query_plane_row(row_at(q, live ? row : 0, ldq, dt), live, d, vec, out + row * (d_pad + PLANE_AUG_COLS), d_pad, dt);
+    float2 s[1];
+    query_plane_rows<1>(q, row, nq, ldq, d, vec, out, d_pad, dt, s);
     if ((threadIdx.x & 31) == 0) tau[row] = live ? neg_inf() : pos_inf();
 }
 
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad, int d_pad,
                        cudaStream_t st, int dt, float2* sq_out) {
-    query_plane_kernel<<<(unsigned)ceil_div(nq_pad, 8), 256, 0, st>>>(
+    query_plane_kernel<<<(unsigned)ceil_div(nq_pad, 8 * QP_ROWS), 256, 0, st>>>(
         q, nq, ldq, d, dt_vec_ok(q, ldq, dt) && d % 4 == 0, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt, sq_out);
     FL_CHECK_LAUNCH();
     return FL_OK;

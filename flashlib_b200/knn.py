@@ -34,6 +34,20 @@ def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+_STREAMS: dict = {}
+
+
+def _stream(device: torch.device) -> torch.cuda.Stream:
+    """The current stream as an object (building one takes 2 us; they are kept by handle)."""
+    key = (device.index, _stream_ptr(device))
+    hit = _STREAMS.get(key)
+    if hit is None:
+        if len(_STREAMS) >= 64:
+            _STREAMS.clear()
+        hit = _STREAMS[key] = torch.cuda.current_stream(device)
+    return hit
+
+
 class _OnDevice:
     """``torch.cuda.device`` for the (usual) case that the tensor's device is current already: no
     context is entered then."""
@@ -73,7 +87,7 @@ class _Built:
         self.stream = _stream_ptr(device)
         self.capture = _capture_id(device)
         self.event = torch.cuda.Event()
-        self.event.record(torch.cuda.current_stream(device))
+        self.event.record(_stream(device))
 
     def __reduce__(self):
         return _nothing, ()            # a copy of an index or its pickle carries no event
@@ -86,7 +100,7 @@ class _Built:
             return
         if _capture_id(self.device) != self.capture:
             return           # a capture may not wait for work outside it; torch.cuda.graph waits for the device first
-        cur = torch.cuda.current_stream(self.device)
+        cur = _stream(self.device)
         cur.wait_event(self.event)
         buf.record_stream(cur)
 
@@ -212,7 +226,12 @@ class DbPlane:
                 buf = torch.empty(nbytes, dtype=torch.uint8, device=db.device)
                 _lib.check(lib.fl_knn_prepare_split_f32(db.data_ptr(), m, d, db.stride(0), buf.data_ptr(),
                                                         nbytes, _stream_ptr(db.device)))
-                split = (buf, _Built(db.device))
+                built = self.built
+                if built.stream == _stream_ptr(db.device) and built.capture == _capture_id(db.device):
+                    built.event.record(_stream(db.device))      # one event for the two of them
+                else:
+                    built = _Built(db.device)
+                split = (buf, built)
             self.split = split             # (only now: another thread must not meet a plane nobody has enqueued yet)
         if split is False:
             return None
@@ -395,10 +414,10 @@ def knn_f32(q: torch.Tensor, db: torch.Tensor, k: int, *, mode: int = _lib.FL_KN
     tensor cores with split hi/lo operands before anything takes the exact CUDA-core pass;
     ``None`` = when the database's split plane exists or is small enough to build."""
     lib = _lib.load()
-    _lib.require_device()
     nq, d = q.shape
     m = db.shape[0]
     dev = q.device
+    _lib.require_device(dev.index)
     if q.dtype != db.dtype or db.dtype not in _DTYPE_CODES:
         raise TypeError(f"knn_f32 takes q and db of one dtype out of fp32 / bf16 / fp16, got {q.dtype} and {db.dtype}")
     resolved, passed, wants_plane, ws_bytes, staged_bytes = _knn_plan(lib, dev.index, nq, m, d, k, mode)
