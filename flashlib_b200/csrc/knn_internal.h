@@ -77,8 +77,7 @@ struct DirectParams {
     int k; int64_t row_offset;
     // inverted-file scan (probed != nullptr): pair i = (query i / nprobe, list probed[i])
     const int32_t* probed; int nprobe; int ivf_nlist; const int64_t* list_offsets;
-    float* out_dist; int32_t* out_idx;       // out_idx (rows) and out_ids (id_map64[row]) are each optional
-    int64_t* out_ids; const int64_t* id_map64;
+    float* out_dist; int32_t* out_idx;
     int32_t* status;         // optional
     // filled in by the launch functions
     int npl, nchunk, lists_per_query; int64_t rows_per_chunk;
@@ -141,9 +140,7 @@ struct PairFinalizeParams {
     const void* db; int64_t m; int64_t ldb; int d; int vec;
     const float2* pools; const int* pool_cnt; const float* pool_tau;
     int cap;                 // slots per pool
-    int npool;               // pools per query: pool i of query q is number q * npool + i, or, with pair_row,
-    const int* pair_row;     //   2 * pair_row[q * npool / 2 + i / 2] + i % 2 (pair_row < 0: none)
-    const int* row_map; int64_t rows_max;    // optional: published id -> row (< 0: padding)
+    int npool;               // pools per query: pool i of query q is number q * npool + i
     int k; float acc; const float* norms; int64_t row_offset;   // scoring error of bf16 operands: as FinalizeParams
     float* out_dist; int32_t* out_idx;
     int* fb_count; int* fb_list; int fb_cap;

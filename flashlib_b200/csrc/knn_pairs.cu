@@ -56,13 +56,7 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t qi = blockIdx.x;
     const void* qp = row_at(p.q, qi, p.ldq, p.dt);
-    auto pool_of = [&](int i) -> int64_t {
-        if (i >= p.npool) return -1;
-        if (p.pair_row == nullptr) return qi * p.npool + i;
-        const int r = __ldg(p.pair_row + qi * (p.npool >> 1) + (i >> 1));
-        return r >= 0 ? (int64_t)r * 2 + (i & 1) : -1;
-    };
-
+    auto pool_of = [&](int i) -> int64_t { return i < p.npool ? qi * p.npool + i : -1; };
     // u = the largest final threshold: every row in no pool scored at most that much
     float u = neg_inf(), qs = 0.f, ls = 0.f;
     for (int i = tid; i < p.npool; i += PF_THREADS) {
@@ -130,11 +124,7 @@ __global__ void __launch_bounds__(PF_THREADS) pairs_finalize_kernel(const PairFi
                     }
                     const float2 v = __ldg(p.pools + (int64_t)s_pool[lo] * p.cap + (idx - s_off[lo]));
                     if (v.x > cut) {
-                        uint32_t raw = __float_as_uint(v.y);
-                        if (p.row_map != nullptr) {
-                            const int mapped = raw < (uint32_t)p.rows_max ? __ldg(p.row_map + raw) : -1;
-                            raw = mapped >= 0 ? (uint32_t)mapped : INVALID_ID;
-                        }
+                        const uint32_t raw = __float_as_uint(v.y);
                         if (raw < (uint32_t)p.m) { sc = v.x; id = raw; tmax = fmaxf(tmax, sc); }
                     }
                 }
