@@ -136,9 +136,13 @@ __global__ void split_x_gather_kernel(const float* __restrict__ x, int64_t ldx, 
 // score's low mantissa bits), so the label is proven when its exact distance is below
 // ||x||^2 - 2 (bound + eps); otherwise the point goes to the `next` list (the next, more precise
 // stage) or, when that is absent or full, to the exact-path list.
+//
+// SPLIT: the scores are those of the split planes, and what their roundings took of the point is summed up here; for plain
+// bf16 operands that comes with ||x||^2 from the pass that rounded the points (xsq).
+template <bool SPLIT>
 __global__ void __launch_bounds__(128) assign_finalize_kernel(
     const float* __restrict__ x, int64_t n, int64_t ldx, const float* __restrict__ c, int K, int64_t ldc, int d,
-    int vec, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, int operands, float acc,
+    int vec, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float2* __restrict__ xsq, float acc,
     const float* __restrict__ norms, int32_t* __restrict__ labels, const int* __restrict__ rows,
     const int* __restrict__ rows_count, int* __restrict__ next_count, int* __restrict__ next_list, int next_cap,
     int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap, int scores_by_point) {
@@ -169,10 +173,12 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
                 const float4 xv = __ldg(reinterpret_cast<const float4*>(xp + t));
                 const float4 p0 = __ldg(reinterpret_cast<const float4*>(c0 + t));
                 const float4 p1 = __ldg(reinterpret_cast<const float4*>(c1 + t));
-                qsq += sq4(xv);
-                const float4 l = bf16_lost4(xv);
-                lost += sq4(l);
-                lost2 += sq4(bf16_lost4(l));
+                if (SPLIT) {
+                    qsq += sq4(xv);
+                    const float4 l = bf16_lost4(xv);
+                    lost += sq4(l);
+                    lost2 += sq4(bf16_lost4(l));
+                }
                 float e0 = xv.x - p0.x, e1 = xv.y - p0.y, e2 = xv.z - p0.z, e3 = xv.w - p0.w;
                 a0 += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
                 e0 = xv.x - p1.x; e1 = xv.y - p1.y; e2 = xv.z - p1.z; e3 = xv.w - p1.w;
@@ -182,15 +188,20 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
             for (int t = sl; t < d; t += 8) {
                 const float xv = __ldg(xp + t);
                 const float e0 = xv - __ldg(c0 + t), e1 = xv - __ldg(c1 + t);
-                const float l = bf16_lost(xv), l2 = bf16_lost(l);
-                qsq += xv * xv; lost += l * l; lost2 += l2 * l2; a0 += e0 * e0; a1 += e1 * e1;
+                if (SPLIT) {
+                    const float l = bf16_lost(xv), l2 = bf16_lost(l);
+                    qsq += xv * xv; lost += l * l; lost2 += l2 * l2;
+                }
+                a0 += e0 * e0; a1 += e1 * e1;
             }
         }
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) {
-            qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
-            lost += __shfl_xor_sync(FULL_MASK, lost, o);
-            lost2 += __shfl_xor_sync(FULL_MASK, lost2, o);
+            if (SPLIT) {
+                qsq += __shfl_xor_sync(FULL_MASK, qsq, o);
+                lost += __shfl_xor_sync(FULL_MASK, lost, o);
+                lost2 += __shfl_xor_sync(FULL_MASK, lost2, o);
+            }
             a0 += __shfl_xor_sync(FULL_MASK, a0, o);
             a1 += __shfl_xor_sync(FULL_MASK, a1, o);
         }
@@ -203,7 +214,12 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
         bool ok = best_i != INVALID_ID;
         if (ok && bound > -1e37f) {
             bound += fabsf(bound) * 3.1e-5f;                       // index bits in the mantissa: 2^-15 relative
-            ok = list_proven(best_d, qsq, bound, score_eps(operands, qsq, lost, lost2, norms, acc),
+            if (!SPLIT) {
+                const float2 x2 = __ldg(xsq + pt);
+                qsq = x2.x;
+                lost = x2.y;
+            }
+            ok = list_proven(best_d, qsq, bound, score_eps(SPLIT ? OPERANDS_SPLIT : OPERANDS_BF16, qsq, lost, lost2, norms, acc),
                              proof_slack(qsq, __ldg(norms + NORM_ROW), d));
         }
         labels[pt] = ok ? (int32_t)best_i : 0;
@@ -538,12 +554,12 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
             FL_CHECK_LAUNCH();
             // ... then, for the undecided ones only, the exact distances to the two half-winners, which
             // need half the lead; what is still open goes to the second stage
-            assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_BF16, acc1, norms, labels, l0_list, l0_count,
+            assign_finalize_kernel<false><<<fin_grid, 128, 0, st>>>(
+                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, xsq, acc1, norms, labels, l0_list, l0_count,
                 l1_count, l1_list, w.l1_cap, fb_count, fb_list, w.fb_cap, 1);
         } else {
-            assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_BF16, acc1, norms, labels, nullptr, nullptr,
+            assign_finalize_kernel<false><<<fin_grid, 128, 0, st>>>(
+                x, n, ldx, c, K, ldc, d, vec, asg_sc, asg_id, xsq, acc1, norms, labels, nullptr, nullptr,
                 nullptr, l1_list, w.l1_cap, fb_count, fb_list, w.fb_cap, 0);
         }
         FL_CHECK_LAUNCH();
@@ -561,8 +577,8 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         tp.tau = tau; tp.status = status;
         rc = launch_assign_tc(tp, asg_sc, asg_id, l1_count, st);
         if (rc != FL_OK) return rc;
-        assign_finalize_kernel<<<fin_grid, 128, 0, st>>>(
-            x, w.l1_cap, ldx, c, K, ldc, d, vec, asg_sc, asg_id, OPERANDS_SPLIT, score_acc_split(d),
+        assign_finalize_kernel<true><<<fin_grid, 128, 0, st>>>(
+            x, w.l1_cap, ldx, c, K, ldc, d, vec, asg_sc, asg_id, nullptr, score_acc_split(d),
             reinterpret_cast<const float*>(cpl3 + w.cl3.off_meta), labels, l1_list, l1_count,
             nullptr, nullptr, 0, fb_count, fb_list, w.fb_cap, 0);
         FL_CHECK_LAUNCH();

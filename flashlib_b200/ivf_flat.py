@@ -238,7 +238,7 @@ def ivf_fine_scan(Qp: torch.Tensor, index: IvfFlatIndex, probed: torch.Tensor, k
                                     (mode in (None, "auto") and k <= 16 and nq * nprobe >= 2048)):
         plane = _tc_plane(index, data, offs)
         ws = torch.empty(tc_bytes, dtype=torch.uint8, device=q.device)
-        status = torch.zeros(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=q.device)
+        status = torch.empty(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=q.device)      # (the call clears the words)
         with torch.cuda.device(q.device):
             _lib.check(lib.fl_ivf_fine_scan_tc_f32(q.data_ptr(), nq, q.stride(0), data.data_ptr(), m, data.stride(0), d,
                                                    offs.data_ptr(), index.nlist, probed.data_ptr(), nprobe, k,

@@ -67,7 +67,8 @@ def _assign_2d(x: torch.Tensor, c: torch.Tensor, out: torch.Tensor, mode: Option
         xplane = _x_plane(x)
         ws_bytes = lib.fl_kmeans_assign_tc_workspace_bytes(n, K, d, 1)
         ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=x.device)
-        status = torch.zeros(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=x.device)
+        # (the call clears the words; without rows it does nothing)
+        status = (torch.empty if n else torch.zeros)(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=x.device)
         _lib.check(lib.fl_kmeans_assign_tc_f32(x.data_ptr(), n, x.stride(0), xplane.data_ptr(), c.data_ptr(), K,
                                                c.stride(0), d, out.data_ptr(), ws.data_ptr(), ws_bytes,
                                                status.data_ptr(), _stream_ptr(x.device)))
@@ -96,7 +97,7 @@ def euclid_assign_triton(x: torch.Tensor, centroids: torch.Tensor, out: Optional
     B, N, D = x.shape
     K = centroids.shape[1]
     assert centroids.shape == (B, K, D), "centroids shape mismatch"
-    _lib.require_device()
+    _lib.require_device(x.device.index)
     if out is None:
         out = torch.empty((B, N), device=x.device, dtype=torch.int32)
     else:
