@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 from .kmeans import euclid_assign_triton, flash_kmeans
-from .knn import _Built, _as_f32_rows, _defer_status_check, _stream_ptr, knn_f32, row_sqnorm
+from .knn import _Built, _as_f32_rows, _as_rows, _defer_status_check, _stream_ptr, knn_f32, row_sqnorm
 
 
 @dataclass
@@ -281,7 +281,14 @@ def flash_ivf_flat_search(index: IvfFlatIndex, Q: torch.Tensor, k: int, *, nprob
     # tensor-core mode proves every row's list of centroids or recomputes it exactly), so the size decides.
     # (no second tensor-core stage here: on a database of a few tiles the exact pass for a handful of
     # unproven rows costs less than the stage's three launches cost every call)
-    _, probed, _ = knn_f32(_as_f32_rows(Qp), _as_f32_rows(index.centroids), nprobe, check_status="deferred", second_stage=False)
+    # 16-bit centroids are searched as they are stored: widened ones would be a new database every time, each with an
+    # operand plane that drives somebody else's out of the cache
+    if Qp.dtype == index.centroids.dtype:
+        qc, cent, coarse = _as_rows(Qp), _as_rows(index.centroids), _lib.FL_KNN_AUTO
+    else:
+        qc, cent = _as_f32_rows(Qp), _as_f32_rows(index.centroids)
+        coarse = _lib.FL_KNN_AUTO if index.centroids.dtype == torch.float32 else _lib.FL_KNN_EXACT_SIMT
+    _, probed, _ = knn_f32(qc, cent, nprobe, mode=coarse, check_status="deferred", second_stage=False)
     mode = {"auto": None, "elementwise": "exact", "gemm": "bf16"}[variant]
     if mode == "bf16" and (k > 16 or index.Dp > 256):
         mode = "exact"

@@ -202,3 +202,33 @@ def test_device_side_build_is_a_stable_partition(m, dim, nlist):
     assert np.array_equal(ids.cpu().numpy(), order)
     assert torch.equal(data.cpu(), x.cpu()[torch.from_numpy(order)])
     assert int(longest.item()) == int(counts.max())
+
+
+@pytest.mark.parametrize("dtype,other", [(torch.bfloat16, False), (torch.float16, False), (torch.bfloat16, True)])
+def test_centroids_of_16_bits_leave_other_planes_alone(monkeypatch, dtype, other):
+    """An index built from 16-bit rows keeps 16-bit centroids (``other``: beside fp32 rows).  A search of many queries
+    makes at most one operand plane of them, once, and drops nobody's."""
+    from flashlib_b200 import knn as knn_mod
+    g = torch.Generator().manual_seed(5)
+    X = torch.randn(20_000, 32, generator=g).cuda()
+    Q = torch.randn(3_000, 32, generator=g).cuda()
+    index = fl.flash_ivf_flat_build(X.to(dtype), 600, nprobe=6, niter=2)
+    assert index.centroids.dtype == dtype
+    if other:
+        index.data = index.data.float()
+    knn_mod.clear_plane_cache()
+    built = []
+    init = knn_mod.DbPlane.__init__
+    monkeypatch.setattr(knn_mod.DbPlane, "__init__", lambda self, db: (built.append(db.dtype), init(self, db))[1])
+    for _ in range(3):
+        vals, ids = fl.flash_ivf_flat_search(index, Q, 5)
+    assert built in ([], [dtype])
+    q, cent = Q.to(index.data.dtype).double(), index.centroids.double()
+    probed = ((q * q).sum(1, keepdim=True) + (cent * cent).sum(1) - 2 * q @ cent.T).topk(6, dim=1, largest=False).indices
+    offs = index.list_offsets.cpu()
+    for i in range(0, 3_000, 300):
+        rows = torch.cat([torch.arange(offs[c], offs[c + 1]) for c in probed[i].tolist()]).cuda()
+        d64 = ((index.data[rows].double() - q[i]) ** 2).sum(1)
+        want = d64.topk(5, largest=False).values
+        # an fp32 sum of 32 squares of rounded differences
+        assert ((vals[i].double() - want).abs() <= 34 * 2.0 ** -24 * want + 1e-12).all()
