@@ -675,9 +675,9 @@ static IvfTcWs ivf_tc_plan(int64_t nq, int nprobe, int nlist, int d, int k) {
     w.off_qplane = take(cur, w.cap_rows * w.pitch * 2);
     w.off_tau = take(cur, w.cap_rows * 4);
     w.off_seed_cls = take(cur, w.cap_rows * 32 * 4);
-    w.off_pools = take(cur, w.cap_rows * tc_taus_per_range() * tc_pair_pool_cap(k) * 8);
-    w.off_part_cnt = take(cur, w.cap_rows * tc_taus_per_range() * 4);
-    w.off_part_tau = take(cur, w.cap_rows * tc_taus_per_range() * 4);
+    w.off_pools = take(cur, w.cap_rows * tc_pair_pools_per_range() * tc_pair_pool_cap(k) * 8);
+    w.off_part_cnt = take(cur, w.cap_rows * tc_pair_pools_per_range() * 4);
+    w.off_part_tau = take(cur, w.cap_rows * tc_pair_pools_per_range() * 4);
     w.off_fblist = take(cur, nq * 4);
     // exact pass over a handful of queries: per-block partial results and a ticket per query
     w.off_x_scratch = take(cur, (int64_t)2 * sm_count() * 16 * 8);
@@ -804,7 +804,7 @@ extern "C" int fl_ivf_fine_scan_tc_f32(const float* q, int64_t nq, int64_t ldq, 
     TcKnnParams tp{};
     tp.qplane = base + w.off_qplane; tp.nq = w.cap_rows; tp.nq_pad = w.cap_rows;
     tp.dbrows = pl + L.pl.off_rows; tp.hnorm = reinterpret_cast<const float*>(pl + L.pl.off_hnorm);
-    tp.m = L.rows_max; tp.m_pad = L.pl.m_pad; tp.d_pad = L.pl.d_pad; tp.K1 = tc_deep_pool_size();
+    tp.m = L.rows_max; tp.m_pad = L.pl.m_pad; tp.d_pad = L.pl.d_pad; tp.d_used = d; tp.K1 = tc_deep_pool_size();
     tp.deep_pools = 0;
     tp.nsplit = 1; tp.tiles_per_split = L.pl.m_pad / IVF_TC_TILE;
     tp.pair_pools = base + w.off_pools;                    // pools in global memory, four ring slots

@@ -540,7 +540,7 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         TcKnnParams tp{};
         tp.qplane = xpl; tp.nq = n; tp.nq_pad = w.n_pad;
         tp.dbrows = cpl + w.cl.off_rows; tp.hnorm = reinterpret_cast<const float*>(cpl + w.cl.off_hnorm);
-        tp.m = K; tp.m_pad = w.cl.m_pad; tp.d_pad = w.cl.d_pad;
+        tp.m = K; tp.m_pad = w.cl.m_pad; tp.d_pad = w.cl.d_pad; tp.d_used = d;
         tp.tau = tau; tp.status = status;
         profile_begin(st);
         rc = launch_assign_tc(tp, asg_sc, asg_id, nullptr, st);
@@ -573,7 +573,7 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         TcKnnParams tp{};
         tp.qplane = xs; tp.nq = w.l1_cap; tp.nq_pad = w.l1_pad;
         tp.dbrows = cpl3 + w.cl3.off_rows; tp.hnorm = reinterpret_cast<const float*>(cpl3 + w.cl3.off_hnorm);
-        tp.m = K; tp.m_pad = w.cl3.m_pad; tp.d_pad = w.cl3.d_pad;
+        tp.m = K; tp.m_pad = w.cl3.m_pad; tp.d_pad = w.cl3.d_pad; tp.d_used = 2 * w.d_pad + d;
         tp.tau = tau; tp.status = status;
         rc = launch_assign_tc(tp, asg_sc, asg_id, l1_count, st);
         if (rc != FL_OK) return rc;

@@ -179,13 +179,14 @@ struct KnnWs {
     int nsplit; int64_t rows_per_split;        // main pass (SIMT: rows; TC: tiles of 256)
     int nsplit_fb; int64_t rows_per_split_fb;  // fallback pass
     int64_t nq_pad; int d_pad; int fb_cap; int fb_bq, fb_blocks;
-    int64_t off_hnorm, off_qplane, off_part_sc, off_part_id, off_part_tau, off_part_cnt, off_seed_cls, off_tau, off_cert, off_norms, off_cnt, off_fblist,
+    int npool;         // published pools of a query
+    int64_t off_hnorm, off_qplane, off_part_sc, off_part_id, off_part_tau, off_part_cnt, off_seed_cls, off_tau, off_lists, off_cert, off_norms, off_cnt, off_fblist,
         off_fbpart_sc, off_fbpart_id, bytes;
     // second stage (split hi/lo planes) for the rows the first proof rejects
     int s2;                                    // 1: planned
     int s2_cap; int64_t s2_pad;                // rows the stage takes (the rest go to the exact path), padded to tiles
     int s2_nsplit; int64_t s2_tiles_per_split; int s2_plen;
-    int64_t off_s2_list, off_s2_qplane, off_s2_tau, off_s2_part_sc, off_s2_part_id, off_s2_part_tau, off_s2_part_cnt;
+    int64_t off_s2_list, off_s2_qplane, off_s2_tau, off_s2_part_sc, off_s2_part_id, off_s2_part_tau, off_s2_part_cnt, off_s2_lists;
 };
 
 static int64_t take(int64_t& cur, int64_t bytes) {
@@ -222,10 +223,11 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.kg = k;
         w.K1 = tc_pool_size(k);
         w.K1f = simt_pool_size(k_real);
-        w.nq_pad = tc_query_rows_padded(nq);
         w.d_pad = (int)round_up(d, 64);
         const int64_t m_pad = round_up(m, 256);
+        w.nq_pad = round_up(nq, 128);
         w.small = !shared_seed && (tc_small(w.nq_pad, m_pad) || d > 512);
+        if (!w.small) w.nq_pad = tc_query_rows_padded(nq);
         if (w.small) {
             w.kg = k_real;                                 // (no pool in shared memory whatever d is)
             tc_small_split(w.nq_pad, m_pad, &w.nsplit, &w.rows_per_split);
@@ -248,20 +250,23 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         w.nsplit_fb = (int)ceil_div(m, w.rows_per_split_fb);
         w.off_hnorm = -1;
         w.off_qplane = take(cur, w.nq_pad * (w.d_pad + PLANE_AUG_COLS) * 2);
-        w.deep = !w.small && tc_use_deep_pools(k, w.d_pad, w.nsplit, w.nq_pad);
+        w.deep = !w.small && tc_use_deep_pools(k, w.d_pad, w.nsplit);
         w.plen = w.deep ? tc_deep_partial_len() : tc_partial_len(k);
         if (w.deep) w.K1 = tc_deep_pool_size();
         if (w.small) {
-            w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)(tc_taus_per_range() * tc_pair_pool_cap(k_real)) * 8);
+            w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)(tc_pair_pools_per_range() * tc_pair_pool_cap(k_real)) * 8);
             w.off_part_id = w.off_part_sc;
         } else {
             w.off_part_sc = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
             w.off_part_id = take(cur, w.nq_pad * w.nsplit * (int64_t)w.plen * 4);
         }
-        w.off_part_tau = take(cur, w.nq_pad * w.nsplit * tc_taus_per_range() * 4);
-        w.off_part_cnt = take(cur, w.nq_pad * w.nsplit * tc_taus_per_range() * 4);
+        w.npool = w.nsplit * (w.small || w.deep ? tc_pair_pools_per_range() : tc_lists_per_range());
+        const int64_t most = w.nq_pad * w.nsplit * (w.small ? tc_pair_pools_per_range() : tc_lists_per_range()) * 4;
+        w.off_part_tau = take(cur, most);
+        w.off_part_cnt = take(cur, most);
         w.off_seed_cls = take(cur, w.nq_pad * (w.seed.splits > 1 ? w.seed.splits : 1) * 32 * 4);
         w.off_tau = take(cur, w.nq_pad * 4);
+        if (!w.small) w.off_lists = take(cur, tc_list_bytes(w.nq_pad / 128 * w.nsplit, k));
         w.off_cert = take(cur, w.nq_pad * 4);
         w.off_norms = take(cur, NORM_WORDS * 4);
         w.off_cnt = take(cur, 1024);
@@ -296,8 +301,9 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
             w.off_s2_tau = take(cur, w.s2_pad * 4);
             w.off_s2_part_sc = take(cur, w.s2_pad * w.s2_nsplit * (int64_t)w.s2_plen * 4);
             w.off_s2_part_id = take(cur, w.s2_pad * w.s2_nsplit * (int64_t)w.s2_plen * 4);
-            w.off_s2_part_tau = take(cur, w.s2_pad * w.s2_nsplit * tc_taus_per_range() * 4);
-            w.off_s2_part_cnt = take(cur, w.s2_pad * w.s2_nsplit * tc_taus_per_range() * 4);
+            w.off_s2_part_tau = take(cur, w.s2_pad * w.s2_nsplit * tc_lists_per_range() * 4);
+            w.off_s2_part_cnt = take(cur, w.s2_pad * w.s2_nsplit * tc_lists_per_range() * 4);
+            w.off_s2_lists = take(cur, tc_list_bytes(w.s2_pad / 128 * w.s2_nsplit, 17));
         }
     } else {
         w.K1 = simt_pool_size(k);
@@ -479,7 +485,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     TcKnnParams tp{};
     tp.qplane = base + w.off_qplane; tp.nq = nq; tp.nq_pad = w.nq_pad;
     tp.dbrows = pl + L.off_rows; tp.hnorm = reinterpret_cast<const float*>(pl + L.off_hnorm);
-    tp.m = m; tp.m_pad = L.m_pad; tp.d_pad = L.d_pad; tp.K1 = w.K1;
+    tp.m = m; tp.m_pad = L.m_pad; tp.d_pad = L.d_pad; tp.d_used = d; tp.K1 = w.K1;
     tp.nsplit = w.nsplit; tp.tiles_per_split = w.rows_per_split;
     tp.part_sc = reinterpret_cast<float*>(base + w.off_part_sc);
     tp.part_id = reinterpret_cast<uint32_t*>(base + w.off_part_id);
@@ -488,6 +494,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     tp.tau = tau; tp.status = status;
     tp.part_tau = reinterpret_cast<float*>(base + w.off_part_tau);
     tp.part_cnt = reinterpret_cast<int*>(base + w.off_part_cnt);
+    tp.lists = base + w.off_lists;
     tp.deep_pools = w.deep;
     tp.seed_cls = seed_cls;
     tp.k = w.kg;
@@ -539,7 +546,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
     // scoring pass left out is bounded by the thresholds it published.
     fp.part_sc = tp.part_sc; fp.part_id = tp.part_id; fp.nsplit = w.nsplit; fp.K1 = w.plen;
     fp.k = k; fp.rerank = fp.K1; fp.row_offset = row_offset;
-    fp.part_tau = tp.part_tau; fp.ntau = w.nsplit * tc_taus_per_range();
+    fp.part_tau = tp.part_tau; fp.ntau = w.npool;
     fp.out_dist = out_dist; fp.out_idx = out_idx;
     fp.verify = 1; fp.operands = OPERANDS_BF16; fp.acc = acc1; fp.norms = norms;
     fp.cert_tau = gnorms != nullptr ? cert : nullptr;
@@ -552,7 +559,7 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
         PairFinalizeParams pf{};
         pf.dt = dt; pf.q = q; pf.ldq = ldq; pf.nq = nq; pf.db = db; pf.m = m; pf.ldb = ldb; pf.d = d; pf.vec = vec;
         pf.pools = static_cast<const float2*>(tp.pair_pools); pf.pool_cnt = tp.part_cnt; pf.pool_tau = tp.part_tau;
-        pf.cap = tc_pair_pool_cap(k); pf.npool = w.nsplit * tc_taus_per_range();
+        pf.cap = tc_pair_pool_cap(k); pf.npool = w.npool;
         pf.k = k; pf.acc = acc1; pf.norms = norms; pf.row_offset = row_offset;
         pf.out_dist = out_dist; pf.out_idx = out_idx;
         pf.fb_count = fb_count; pf.fb_list = fb_list; pf.fb_cap = w.fb_cap;
@@ -578,19 +585,20 @@ static int knn_tc_phases(int phases, const void* q, int64_t nq, int64_t ldq, con
         TcKnnParams t2{};
         t2.qplane = base + w.off_s2_qplane; t2.nq = w.s2_cap; t2.nq_pad = w.s2_pad;
         t2.dbrows = pl3 + L3.off_rows; t2.hnorm = reinterpret_cast<const float*>(pl3 + L3.off_hnorm);
-        t2.m = m; t2.m_pad = L3.m_pad; t2.d_pad = L3.d_pad; t2.K1 = tc_pool_size(17);
+        t2.m = m; t2.m_pad = L3.m_pad; t2.d_pad = L3.d_pad; t2.d_used = 2 * L.d_pad + d; t2.K1 = tc_pool_size(17);
         t2.nsplit = w.s2_nsplit; t2.tiles_per_split = w.s2_tiles_per_split;
         t2.part_sc = reinterpret_cast<float*>(base + w.off_s2_part_sc);
         t2.part_id = reinterpret_cast<uint32_t*>(base + w.off_s2_part_id);
         t2.part_tau = reinterpret_cast<float*>(base + w.off_s2_part_tau);
         t2.part_cnt = reinterpret_cast<int*>(base + w.off_s2_part_cnt);
+        t2.lists = base + w.off_s2_lists;
         t2.tau = tau2; t2.status = status; t2.k = k; t2.big_pools = 1; t2.nq_dev = s2_count;
         rc = launch_knn_tc_scoring(t2, st);
         if (rc != FL_OK) return rc;
         FinalizeParams f2 = fp;
         f2.qlist = s2_list; f2.count_dev = s2_count; f2.count = w.s2_cap;
         f2.part_sc = t2.part_sc; f2.part_id = t2.part_id; f2.nsplit = w.s2_nsplit; f2.K1 = w.s2_plen;
-        f2.rerank = f2.K1; f2.part_tau = t2.part_tau; f2.ntau = w.s2_nsplit * tc_taus_per_range();
+        f2.rerank = f2.K1; f2.part_tau = t2.part_tau; f2.ntau = w.s2_nsplit * tc_lists_per_range();
         f2.part_cnt = t2.part_cnt; f2.operands = OPERANDS_SPLIT; f2.acc = acc2; f2.norms = norms3; f2.cert_tau = nullptr;
         f2.next_count = nullptr; f2.next_list = nullptr; f2.next_cap = 0;
         rc = launch_knn_finalize_big(f2, w.s2_cap, st);
@@ -974,7 +982,7 @@ extern "C" int fl_debug_knn_tc_scores(const float* q, int64_t nq, int64_t ldq, i
                                       int32_t* status, void* stream) {
     FL_CHECK_ARG(q && plane && scores && ws && nq >= 1 && nq <= 128 && m >= 1 && d >= 1, "fl_debug_knn_tc_scores: bad arguments");
     if (d > 256 || tc_knn_supported(nq, m, d, 10) != FL_OK) { set_error("fl_debug_knn_tc_scores: unsupported shape"); return FL_EUNSUPPORTED; }
-    const KnnWs w = knn_ws_plan(nq, m, d, 10, FL_KNN_BF16_RERANK);
+    const KnnWs w = knn_ws_plan(nq, m, d, 10, FL_KNN_BF16_RERANK, 0, 1);      // (never the small-problem plan: no lists there)
     if (ws_bytes < w.bytes) { set_error("fl_debug_knn_tc_scores: workspace too small"); return FL_EWORKSPACE; }
     const PlaneLayout L = plane_layout(m, d);
     FL_CHECK_ARG(ld_scores >= L.m_pad, "fl_debug_knn_tc_scores: ld_scores must cover the padded row count %lld", (long long)L.m_pad);
@@ -990,11 +998,12 @@ extern "C" int fl_debug_knn_tc_scores(const float* q, int64_t nq, int64_t ldq, i
     TcKnnParams tp{};
     tp.qplane = base + w.off_qplane; tp.nq = nq; tp.nq_pad = w.nq_pad;
     tp.dbrows = pl + L.off_rows; tp.hnorm = reinterpret_cast<const float*>(pl + L.off_hnorm);
-    tp.m = m; tp.m_pad = L.m_pad; tp.d_pad = L.d_pad; tp.K1 = w.K1;
+    tp.m = m; tp.m_pad = L.m_pad; tp.d_pad = L.d_pad; tp.d_used = d; tp.K1 = w.K1;
     tp.nsplit = w.nsplit; tp.tiles_per_split = w.rows_per_split;
     tp.part_sc = reinterpret_cast<float*>(base + w.off_part_sc);
     tp.part_id = reinterpret_cast<uint32_t*>(base + w.off_part_id);
     tp.tau = tau; tp.status = status;
+    tp.lists = base + w.off_lists;
     tp.part_tau = reinterpret_cast<float*>(base + w.off_part_tau);
     return launch_knn_tc_debug(tp, scores, ld_scores, st);
 }

@@ -34,7 +34,7 @@ int launch_knn_finalize(const FinalizeParams& p, int64_t max_slots, cudaStream_t
 // ------------------------------------------------------------------------------------
 // Finalisation of the large-k tensor-core pools: one block per query.
 //
-// The scoring pass published, per (query, range, warpgroup), a pool of up to 256 (score, row)
+// The scoring pass published, per (query, range, warpgroup), a list of up to 128 (score, row)
 // entries with its entry count and final threshold; every row it did not publish scored at most
 // u = the largest threshold.  The block gathers the entries scoring above u (the others can
 // never satisfy the proof), sorts them by score, re-scores the best BIG_RERANK with exact fp32
@@ -42,7 +42,7 @@ int launch_knn_finalize(const FinalizeParams& p, int64_t max_slots, cudaStream_t
 // lies below qsq - 2 (bound + eps), bound = max(u, best score that was not re-scored).
 // Otherwise (or when more than BIG_CAND entries survive) the query is queued for the exact path.
 // ------------------------------------------------------------------------------------
-constexpr int BIG_THREADS = 256, BIG_CAND = 2048, BIG_RERANK = 256, BIG_POOL = 256;
+constexpr int BIG_THREADS = 256, BIG_CAND = 2048, BIG_RERANK = 256, BIG_POOL = 128;
 
 static __device__ __forceinline__ void finalize_big_slot(const FinalizeParams& p, const int64_t slot) {
     __shared__ float s_key[BIG_CAND];
@@ -93,8 +93,14 @@ static __device__ __forceinline__ void finalize_big_slot(const FinalizeParams& p
         __syncthreads();
         if (tid == 0) s_n = 0;
         __syncthreads();
-        for (int pi = warp; pi < p.ntau; pi += BIG_THREADS / 32) {
-            int cnt = p.part_cnt[slot * p.ntau + pi];
+        // (the counts of this warp's next 32 pools in one read, so that a pool costs one memory round trip)
+        int counts = 0;
+        for (int pi = warp, turn = 0; pi < p.ntau; pi += BIG_THREADS / 32, ++turn) {
+            if ((turn & 31) == 0) {
+                const int mine = pi + lane * (BIG_THREADS / 32);
+                counts = mine < p.ntau ? p.part_cnt[slot * p.ntau + mine] : 0;
+            }
+            int cnt = __shfl_sync(FULL_MASK, counts, turn & 31);
             cnt = cnt < BIG_POOL ? cnt : BIG_POOL;
             const float* psc = p.part_sc + (slot * p.ntau + pi) * (int64_t)BIG_POOL;
             const uint32_t* pid = p.part_id + (slot * p.ntau + pi) * (int64_t)BIG_POOL;
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(BIG_THREADS) knn_finalize_big_kernel(FinalizeP
 
 int launch_knn_finalize_big(const FinalizeParams& p, int64_t max_slots, cudaStream_t st) {
     if (max_slots <= 0) return FL_OK;
-    FL_CHECK_ARG(p.part_cnt && p.part_tau && p.K1 == 2 * BIG_POOL && p.d <= 512 && p.k <= BIG_RERANK && p.count == max_slots,
+    FL_CHECK_ARG(p.part_cnt && p.part_tau && p.K1 == 4 * BIG_POOL && p.d <= 512 && p.k <= BIG_RERANK && p.count == max_slots,
                  "large-k finalisation: bad parameters");
     int64_t grid = max_slots;
     if (p.count_dev != nullptr && grid > (int64_t)sm_count() * 4) grid = (int64_t)sm_count() * 4;

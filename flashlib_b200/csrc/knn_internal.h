@@ -158,12 +158,13 @@ struct TcKnnParams {
     const void* dbrows;      // bf16 [m_pad][d_pad]
     const float* hnorm;      // f32 [m_pad]
     int64_t m, m_pad; int d_pad;
+    int d_used;              // columns before the first that is zero in every row (0: not known, d_pad)
     int K1;                  // entries a pool keeps (informational: fixed by the kernel mode)
     int nsplit; int64_t tiles_per_split;   // database tiles of 256 rows per split
     float* part_sc; uint32_t* part_id;     // [nq_pad][nsplit][tc_partial_len]
     float* tau;              // f32 [nq_pad], running per-query thresholds, -inf initialised
-    float* part_tau;         // f32 [nq_pad][nsplit][tc_taus_per_range]: thresholds each (query, range) ended with
-    int* part_cnt;           // large-k pools only: i32 [nq_pad][nsplit][tc_taus_per_range] entries per pool
+    float* part_tau;         // f32 [nq_pad][nsplit][pools per range]: thresholds each (query, range) ended with
+    int* part_cnt;           // large-k pools only: i32 [nq_pad][nsplit][pools per range] entries per pool
     float* seed_cls;         // f32 [nq_pad][max(1, seed_splits)][32] scratch of the threshold-seeding pass (nullptr: no seeding)
     int seed_tiles, seed_splits, seed_rank;   // > 0: sample and rank of tc_seed_plan
     int deep_pools;          // 1: pools keep tc_deep_pool_size() entries and publish tc_deep_partial_len() per
@@ -176,8 +177,9 @@ struct TcKnnParams {
     int item_tile_cap;       // seeding pass over item tables: tiles of every item's range it samples
     const int* item_order;   // optional, with item tables: order in which the items are dealt to the CTAs
     void* pair_pools;        // optional: pools kept in global memory as (score f32, row u32) pairs,
-                             //   [nq_pad][nsplit][tc_taus_per_range][tc_pair_pool_cap(k)]; entry counts go to
+                             //   [nq_pad][nsplit][pools per range][tc_pair_pool_cap(k)]; entry counts go to
                              //   part_cnt, thresholds to part_tau, part_sc / part_id are not used
+    void* lists;             // scratch of the scoring pass (tc_list_bytes), unless it uses pair_pools or deep_pools
     int k;                   // neighbours wanted: selects the pool geometry (tc_knn_big)
     int big_pools;           // 1: the large global-memory pools whatever k is (no pool in shared memory:
                              //    room for a query tile of up to 384 feature columns)
@@ -191,10 +193,13 @@ int tc_pool_size(int k);
 // Entries the tensor-core pass publishes per (query, range): a multiple of the pool size.
 int tc_partial_len(int k);
 int tc_deep_pool_size();
-int tc_use_deep_pools(int k, int d_pad, int nsplit, int64_t nq_pad);
+int tc_use_deep_pools(int k, int d_pad, int nsplit);
 int tc_deep_partial_len();
-// Thresholds the tensor-core pass publishes per (query, range).
-int tc_taus_per_range();
+// Pools, each with its threshold, that the tensor-core pass publishes per (query, range): the plain modes' lists, and the
+// deep pools and pair pools.
+int tc_lists_per_range();
+int tc_pair_pools_per_range();
+int64_t tc_list_bytes(int64_t items, int k);
 // Slots of a (query row, warpgroup) pool in the global pair-pool modes.
 int tc_pair_pool_cap(int k);
 // Calls bound by latencies rather than by the tensor pipe, their row ranges, and the seeding sample of any
@@ -229,9 +234,9 @@ int tc_debug_active();       // 1 while experiment flags are set
 int tc_prof_read(unsigned long long* host_out, int words);
 int launch_knn_tc_debug(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cudaStream_t st);
 void tc_split_plan(int64_t nq_pad, int64_t m_pad, int k, int* nsplit, int64_t* tiles_per_split);
-int tc_pair_enabled(int64_t nq_pad, int k);
-// Query rows of the bf16 query plane for nq queries: whole tiles of 128 (whole pairs of tiles when
-// CTA pairs are requested).
+int tc_pair_enabled(int64_t nq_pad);
+// Query rows of the bf16 query plane for nq queries outside the small-problem plan: whole tiles of 128, or whole
+// pairs of tiles.
 int64_t tc_query_rows_padded(int64_t nq);
 int launch_knn_tc(const TcKnnParams& p, cudaStream_t st);
 // k-means assignment on the same pipeline: asg_sc [nq_pad][2][2] (best, second-best score per

@@ -7,16 +7,23 @@
 // side, -||x||^2/2 split into three bf16 terms on the database side), so one extra K=16 MMA
 // step makes every accumulator element the score
 //     s = <q, x> - ||x||^2 / 2          (larger = closer)
-// and the epilogue only compares: scores above a row's threshold feed that query's
-// candidate pool in shared memory.  Nothing of the 128 x 256 score tile ever reaches global
-// memory; per query and range only the two warpgroups' pools (32 entries each, 12 kept at a
-// compaction; deeper or global-memory pools in the modes described below) and their final
-// thresholds are written, unsorted.
+// and the epilogue only compares: column groups with a score above a row's threshold go to a queue of
+// that row's thread, and from there the scores that still pass to the row's candidate list, both
+// in scratch that stays in the L2.  Nothing of the 128 x 256 score tile is stored; per query and
+// range only the four warpgroups' lists (16 entries each; deeper or other pools in the modes
+// described below) and their final thresholds are published, unsorted.
 //
-// Warp roles (320 threads): warps 0-7 epilogue in two warpgroups (group g takes columns
-// 128g..128g+127 of every accumulator; warp w reads TMEM lanes 32(w%4)..32(w%4)+31, one query
-// row per thread, and keeps a pool per row), warp 8 TMA producer, warp 9 MMA issuer and TMEM
-// owner.
+// Warp roles of the list modes (608 threads): warps 0-15 epilogue in four warpgroups (group g takes
+// columns 64g..64g+63 of every accumulator; warp w reads TMEM lanes 32(w%4)..32(w%4)+31, one query
+// row per thread, and keeps a list per row), warp 16 TMA producer, warps 17 and 18 MMA issuers (every
+// other tile each; warp 17 owns the TMEM allocation).  The other modes (352 threads) have two epilogue
+// warpgroups of 128 columns.  What bounds the list modes, 10 000 x 1M x 128, k = 10 (scoring pass 2.56 ms
+// with two warpgroups, pools in shared memory and one issuing lane): 1 152 cycles of tensor core a tile,
+// which run at about 1.6 PFLOP/s before the power limit, and the epilogue's ALU pipe beside it
+// (half a three-input maximum a score, 16 lanes a cycle): 2.05 ms; its screening alone would allow 1.74,
+// the MMAs alone 1.63.  Four warpgroups because two warps a scheduler leave half of that pipe idle; the queue
+// because a flagged group costs a warp 10 instructions that way, and 40 when its scores are compared and
+// appended on the spot (2.36 ms), wherever its lanes' scores then go.
 // Every wait is bounded; a wait that gives up raises a CTA-wide abort flag, records where
 // it happened in the status words and every role falls through to the common exit.
 #include "knn_internal.h"
@@ -32,15 +39,19 @@ constexpr int TC_BM = 128;            // queries per tile (MMA M)
 constexpr int TC_BN = 256;            // database rows per tile (MMA N)
 constexpr int TC_BK = 64;             // bf16 features per shared-memory chunk (128 bytes)
 constexpr int TC_NWG = 2;             // epilogue warpgroups; group g owns columns 128g.. of every tile
-constexpr int TC_K1 = 12;             // entries a (query, warpgroup) pool keeps at compaction
-constexpr int TC_CAP = 32;            // pool capacity before compaction
-constexpr int TC_PSTR = TC_CAP + 1;   // padded pool row stride (bank spread); the extra slot is scratch
-constexpr int TC_BIG_K1 = 128;        // large-k mode (16 < k <= 128): pools live in global memory,
-constexpr int TC_BIG_CAP = 256;       // directly in the published-pool buffers
+constexpr int TC_LIST_NWG = 4;        // ... of the list modes: columns 64g..
+constexpr int TC_LIST_PUB = 16, TC_LIST_K1 = 16, TC_LIST_CAP = 32;            // list modes: entries published, kept at a
+constexpr int TC_BIG_PUB = 128, TC_BIG_K1 = 128, TC_BIG_CAP = 256;            // compaction, working capacity (k <= 16; beyond)
+// List modes: queue of flagged column groups of an epilogue thread, slots of 8 scores and a row number (48 bytes).  Emptied by
+// all warps of the CTA at every TC_QUEUE_EVERY-th tile, and by a warp that could overflow with the next tile's 8.
+constexpr int TC_QUEUE_EVERY = 64, TC_QUEUE_SLOTS = 24, TC_QUEUE_SLOT_BYTES = 48, TC_QUEUE_FULL = TC_QUEUE_SLOTS - 8;
+constexpr int TC_QUEUE_BYTES = TC_QUEUE_SLOTS * TC_QUEUE_SLOT_BYTES;
 constexpr int TC_MID_K1 = 24;         // deep-pool mode: a query has few pools (inverted-file scan: two per
 constexpr int TC_MID_CAP = 48;        // probed list), so each must reach further below the k-th neighbour
 constexpr int TC_MID_PUB = 64;        // published entries per pool in that mode (padded)
-constexpr int TC_THREADS = (4 * TC_NWG + 2) * 32;
+constexpr int TC_MMA_WARPS = 2;       // MMA issuers; issuer j owns accumulator j, i.e. every other tile
+constexpr int TC_THREADS = (4 * TC_NWG + 1 + TC_MMA_WARPS) * 32;
+constexpr int TC_LIST_THREADS = (4 * TC_LIST_NWG + 1 + TC_MMA_WARPS) * 32;
 constexpr int TC_A_CHUNK = TC_BM * 128;   // bytes of one K-chunk of the query tile
 constexpr int TC_A_AUG = TC_BM * 32;      // bytes of the query tile's 16 norm columns
 constexpr int TC_B_CHUNK = TC_BN * 128;   // bytes of one K-chunk of a database tile
@@ -59,7 +70,7 @@ struct TcSmemPlan {
 };
 
 // nabuf: query-tile buffers (2: the next item's tile is loaded while the current item is scored).
-static TcSmemPlan tc_smem_plan(int d_pad, int smem_limit, int pool_stride = TC_PSTR, int slot_bytes = TC_B_STAGE, int nabuf = 1) {
+static TcSmemPlan tc_smem_plan(int d_pad, int smem_limit, int pool_stride, int slot_bytes = TC_B_STAGE, int nabuf = 1) {
     TcSmemPlan s{};
     s.nkc = d_pad / TC_BK;
     int cur = 0;
@@ -96,6 +107,7 @@ __device__ unsigned long long g_tc_prof[160 * TC_PROF_WORDS];
 
 struct TcKernelParams {
     int n_qtiles, n_tiles, nsplit, tiles_per_split, nkc, nstage;
+    int last_steps;          // K = 16 steps of a tile's last chunk that hold features at all (1 to 4)
     int nabuf;               // query-tile buffers in shared memory (1 or 2)
     int stream_a;            // 1: the query tile is not resident; its chunk travels with every database chunk
     int off_b, off_pool_sc, off_pool_id, off_bar;
@@ -113,6 +125,7 @@ struct TcKernelParams {
     const int* item_order;   // optional, with item tables: the CTAs walk item item_order[i] in place of item i
                              //   (longest ranges first, so that the round-robin deal comes out even)
     float* seed_cls;         // seeding output: [nq_pad][nsplit][TC_NWG][16] class maxima
+    void* lists;             // list modes: working lists of every CTA, tc_list_bytes()
     float2* gpool;           // global-pool modes: (score, row) pairs, [nq_pad][nsplit][TC_NWG][CAP]
     float* asg_sc; uint32_t* asg_id;   // assignment mode outputs: [rows][TC_NWG] x (best, second) / centroid
     int32_t* status;
@@ -122,8 +135,8 @@ struct TcKernelParams {
                              // after the MMA lane has, wait twice as long, so the status names the wait
                              // nearest to the cause.
     int tile_stride;         // database tile actually read for loop index t is t * tile_stride (1 outside seeding)
-    int dbg_flags;           // timing experiments (results invalid): 1 skip pass 2, 2 skip the
-                             // reductions of pass 1, 4 skip the tensor-memory loads too, 8 skip the
+    int dbg_flags;           // timing experiments (results invalid): 1 flag nothing, 4 skip the
+                             // screening too, 8 skip the
                              // norm-column MMA step, 16 issue no MMA at all (operand streaming only);
                              // 32 the producer leaves out its fourth operand load, so the MMA lane's
                              // wait for it runs out (host-visible test of the bounded-wait exit)
@@ -150,25 +163,8 @@ __device__ __forceinline__ void tc_report_timeout(int32_t* status, int role, int
     }
 }
 
-// Compacts the pools of the rows named in `need` (one bit per lane = row of this warp).
-// Kept out of line: compaction is rare and the sorting network is large.
-// `stride` = elements between the pools of consecutive rows.
-template <int CAP, int K1>
-static __device__ __noinline__ float2 tc_compact_rows(unsigned need, float* warp_sc, uint32_t* warp_id, int64_t stride,
-                                                      int cnt, float tau) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    while (need) {
-        const int src = __ffs(need) - 1;
-        need &= need - 1;
-        const int n = __shfl_sync(FULL_MASK, cnt, src);
-        const float thr = warp_pool_compact<(CAP + 31) / 32>(warp_sc + src * stride, warp_id + src * stride, n, K1);
-        if (lane == src) { cnt = min(n, K1); tau = fmaxf(tau, thr); }
-    }
-    return make_float2(__int_as_float(cnt), tau);
-}
-
-// Same for pools stored as (score, row) pairs of 8 bytes (the deep-pool mode), `stride` pairs apart.
+// Compacts the pools of the rows named in `need` (one bit per lane = row of this warp): (score, row) pairs of 8 bytes,
+// `stride` pairs from row to row.  Kept out of line: compaction is rare and the sorting network is large.
 template <int CAP, int K1>
 static __device__ __noinline__ float2 tc_compact_rows_pairs(unsigned need, float2* warp_pool, int stride, int cnt, float tau) {
     constexpr int NPL = (CAP + 31) / 32;
@@ -202,6 +198,26 @@ static __device__ __noinline__ float2 tc_compact_rows_pairs(unsigned need, float
     return make_float2(__int_as_float(cnt), tau);
 }
 
+// Appends the scores of x[0..7] (rows col0 ..) that exceed tau at ADDR, which moves on: the 8 comparisons first
+// (independent), then the predicated stores, so that only the address increments form a chain.
+#define FL_APPEND(ST, ADD, C, ADDR)                                                                                    \
+    asm volatile(                                                                                                      \
+        "{\n\t.reg .pred p0, p1, p2, p3, p4, p5, p6, p7;\n\t.reg .b32 c;\n\t"                                         \
+        "setp.gt.f32 p0, %3, %1;\n\tsetp.gt.f32 p1, %4, %1;\n\tsetp.gt.f32 p2, %5, %1;\n\tsetp.gt.f32 p3, %6, %1;\n\t" \
+        "setp.gt.f32 p4, %7, %1;\n\tsetp.gt.f32 p5, %8, %1;\n\tsetp.gt.f32 p6, %9, %1;\n\tsetp.gt.f32 p7, %10, %1;\n\t" \
+        "@p0 " ST " [%0], {%3, %2};\n\t@p0 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 1;\n\t"                              \
+        "@p1 " ST " [%0], {%4, c};\n\t@p1 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 2;\n\t"                               \
+        "@p2 " ST " [%0], {%5, c};\n\t@p2 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 3;\n\t"                               \
+        "@p3 " ST " [%0], {%6, c};\n\t@p3 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 4;\n\t"                               \
+        "@p4 " ST " [%0], {%7, c};\n\t@p4 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 5;\n\t"                               \
+        "@p5 " ST " [%0], {%8, c};\n\t@p5 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 6;\n\t"                               \
+        "@p6 " ST " [%0], {%9, c};\n\t@p6 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 7;\n\t"                               \
+        "@p7 " ST " [%0], {%10, c};\n\t@p7 " ADD " %0, %0, 8;\n\t}"                                                  \
+        : "+" C(ADDR)                                                                                                  \
+        : "r"(__float_as_uint(tau)), "r"(col0), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]),      \
+          "r"(x[6]), "r"(x[7])                                                                                         \
+        : "memory")
+
 // MODE 1 (TC_MODE_SEED) turns the kernel into the threshold-seeding pass: it scans a strided sample of
 // the database tiles and, instead of pools, keeps 16 running maxima per query row over
 // disjoint column classes; their minimum is a score that 16 distinct rows reach, i.e. a valid
@@ -212,18 +228,14 @@ static __device__ __noinline__ float2 tc_compact_rows_pairs(unsigned need, float
 // score of its row in registers (the column index rides in the low 7 mantissa bits of the
 // score) and no pool is touched.
 //
-// MODE 3 (TC_MODE_KNN_BIG) is MODE 0 for 16 < k <= 128: pools of 256 entries (128 kept) that do not
-// fit shared memory; they live in global memory, in place in the published-pool buffers (appends
-// are predicated stores, compaction reads them back through the L2), and each pool's entry
-// count is published with it.
+// MODE 3 (TC_MODE_KNN_BIG) is MODE 0 for 16 < k <= 112 (lists of 256, 128 kept and published).
 //
 // MODE 4 (TC_MODE_KNN_MID) is MODE 0 with deeper pools in shared memory (24 of 48 kept, 64
 // published): for callers whose queries have only a few pools each (a small database scored as
 // one range; the inverted-file scan, where a query row meets only the tiles of one list).  There a
-// row has a candidate in most tiles, which the screen-then-revisit epilogue of MODE 0 handles
-// badly (every group of columns ends up revisited, one latency-bound step each); this mode
-// compares every score against the row's threshold and appends the passing ones with predicated
-// 8-byte stores -- three instructions per score, no branch, no second pass.
+// row has a candidate in most tiles, so queueing whole groups would store most of the scores; this mode
+// compares the scores of flagged groups against the row's threshold on the spot and appends the passing
+// ones with predicated 8-byte stores.
 //
 // MODE 5 (TC_MODE_KNN_GPOOL) is MODE 4 with the pools in global memory, as (score, row) pairs in
 // the buffer the finalisation reads (64 slots per (query row, warpgroup), 24 kept at a
@@ -231,15 +243,10 @@ static __device__ __noinline__ float2 tc_compact_rows_pairs(unsigned need, float
 // slots deep -- two whole tiles, where MODE 4 has room for one and stalls on every load -- and
 // nothing is copied out when an item ends.  The inverted-file scan runs in this mode.
 //
-// MODE 6 (TC_MODE_KNN_GS) is MODE 0 with its small pools (32 slots, 12 kept) in global memory, in
-// place in the published-pool buffers like MODE 3: appends are rare in MODE 0 (about a hundred per
-// query row and launch), so their stores and the compactions' reads can afford the L2, and the
-// 67 KB of shared memory the pools took go to the TMA ring (four slots instead of three at 128
-// features, four instead of two at 256).
-//
 // MODE 7 (TC_MODE_KNN_GPOOL_BIG) is MODE 5 with 256 slots, 128 kept, for 16 < k <= 112.
 constexpr int TC_MODE_KNN = 0, TC_MODE_SEED = 1, TC_MODE_ASSIGN = 2, TC_MODE_KNN_BIG = 3, TC_MODE_KNN_MID = 4,
-              TC_MODE_KNN_GPOOL = 5, TC_MODE_KNN_GS = 6, TC_MODE_KNN_GPOOL_BIG = 7;
+              TC_MODE_KNN_GPOOL = 5, TC_MODE_KNN_GPOOL_BIG = 7;
+constexpr bool tc_list_mode(int mode) { return mode == TC_MODE_KNN || mode == TC_MODE_KNN_BIG; }
 constexpr int TC_GP_K1 = 24, TC_GP_CAP = 64;
 //
 // PAIR: two CTAs of a cluster work as one (tcgen05 cta_group::2).  CTA r of the pair owns query
@@ -250,10 +257,12 @@ constexpr int TC_GP_K1 = 24, TC_GP_CAP = 64;
 // Operand and accumulator barriers live in the leader; "slot free", "query tile free" and
 // "accumulator full" are committed to both CTAs.
 template <bool DBG, int MODE, bool PAIR = false>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(tc_list_mode(MODE) ? TC_LIST_THREADS : TC_THREADS, 1)
 knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_aug,
               const __grid_constant__ CUtensorMap map_db, const __grid_constant__ CUtensorMap map_db_aug,
               const TcKernelParams p) {
+    constexpr bool LIST = tc_list_mode(MODE);
+    constexpr int NWG = LIST ? TC_LIST_NWG : TC_NWG, COLS = TC_BN / NWG;
     extern __shared__ uint8_t smem_raw[];
     // the swizzled operand tiles need 1024-byte aligned shared memory
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -262,13 +271,12 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const uint32_t a_aug_addr = sbase + p.nkc * TC_A_CHUNK;       // 4 KB: the query tile's norm columns
     const uint32_t b_addr = sbase + p.off_b;                      // nstage slots of 40 KB
     float* pool_sc = reinterpret_cast<float*>(smem + p.off_pool_sc);
-    uint32_t* pool_id = reinterpret_cast<uint32_t*>(smem + p.off_pool_id);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.off_bar);
     // barrier slots: [0, 6) full, [6, 12) empty, 12 a_full, 13 a_empty, 14-15 tmem_full, 16-17 tmem_empty,
-    // 18 a_full / 19 a_empty of the second query-tile buffer
+    // 18 a_full / 19 a_empty of the second query-tile buffer, 22-23 turn of MMA warp 0 / 1
     const uint32_t bar0 = smem_u32(bars);
     auto BAR = [&](int i) { return bar0 + 8u * i; };
-    constexpr int B_FULL = 0, B_EMPTY = 6, B_AFULL = 12, B_AEMPTY = 13, B_TFULL = 14, B_TEMPTY = 16;
+    constexpr int B_FULL = 0, B_EMPTY = 6, B_AFULL = 12, B_AEMPTY = 13, B_TFULL = 14, B_TEMPTY = 16, B_TURN = 22;
     // Query-tile buffer of item number i of this CTA: buffer i % nabuf, used for the (i / nabuf)-th time.
     const uint32_t a_stride = (uint32_t)(p.nkc * TC_A_CHUNK + TC_A_AUG);
     const bool two_a = !PAIR && p.nabuf == 2;
@@ -299,14 +307,15 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     if (tid == 0) {
         for (int i = 0; i < TC_MAX_STAGES; ++i) { mbar_init(BAR(B_FULL + i), 1); mbar_init(BAR(B_EMPTY + i), 1); }
         mbar_init(BAR(B_AFULL), 1);
-        mbar_init(BAR(B_AEMPTY), 1);
+        mbar_init(BAR(B_AEMPTY), TC_MMA_WARPS);
         mbar_init(BAR(18), 1);
-        mbar_init(BAR(19), 1);
-        for (int i = 0; i < 2; ++i) { mbar_init(BAR(B_TFULL + i), 1); mbar_init(BAR(B_TEMPTY + i), 4 * TC_NWG * OPERAND_CTAS); }
+        mbar_init(BAR(19), TC_MMA_WARPS);
+        for (int i = 0; i < TC_MMA_WARPS; ++i) mbar_init(BAR(B_TURN + i), 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(BAR(B_TFULL + i), 1); mbar_init(BAR(B_TEMPTY + i), 4 * NWG * OPERAND_CTAS); }
         *abort_flag = 0;
         fence_barrier_init();
     }
-    constexpr int W_PRODUCER = 4 * TC_NWG, W_MMA = 4 * TC_NWG + 1;
+    constexpr int W_PRODUCER = 4 * NWG, W_MMA = 4 * NWG + 1;
     if (warp == W_PRODUCER && lane == 0) {
         prefetch_tensormap(&map_q); prefetch_tensormap(&map_q_aug);
         prefetch_tensormap(&map_db); prefetch_tensormap(&map_db_aug);
@@ -337,83 +346,114 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
     if (warp == W_PRODUCER) {
         // ------------------------------ TMA producer --------------------------------------
-        if (lane == 0) {
-            uint32_t fill = 0;     // database chunks issued so far
-            uint32_t item_no = 0;
-            bool ok = true;
-            TC_PROF(long long prof_a = 0;)
-            // loads of a pair are credited to the leader's barrier, which expects both CTAs' bytes
-            auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
-                if (PAIR) tma_load_2d_pair(dst, map, c0, c1, bar); else tma_load_2d(dst, map, c0, c1, bar);
-            };
-            for (int it = it_first; it < n_items && ok; it += it_step, ++item_no) {
-                const int itp = p.item_order != nullptr ? __ldg(p.item_order + it) : it;
-                const int split = itp / n_units, unit = itp - split * n_units;
-                const int qt = PAIR ? 2 * unit + (int)cta_rank : unit;
-                int t0, t1;
-                tc_item_range(p, itp, split, t0, t1);
-                const uint32_t ab = a_buf(item_no), a_off = ab * a_stride;
-                if (!stream_a) {
-                    if (!mbar_wait(a_empty_bar(ab), a_phase(item_no) ^ 1u, abort_flag, 2 * p.wait_ns, p.wait_hint_ns)) {
-                        tc_report_timeout(p.status, 4, ab ? 19 : B_AEMPTY); ok = false; break;
-                    }
+        // (the whole warp walks the loop and an elected lane issues, as in the MMA warps: from a `lane == 0`
+        // branch a 128-feature tile's three loads and two waits took 1 500 cycles)
+        const uint32_t elected = elect_one();
+        int s = 0;             // ring slot and its phase
+        uint32_t ph = 0;
+        int fill = 0;
+        uint32_t item_no = 0;
+        bool ok = true;
+        TC_PROF(long long prof_a = 0;)
+        // loads of a pair are credited to the leader's barrier, which expects both CTAs' bytes
+        auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+            if (PAIR) tma_load_2d_pair(dst, map, c0, c1, bar); else tma_load_2d(dst, map, c0, c1, bar);
+        };
+        auto wait = [&](uint32_t bar, int name, uint32_t parity) {
+            const bool got = __all_sync(FULL_MASK, mbar_wait(bar, parity, abort_flag, 2 * p.wait_ns, p.wait_hint_ns));
+            if (!got && lane == 0) tc_report_timeout(p.status, 4, name);
+            return got;
+        };
+        for (int it = it_first; it < n_items && ok; it += it_step, ++item_no) {
+            const int itp = p.item_order != nullptr ? __ldg(p.item_order + it) : it;
+            const int split = itp / n_units, unit = itp - split * n_units;
+            const int qt = PAIR ? 2 * unit + (int)cta_rank : unit;
+            int t0, t1;
+            tc_item_range(p, itp, split, t0, t1);
+            const uint32_t ab = a_buf(item_no), a_off = ab * a_stride;
+            if (!stream_a) {
+                ok = wait(a_empty_bar(ab), ab ? 19 : B_AEMPTY, a_phase(item_no) ^ 1u);
+                if (!ok) break;
+                if (elected) {
                     if (leader) mbar_expect_tx(a_full_bar(ab), (p.nkc * TC_A_CHUNK + TC_A_AUG) * OPERAND_CTAS);
                     for (int kc = 0; kc < p.nkc; ++kc)
                         load(a_addr + a_off + kc * TC_A_CHUNK, &map_q, kc * TC_BK, qt * TC_BM, a_full_bar(ab));
                     load(a_aug_addr + a_off, &map_q_aug, d_pad, qt * TC_BM, a_full_bar(ab));
                 }
-                const int nt = t1 - t0;
-                const int rot = (int)(((int64_t)unit * nt) / n_units);
-                for (int i = 0; i < nt && ok; ++i) {
-                    // Query tiles walk their range from different starting tiles, so the CTAs of a
-                    // wave do not all ask the L2 for the same lines at the same moment.
-                    const int t = t0 + (i + rot < nt ? i + rot : i + rot - nt);
-                    for (int kc = 0; kc < p.nkc; ++kc, ++fill) {
-                        const int s = fill % p.nstage;
-                        const uint32_t ph = (fill / p.nstage) & 1;
-                        TC_PROF(const long long c0 = clock64();)
-                        if (!mbar_wait(BAR(B_EMPTY + s), ph ^ 1, abort_flag, 2 * p.wait_ns, p.wait_hint_ns)) {
-                            tc_report_timeout(p.status, 4, B_EMPTY + s); ok = false; break;
-                        }
-                        TC_PROF(prof_a += clock64() - c0;)
+                __syncwarp();
+            }
+            const int nt = t1 - t0;
+            const int rot = (int)(((int64_t)unit * nt) / n_units);
+            for (int i = 0; i < nt && ok; ++i) {
+                // Query tiles walk their range from different starting tiles, so the CTAs of a
+                // wave do not all ask the L2 for the same lines at the same moment.
+                const int t = t0 + (i + rot < nt ? i + rot : i + rot - nt);
+                const int row0 = t * p.tile_stride * TC_BN + (int)cta_rank * B_ROWS;
+                for (int kc = 0; kc < p.nkc; ++kc, ++fill) {
+                    TC_PROF(const long long c0 = clock64();)
+                    ok = wait(BAR(B_EMPTY + s), B_EMPTY + s, ph ^ 1u);
+                    if (!ok) break;
+                    TC_PROF(prof_a += clock64() - c0;)
+                    if (elected && !(DBG && (p.dbg_flags & 32) && fill == 3)) {       // (32: this slot never fills)
                         const bool last = (kc == p.nkc - 1);
-                        const int row0 = t * p.tile_stride * TC_BN + (int)cta_rank * B_ROWS;
-                        if (DBG && (p.dbg_flags & 32) && fill == 3) continue;   // this slot never fills
-                        const uint32_t slot = b_addr + s * slot_bytes;
+                        const uint32_t slot = b_addr + s * slot_bytes, full = BAR(B_FULL + s);
                         if (leader) {
                             uint32_t bytes = (last ? SLOT_B_BYTES : SLOT_CHUNK) * OPERAND_CTAS;
                             if (stream_a) bytes += TC_A_CHUNK + (last ? TC_A_AUG : 0);
-                            mbar_expect_tx(BAR(B_FULL + s), bytes);
+                            mbar_expect_tx(full, bytes);
                         }
-                        load(slot, &map_db, kc * TC_BK, row0, BAR(B_FULL + s));
-                        if (last) load(slot + SLOT_CHUNK, &map_db_aug, d_pad, row0, BAR(B_FULL + s));
+                        load(slot, &map_db, kc * TC_BK, row0, full);
+                        if (last) load(slot + SLOT_CHUNK, &map_db_aug, d_pad, row0, full);
                         if (stream_a) {
-                            load(slot + SLOT_B_BYTES, &map_q, kc * TC_BK, qt * TC_BM, BAR(B_FULL + s));
-                            if (last) load(slot + SLOT_B_BYTES + TC_A_CHUNK, &map_q_aug, d_pad, qt * TC_BM, BAR(B_FULL + s));
+                            load(slot + SLOT_B_BYTES, &map_q, kc * TC_BK, qt * TC_BM, full);
+                            if (last) load(slot + SLOT_B_BYTES + TC_A_CHUNK, &map_q_aug, d_pad, qt * TC_BM, full);
                         }
                     }
+                    __syncwarp();
+                    if (++s == p.nstage) { s = 0; ph ^= 1u; }
                 }
             }
-            TC_PROF(if (blockIdx.x < 160) g_tc_prof[blockIdx.x * TC_PROF_WORDS + 0] = prof_a;)
-            if (!ok) {
-                // give copies already in flight a bounded time to land before the CTA exits
-                const uint64_t t_start = globaltimer_ns();
-                while (globaltimer_ns() - t_start < 2000000ull) { }
-            }
         }
-    } else if (warp == W_MMA) {
+        TC_PROF(if (lane == 0 && blockIdx.x < 160) g_tc_prof[blockIdx.x * TC_PROF_WORDS + 0] = prof_a;)
+        if (!ok) {
+            // give copies already in flight a bounded time to land before the CTA exits
+            const uint64_t t_start = globaltimer_ns();
+            while (globaltimer_ns() - t_start < 2000000ull) { }
+        }
+    } else if (warp >= W_MMA && warp < W_MMA + TC_MMA_WARPS) {
         // ------------------------------ MMA issuer -----------------------------------------
-        if (lane == 0 && leader) {
+        // Bound by the serial cost of issuing, which must stay below the tensor core's 128 cycles a K = 16 step.
+        // Two things keep it there.  A whole warp walks the loop and one elected lane issues: from a `lane == 0`
+        // branch a chunk of four MMAs took 682 cycles however narrow they were (operands moved to uniform
+        // registers under divergence), elected and unrolled 410.  And two warps take turns by tile: a wait that
+        // succeeds at once and a commit cost about 200 cycles each, so one warp needs 1 450 cycles for the nine
+        // steps of a 128-feature tile (1 152 cycles of tensor core).  A warp hands the turn on with its last MMA: its
+        // commits and its wait for the accumulator fall into the other's turn.  (The turn also keeps the waits on
+        // the ring in order: a slot's barrier is only asked about a phase when the one before has completed.)
+        // Scoring of 10 000 x 1M x 128, one CTA a tile and the epilogue of before: 2.55 ms -> 2.22.
+        if (leader) {
             constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * TC_BM : TC_BM, TC_BN);
+            const uint32_t elected = elect_one();
             auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
                 if (DBG && (p.dbg_flags & 16)) return;     // timing experiment: operand streaming only
                 if (PAIR) umma_bf16_pair(d, a, b, idesc, acc); else umma_bf16(d, a, b, idesc, acc);
             };
             auto commit = [&](uint32_t bar) { if (PAIR) umma_commit_pair(bar); else umma_commit(bar); };
-            uint32_t use = 0;      // database chunks consumed so far
-            uint32_t tile_no = 0;  // tiles issued so far (accumulator ring position)
+            // all lanes wait; a lane that gave up takes the others with it
+            auto wait = [&](int bar, uint32_t parity) {
+                const bool got = __all_sync(FULL_MASK, mbar_wait(BAR(bar), parity, abort_flag, p.wait_ns, p.wait_hint_ns));
+                if (!got && lane == 0) tc_report_timeout(p.status, 5, bar);
+                return got;
+            };
+            const int b = warp - W_MMA;            // this warp's accumulator and tiles
+            const uint32_t d_tmem = tmem_base + b * TC_BN;
+            int s = 0;             // ring slot of the current tile's first chunk and its phase
+            uint32_t ph = 0;
+            uint32_t tile_no = 0;  // tiles so far, the other warp's included
             uint32_t item_no = 0;
+            uint32_t turn = b == 0 ? 1u : 0u;      // the first turn is warp 0's without being handed to it
             bool ok = true;
+            auto skip = [&](int chunks) { for (s += chunks; s >= p.nstage; s -= p.nstage) ph ^= 1u; };
             TC_PROF(long long prof_full = 0; long long prof_tempty = 0;)
             for (int it = it_first; it < n_items && ok; it += it_step, ++item_no) {
                 const int itp = p.item_order != nullptr ? __ldg(p.item_order + it) : it;
@@ -421,82 +461,131 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 int t0, t1;
                 tc_item_range(p, itp, split, t0, t1);
                 const uint32_t ab = a_buf(item_no), a_off = ab * a_stride;
-                if (!stream_a && !mbar_wait(a_full_bar(ab), a_phase(item_no), abort_flag, p.wait_ns, p.wait_hint_ns)) {
-                    tc_report_timeout(p.status, 5, ab ? 18 : B_AFULL); ok = false; break;
+                if (!stream_a) {
+                    ok = wait(ab ? 18 : B_AFULL, a_phase(item_no));
+                    if (!ok) break;
                 }
                 for (int t = t0; t < t1 && ok; ++t, ++tile_no) {
-                    const int b = tile_no & 1;
+                    if ((int)(tile_no & 1) != b) { skip(p.nkc); continue; }
                     TC_PROF(const long long c0 = clock64();)
-                    if (!mbar_wait(BAR(B_TEMPTY + b), ((tile_no >> 1) & 1) ^ 1, abort_flag, p.wait_ns, p.wait_hint_ns)) {
-                        tc_report_timeout(p.status, 5, B_TEMPTY + b); ok = false; break;
-                    }
+                    ok = wait(B_TEMPTY + b, ((tile_no >> 1) & 1) ^ 1);
+                    if (!ok) break;
                     TC_PROF(prof_tempty += clock64() - c0;)
-                    tc_fence_after_sync();
-                    const uint32_t d_tmem = tmem_base + b * TC_BN;
-                    for (int kc = 0; kc < p.nkc; ++kc, ++use) {
-                        const int s = use % p.nstage;
-                        const uint32_t ph = (use / p.nstage) & 1;
+                    ok = wait(B_TURN + b, turn);
+                    if (!ok) break;
+                    turn ^= 1u;
+                    for (int kc = 0; kc < p.nkc; ++kc) {
                         TC_PROF(const long long c1 = clock64();)
-                        if (!mbar_wait(BAR(B_FULL + s), ph, abort_flag, p.wait_ns, p.wait_hint_ns)) {
-                            tc_report_timeout(p.status, 5, B_FULL + s); ok = false; break;
-                        }
+                        ok = wait(B_FULL + s, ph);
+                        if (!ok) break;
                         TC_PROF(prof_full += clock64() - c1;)
                         tc_fence_after_sync();
-                        const uint32_t slot = b_addr + s * slot_bytes;
-                        const bool last = kc == p.nkc - 1;
-                        const uint64_t da = umma_desc(stream_a ? slot + SLOT_B_BYTES : a_addr + a_off + kc * TC_A_CHUNK);
-                        const uint64_t db = umma_desc(slot);
-#pragma unroll
-                        for (int k4 = 0; k4 < TC_BK / 16; ++k4) {
+                        if (elected) {
+                            const uint32_t slot = b_addr + s * slot_bytes;
+                            const bool last = kc == p.nkc - 1;
+                            const uint64_t da = umma_desc(stream_a ? slot + SLOT_B_BYTES : a_addr + a_off + kc * TC_A_CHUNK);
+                            const uint64_t db = umma_desc(slot);
                             // +32 bytes per 16-feature step inside the 128-byte swizzled row
-                            mma(d_tmem, da + 2 * k4, db + 2 * k4, (kc | k4) != 0 ? 1u : 0u);
+                            mma(d_tmem, da, db, kc != 0 ? 1u : 0u);
+                            if (!last || p.last_steps == TC_BK / 16) {
+#pragma unroll
+                                for (int k4 = 1; k4 < TC_BK / 16; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u);
+                            } else {
+                                // columns of zeros beyond the last feature: 96 features take 7 steps with the norm
+                                // columns in place of 9
+                                for (int k4 = 1; k4 < p.last_steps; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u);
+                            }
+                            if (last && !(DBG && (p.dbg_flags & 8))) {
+                                // norm columns: ones x split(-||x||^2/2), 32-byte rows, 32-byte swizzle
+                                const uint32_t a_aug = stream_a ? slot + SLOT_B_BYTES + TC_A_CHUNK : a_aug_addr + a_off;
+                                mma(d_tmem, umma_desc_sw32(a_aug), umma_desc_sw32(slot + SLOT_CHUNK), 1u);
+                            }
+                            if (last) mbar_arrive(BAR(B_TURN + (b ^ 1)));
+                            commit(BAR(B_EMPTY + s));   // slot reusable once these MMAs retire
+                            if (last) commit(BAR(B_TFULL + b));
                         }
-                        if (last && !(DBG && (p.dbg_flags & 8))) {
-                            // norm columns: ones x split(-||x||^2/2), 32-byte rows, 32-byte swizzle
-                            const uint32_t a_aug = stream_a ? slot + SLOT_B_BYTES + TC_A_CHUNK : a_aug_addr + a_off;
-                            mma(d_tmem, umma_desc_sw32(a_aug), umma_desc_sw32(slot + SLOT_CHUNK), 1u);
-                        }
-                        commit(BAR(B_EMPTY + s));   // slot reusable once these MMAs retire
+                        __syncwarp();
+                        skip(1);
                     }
-                    if (ok) commit(BAR(B_TFULL + b));
                 }
-                if (ok && !stream_a) commit(a_empty_bar(ab));     // query tile buffer reusable
+                if (ok && !stream_a && elected) commit(a_empty_bar(ab));     // query tile buffer reusable (both warps' word)
+                __syncwarp();
             }
-            TC_PROF(if (blockIdx.x < 160) {
+            TC_PROF(if (lane == 0 && b == 0 && blockIdx.x < 160) {
                 g_tc_prof[blockIdx.x * TC_PROF_WORDS + 1] = prof_full;
                 g_tc_prof[blockIdx.x * TC_PROF_WORDS + 2] = prof_tempty;
             })
         }
-    } else {
+    } else if (warp < W_PRODUCER) {
         // ------------------------------ epilogue warps --------------------------------------
-        // warp = 4 * warpgroup + TMEM lane quarter; warpgroup g reads columns 128g .. 128g+127 of
+        // warp = 4 * warpgroup + TMEM lane quarter; warpgroup g reads columns COLS g .. COLS (g + 1) - 1 of
         // every accumulator and keeps its own pool per query row.
         const int wg = warp >> 2, quarter = warp & 3;
         constexpr bool BIG = (MODE == TC_MODE_KNN_BIG);
-        constexpr bool GS = (MODE == TC_MODE_KNN_GS);
-        constexpr bool GLOB = BIG || GS;                 // pools addressed in global memory
         constexpr bool MID = (MODE == TC_MODE_KNN_MID);
         constexpr bool GPB = (MODE == TC_MODE_KNN_GPOOL_BIG);
         constexpr bool GP = (MODE == TC_MODE_KNN_GPOOL) || GPB;
-        constexpr int CAP = (BIG || GPB) ? TC_BIG_CAP : MID ? TC_MID_CAP : GP ? TC_GP_CAP : TC_CAP;
-        constexpr int K1 = (BIG || GPB) ? TC_BIG_K1 : MID ? TC_MID_K1 : GP ? TC_GP_K1 : TC_K1;
-        constexpr int PSTR = CAP + 1;                    // shared pools: padded stride, slot CAP is scratch
-        constexpr int PUB = BIG ? TC_BIG_CAP : MID ? TC_MID_PUB : TC_CAP;   // published entries per pool
-        // pool of lane 0's row and distance (elements) between the pools of consecutive rows
-        float* warp_sc = pool_sc + warp * 32 * PSTR;
-        uint32_t* warp_id = pool_id + warp * 32 * PSTR;
-        int64_t pstride = PSTR;
-        float* my_sc = warp_sc + lane * PSTR;
-        uint32_t* my_id = warp_id + lane * PSTR;
+        constexpr int CAP = (BIG || GPB) ? TC_BIG_CAP : LIST ? TC_LIST_CAP : MID ? TC_MID_CAP : TC_GP_CAP;
+        constexpr int K1 = (BIG || GPB) ? TC_BIG_K1 : LIST ? TC_LIST_K1 : MID ? TC_MID_K1 : TC_GP_K1;
+        constexpr int PSTR = CAP + 1;                    // shared pools: padded stride
+        constexpr int PUB = BIG ? TC_BIG_PUB : LIST ? TC_LIST_PUB : TC_MID_PUB;   // published entries per pool
         const uint32_t lane_taddr = tmem_base + (uint32_t(quarter * 32) << 16);
         uint32_t tile_no = 0;
         bool ok = true;
-        TC_PROF(long long prof_tfull = 0; long long prof_rare = 0; long long prof_cc = 0;
+        TC_PROF(long long prof_tfull = 0; long long prof_rare = 0; long long prof_cc = 0; long long prof_flush = 0;
                 unsigned prof_groups = 0; unsigned prof_compact = 0; unsigned prof_append = 0;
                 const long long prof_t0 = clock64();)
         // hands accumulator b back to the MMA lane (of the leader, for a pair)
         auto release_acc = [&](int b) {
             if (PAIR) mbar_arrive_cluster(BAR(B_TEMPTY + b), 0u); else mbar_arrive(BAR(B_TEMPTY + b));
+        };
+        // List modes: this thread's queue of flagged groups and its row's working list, both its CTA's own scratch.
+        float tau = neg_inf();
+        int cnt = 0;
+        char* const scratch = static_cast<char*>(p.lists) + ((int64_t)blockIdx.x * (4 * NWG) + warp) * (32 * (TC_QUEUE_BYTES + CAP * 8));
+        float2* const warp_list = reinterpret_cast<float2*>(scratch + 32 * TC_QUEUE_BYTES);
+        const uint64_t queue = reinterpret_cast<uint64_t>(scratch + lane * TC_QUEUE_BYTES);
+        uint64_t queue_end = queue;
+        // The queued scores that still pass move to the lists, every lane its own group a step.
+        auto flush = [&]() {
+            TC_PROF(const long long cf0 = clock64();)
+            const uint32_t bytes = (uint32_t)(queue_end - queue), most = __reduce_max_sync(FULL_MASK, bytes);
+            float2* const list = warp_list + lane * CAP;
+#pragma unroll 1
+            for (uint32_t o0 = 0; o0 < most; o0 += 2 * TC_QUEUE_SLOT_BYTES) {
+                float4 x[2][2];
+                uint32_t first[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const uint32_t o = o0 + u * TC_QUEUE_SLOT_BYTES;
+                    x[u][0] = x[u][1] = make_float4(neg_inf(), neg_inf(), neg_inf(), neg_inf());
+                    first[u] = 0;
+                    if (o < bytes) {
+                        const float4* slot = reinterpret_cast<const float4*>(queue + o);
+                        x[u][0] = slot[0];
+                        x[u][1] = slot[1];
+                        first[u] = *reinterpret_cast<const uint32_t*>(slot + 2);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (u > 0 && o0 + u * TC_QUEUE_SLOT_BYTES >= most) break;
+                    const unsigned need = __ballot_sync(FULL_MASK, cnt > CAP - 8);
+                    if (need) {
+                        TC_PROF(prof_compact += __popc(need); const long long cc0 = clock64();)
+                        const float2 cr = tc_compact_rows_pairs<CAP, K1>(need, warp_list, CAP, cnt, tau);
+                        TC_PROF(prof_cc += clock64() - cc0;)
+                        cnt = __float_as_int(cr.x);
+                        tau = cr.y;
+                    }
+                    const float sv[8] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w, x[u][1].x, x[u][1].y, x[u][1].z, x[u][1].w};
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (sv[j] > tau) list[cnt++] = make_float2(sv[j], __uint_as_float(first[u] + j));
+                }
+            }
+            queue_end = queue;
+            TC_PROF(prof_flush += clock64() - cf0;)
         };
         for (int it = it_first; it < n_items && ok; it += it_step) {
             const int itp = p.item_order != nullptr ? __ldg(p.item_order + it) : it;
@@ -513,16 +602,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 qidx = __ldg(p.row_query + qrow);
                 if (qidx >= 0) tau_in = fmaxf(tau_in, __ldcg(p.tau_q + qidx));
             }
-            if (GLOB) {
-                pstride = (int64_t)p.nsplit * TC_NWG * CAP;
-                const int64_t o = (((int64_t)(qt * TC_BM + quarter * 32) * p.nsplit + split) * TC_NWG + wg) * CAP;
-                warp_sc = p.part_sc + o;
-                warp_id = p.part_id + o;
-                my_sc = warp_sc + lane * pstride;
-                my_id = warp_id + lane * pstride;
-            }
-            float tau = tau_in;
-            int cnt = 0;
+            tau = tau_in;
+            cnt = 0;
             float cls[16];
 #pragma unroll
             for (int c = 0; c < 16; ++c) cls[c] = neg_inf();
@@ -542,8 +623,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 TC_PROF(prof_tfull += clock64() - c0;)
                 tc_fence_after_sync();
                 // this warpgroup's half of the accumulator columns / of the tile's database rows
-                const uint32_t tile_taddr = lane_taddr + b * TC_BN + wg * (TC_BN / TC_NWG);
-                const uint32_t row_base = (uint32_t)t * TC_BN + wg * (TC_BN / TC_NWG);
+                const uint32_t tile_taddr = lane_taddr + b * TC_BN + wg * COLS;
+                const uint32_t row_base = (uint32_t)t * TC_BN + wg * COLS;
 
                 // Pass 1, branch free: stream the 256 scores of this thread's query row through
                 // registers, 64 columns per wait, and note which groups of 8 columns hold a score
@@ -621,9 +702,9 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 if (GP || MID) {
                     // This row's pool of (score, row) pairs -- in global memory (GP) or shared memory (MID) --
                     // and the address of its next free slot.
-                    float2* warp_pool = GP ? p.gpool + (((int64_t)(qt * TC_BM + quarter * 32) * p.nsplit + split) * TC_NWG + wg) * CAP
+                    float2* warp_pool = GP ? p.gpool + (((int64_t)(qt * TC_BM + quarter * 32) * p.nsplit + split) * NWG + wg) * CAP
                                            : reinterpret_cast<float2*>(pool_sc) + warp * 32 * PSTR;
-                    const int gstride = GP ? p.nsplit * TC_NWG * CAP : PSTR;      // pairs between the pools of consecutive rows
+                    const int gstride = GP ? p.nsplit * NWG * CAP : PSTR;      // pairs between the pools of consecutive rows
                     const uint64_t my_addr = reinterpret_cast<uint64_t>(warp_pool + (int64_t)lane * gstride);
                     const uint32_t my_saddr = MID ? smem_u32(warp_pool + lane * gstride) : 0u;
                     tmem_ld_32x32b_x32(tile_taddr, va);
@@ -677,26 +758,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                                 // the address increments form a chain
                                 const uint32_t col0 = row_base + slice * 32 + g * 8;
                                 const uint32_t* x = v + g * 8;
-#define FL_APPEND(ST, ADD, C, ADDR)                                                                                    \
-    asm volatile(                                                                                                      \
-        "{\n\t.reg .pred p0, p1, p2, p3, p4, p5, p6, p7;\n\t.reg .b32 c;\n\t"                                         \
-        "setp.gt.f32 p0, %3, %1;\n\tsetp.gt.f32 p1, %4, %1;\n\tsetp.gt.f32 p2, %5, %1;\n\tsetp.gt.f32 p3, %6, %1;\n\t" \
-        "setp.gt.f32 p4, %7, %1;\n\tsetp.gt.f32 p5, %8, %1;\n\tsetp.gt.f32 p6, %9, %1;\n\tsetp.gt.f32 p7, %10, %1;\n\t" \
-        "@p0 " ST " [%0], {%3, %2};\n\t@p0 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 1;\n\t"                              \
-        "@p1 " ST " [%0], {%4, c};\n\t@p1 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 2;\n\t"                               \
-        "@p2 " ST " [%0], {%5, c};\n\t@p2 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 3;\n\t"                               \
-        "@p3 " ST " [%0], {%6, c};\n\t@p3 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 4;\n\t"                               \
-        "@p4 " ST " [%0], {%7, c};\n\t@p4 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 5;\n\t"                               \
-        "@p5 " ST " [%0], {%8, c};\n\t@p5 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 6;\n\t"                               \
-        "@p6 " ST " [%0], {%9, c};\n\t@p6 " ADD " %0, %0, 8;\n\tadd.u32 c, %2, 7;\n\t"                               \
-        "@p7 " ST " [%0], {%10, c};\n\t@p7 " ADD " %0, %0, 8;\n\t}"                                                  \
-        : "+" C(ADDR)                                                                                                  \
-        : "r"(__float_as_uint(tau)), "r"(col0), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]),      \
-          "r"(x[6]), "r"(x[7])                                                                                         \
-        : "memory")
                                 if (MID) FL_APPEND("st.shared.v2.b32", "add.u32", "r", saddr);
                                 else FL_APPEND("st.global.v2.b32", "add.u64", "l", waddr);
-#undef FL_APPEND
                             }
                         };
                         append(va, 0);
@@ -709,6 +772,21 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                     }
                     continue;
                 }
+                // All 128 scores of this thread's query row into registers, and the accumulator back to the MMA warps
+                // at once: it is theirs again after about 300 cycles, where reading it in two halves, screening
+                // and coming back for the flagged groups held it for 1 000 to 1 500 -- with two accumulators and 1 152
+                // cycles of MMA a tile, that was what paced the kernel.
+                // List modes.  All 64 scores of this thread's row into registers and the accumulator back to the MMA
+                // warps at once; then which groups of 8 columns hold a score above the row's threshold (branch free).
+                // A flagged group goes to the thread's queue as it is, without a look at the single scores.
+                tmem_ld_32x32b_x32(tile_taddr, va);
+                tmem_ld_32x32b_x32(tile_taddr + 32, vb);
+                tmem_ld_wait();
+                reg_fence32(va);
+                reg_fence32(vb);
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) release_acc(b);
                 unsigned hits = 0;
                 auto scan = [&](uint32_t (&v)[32], int slice) {
 #pragma unroll
@@ -730,230 +808,117 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                     }
                 };
                 if (!DBG || !(p.dbg_flags & 4)) {
-                    tmem_ld_32x32b_x32(tile_taddr, va);
-                    tmem_ld_32x32b_x32(tile_taddr + 32, vb);
-                    tmem_ld_wait();
-                    reg_fence32(va);
-                    reg_fence32(vb);
-                    tmem_ld_32x32b_x32(tile_taddr + 64, vc);
-                    tmem_ld_32x32b_x32(tile_taddr + 96, vd);
                     scan(va, 0);
                     scan(vb, 1);
-                    tmem_ld_wait();
-                    reg_fence32(vc);
-                    reg_fence32(vd);
-                    scan(vc, 2);
-                    scan(vd, 3);
                 }
                 if (DBG && (p.dbg_flags & 1)) hits = 0;
-
-                // Pass 2, rare.  A lane seldom has more than one flagged group in a tile, so the
-                // work is split in two: (a) a small loop copies every flagged group from tensor
-                // memory and each flagged lane keeps the 8 scores of its first flagged group in
-                // registers -- after that the accumulator goes back to the MMA warp; (b) all lanes
-                // handle their kept group together in one straight-line step (a lone warp pays a
-                // few cycles per instruction, so once per tile beats once per group).  Further
-                // flagged groups of the same lane ("late") are handled one by one before (b).
-                unsigned wm = __reduce_or_sync(FULL_MASK, hits);
+                const unsigned wm = __reduce_or_sync(FULL_MASK, hits);
                 if (wm) {
-                    TC_PROF(const long long cr0 = clock64();)
-                    float sv[8];
+                    TC_PROF(const long long cr0 = clock64(); prof_groups += __popc(wm);)
+                    auto enqueue = [&](uint32_t (&v)[32], int slice) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) sv[j] = neg_inf();
-                    uint32_t scb = 0;
-                    bool have = false;
-                    unsigned late = 0;
-                    do {
-                        // four flagged groups per round trip: a copy from tensor memory takes a few
-                        // hundred cycles and tcgen05.wait::ld waits for all copies in flight
-                        int gs[4];
-                        bool live[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int f = __ffs(wm) - 1;          // -1 when no group is left
-                            live[k] = f >= 0;
-                            gs[k] = f >= 0 ? f : 0;
-                            wm &= wm - 1;                         // 0 stays 0
+                        for (int g = 0; g < 4; ++g) {
+                            const unsigned bit = 1u << (slice * 4 + g);
+                            if (!(wm & bit)) continue;                        // (uniform)
+                            const uint32_t* x = v + g * 8;
+                            asm volatile(
+                                "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+                                "@p st.global.v4.b32 [%0], {%3, %4, %5, %6};\n\t"
+                                "@p st.global.v4.b32 [%0+16], {%7, %8, %9, %10};\n\t"
+                                "@p st.global.b32 [%0+32], %2;\n\t@p add.u64 %0, %0, %11;\n\t}"
+                                : "+l"(queue_end)
+                                : "r"(hits & bit), "r"(row_base + slice * 32 + g * 8), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]),
+                                  "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "n"(TC_QUEUE_SLOT_BYTES)
+                                : "memory");
                         }
-                        uint32_t rn[4][8];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) tmem_ld_32x32b_x8(tile_taddr + gs[k] * 8, rn[k]);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) reg_fence8(rn[k]);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const bool mine = live[k] && ((hits >> gs[k]) & 1u);
-                            const bool take = mine && !have;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) sv[j] = take ? __uint_as_float(rn[k][j]) : sv[j];
-                            scb = take ? row_base + gs[k] * 8 : scb;
-                            late |= (mine && have) ? (1u << gs[k]) : 0u;
-                            have = have || mine;
-                            TC_PROF(prof_groups += live[k] ? 1 : 0;)
-                        }
-                    } while (wm);
-                    unsigned wl = __reduce_or_sync(FULL_MASK, late);
-#pragma unroll 1
-                    while (wl) {
-                        const int g = __ffs(wl) - 1;
-                        wl &= wl - 1;
-                        const unsigned need = __ballot_sync(FULL_MASK, cnt > CAP - 8);
-                        if (need) {
-                            TC_PROF(prof_compact += __popc(need);)
-                            const float2 cr = tc_compact_rows<CAP, K1>(need, warp_sc, warp_id, pstride, cnt, tau);
-                            cnt = __float_as_int(cr.x);
-                            tau = cr.y;
-                        }
-                        uint32_t r[8];
-                        tmem_ld_32x32b_x8(tile_taddr + g * 8, r);
-                        tmem_ld_wait();
-                        reg_fence8(r);
-                        unsigned pm = 0;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) pm |= (__uint_as_float(r[j]) > tau) ? (1u << j) : 0u;
-                        pm = ((late >> g) & 1u) ? pm : 0u;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const bool pass = (pm >> j) & 1u;
-                            const int pos = pass ? cnt + __popc(pm & ((1u << j) - 1u)) : CAP;
-                            if (!GLOB || pass) {      // shared pools: slot CAP is the row's scratch slot
-                                my_sc[pos] = __uint_as_float(r[j]);
-                                my_id[pos] = row_base + g * 8 + j;
-                            }
-                        }
-                        cnt += __popc(pm);
-                        TC_PROF(prof_append += __popc(pm);)
-                    }
-                    // every flagged score is in registers or in a pool: hand the accumulator back
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) release_acc(b);
-                    // (b) all lanes at once
-                    const unsigned need = __ballot_sync(FULL_MASK, cnt > CAP - 8);
-                    if (need) {
-                        TC_PROF(prof_compact += __popc(need); const long long cc0 = clock64();)
-                        const float2 cr = tc_compact_rows<CAP, K1>(need, warp_sc, warp_id, pstride, cnt, tau);
-                        TC_PROF(prof_cc += clock64() - cc0;)
-                        cnt = __float_as_int(cr.x);
-                        tau = cr.y;
-                    }
-                    unsigned pm = 0;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) pm |= (sv[j] > tau) ? (1u << j) : 0u;   // sv is -inf without a kept group
-                    const int np = __popc(pm);
-                    if (!__any_sync(FULL_MASK, np > 1)) {
-                        // at most one passing score per lane: it is the maximum of the group
-                        const float mx = fmaxf(fmax3(sv[0], sv[1], sv[2]), fmax3(fmax3(sv[3], sv[4], sv[5]), sv[6], sv[7]));
-                        const int pos = np ? cnt : CAP;
-                        if (!GLOB || np) {
-                            my_sc[pos] = mx;
-                            my_id[pos] = scb + (__ffs(pm) - 1);
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const bool pass = (pm >> j) & 1u;
-                            const int pos = pass ? cnt + __popc(pm & ((1u << j) - 1u)) : CAP;
-                            if (!GLOB || pass) {
-                                my_sc[pos] = sv[j];
-                                my_id[pos] = scb + j;
-                            }
-                        }
-                    }
-                    cnt += np;
-                    TC_PROF(prof_append += np;)
+                    };
+                    enqueue(va, 0);
+                    enqueue(vb, 1);
                     TC_PROF(prof_rare += clock64() - cr0;)
-                } else {
-                    // nothing flagged: hand the accumulator back right away
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) release_acc(b);
                 }
+                const bool full = (uint32_t)(queue_end - queue) > (uint32_t)(TC_QUEUE_FULL * TC_QUEUE_SLOT_BYTES);
+                if ((tile_no & (TC_QUEUE_EVERY - 1)) == TC_QUEUE_EVERY - 1 || __any_sync(FULL_MASK, full)) flush();
             }
+            if (LIST) flush();
             if (!ok) break;
             if (MODE == TC_MODE_ASSIGN) {
-                const int64_t o = qrow * TC_NWG + wg;
+                const int64_t o = qrow * NWG + wg;
                 p.asg_sc[2 * o] = b1;
                 p.asg_sc[2 * o + 1] = b2;
-                p.asg_id[o] = (uint32_t)tbest * TC_BN + wg * (TC_BN / TC_NWG) + (__float_as_uint(b1) & 0x7Fu);
+                p.asg_id[o] = (uint32_t)tbest * TC_BN + wg * (TC_BN / NWG) + (__float_as_uint(b1) & 0x7Fu);
                 continue;
             }
             if (MODE == TC_MODE_SEED) {
-                float4* o = reinterpret_cast<float4*>(p.seed_cls + ((qrow * p.nsplit + split) * TC_NWG + wg) * 16);
+                float4* o = reinterpret_cast<float4*>(p.seed_cls + ((qrow * p.nsplit + split) * NWG + wg) * 16);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) o[c] = make_float4(cls[4 * c], cls[4 * c + 1], cls[4 * c + 2], cls[4 * c + 3]);
                 continue;
             }
-            // end of the item: publish every row's pool as it stands (up to TC_CAP entries, the rest
-            // padded) and the row's threshold.  The pool is not sorted here: the finalize kernel
-            // merges the published entries anyway.
-            if (BIG) {
-                // the pools already are the published buffers
-                p.part_cnt[(qrow * p.nsplit + split) * TC_NWG + wg] = cnt;
-                p.part_tau[(qrow * p.nsplit + split) * TC_NWG + wg] = tau;
-                if (tau > tau_in) __stcg(p.tau + qrow, tau);
-                continue;
-            }
-            if (GS) {
-                // the pools already are the published buffers: pad the unused slots
-                for (int e = cnt; e < CAP; ++e) { my_sc[e] = neg_inf(); my_id[e] = INVALID_ID; }
-                p.part_tau[(qrow * p.nsplit + split) * TC_NWG + wg] = tau;
+            // end of the item: publish every row's pool (the rest of its slots padded, or its entry count beside it) and
+            // the row's threshold.  Nothing is sorted here: the finalisation merges the published entries anyway.
+            if (LIST) {
+                const unsigned need = __ballot_sync(FULL_MASK, cnt > PUB);
+                if (need) {
+                    const float2 cr = tc_compact_rows_pairs<CAP, K1>(need, warp_list, CAP, cnt, tau);
+                    cnt = __float_as_int(cr.x);
+                    tau = cr.y;
+                }
+                __syncwarp();
+                const int64_t o = (qrow * p.nsplit + split) * NWG + wg;
+                p.part_tau[o] = tau;
+                if (BIG) p.part_cnt[o] = cnt;
+                constexpr int PER = PUB < 32 ? PUB : 32, ROWS = 32 / PER;        // lanes a row, rows a step
+#pragma unroll 2
+                for (int r0 = 0; r0 < 32; r0 += ROWS) {
+                    const int src = r0 + lane / PER;
+                    const int n = __shfl_sync(FULL_MASK, cnt, src);
+                    const int64_t q = (int64_t)qt * TC_BM + quarter * 32 + src;
+                    const int64_t to = ((q * p.nsplit + split) * NWG + wg) * PUB;
+#pragma unroll
+                    for (int e = lane % PER; e < PUB; e += PER) {
+                        if (BIG && e >= n) break;
+                        const float2 v = e < n ? warp_list[src * CAP + e] : make_float2(neg_inf(), __uint_as_float(INVALID_ID));
+                        p.part_sc[to + e] = v.x;
+                        p.part_id[to + e] = __float_as_uint(v.y);
+                    }
+                }
+                __syncwarp();
                 if (tau > tau_in) __stcg(p.tau + qrow, tau);
                 continue;
             }
             if (GP) {
                 // the pools already are the published buffers
-                p.part_cnt[(qrow * p.nsplit + split) * TC_NWG + wg] = cnt;
-                p.part_tau[(qrow * p.nsplit + split) * TC_NWG + wg] = tau;
+                p.part_cnt[(qrow * p.nsplit + split) * NWG + wg] = cnt;
+                p.part_tau[(qrow * p.nsplit + split) * NWG + wg] = tau;
                 if (tau > tau_in) __stcg(p.tau + qrow, tau);
                 if (qidx >= 0 && tau > tau_in) atomic_max_f32(p.tau_q + qidx, tau);
                 continue;
             }
             __syncwarp();
-            if (MID) {
-                const float2* warp_pool = reinterpret_cast<const float2*>(pool_sc) + warp * 32 * PSTR;
-#pragma unroll 1
-                for (int src = 0; src < 32; ++src) {
-                    const int n = __shfl_sync(FULL_MASK, cnt, src);
-                    const float2* row = warp_pool + src * PSTR;
-                    const int64_t q = (int64_t)qt * TC_BM + quarter * 32 + src;
-                    const int64_t o = ((q * p.nsplit + split) * TC_NWG + wg) * PUB;
-#pragma unroll
-                    for (int e = lane; e < PUB; e += 32) {
-                        const float2 v = e < n ? row[e] : make_float2(neg_inf(), __uint_as_float(INVALID_ID));
-                        p.part_sc[o + e] = v.x;
-                        p.part_id[o + e] = __float_as_uint(v.y);
-                    }
-                }
-                p.part_tau[(qrow * p.nsplit + split) * TC_NWG + wg] = tau;
-                if (tau > tau_in) __stcg(p.tau + qrow, tau);
-                if (qidx >= 0 && tau > tau_in) atomic_max_f32(p.tau_q + qidx, tau);
-            } else {
+            const float2* warp_pool = reinterpret_cast<const float2*>(pool_sc) + warp * 32 * PSTR;
 #pragma unroll 1
             for (int src = 0; src < 32; ++src) {
                 const int n = __shfl_sync(FULL_MASK, cnt, src);
-                const float* rsc = warp_sc + src * PSTR;
-                const uint32_t* rid = warp_id + src * PSTR;
+                const float2* row = warp_pool + src * PSTR;
                 const int64_t q = (int64_t)qt * TC_BM + quarter * 32 + src;
-                const int64_t o = ((q * p.nsplit + split) * TC_NWG + wg) * PUB;
+                const int64_t o = ((q * p.nsplit + split) * NWG + wg) * PUB;
 #pragma unroll
                 for (int e = lane; e < PUB; e += 32) {
-                    p.part_sc[o + e] = e < n ? rsc[e] : neg_inf();
-                    p.part_id[o + e] = e < n ? rid[e] : INVALID_ID;
+                    const float2 v = e < n ? row[e] : make_float2(neg_inf(), __uint_as_float(INVALID_ID));
+                    p.part_sc[o + e] = v.x;
+                    p.part_id[o + e] = __float_as_uint(v.y);
                 }
             }
-            p.part_tau[(qrow * p.nsplit + split) * TC_NWG + wg] = tau;
+            p.part_tau[(qrow * p.nsplit + split) * NWG + wg] = tau;
             if (tau > tau_in) __stcg(p.tau + qrow, tau);
             if (qidx >= 0 && tau > tau_in) atomic_max_f32(p.tau_q + qidx, tau);
-            }
         }
         TC_PROF(
         if (warp == 0 && lane == 0 && blockIdx.x < 160) {
             unsigned long long* pr = g_tc_prof + blockIdx.x * TC_PROF_WORDS;
             pr[3] = prof_tfull; pr[4] = prof_rare; pr[5] = prof_groups; pr[6] = prof_compact; pr[7] = prof_append;
             pr[8] = clock64() - prof_t0; pr[9] = tile_no;
-            pr[10] = 0; pr[11] = prof_cc;
+            pr[10] = prof_flush; pr[11] = prof_cc;
         }
         )
     }
@@ -1105,20 +1070,27 @@ static int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int c
     return FL_OK;
 }
 
+// Scratch of the list modes: a working list per epilogue thread of every CTA that `items` work items can occupy.
+int64_t tc_list_bytes(int64_t items, int k) {
+    const int64_t ctas = items < sm_count() ? items : sm_count();
+    return ctas * 4 * TC_LIST_NWG * 32 * (TC_QUEUE_BYTES + (tc_knn_big(k) ? TC_BIG_CAP : TC_LIST_CAP) * 8);
+}
 int tc_knn_big(int k) { return k > 16 ? 1 : 0; }
-int tc_pool_size(int k) { return tc_knn_big(k) ? TC_BIG_K1 : TC_K1; }
-int tc_partial_len(int k) { return TC_NWG * (tc_knn_big(k) ? TC_BIG_CAP : TC_CAP); }
+int tc_pool_size(int k) { return tc_knn_big(k) ? TC_BIG_K1 : TC_LIST_K1; }
+int tc_partial_len(int k) { return TC_LIST_NWG * (tc_knn_big(k) ? TC_BIG_PUB : TC_LIST_PUB); }
+static int tc_pair_requested();
 // Deep pools for plain k <= 16 scoring when the whole database is one range, i.e. a query ends up
 // with just two pools: the larger of two 12th-best scores sits too close to the k-th neighbour
 // for the proof (a quarter of the rows of a 1M x 1M self-kNN failed it).  With three ranges the
 // shallow pools prove every row of the benchmark mixture and are faster.  Needs the 128-feature
 // shared-memory budget.
-int tc_use_deep_pools(int k, int d_pad, int nsplit, int64_t nq_pad) {
-    return !tc_knn_big(k) && d_pad <= 128 && nsplit == 1 && !tc_pair_enabled(nq_pad, k);
+int tc_use_deep_pools(int k, int d_pad, int nsplit) {
+    return !tc_knn_big(k) && d_pad <= 128 && nsplit == 1 && tc_pair_requested() <= 0;
 }
 int tc_deep_pool_size() { return TC_MID_K1; }
 int tc_deep_partial_len() { return TC_NWG * TC_MID_PUB; }
-int tc_taus_per_range() { return TC_NWG; }
+int tc_pair_pools_per_range() { return TC_NWG; }
+int tc_lists_per_range() { return TC_LIST_NWG; }
 int tc_pair_pool_cap(int k) { return tc_knn_big(k) ? TC_BIG_CAP : TC_GP_CAP; }
 
 int tc_knn_supported(int64_t nq, int64_t m, int d, int k) {
@@ -1148,22 +1120,24 @@ int tc_knn_auto(int64_t nq, int64_t m, int d, int k) {
     return direct_estimate_us(nq, m, d) > tc;
 }
 
-// CTA pairs (cta_group::2) for plain k <= 16 scoring.  Measured on the 1M x 128 benchmark they are
-// 7 % slower than single CTAs (the leader's MMA reads half of every database tile from the peer's
-// shared memory and waits for both CTAs' epilogues), so they are off unless FLASHLIB_B200_TC_PAIR=1.
-int tc_pair_requested() {
-    static int on = -1;
-    if (on < 0) { const char* e = getenv("FLASHLIB_B200_TC_PAIR"); on = (e && atoi(e) != 0) ? 1 : 0; }
-    return on;
+// CTA pairs (cta_group::2) in the list modes: each CTA of a pair loads half of every database tile, which halves what the
+// L2 delivers to the SMs -- one CTA alone asks for 64 bytes a cycle, about all there is (10 000 x 1M x 128: scoring
+// 2.16 ms alone, 2.05 in pairs; with an epilogue that only reads the accumulators 1.87 and 1.63).  They need an even
+// number of query tiles, so an odd one is padded: 11 % more work at nine tiles, the fewest that come here
+// (tc_small), and less from there on.  FLASHLIB_B200_TC_PAIR=0/1 overrides.
+static int tc_pair_requested() {
+    static int v = -2;
+    if (v == -2) { const char* e = getenv("FLASHLIB_B200_TC_PAIR"); v = e ? (atoi(e) != 0 ? 1 : 0) : -1; }
+    return v;
 }
-// Pairs need an even number of query tiles (tc_query_rows_padded provides it).
-int tc_pair_enabled(int64_t nq_pad, int k) {
-    return tc_pair_requested() && !tc_knn_big(k) && (nq_pad / TC_BM) % 2 == 0 && nq_pad / TC_BM >= 2;
+int tc_pair_enabled(int64_t nq_pad) { return tc_pair_requested() != 0 && (nq_pad / TC_BM) % 2 == 0; }
+int64_t tc_query_rows_padded(int64_t nq) {
+    const bool even = tc_pair_requested() < 0 ? nq > 8 * TC_BM : tc_pair_requested() != 0;
+    return round_up(nq, even ? 2 * TC_BM : TC_BM);
 }
-int64_t tc_query_rows_padded(int64_t nq) { return round_up(nq, tc_pair_requested() ? 2 * TC_BM : TC_BM); }
 
 void tc_split_plan(int64_t nq_pad, int64_t m_pad, int k, int* nsplit, int64_t* tiles_per_split) {
-    const bool pair = tc_pair_enabled(nq_pad, k) != 0;
+    const bool pair = tc_pair_enabled(nq_pad) != 0;
     // work units that walk a range together, and how many of them the GPU runs at once
     const int64_t n_qtiles = pair ? nq_pad / TC_BM / 2 : nq_pad / TC_BM;
     const int64_t n_tiles = m_pad / TC_BN;
@@ -1227,7 +1201,7 @@ void tc_debug_set(int flags, unsigned wait_us) {
 // 1 000 554 -> 460; 3 000 1 240 -> 1 265), beyond that up to 64 tiles of work per SM (10 000 x 100 000
 // x 64, 208 tiles per SM: 507 -> 771).
 int tc_small(int64_t nq_pad, int64_t m_pad) {
-    if (tc_pair_requested()) return 0;
+    if (tc_pair_requested() > 0) return 0;
     const int64_t n_qtiles = nq_pad / TC_BM;
     return n_qtiles <= 8 || n_qtiles * (m_pad / TC_BN) <= 64 * (int64_t)sm_count();
 }
@@ -1266,7 +1240,7 @@ void tc_seed_plan(int64_t nq_pad, int64_t m_pad, int k, TcSeedPlan* w) {
     const int64_t aim = k <= 16 ? 10 * k + 200 : 6 * k + 50 > 250 ? 6 * k + 50 : 250;
     int64_t tiles = ceil_div(w->rank * n_tiles, aim);
     if (tiles < 16) tiles = 16;
-    if (n_qtiles > 8 && k <= 16 && tiles > 96) tiles = 96;       // (the scoring pass of many query tiles tightens them itself)
+    if (n_qtiles > 8 && k <= 16 && tiles > 192) tiles = 192;      // (the scoring pass of many query tiles tightens them itself)
     if (tiles > n_tiles) tiles = n_tiles;
     w->dense = tiles * 8 >= n_tiles;
     if (w->dense) w->rank = k + 6;
@@ -1312,18 +1286,13 @@ struct TcLaunch {
     TcSmemPlan sp;
     TcKernelParams kp;
     int seed_tiles, seed_rank;
-    bool big, mid, gs, gpb;
+    bool big, mid, gpb;
 };
 
-// Plain k <= 16 scoring with the small pools in global memory (mode KNN_GS) instead of shared memory.
-// Measured on 1M rows x 10 000 queries: 8 % slower at 128 features (2.86 vs 2.65 ms: the three-slot ring
-// was not what held the kernel back, and compactions through the L2 cost more), 12 % faster at 192 and
-// 21 % faster at 256 features (4.83 vs 5.85 ms), where pools in shared memory leave only two ring
-// slots.  So: beyond 128 features.  FLASHLIB_B200_TC_GS=0/1 overrides.
-static int tc_gs_requested(int d_pad) {
-    static int v = -2;
-    if (v == -2) { const char* e = getenv("FLASHLIB_B200_TC_GS"); v = e ? (atoi(e) != 0 ? 1 : 0) : -1; }
-    return v >= 0 ? v : (d_pad > 128 ? 1 : 0);
+static int tc_last_steps(const TcKnnParams& p) {
+    if (p.d_used <= 0) return TC_BK / 16;
+    const int rest = p.d_used - (p.d_pad - TC_BK);                 // features in the last chunk
+    return rest <= 16 ? 1 : (rest + 15) / 16;
 }
 
 // Everything a launch needs: tensor maps, shared-memory plan, kernel parameters and the size of
@@ -1333,9 +1302,6 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     L->big = (tc_knn_big(p.k) != 0 || p.big_pools != 0) && p.pair_pools == nullptr;
     L->gpb = p.pair_pools != nullptr && tc_knn_big(p.k) != 0;
     L->mid = p.deep_pools != 0;
-    const TcExperiment& ex0 = tc_experiment();
-    L->gs = !L->big && !L->mid && p.pair_pools == nullptr && dbg == nullptr && ex0.flags == 0 && p.row_query == nullptr &&
-            p.item_t0 == nullptr && !tc_pair_enabled(p.nq_pad, p.k) && tc_gs_requested(p.d_pad) != 0;
     const int pitch = p.d_pad + PLANE_AUG_COLS;
     int rc = cached_map_bf16(&L->map_q, p.qplane, p.nq_pad, pitch, TC_BK, TC_BM);
     if (rc == FL_OK) rc = cached_map_bf16(&L->map_q_aug, p.qplane, p.nq_pad, pitch, PLANE_AUG_COLS, TC_BM);
@@ -1346,7 +1312,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     // a query tile of more than 512 features is streamed with the database chunks
     const bool stream = p.d_pad > 512;
     FL_CHECK_ARG(!stream || p.pair_pools != nullptr, "tensor-core kNN launch: more than 512 features go with pair pools");
-    L->sp = tc_smem_plan(p.d_pad, smem_optin_bytes(), (L->big || L->gs || p.pair_pools != nullptr) ? 0 : L->mid ? TC_MID_CAP + 1 : TC_PSTR,
+    L->sp = tc_smem_plan(p.d_pad, smem_optin_bytes(), L->mid ? TC_MID_CAP + 1 : 0,
                          stream ? TC_STREAM_STAGE : TC_B_STAGE, stream ? 0 : 1);
     if (L->sp.nstage < 2) { set_error("tensor-core kNN: feature dimension %d leaves no room for the TMA ring", p.d_pad); return FL_EUNSUPPORTED; }
     const TcExperiment& ex = tc_experiment();
@@ -1356,6 +1322,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     kp.n_tiles = (int)(p.m_pad / TC_BN);
     kp.nsplit = p.nsplit;
     kp.tiles_per_split = (int)p.tiles_per_split;
+    kp.last_steps = tc_last_steps(p);
     kp.nkc = L->sp.nkc; kp.nstage = L->sp.nstage;
     kp.stream_a = stream ? 1 : 0;
     kp.off_b = L->sp.off_b; kp.off_pool_sc = L->sp.off_pool_sc; kp.off_pool_id = L->sp.off_pool_id;
@@ -1364,6 +1331,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     kp.tau = p.tau; kp.part_tau = p.part_tau; kp.status = p.status; kp.dbg_scores = dbg; kp.dbg_ld = dbg_ld;
     kp.part_cnt = p.part_cnt;
     kp.gpool = reinterpret_cast<float2*>(p.pair_pools);
+    kp.lists = p.lists;
     kp.seed_cls = p.seed_cls;
     kp.nq_dev = p.nq_dev; kp.item_t0 = p.item_t0; kp.item_t1 = p.item_t1; kp.item_order = p.item_order;
     kp.row_query = p.row_query; kp.tau_q = p.tau_q;
@@ -1374,7 +1342,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     // Seeding sample.  The threshold is the seed_rank-th largest of 32 class maxima, which sits
     // near rank 32 ln(32 / (32 - seed_rank)) of the sample, hence near that figure times
     // n_tiles / seed_tiles of the whole database.
-    //  k <= 16: the pools tighten the threshold quickly; one tile in 16 (at most 64 tiles, 96 for the
+    //  k <= 16: the pools tighten the threshold quickly; one tile in 16 (at most 64 tiles, 192 for the
     //           largest databases), k + 6 rows guaranteed.
     //  large k: the pools seldom fill, so the seeded threshold is what filters.  Aim at about
     //           rank 6 k of the database: loose enough that the k-th neighbour's error band
@@ -1394,10 +1362,10 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
 int tc_seed_tiles(int64_t m_pad, int k) {
     const int n_tiles = (int)(m_pad / TC_BN);
     const TcExperiment& ex = tc_experiment();
-    // one tile in 16, at most 64 -- 96 for the largest databases (measured on 3 907 tiles x 10 000
-    // queries: 64 tiles 2.795 ms per step, 96 2.767, 128 2.777, 160 2.797; on 489-tile shards x 80 000
-    // queries the 30 tiles of the rule beat 16 and 48)
-    int seed_tiles = n_tiles >= 3072 ? 96 : n_tiles >= 1024 ? 64 : n_tiles / 16;
+    // one tile in 16, at most 64 -- 192 for the largest databases (measured on 3 907 tiles x 10 000
+    // queries: 64 tiles 2.490 ms per step, 96 2.455, 128 2.385, 192 2.361, 256 2.391; on 489-tile shards x 80 000
+    // queries, with the epilogue of before, the 30 tiles of the rule beat 16 and 48)
+    int seed_tiles = n_tiles >= 3072 ? 192 : n_tiles >= 1024 ? 64 : n_tiles / 16;
 
     if (tc_knn_big(k)) {
         const double sample_rank = k >= 64 ? 22.2 : 9.2;
@@ -1477,7 +1445,7 @@ int launch_knn_tc_seed_select(const TcKnnParams& p, const TcSeedMargin& mg, cuda
 // Main scoring launch (thresholds in p.tau as they stand).
 static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cudaStream_t st) {
     const bool gp = p.pair_pools != nullptr;
-    FL_CHECK_ARG(p.part_tau && (gp ? p.part_cnt != nullptr : (p.part_sc && p.part_id)), "tensor-core kNN launch with a null buffer");
+    FL_CHECK_ARG(p.part_tau && (gp ? p.part_cnt != nullptr : (p.part_sc && p.part_id && (p.lists || p.deep_pools))), "tensor-core kNN launch with a null buffer");
     TcLaunch L;
     int rc = tc_prepare(p, dbg, dbg_ld, &L);
     if (rc != FL_OK) return rc;
@@ -1492,10 +1460,9 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
     const int pitch = p.d_pad + PLANE_AUG_COLS;
     const int items = kp.n_qtiles * kp.nsplit;
     const int grid = items < sm_count() ? items : sm_count();
-    // CTA pairs (cta_group::2): plain k <= 16 scoring over uniform ranges, an even number of query
-    // tiles, at least one pair-item per cluster of a full grid.  FLASHLIB_B200_TC_PAIR=0/1 overrides.
+    // CTA pairs (cta_group::2): list modes over uniform ranges and an even number of query tiles.
     const bool pair = !gp && !mid && dbg == nullptr && p.item_t0 == nullptr && p.nq_dev == nullptr &&
-                      tc_pair_enabled(p.nq_pad, p.k);
+                      tc_pair_enabled(p.nq_pad);
     if (L.gpb) {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
         knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
@@ -1507,18 +1474,19 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
         rc = cached_map_bf16(&map_db_h, p.dbrows, p.m_pad, pitch, TC_BK, TC_BN / 2);
         if (rc == FL_OK) rc = cached_map_bf16(&map_db_aug_h, p.dbrows, p.m_pad, pitch, PLANE_AUG_COLS, TC_BN / 2);
         if (rc != FL_OK) return rc;
-        const TcSmemPlan spp = tc_smem_plan(p.d_pad, smem_optin_bytes(), TC_PSTR, TC_B_STAGE / 2);
+        const TcSmemPlan spp = tc_smem_plan(p.d_pad, smem_optin_bytes(), 0, TC_B_STAGE / 2);
         TcKernelParams kq = kp;
         kq.nstage = spp.nstage; kq.off_b = spp.off_b; kq.off_pool_sc = spp.off_pool_sc; kq.off_pool_id = spp.off_pool_id;
         kq.off_bar = spp.off_bar;
         const int pair_items = (kp.n_qtiles / 2) * kp.nsplit;
         int clusters = sm_count() / 2;
         if (clusters > pair_items) clusters = pair_items;
-        auto kern = kp.dbg_flags != 0 ? knn_tc_kernel<true, TC_MODE_KNN, true> : knn_tc_kernel<false, TC_MODE_KNN, true>;
+        auto kern = big ? knn_tc_kernel<false, TC_MODE_KNN_BIG, true>
+                        : kp.dbg_flags != 0 ? knn_tc_kernel<true, TC_MODE_KNN, true> : knn_tc_kernel<false, TC_MODE_KNN, true>;
         FL_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, spp.bytes));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(2 * clusters));
-        cfg.blockDim = dim3(TC_THREADS);
+        cfg.blockDim = dim3(TC_LIST_THREADS);
         cfg.dynamicSmemBytes = (size_t)spp.bytes;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -1532,16 +1500,13 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
         knn_tc_kernel<false, TC_MODE_KNN_MID><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     } else if (big) {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<false, TC_MODE_KNN_BIG><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
-    } else if (L.gs) {
-        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<false, TC_MODE_KNN_GS><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
+        knn_tc_kernel<false, TC_MODE_KNN_BIG><<<grid, TC_LIST_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     } else if (dbg != nullptr || kp.dbg_flags != 0) {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<true, TC_MODE_KNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<true, TC_MODE_KNN><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
+        knn_tc_kernel<true, TC_MODE_KNN><<<grid, TC_LIST_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     } else {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<false, TC_MODE_KNN><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
+        knn_tc_kernel<false, TC_MODE_KNN><<<grid, TC_LIST_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     }
     FL_CHECK_LAUNCH();
     return FL_OK;
@@ -1596,12 +1561,14 @@ int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, cons
     kp.n_tiles = (int)(p.m_pad / TC_BN);
     kp.nsplit = 1;
     kp.tiles_per_split = kp.n_tiles;
+    kp.last_steps = tc_last_steps(p);
     kp.nkc = sp.nkc; kp.nstage = sp.nstage;
     kp.off_b = sp.off_b; kp.off_pool_sc = sp.off_pool_sc; kp.off_pool_id = sp.off_pool_id; kp.off_bar = sp.off_bar;
     kp.nq_pad = p.nq_pad; kp.tau = p.tau; kp.status = p.status;
     kp.asg_sc = asg_sc; kp.asg_id = asg_id;
     kp.nq_dev = nq_dev;
-    kp.tile_stride = 1; kp.wait_hint_ns = 1000u;
+    kp.tile_stride = 1; kp.wait_hint_ns = tc_experiment().hint_ns;
+    kp.wait_ns = tc_experiment().wait_ns;      // (a limit of zero gives up after a few microseconds of waiting)
     const int grid = kp.n_qtiles < sm_count() ? kp.n_qtiles : sm_count();
     FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_ASSIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
     knn_tc_kernel<false, TC_MODE_ASSIGN><<<grid, TC_THREADS, sp.bytes, st>>>(map_q, map_q_aug, map_db, map_db_aug, kp);
