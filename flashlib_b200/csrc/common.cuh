@@ -308,10 +308,29 @@ __device__ __forceinline__ float4 bf16_lost4(float4 v, uint2 w) {
                        v.z - __uint_as_float(w.y << 16), v.w - __uint_as_float(w.y & 0xffff0000u));
 }
 
+// The same for operands in fp16 (saturating: what lies beyond 65 504 is lost and counted, NaN too).
+__device__ __forceinline__ uint2 f16x4_bits(float4 v) {
+    auto fit = [](float x) { return fminf(fmaxf(x, -65504.f), 65504.f); };
+    const __half2 a = __floats2half2_rn(fit(v.x), fit(v.y)), b = __floats2half2_rn(fit(v.z), fit(v.w));
+    uint2 w;
+    w.x = *reinterpret_cast<const uint32_t*>(&a);
+    w.y = *reinterpret_cast<const uint32_t*>(&b);
+    return w;
+}
+__device__ __forceinline__ float4 f16_lost4(float4 v, uint2 w) {
+    return make_float4(v.x - f16_bits_to_f32((unsigned short)(w.x & 0xffffu)), v.y - f16_bits_to_f32((unsigned short)(w.x >> 16)),
+                       v.z - f16_bits_to_f32((unsigned short)(w.y & 0xffffu)), v.w - f16_bits_to_f32((unsigned short)(w.y >> 16)));
+}
+// Operand format of a plane (FMT_*): the values to store, and what storing them takes away.
+constexpr uint32_t FMT_BF16 = 0, FMT_F16 = 1;
+__device__ __forceinline__ uint2 operand4_bits(float4 v, uint32_t fmt) { return fmt == FMT_F16 ? f16x4_bits(v) : bf16x4_bits(v); }
+__device__ __forceinline__ float4 operand4_lost(float4 v, uint2 w, uint32_t fmt) { return fmt == FMT_F16 ? f16_lost4(v, w) : bf16_lost4(v, w); }
+
 // Largest norms over the rows of a database, left by the passes that write its operand planes: of the rows x, of what
-// one rounding to bf16 takes from them (x - hi) and of what the second half of a split plane still misses
-// (x - hi - lo).
-enum { NORM_ROW = 0, NORM_LOST = 1, NORM_LOST2 = 2, NORM_WORDS = 4 };
+// one rounding to the operands' format takes from them (x - hi) and of what the second half of a split plane still misses
+// (x - hi - lo).  The word after them holds the operand format of planes that choose it (kmeans_tc.cu, ivf_tc.cu).
+enum { NORM_ROW = 0, NORM_LOST = 1, NORM_LOST2 = 2, NORM_FMT = 3, NORM_WORDS = 4 };
+__device__ __forceinline__ uint32_t operand_format(const float* norms) { return __float_as_uint(__ldg(norms + NORM_FMT)); }
 
 // Bound on |score - (<q,x> - ||x||^2/2)| over the rows behind `norms`, from the rounding that happened to this query
 // (sums of squares: qsq of its values, lost of q - hi, lost2 of q - hi - lo) and to those rows.  With
@@ -319,6 +338,7 @@ enum { NORM_ROW = 0, NORM_LOST = 1, NORM_LOST2 = 2, NORM_WORDS = 4 };
 // Whatever the values, no constant is assumed: a bf16 rounding may move a value by 2^-8 of itself, and where
 // all roundings go one way the product is off by nearly 2^-7 ||q|| ||x||; on ordinary data the norms give
 // half of that.  Nothing is lost where the rows are stored as bf16.  `acc`: see score_acc().
+// OPERANDS_BF16 stands for one rounding, to bf16 or fp16: `lost` and the norms are those of the one that happened.
 constexpr int OPERANDS_F32 = 0, OPERANDS_BF16 = 1, OPERANDS_SPLIT = 2;
 __device__ __forceinline__ float score_eps(int operands, float qsq, float lost, float lost2, const float* __restrict__ norms, float acc) {
     const float qn = sqrtf(qsq), xn = __ldg(norms + NORM_ROW);

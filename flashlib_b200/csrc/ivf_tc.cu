@@ -78,26 +78,28 @@ __global__ void ivf_row_map_kernel(const int64_t* __restrict__ list_offsets, con
     for (int r = threadIdx.x; r < len; r += blockDim.x) row_map[p0 + r] = (int)(r0 + r);
 }
 
-// One warp per plane row: bf16 features, the split -||x||^2/2 columns, half norm, largest norms.  rows_max is a multiple of the block's rows.
+// One warp per plane row: features in the plane's operand format, the split -||x||^2/2 columns, half norm, largest norms.  rows_max is a multiple of the block's rows.
 __global__ void ivf_plane_rows_kernel(const float* __restrict__ data, int64_t ld, int d, const int* __restrict__ row_map,
                                       int64_t rows_max, __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                      unsigned int* __restrict__ norm_bits, int d_pad) {
+                                      unsigned int* __restrict__ norm_bits, int d_pad, int vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int pitch = d_pad + PLANE_AUG_COLS;
     __nv_bfloat16* o = rows + row * pitch;
     const int src = __ldg(row_map + row);
     float sq[2] = {0.f, 0.f};                   // NORM_ROW, NORM_LOST
+    const uint32_t fmt = norm_bits[NORM_FMT];
     if (src < 0) {
         for (int c = lane; c < pitch; c += 32) o[c] = __float2bfloat16_rn(c == d_pad ? -3.0e38f : 0.f);
         if (lane == 0) hnorm[row] = pos_inf();
     } else {
         const float* p = data + (int64_t)src * ld;
-        for (int c = lane; c < d_pad; c += 32) {
-            const float v = (c < d) ? __ldg(p + c) : 0.f, l = bf16_lost(v);
-            sq[0] += v * v;
-            sq[1] += l * l;
-            o[c] = __float2bfloat16_rn(v);
+        for (int c = lane * 4; c < d_pad; c += 128) {
+            const float4 v = ld_row4(p, c, d, vec, DT_F32);
+            const uint2 b = operand4_bits(v, fmt);
+            sq[0] += sq4(v);
+            sq[1] += sq4(operand4_lost(v, b, fmt));
+            *reinterpret_cast<uint2*>(o + c) = b;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -164,13 +166,14 @@ __global__ void __launch_bounds__(256) ivf_tc_item_order_kernel(const int* __res
     if (mine && sub == 0) order[place] = i;
 }
 
-// One warp per gathered query row (grid-stride over the live rows): the bf16 row of the pair's
+// One warp per gathered query row (grid-stride over the live rows): the 16-bit row of the pair's
 // query with ones in the norm columns and a -inf starting threshold; rows without a pair are
 // zero and get a +inf threshold, so nothing is ever a candidate for them.
 __global__ void ivf_tc_gather_kernel(const float* __restrict__ q, int64_t ldq, int d, int nprobe,
                                      const int* __restrict__ grow, const int* __restrict__ live_rows,
                                      __nv_bfloat16* __restrict__ qplane, float* __restrict__ tau,
-                                     int* __restrict__ row_query, int d_pad) {
+                                     int* __restrict__ row_query, int d_pad, int vec, const float* __restrict__ norms) {
+    const uint32_t fmt = operand_format(norms);
     const int lane = threadIdx.x & 31;
     const int pitch = d_pad + PLANE_AUG_COLS;
     const int live = *live_rows;
@@ -184,17 +187,20 @@ __global__ void ivf_tc_gather_kernel(const float* __restrict__ q, int64_t ldq, i
             continue;
         }
         const float* src = q + (int64_t)(pair / nprobe) * ldq;
-        for (int c = lane; c < d_pad; c += 32) o[c] = __float2bfloat16_rn(c < d ? __ldg(src + c) : 0.f);
+        for (int c = lane * 4; c < d_pad; c += 128)
+            *reinterpret_cast<uint2*>(o + c) = operand4_bits(ld_row4(src, c, d, vec, DT_F32), fmt);
         if (lane < PLANE_AUG_COLS) o[d_pad + lane] = __float2bfloat16_rn(lane < 3 ? 1.f : 0.f);
         if (lane == 0) { tau[r] = neg_inf(); row_query[r] = pair / nprobe; }
     }
 }
 
-// ||q||^2 and the square of what rounding q to bf16 takes from it (all lanes of a warp).
-__device__ __forceinline__ void ivf_query_norms(const float* __restrict__ qp, int d, float& qsq, float& lost) {
+// ||q||^2 and the square of what rounding q to the operands' format takes from it (all lanes of a warp).
+__device__ __forceinline__ void ivf_query_norms(const float* __restrict__ qp, int d, uint32_t fmt, float& qsq, float& lost) {
     qsq = lost = 0.f;
     for (int c = threadIdx.x & 31; c < d; c += 32) {
-        const float v = __ldg(qp + c), l = bf16_lost(v);
+        const float v = __ldg(qp + c);
+        const float4 v4 = make_float4(v, 0.f, 0.f, 0.f);
+        const float l = operand4_lost(v4, operand4_bits(v4, fmt), fmt).x;
         qsq += v * v;
         lost += l * l;
     }
@@ -266,7 +272,7 @@ __global__ void __launch_bounds__(128) ivf_tc_seed_select_kernel(const float* __
         pick = __shfl_sync(FULL_MASK, key[0], rank - 1);     // -inf while fewer than `rank` rows were sampled
     }
     float qsq, lost;
-    ivf_query_norms(q + qi * ldq, d, qsq, lost);
+    ivf_query_norms(q + qi * ldq, d, operand_format(norms), qsq, lost);
     if (pick > neg_inf())
         pick -= 2.f * score_eps(OPERANDS_BF16, qsq, lost, 0.f, norms, acc) + proof_slack(qsq, __ldg(norms + NORM_ROW), d);
     // (NaN where a row's norm or the query is not finite: no score would exceed it)
@@ -402,7 +408,7 @@ __global__ void __launch_bounds__(128) ivf_tc_finalize_kernel(
     if (qi >= nq) return;
     const float* qp = q + qi * ldq;
     float qsq, lost;
-    ivf_query_norms(qp, d, qsq, lost);
+    ivf_query_norms(qp, d, operand_format(norms), qsq, lost);
     const float eps = score_eps(OPERANDS_BF16, qsq, lost, 0.f, norms, acc);
     const float slack = proof_slack(qsq, __ldg(norms + NORM_ROW), d);
 
@@ -717,6 +723,8 @@ extern "C" int fl_ivf_prepare_f32(const float* data, int64_t m, int64_t ldd, int
     int* row_map = reinterpret_cast<int*>(base + L.off_row_map);
     FL_CHECK_CUDA(cudaMemsetAsync(row_map, 0xFF, (size_t)L.rows_max * 4, st));
     FL_CHECK_CUDA(cudaMemsetAsync(base + L.pl.off_meta, 0, 1024, st));
+    int rc = launch_operand_format(data, m, ldd, d, reinterpret_cast<uint32_t*>(base + L.pl.off_meta) + NORM_FMT, st);
+    if (rc != FL_OK) return rc;
     ivf_tile_scan_kernel<<<1, 1024, 0, st>>>(list_offsets, nlist, tile_off);
     FL_CHECK_LAUNCH();
     ivf_row_map_kernel<<<(unsigned)nlist, 256, 0, st>>>(list_offsets, tile_off, row_map);
@@ -725,7 +733,7 @@ extern "C" int fl_ivf_prepare_f32(const float* data, int64_t m, int64_t ldd, int
     ivf_plane_rows_kernel<<<(unsigned)ceil_div(L.rows_max, wpb), wpb * 32, 0, st>>>(
         data, ldd, d, row_map, L.rows_max, reinterpret_cast<__nv_bfloat16*>(base + L.pl.off_rows),
         reinterpret_cast<float*>(base + L.pl.off_hnorm), reinterpret_cast<unsigned int*>(base + L.pl.off_meta),
-        L.pl.d_pad);
+        L.pl.d_pad, dt_vec_ok(data, ldd, DT_F32) && d % 4 == 0);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
@@ -797,12 +805,13 @@ extern "C" int fl_ivf_fine_scan_tc_f32(const float* q, int64_t nq, int64_t ldq, 
     profile_mark(st);      // 2: gathered query plane
     ivf_tc_gather_kernel<<<(unsigned)(8 * sm_count()), 256, 0, st>>>(
         q, ldq, d, nprobe, grow, live_rows, reinterpret_cast<__nv_bfloat16*>(base + w.off_qplane), tau,
-        reinterpret_cast<int*>(base + w.off_row_query), w.d_pad);
+        reinterpret_cast<int*>(base + w.off_row_query), w.d_pad, dt_vec_ok(q, ldq, DT_F32) && d % 4 == 0, norms);
     FL_CHECK_LAUNCH();
     float* tau_q = reinterpret_cast<float*>(base + w.off_tau_q);
 
     TcKnnParams tp{};
     tp.qplane = base + w.off_qplane; tp.nq = w.cap_rows; tp.nq_pad = w.cap_rows;
+    tp.fmt = reinterpret_cast<const uint32_t*>(norms) + NORM_FMT;
     tp.dbrows = pl + L.pl.off_rows; tp.hnorm = reinterpret_cast<const float*>(pl + L.pl.off_hnorm);
     tp.m = L.rows_max; tp.m_pad = L.pl.m_pad; tp.d_pad = L.pl.d_pad; tp.d_used = d; tp.K1 = tc_deep_pool_size();
     tp.deep_pools = 0;

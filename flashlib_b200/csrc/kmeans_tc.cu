@@ -362,7 +362,7 @@ struct AssignTcWs {
     int l1_cap; int64_t l1_pad; int pitch3;
     int nsplit_fb; int64_t rows_per_split_fb; int fb_bq, fb_blocks;
     PlaneLayout cl, cl3;
-    int64_t off_cplane, off_cplane3, off_xplane, off_xsq, off_xsplit, off_asg_sc, off_asg_id, off_tau, off_cnt, off_l0list, off_l1list,
+    int64_t off_cplane, off_cplane3, off_xplane, off_xsq, off_xfmt, off_xsplit, off_asg_sc, off_asg_id, off_tau, off_cnt, off_l0list, off_l1list,
         off_fblist, off_fblist2, off_fbpart_sc, off_fbpart_id, off_fbdist, bytes;
 };
 
@@ -401,6 +401,7 @@ static AssignTcWs assign_tc_plan(int64_t n, int K, int d, int have_xplane) {
     w.off_cplane3 = w.split ? take(cur, w.cl3.bytes) : -1;
     w.off_xplane = have_xplane ? -1 : take(cur, w.n_pad * w.pitch * 2);
     w.off_xsq = have_xplane ? -1 : take(cur, w.n_pad * 8);
+    w.off_xfmt = have_xplane ? -1 : take(cur, 4);
     w.off_xsplit = w.split ? take(cur, w.l1_pad * w.pitch3 * 2) : -1;
     w.off_asg_sc = take(cur, w.n_pad * 4 * 4);
     w.off_asg_id = take(cur, w.n_pad * 2 * 4);
@@ -453,10 +454,15 @@ int assign_tc_supported(int64_t n, int K, int d) {
 
 using namespace fl;
 
+static int64_t xplane_fmt_offset(int64_t n, int d) {
+    return round_up(round_up(n, 128) * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024) + round_up(n, 128) * 8;
+}
+
 extern "C" int64_t fl_kmeans_xplane_bytes(int64_t n, int d) {
     if (n < 1 || d < 1) return 0;
-    // the bf16 rows, then ||x||^2 of every row and the square of the norm of what rounding took of it (f32 [n_pad][2])
-    return round_up(round_up(n, 128) * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024) + round_up(n, 128) * 8;
+    // the 16-bit rows, then ||x||^2 of every row and the square of the norm of what rounding took of it (f32 [n_pad][2]), then
+    // the operand format
+    return xplane_fmt_offset(n, d) + 1024;
 }
 
 extern "C" int fl_kmeans_prepare_x_f32(const float* x, int64_t n, int d, int64_t ldx, void* xplane,
@@ -466,7 +472,10 @@ extern "C" int fl_kmeans_prepare_x_f32(const float* x, int64_t n, int d, int64_t
     const int64_t n_pad = round_up(n, 128);
     // the rows' norms (the scoring error bound of a point needs its own) come from the same read
     float2* xsq = reinterpret_cast<float2*>(static_cast<char*>(xplane) + round_up(n_pad * (round_up(d, 64) + PLANE_AUG_COLS) * 2, 1024));
-    return launch_query_plane(x, n, ldx, d, xplane, n_pad, (int)round_up(d, 64), (cudaStream_t)stream, DT_F32, xsq);
+    uint32_t* fmt = reinterpret_cast<uint32_t*>(static_cast<char*>(xplane) + xplane_fmt_offset(n, d));
+    const int rc = launch_operand_format(x, n, ldx, d, fmt, (cudaStream_t)stream);
+    if (rc != FL_OK) return rc;
+    return launch_query_plane(x, n, ldx, d, xplane, n_pad, (int)round_up(d, 64), (cudaStream_t)stream, DT_F32, xsq, fmt);
 }
 
 extern "C" int64_t fl_kmeans_assign_tc_workspace_bytes(int64_t n, int K, int d, int have_xplane) {
@@ -474,8 +483,8 @@ extern "C" int64_t fl_kmeans_assign_tc_workspace_bytes(int64_t n, int K, int d, 
     return assign_tc_plan(n, K, d, have_xplane).bytes;
 }
 
-// Two stages.  (1) plain bf16 planes: every point is scored against every centroid; labels the
-// proof accepts (scoring error about 0.0037 ||x|| max||c||) are final.  (2) d <= 128: the unproven points
+// Two stages.  (1) planes of one rounding: every point is scored against every centroid; labels the
+// proof accepts (scoring error about 0.0005 ||x|| max||c|| in fp16, which almost all data takes, 0.0037 in bf16) are final.  (2) d <= 128: the unproven points
 // (a device-side list) are gathered into split planes and scored again, error about 6e-5: nearly all of
 // the rest is proven.  What is left takes the exact CUDA-core path.
 extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, const float* c,
@@ -493,27 +502,33 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     char* base = static_cast<char*>(ws);
     if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
 
+    // sample plane (query side), whose operand format the plain centroid plane shares
+    const char* xpl = static_cast<const char*>(xplane);
+    const float2* xsq;
+    const uint32_t* fmt;
+    int rc;
+    if (!xpl) {
+        float2* xs = reinterpret_cast<float2*>(base + w.off_xsq);
+        uint32_t* f = reinterpret_cast<uint32_t*>(base + w.off_xfmt);
+        rc = launch_operand_format(x, n, ldx, d, f, st);
+        if (rc == FL_OK) rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs, f);
+        if (rc != FL_OK) return rc;
+        xpl = base + w.off_xplane;
+        xsq = xs;
+        fmt = f;
+    } else {
+        xsq = reinterpret_cast<const float2*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
+        fmt = reinterpret_cast<const uint32_t*>(xpl + xplane_fmt_offset(n, d));
+    }
     // centroid planes (database side): plain, and split for the second stage
     char* cpl = base + w.off_cplane;
-    int rc = launch_plane_build(c, K, d, ldc, cpl, st);
+    rc = launch_plane_build(c, K, d, ldc, cpl, st, DT_F32, fmt);
     if (rc != FL_OK) return rc;
     char* cpl3 = nullptr;
     if (w.split) {
         cpl3 = base + w.off_cplane3;
         rc = launch_split_db_plane(c, K, d, ldc, cpl3, st);
         if (rc != FL_OK) return rc;
-    }
-    // sample plane (query side)
-    const char* xpl = static_cast<const char*>(xplane);
-    const float2* xsq;
-    if (!xpl) {
-        float2* xs = reinterpret_cast<float2*>(base + w.off_xsq);
-        rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs);
-        if (rc != FL_OK) return rc;
-        xpl = base + w.off_xplane;
-        xsq = xs;
-    } else {
-        xsq = reinterpret_cast<const float2*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
     }
     int* counters = reinterpret_cast<int*>(base + w.off_cnt);
     int* fb_count = counters;          // points for the exact path
@@ -533,13 +548,14 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     const float* norms = reinterpret_cast<const float*>(cpl + w.cl.off_meta);
     const float acc1 = score_acc(d + PLANE_AUG_COLS);
 
-    // ---- stage 1: plain bf16 ---------------------------------------------------------------
+    // ---- stage 1: one rounding, to the samples' operand format ---------------------------------------------------------------
     {
         rc = launch_fill_f32(tau, w.n_pad, -INFINITY, st);
         if (rc != FL_OK) return rc;
         TcKnnParams tp{};
         tp.qplane = xpl; tp.nq = n; tp.nq_pad = w.n_pad;
         tp.dbrows = cpl + w.cl.off_rows; tp.hnorm = reinterpret_cast<const float*>(cpl + w.cl.off_hnorm);
+        tp.fmt = fmt;
         tp.m = K; tp.m_pad = w.cl.m_pad; tp.d_pad = w.cl.d_pad; tp.d_used = d;
         tp.tau = tau; tp.status = status;
         profile_begin(st);

@@ -40,7 +40,7 @@ constexpr float SIMT_EPS_REL = 4e-6f;
 // rounding took.
 template <int N>
 __device__ __forceinline__ void query_plane_rows(const void* q, int64_t row, int64_t nq, int64_t ldq, int d, int vec,
-                                                 __nv_bfloat16* out, int d_pad, int dt, float2 (&s)[N]) {
+                                                 __nv_bfloat16* out, int d_pad, int dt, float2 (&s)[N], uint32_t fmt = FMT_BF16) {
     const int lane = threadIdx.x & 31, pitch = d_pad + PLANE_AUG_COLS;
     const void* p[N];
     bool live[N];
@@ -61,9 +61,10 @@ __device__ __forceinline__ void query_plane_rows(const void* q, int64_t row, int
         }
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            const uint2 w = bf16x4_bits(v[i]);
+            // (the columns beyond the features stay bf16, as the norm terms they meet)
+            const uint2 w = operand4_bits(v[i], c < d ? fmt : FMT_BF16);
             *reinterpret_cast<uint2*>(o + i * pitch + c) = w;
-            if (c < d) { s[i].x += sq4(v[i]); s[i].y += sq4(bf16_lost4(v[i], w)); }
+            if (c < d) { s[i].x += sq4(v[i]); s[i].y += sq4(operand4_lost(v[i], w, fmt)); }
         }
     }
 }
@@ -74,11 +75,12 @@ __device__ __forceinline__ void query_plane_rows(const void* q, int64_t row, int
 constexpr int QP_ROWS = 2;
 __global__ void __launch_bounds__(256) query_plane_kernel(const void* __restrict__ q, int64_t nq, int64_t ldq, int d, int vec,
                                                           __nv_bfloat16* __restrict__ out, int64_t nq_pad, int d_pad, int dt,
-                                                          float2* __restrict__ sq_out) {
+                                                          float2* __restrict__ sq_out, const uint32_t* __restrict__ fmt_word) {
+    const uint32_t fmt = fmt_word != nullptr ? __ldg(fmt_word) : FMT_BF16;
     const int64_t row = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * QP_ROWS;
     if (row >= nq_pad) return;
     float2 s[QP_ROWS];
-    query_plane_rows<QP_ROWS>(q, row, nq, ldq, d, vec, out, d_pad, dt, s);
+    query_plane_rows<QP_ROWS>(q, row, nq, ldq, d, vec, out, d_pad, dt, s, fmt);
     if (sq_out == nullptr) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -113,9 +115,9 @@ __global__ void __launch_bounds__(256) knn_prep_kernel(const void* __restrict__ 
 }
 
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad, int d_pad,
-                       cudaStream_t st, int dt, float2* sq_out) {
+                       cudaStream_t st, int dt, float2* sq_out, const uint32_t* fmt) {
     query_plane_kernel<<<(unsigned)ceil_div(nq_pad, 8 * QP_ROWS), 256, 0, st>>>(
-        q, nq, ldq, d, dt_vec_ok(q, ldq, dt) && d % 4 == 0, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt, sq_out);
+        q, nq, ldq, d, dt_vec_ok(q, ldq, dt) && d % 4 == 0, reinterpret_cast<__nv_bfloat16*>(qplane), nq_pad, d_pad, dt, sq_out, fmt);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }

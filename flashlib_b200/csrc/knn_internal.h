@@ -157,6 +157,7 @@ struct TcKnnParams {
     int64_t nq, nq_pad;
     const void* dbrows;      // bf16 [m_pad][d_pad]
     const float* hnorm;      // f32 [m_pad]
+    const uint32_t* fmt;     // optional: operand format of the feature columns of both planes (FMT_*, device; bf16 without)
     int64_t m, m_pad; int d_pad;
     int d_used;              // columns before the first that is zero in every row (0: not known, d_pad)
     int K1;                  // entries a pool keeps (informational: fixed by the kernel mode)
@@ -260,10 +261,13 @@ int launch_split_query_gather(const float* x, int64_t ldx, int d, const int* row
 // bf16 query plane [nq_pad][d_pad + 16] (features zero padded, ones in the norm columns) from fp32 queries;
 // sq_out (optional): ||q||^2 of every query and the square of the norm of what its rounding took.
 int launch_query_plane(const void* q, int64_t nq, int64_t ldq, int d, void* qplane, int64_t nq_pad,
-                       int d_pad, cudaStream_t st, int dt = DT_F32, float2* sq_out = nullptr);
+                       int d_pad, cudaStream_t st, int dt = DT_F32, float2* sq_out = nullptr, const uint32_t* fmt = nullptr);
+// Picks the operand format (FMT_*) that loses less of a sample of the rows and writes it to *fmt.
+int launch_operand_format(const float* x, int64_t n, int64_t ld, int d, uint32_t* fmt, cudaStream_t st);
 
 // Small helpers shared by the entry points.
-int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt = DT_F32);
+int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt = DT_F32,
+                       const uint32_t* fmt = nullptr);
 int launch_status_publish(const int32_t* status, int32_t* host, cudaStream_t st);
 int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t st);
 int launch_ivf_group(const int32_t* probed, int64_t npairs, int nlist, int bq, const int64_t* list_offsets, int* cnt,

@@ -107,6 +107,7 @@ __device__ unsigned long long g_tc_prof[160 * TC_PROF_WORDS];
 
 struct TcKernelParams {
     int n_qtiles, n_tiles, nsplit, tiles_per_split, nkc, nstage;
+    const uint32_t* fmt;     // operand format of the feature columns (FMT_*; null: bf16)
     int last_steps;          // K = 16 steps of a tile's last chunk that hold features at all (1 to 4)
     int nabuf;               // query-tile buffers in shared memory (1 or 2)
     int stream_a;            // 1: the query tile is not resident; its chunk travels with every database chunk
@@ -432,9 +433,11 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         // the ring in order: a slot's barrier is only asked about a phase when the one before has completed.)
         // Scoring of 10 000 x 1M x 128, one CTA a tile and the epilogue of before: 2.55 ms -> 2.22.
         if (leader) {
-            constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * TC_BM : TC_BM, TC_BN);
+            // the norm columns are bf16 whatever the features are (a step of their own: one format within an MMA)
+            constexpr uint32_t idesc_norm = umma_idesc_bf16(PAIR ? 2 * TC_BM : TC_BM, TC_BN);
+            const uint32_t idesc_feat = p.fmt != nullptr && __ldg(p.fmt) == FMT_F16 ? umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, TC_BN) : idesc_norm;
             const uint32_t elected = elect_one();
-            auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+            auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t acc, uint32_t idesc) {
                 if (DBG && (p.dbg_flags & 16)) return;     // timing experiment: operand streaming only
                 if (PAIR) umma_bf16_pair(d, a, b, idesc, acc); else umma_bf16(d, a, b, idesc, acc);
             };
@@ -486,19 +489,19 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                             const uint64_t da = umma_desc(stream_a ? slot + SLOT_B_BYTES : a_addr + a_off + kc * TC_A_CHUNK);
                             const uint64_t db = umma_desc(slot);
                             // +32 bytes per 16-feature step inside the 128-byte swizzled row
-                            mma(d_tmem, da, db, kc != 0 ? 1u : 0u);
+                            mma(d_tmem, da, db, kc != 0 ? 1u : 0u, idesc_feat);
                             if (!last || p.last_steps == TC_BK / 16) {
 #pragma unroll
-                                for (int k4 = 1; k4 < TC_BK / 16; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u);
+                                for (int k4 = 1; k4 < TC_BK / 16; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u, idesc_feat);
                             } else {
                                 // columns of zeros beyond the last feature: 96 features take 7 steps with the norm
                                 // columns in place of 9
-                                for (int k4 = 1; k4 < p.last_steps; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u);
+                                for (int k4 = 1; k4 < p.last_steps; ++k4) mma(d_tmem, da + 2 * k4, db + 2 * k4, 1u, idesc_feat);
                             }
                             if (last && !(DBG && (p.dbg_flags & 8))) {
                                 // norm columns: ones x split(-||x||^2/2), 32-byte rows, 32-byte swizzle
                                 const uint32_t a_aug = stream_a ? slot + SLOT_B_BYTES + TC_A_CHUNK : a_aug_addr + a_off;
-                                mma(d_tmem, umma_desc_sw32(a_aug), umma_desc_sw32(slot + SLOT_CHUNK), 1u);
+                                mma(d_tmem, umma_desc_sw32(a_aug), umma_desc_sw32(slot + SLOT_CHUNK), 1u, idesc_norm);
                             }
                             if (last) mbar_arrive(BAR(B_TURN + (b ^ 1)));
                             commit(BAR(B_EMPTY + s));   // slot reusable once these MMAs retire
@@ -1322,7 +1325,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     kp.n_tiles = (int)(p.m_pad / TC_BN);
     kp.nsplit = p.nsplit;
     kp.tiles_per_split = (int)p.tiles_per_split;
-    kp.last_steps = tc_last_steps(p);
+    kp.last_steps = tc_last_steps(p); kp.fmt = p.fmt;
     kp.nkc = L->sp.nkc; kp.nstage = L->sp.nstage;
     kp.stream_a = stream ? 1 : 0;
     kp.off_b = L->sp.off_b; kp.off_pool_sc = L->sp.off_pool_sc; kp.off_pool_id = L->sp.off_pool_id;
@@ -1561,7 +1564,7 @@ int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, cons
     kp.n_tiles = (int)(p.m_pad / TC_BN);
     kp.nsplit = 1;
     kp.tiles_per_split = kp.n_tiles;
-    kp.last_steps = tc_last_steps(p);
+    kp.last_steps = tc_last_steps(p); kp.fmt = p.fmt;
     kp.nkc = sp.nkc; kp.nstage = sp.nstage;
     kp.off_b = sp.off_b; kp.off_pool_sc = sp.off_pool_sc; kp.off_pool_id = sp.off_pool_id; kp.off_bar = sp.off_bar;
     kp.nq_pad = p.nq_pad; kp.tau = p.tau; kp.status = p.status;

@@ -43,7 +43,9 @@ __global__ void rownorm_kernel(const float* __restrict__ x, int64_t n, int d, in
 // rows allow them (vec) and 8-byte writes.
 __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d, int64_t ld,
                                    __nv_bfloat16* __restrict__ rows, float* __restrict__ hnorm,
-                                   unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int dt, int vec) {
+                                   unsigned int* __restrict__ norm_bits, int64_t m_pad, int d_pad, int dt, int vec,
+                                   const uint32_t* __restrict__ fmt_word) {
+    const uint32_t fmt = fmt_word != nullptr ? __ldg(fmt_word) : FMT_BF16;
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int pitch = d_pad + PLANE_AUG_COLS;
@@ -56,9 +58,9 @@ __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d
         const void* p = row_at(db, row, ld, dt);
         for (int c = lane * 4; c < d_pad; c += 128) {
             const float4 v = ld_row4(p, c, d, vec, dt);
-            const uint2 w = bf16x4_bits(v);
+            const uint2 w = operand4_bits(v, fmt);
             sq[0] += sq4(v);
-            sq[1] += sq4(bf16_lost4(v, w));
+            sq[1] += sq4(operand4_lost(v, w, fmt));
             *reinterpret_cast<uint2*>(o + c) = w;
         }
 #pragma unroll
@@ -70,6 +72,46 @@ __global__ void plane_build_kernel(const void* __restrict__ db, int64_t m, int d
         write_norm_columns(o + d_pad, sq[0], PLANE_AUG_COLS);
     }
     block_norms_update(norm_bits, sq);
+}
+
+// Operand format of a set of fp32 rows, from FMT_SAMPLE of them spread over the set: fp16 where it loses less than half
+// as much as bf16 (eight times less on values between 2^-14 and 65 504, which rows mostly are), bf16 where values lie beyond
+// fp16's range, or NaN or infinities make the comparison fail.  Only speed hangs on the choice: what rounding
+// takes from each row is measured by the pass that does it, in either format, and the proofs build on that.
+constexpr int FMT_SAMPLE = 128;
+__global__ void __launch_bounds__(1024) operand_format_kernel(const float* __restrict__ x, int64_t n, int64_t ld, int d,
+                                                              uint32_t* __restrict__ fmt) {
+    __shared__ float s_b[32], s_h[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t count = n < FMT_SAMPLE ? n : FMT_SAMPLE;
+    float lb = 0.f, lh = 0.f;
+    for (int64_t i = warp; i < count; i += 32) {
+        const float* p = x + (i * n / count) * ld;
+        for (int c = lane; c < d; c += 32) {
+            const float v = __ldg(p + c);
+            const float4 v4 = make_float4(v, 0.f, 0.f, 0.f);
+            const float b = bf16_lost(v), h = f16_lost4(v4, f16x4_bits(v4)).x;
+            lb += b * b;
+            lh += h * h;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lb += __shfl_xor_sync(FULL_MASK, lb, o);
+        lh += __shfl_xor_sync(FULL_MASK, lh, o);
+    }
+    if (lane == 0) { s_b[warp] = lb; s_h[warp] = lh; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float b = 0.f, h = 0.f;
+        for (int w = 0; w < 32; ++w) { b += s_b[w]; h += s_h[w]; }
+        *fmt = h < 0.25f * b ? FMT_F16 : FMT_BF16;
+    }
+}
+int launch_operand_format(const float* x, int64_t n, int64_t ld, int d, uint32_t* fmt, cudaStream_t st) {
+    operand_format_kernel<<<1, 1024, 0, st>>>(x, n, ld, d, fmt);
+    FL_CHECK_LAUNCH();
+    return FL_OK;
 }
 
 PlaneLayout plane_layout(int64_t m, int d) {
@@ -85,7 +127,7 @@ PlaneLayout plane_layout(int64_t m, int d) {
 }
 
 // Fills `plane` (layout plane_layout(m, d)) for the fp32 rows of db.
-int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt) {
+int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane, cudaStream_t st, int dt, const uint32_t* fmt) {
     const PlaneLayout L = plane_layout(m, d);
     char* base = static_cast<char*>(plane);
     FL_CHECK_CUDA(cudaMemsetAsync(base + L.off_meta, 0, 1024, st));
@@ -93,7 +135,7 @@ int launch_plane_build(const void* db, int64_t m, int d, int64_t ld, void* plane
     plane_build_kernel<<<(unsigned)ceil_div(L.m_pad, wpb), wpb * 32, 0, st>>>(
         db, m, d, ld, reinterpret_cast<__nv_bfloat16*>(base + L.off_rows),
         reinterpret_cast<float*>(base + L.off_hnorm), reinterpret_cast<unsigned int*>(base + L.off_meta),
-        L.m_pad, L.d_pad, dt, dt_vec_ok(db, ld, dt) && d % 4 == 0);
+        L.m_pad, L.d_pad, dt, dt_vec_ok(db, ld, dt) && d % 4 == 0, fmt);
     FL_CHECK_LAUNCH();
     return FL_OK;
 }
