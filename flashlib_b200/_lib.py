@@ -115,6 +115,11 @@ SIGNATURES = {
     "fl_kmeans_lloyd_words": (c_int, []),
     "fl_kmeans_lloyd_f32": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "fl_kmeans_lloyd_tc_supported": (c_int, [c_int64, c_int, c_int]),
+    "fl_kmeans_lloyd_tc_workspace_bytes": (c_int64, [c_int64, c_int, c_int]),
+    "fl_kmeans_lloyd_tc_f32": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                                       c_void_p, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                       c_void_p, c_void_p]),
     "fl_kmeans_lloyd_pick": (c_int, [c_int, c_int64, c_int, c_int]),
     "fl_kmeans_assign_pick": (c_int, [c_int, c_int64, c_int, c_int]),
     "fl_ivf_fine_scan_workspace_bytes": (c_int64, [c_int64, c_int, c_int, c_int64, c_int, c_int]),

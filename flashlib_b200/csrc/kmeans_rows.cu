@@ -370,15 +370,16 @@ int launch_kmeans_rows(const float* x, int batch, int64_t n, int64_t ldx, int64_
 }
 
 // Control words of a Lloyd loop on the device: converged flag, blocks finished, largest shift (float bits).
-enum { LLOYD_DONE = 0, LLOYD_BLOCKS = 1, LLOYD_SHIFT = 2, LLOYD_WORDS = 4 };
 
-// New centroids, one warp per centroid; clears the sums when the next iteration adds every row again.  With
+// New centroids, one warp per centroid (and, with `shift`, how far each moved); clears the sums when the next iteration adds
+// every row again.  With
 // tol > 0 the last block to finish compares the largest shift with it and tells the host, in pinned
 // memory, how many iterations are finished; negated when the loop has converged.
 __global__ void __launch_bounds__(256) kmeans_step_kernel(float* __restrict__ sums, int32_t* __restrict__ cnts,
                                                           const float* __restrict__ old_c, float* __restrict__ new_c,
                                                           int64_t KB, int d, int clear, float tol, int it,
-                                                          unsigned* __restrict__ ctl, volatile int32_t* host) {
+                                                          unsigned* __restrict__ ctl, volatile int32_t* host,
+                                                          float* __restrict__ shift_out) {
     if (tol > 0.f && ctl[LLOYD_DONE] != 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t j = (int64_t)blockIdx.x * 8 + warp;
@@ -396,9 +397,11 @@ __global__ void __launch_bounds__(256) kmeans_step_kernel(float* __restrict__ su
         __syncwarp();
         if (clear && lane == 0) cnts[j] = 0;
     }
-    if (!(tol > 0.f)) return;
+    if (!(tol > 0.f) && shift_out == nullptr) return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+    if (shift_out != nullptr && lane == 0 && j < KB) shift_out[j] = sqrtf(s);
+    if (!(tol > 0.f)) return;
     __shared__ unsigned shift[8];
     if (lane == 0) shift[warp] = __float_as_uint(fabsf(sqrtf(s)));      // NaN orders above every number
     __syncthreads();
@@ -418,8 +421,16 @@ __global__ void __launch_bounds__(256) kmeans_step_kernel(float* __restrict__ su
     host[0] = done ? -(it + 1) : it + 1;
 }
 
+int launch_kmeans_step(float* sums, int32_t* cnts, const float* old_c, float* new_c, int64_t KB, int d, int clear, float tol, int it,
+                       int32_t* ctl, int32_t* host, float* shift, cudaStream_t st) {
+    kmeans_step_kernel<<<(unsigned)ceil_div(KB, 8), 256, 0, st>>>(sums, cnts, old_c, new_c, KB, d, clear, tol, it,
+                                                                  reinterpret_cast<unsigned*>(ctl), host, shift);
+    FL_CHECK_LAUNCH();
+    return FL_OK;
+}
+
 // Waits until the device has finished `want` iterations or converged, or the stream has stopped.
-static void lloyd_wait(const int32_t* host, int want, cudaStream_t st) {
+void lloyd_wait(const int32_t* host, int want, cudaStream_t st) {
     for (unsigned spin = 1;; ++spin) {
         const int v = __atomic_load_n(host, __ATOMIC_ACQUIRE);
         if (v < 0 || v >= want) return;
@@ -492,9 +503,11 @@ extern "C" int fl_kmeans_lloyd_f32(const float* x, int batch, int64_t n, int64_t
             if (test) cudaStreamSynchronize(st);       // launched steps still write to `host`
             return rc;
         }
-        kmeans_step_kernel<<<(unsigned)ceil_div(KB, 8), 256, 0, st>>>(sums, cnts, cur, nxt, KB, d, (it + 1) % refresh == 0, tol, it,
-                                                                      reinterpret_cast<unsigned*>(ctl), host);
-        FL_CHECK_LAUNCH();
+        const int rs = launch_kmeans_step(sums, cnts, cur, nxt, KB, d, (it + 1) % refresh == 0, tol, it, ctl, host, nullptr, st);
+        if (rs != FL_OK) {
+            if (test) cudaStreamSynchronize(st);
+            return rs;
+        }
         float* t = cur; cur = nxt; nxt = t;
     }
     *n_iter = iters;

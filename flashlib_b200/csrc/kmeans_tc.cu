@@ -4,6 +4,7 @@
 // queues the points it cannot prove for the exact CUDA-core path.
 #include "knn_internal.h"
 #include "pool.cuh"
+#include "kmeans_rows.h"
 #include <cuda_bf16.h>
 
 namespace fl {
@@ -243,12 +244,26 @@ __global__ void __launch_bounds__(128) assign_finalize_kernel(
 // sample row and no centroid is read -- 32 bytes per point instead of its 4 d -- at the price of a
 // lead of 2 eps where the exact re-scoring of assign_finalize_kernel needs eps; what the lead does
 // not decide goes to the `next` list (the second stage, whose bound is a hundred times smaller).
+//
+// Inside a Lloyd loop (live.rows: the points this iteration scores at all, or all of them) a proven point also gets its
+// bounds for the next iterations: at most `x` from its centroid, at least `y` from every other one.
+struct LivePoints {
+    const int* rows;         // listed points and their number (device), or, when *count is negative, all n of them
+    const int* count;
+    float2* bounds;
+};
 __global__ void __launch_bounds__(256) assign_by_lead_kernel(
     int64_t n, int K, int d, const float* __restrict__ asg_sc, const uint32_t* __restrict__ asg_id, const float2* __restrict__ xsq,
     float acc, const float* __restrict__ norms, int32_t* __restrict__ labels, int* __restrict__ next_count,
-    int* __restrict__ next_list, int next_cap, int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap) {
-    const int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int* __restrict__ next_list, int next_cap, int* __restrict__ fb_count, int* __restrict__ fb_list, int fb_cap,
+    const LivePoints live) {
+    int64_t pt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pt >= n) return;
+    const int listed = live.count != nullptr ? __ldg(live.count) : -1;
+    if (listed >= 0) {
+        if (pt >= listed) return;
+        pt = __ldg(live.rows + pt);
+    }
     const float4 sc = __ldg(reinterpret_cast<const float4*>(asg_sc + pt * 4));   // b1_0, b2_0, b1_1, b2_1
     const uint2 ids = __ldg(reinterpret_cast<const uint2*>(asg_id + pt * 2));
     const bool v0 = ids.x < (uint32_t)K && sc.x > -1e37f;   // false: no real centroid in that half
@@ -263,8 +278,16 @@ __global__ void __launch_bounds__(256) assign_by_lead_kernel(
         const float2 x2 = __ldg(xsq + pt);
         const float q2 = x2.x, eps = score_eps(OPERANDS_BF16, q2, x2.y, 0.f, norms, acc);
         // the column index rides in the low mantissa bits of both scores: 2^-15 relative each
-        const float lead = (best - fabsf(best) * 3.1e-5f) - (second + fabsf(second) * 3.1e-5f);
-        ok = lead > 2.f * eps + proof_slack(q2, __ldg(norms + NORM_ROW), d);
+        const float lo = best - fabsf(best) * 3.1e-5f, hi = second + fabsf(second) * 3.1e-5f;
+        const float slack = proof_slack(q2, __ldg(norms + NORM_ROW), d);
+        ok = lo - hi > 2.f * eps + slack;
+        if (live.bounds != nullptr) {
+            // squared distances from the scores, both ends of the error band (no bounds for a point that is not proven)
+            const float du = q2 - 2.f * (lo - eps) + slack, dl = q2 - 2.f * (hi + eps) - slack;
+            live.bounds[pt] = ok ? make_float2(__fsqrt_ru(fmaxf(du, 0.f)), dl > 0.f ? __fsqrt_rd(dl) : 0.f) : make_float2(pos_inf(), 0.f);
+        }
+    } else if (live.bounds != nullptr) {
+        live.bounds[pt] = make_float2(pos_inf(), 0.f);
     }
     labels[pt] = ok ? (int32_t)best_i : 0;
     if (!ok) {
@@ -277,6 +300,103 @@ __global__ void __launch_bounds__(256) assign_by_lead_kernel(
             const int i = atomicAdd(fb_count, 1);
             if (i < fb_cap) fb_list[i] = (int)pt;
         }
+    }
+}
+
+// Which points of a Lloyd iteration need their scores at all (Hamerly, "Making k-means even faster", SDM 2010).  Since the
+// bounds of a point were taken its own centroid has moved by shift[label] and no other by more than the largest shift of
+// the others: while the upper bound so widened stays below the lower one, the label cannot have changed.  The sums are
+// rounded against the point, and `shift` -- an fp32 norm of up to 128 differences -- counts 2 10^-5 more than it says.
+// The rest is listed; when that is more than `most`, all points are scored in place instead (count[0] < 0) and nothing
+// is gathered.  count: [0] points listed or -1, [1] rows of the gathered pass, [2] rows of the pass in place, [3] blocks
+// done, [4] points found (cleared by the caller).
+// Bound by HBM: 20 bytes a point.
+constexpr int BOUNDS_THREADS = 256, BOUNDS_PER = 4;
+__global__ void __launch_bounds__(BOUNDS_THREADS) lloyd_bounds_kernel(int64_t n, int K, const int32_t* __restrict__ labels,
+                                                                      float2* __restrict__ bounds, const float* __restrict__ shift,
+                                                                      const int32_t* __restrict__ done, int most,
+                                                                      int* __restrict__ list, int* __restrict__ count) {
+    __shared__ float s_m1[BOUNDS_THREADS / 32], s_m2[BOUNDS_THREADS / 32];
+    __shared__ int s_at[BOUNDS_THREADS / 32], s_n[BOUNDS_THREADS / 32], s_base;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the largest shift, whose it is, and the largest of the others; a shift that is no number counts as infinite
+    float m1 = -1.f, m2 = -1.f;
+    int at = -1;
+    auto fold = [&](float a1, int aa, float a2) {
+        if (a1 > m1) { m2 = fmaxf(m1, a2); m1 = a1; at = aa; } else m2 = fmaxf(m2, a1);
+    };
+    auto moved = [&](int j) { const float s = __ldg(shift + j); return s >= 0.f ? s : pos_inf(); };
+    for (int j = tid; j < K; j += BOUNDS_THREADS) fold(moved(j), j, -1.f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float a1 = __shfl_xor_sync(FULL_MASK, m1, o), a2 = __shfl_xor_sync(FULL_MASK, m2, o);
+        const int aa = __shfl_xor_sync(FULL_MASK, at, o);
+        fold(a1, aa, a2);
+    }
+    if (lane == 0) { s_m1[warp] = m1; s_m2[warp] = m2; s_at[warp] = at; }
+    __syncthreads();
+    m1 = m2 = -1.f;
+    at = -1;
+    for (int w = 0; w < BOUNDS_THREADS / 32; ++w) fold(s_m1[w], s_at[w], s_m2[w]);
+    constexpr float MORE = 1.00002f;
+    m1 = __fmul_ru(fmaxf(m1, 0.f), MORE);
+    m2 = __fmul_ru(fmaxf(m2, 0.f), MORE);
+    const bool stop = done != nullptr && *done != 0;
+    for (int64_t base = (int64_t)blockIdx.x * (BOUNDS_THREADS * BOUNDS_PER); base < n && !stop;
+         base += (int64_t)gridDim.x * (BOUNDS_THREADS * BOUNDS_PER)) {
+        bool live[BOUNDS_PER];
+        int mine = 0;
+#pragma unroll
+        for (int i = 0; i < BOUNDS_PER; ++i) {
+            const int64_t pt = base + i * BOUNDS_THREADS + tid;
+            live[i] = false;
+            if (pt < n) {
+                const int lab = __ldg(labels + pt);               // (-1 where no distance is a number)
+                float2 b = bounds[pt];
+                b.x = __fadd_ru(b.x, lab >= 0 ? __fmul_ru(moved(lab), MORE) : pos_inf());
+                b.y = __fsub_rd(b.y, lab == at ? m2 : m1);
+                live[i] = !(b.x < b.y);
+                if (!live[i]) bounds[pt] = b;         // (a listed point gets new ones, or none)
+            }
+            mine += live[i] ? 1 : 0;
+        }
+        int before = mine;                            // of this warp's lanes, then of the block's warps
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(FULL_MASK, before, o);
+            if (lane >= o) before += t;
+        }
+        if (lane == 31) s_n[warp] = before;
+        __syncthreads();
+        if (tid == 0) {
+            int total = 0;
+            for (int w = 0; w < BOUNDS_THREADS / 32; ++w) { const int t = s_n[w]; s_n[w] = total; total += t; }
+            s_base = total > 0 ? atomicAdd(count + 4, total) : 0;
+        }
+        __syncthreads();
+        int pos = s_base + s_n[warp] + before - mine;
+#pragma unroll
+        for (int i = 0; i < BOUNDS_PER; ++i)
+            if (live[i]) list[pos++] = (int)(base + i * BOUNDS_THREADS + tid);
+        __syncthreads();
+    }
+    if (tid != 0) return;
+    __threadfence();
+    if (atomicAdd(count + 3, 1) != (int)gridDim.x - 1) return;
+    const int found = atomicAdd(count + 4, 0);
+    const bool all = found > most;
+    count[0] = all ? -1 : found;
+    count[1] = all ? 0 : found;
+    count[2] = all ? (int)n : 0;
+}
+
+// Plane rows of the listed points side by side (a warp copies one, 16 bytes a lane; rows are multiples of 32 bytes).
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ plane, int words, const int* __restrict__ list,
+                                                          const int* __restrict__ count, uint4* __restrict__ out) {
+    const int lane = threadIdx.x & 31, live = __ldg(count), warps = (gridDim.x * blockDim.x) >> 5;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < live; r += warps) {
+        const uint4* src = plane + (int64_t)__ldg(list + r) * words;
+        for (int c = lane; c < words; c += 32) out[(int64_t)r * words + c] = __ldg(src + c);
     }
 }
 
@@ -362,7 +482,7 @@ struct AssignTcWs {
     int l1_cap; int64_t l1_pad; int pitch3;
     int nsplit_fb; int64_t rows_per_split_fb; int fb_bq, fb_blocks;
     PlaneLayout cl, cl3;
-    int64_t off_cplane, off_cplane3, off_xplane, off_xsq, off_xfmt, off_xsplit, off_asg_sc, off_asg_id, off_tau, off_cnt, off_l0list, off_l1list,
+    int64_t off_cplane, off_cplane3, off_xplane, off_xsq, off_xfmt, off_xsplit, off_asg_sc, off_asg_id, off_cnt, off_l0list, off_l1list,
         off_fblist, off_fblist2, off_fbpart_sc, off_fbpart_id, off_fbdist, bytes;
 };
 
@@ -405,7 +525,6 @@ static AssignTcWs assign_tc_plan(int64_t n, int K, int d, int have_xplane) {
     w.off_xsplit = w.split ? take(cur, w.l1_pad * w.pitch3 * 2) : -1;
     w.off_asg_sc = take(cur, w.n_pad * 4 * 4);
     w.off_asg_id = take(cur, w.n_pad * 2 * 4);
-    w.off_tau = take(cur, w.n_pad * 4);
     w.off_cnt = take(cur, 1024);
     w.off_l0list = take(cur, (w.split ? n : 1) * 4);
     w.off_l1list = take(cur, (int64_t)(w.l1_cap > 0 ? w.l1_cap : 1) * 4);
@@ -487,39 +606,13 @@ extern "C" int64_t fl_kmeans_assign_tc_workspace_bytes(int64_t n, int K, int d, 
 // proof accepts (scoring error about 0.0005 ||x|| max||c|| in fp16, which almost all data takes, 0.0037 in bf16) are final.  (2) d <= 128: the unproven points
 // (a device-side list) are gathered into split planes and scored again, error about 6e-5: nearly all of
 // the rest is proven.  What is left takes the exact CUDA-core path.
-extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, const float* c,
-                                       int K, int64_t ldc, int d, int32_t* labels, void* ws, int64_t ws_bytes,
-                                       int32_t* status, void* stream) {
-    FL_CHECK_ARG(n >= 0 && K >= 1 && d >= 1 && ldx >= d && ldc >= d, "fl_kmeans_assign_tc_f32: bad shape");
-    if (!assign_tc_supported(n > 0 ? n : 1, K, d)) { set_error("fl_kmeans_assign_tc_f32: d=%d > 256 is not supported", d); return FL_EUNSUPPORTED; }
-    if (n == 0) return FL_OK;
-    FL_CHECK_ARG(x && c && labels && ws, "fl_kmeans_assign_tc_f32: null pointer");
-    FL_CHECK_ARG((reinterpret_cast<uintptr_t>(ws) & 255) == 0, "fl_kmeans_assign_tc_f32: workspace must be 256-byte aligned");
-    FL_CHECK_ARG(n < (1ll << 31), "fl_kmeans_assign_tc_f32: more than 2^31 rows");
-    const AssignTcWs w = assign_tc_plan(n, K, d, xplane != nullptr);
-    if (ws_bytes < w.bytes) { set_error("fl_kmeans_assign_tc_f32: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes); return FL_EWORKSPACE; }
-    cudaStream_t st = (cudaStream_t)stream;
-    char* base = static_cast<char*>(ws);
-    if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
-
-    // sample plane (query side), whose operand format the plain centroid plane shares
-    const char* xpl = static_cast<const char*>(xplane);
-    const float2* xsq;
-    const uint32_t* fmt;
+//
+// live: inside a Lloyd loop, the points to score (n in place, or the listed ones through `gathered`, room for
+// gathered_rows plane rows); needs the second stage (d <= 128) and a sample plane.
+static int assign_tc_run(const float* x, int64_t n, int64_t ldx, const char* xpl, const float2* xsq, const uint32_t* fmt, const float* c,
+                         int K, int64_t ldc, int d, int32_t* labels, char* base, const AssignTcWs& w, const LivePoints& live,
+                         void* gathered, int64_t gathered_rows, int32_t* status, cudaStream_t st) {
     int rc;
-    if (!xpl) {
-        float2* xs = reinterpret_cast<float2*>(base + w.off_xsq);
-        uint32_t* f = reinterpret_cast<uint32_t*>(base + w.off_xfmt);
-        rc = launch_operand_format(x, n, ldx, d, f, st);
-        if (rc == FL_OK) rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs, f);
-        if (rc != FL_OK) return rc;
-        xpl = base + w.off_xplane;
-        xsq = xs;
-        fmt = f;
-    } else {
-        xsq = reinterpret_cast<const float2*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
-        fmt = reinterpret_cast<const uint32_t*>(xpl + xplane_fmt_offset(n, d));
-    }
     // centroid planes (database side): plain, and split for the second stage
     char* cpl = base + w.off_cplane;
     rc = launch_plane_build(c, K, d, ldc, cpl, st, DT_F32, fmt);
@@ -541,7 +634,6 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     const int vecx = (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int vecc = (ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(c) & 15) == 0);
     const int vec = vecx && vecc && (d % 4 == 0);
-    float* tau = reinterpret_cast<float*>(base + w.off_tau);
     float* asg_sc = reinterpret_cast<float*>(base + w.off_asg_sc);
     uint32_t* asg_id = reinterpret_cast<uint32_t*>(base + w.off_asg_id);
     const unsigned fin_grid = (unsigned)(4 * sm_count());      // grid-stride finalisation
@@ -550,23 +642,30 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
 
     // ---- stage 1: one rounding, to the samples' operand format ---------------------------------------------------------------
     {
-        rc = launch_fill_f32(tau, w.n_pad, -INFINITY, st);
-        if (rc != FL_OK) return rc;
         TcKnnParams tp{};
         tp.qplane = xpl; tp.nq = n; tp.nq_pad = w.n_pad;
         tp.dbrows = cpl + w.cl.off_rows; tp.hnorm = reinterpret_cast<const float*>(cpl + w.cl.off_hnorm);
         tp.fmt = fmt;
         tp.m = K; tp.m_pad = w.cl.m_pad; tp.d_pad = w.cl.d_pad; tp.d_used = d;
-        tp.tau = tau; tp.status = status;
+        tp.status = status;
         profile_begin(st);
-        rc = launch_assign_tc(tp, asg_sc, asg_id, nullptr, st);
+        rc = launch_assign_tc(tp, asg_sc, asg_id, live.count != nullptr ? live.count + 2 : nullptr, st);
+        if (rc == FL_OK && live.count != nullptr) {
+            // the listed points, gathered; their scores go where the pass in place would have put them
+            gather_rows_kernel<<<(unsigned)(8 * sm_count()), 256, 0, st>>>(reinterpret_cast<const uint4*>(xpl), w.pitch / 8, live.rows,
+                                                                          live.count + 1, static_cast<uint4*>(gathered));
+            FL_CHECK_LAUNCH();
+            TcKnnParams tg = tp;
+            tg.qplane = gathered; tg.nq = gathered_rows; tg.nq_pad = round_up(gathered_rows, 128);
+            rc = launch_assign_tc(tg, asg_sc, asg_id, live.count + 1, st, live.rows);
+        }
         profile_end(st);
         if (rc != FL_OK) return rc;
         if (w.split) {
             // a second, far more precise stage follows: decide what the scores' lead decides
             // without touching the rows
             assign_by_lead_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(
-                n, K, d, asg_sc, asg_id, xsq, acc1, norms, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap);
+                n, K, d, asg_sc, asg_id, xsq, acc1, norms, labels, l0_count, l0_list, (int)n, fb_count, fb_list, w.fb_cap, live);
             FL_CHECK_LAUNCH();
             // ... then, for the undecided ones only, the exact distances to the two half-winners, which
             // need half the lead; what is still open goes to the second stage
@@ -590,7 +689,7 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
         tp.qplane = xs; tp.nq = w.l1_cap; tp.nq_pad = w.l1_pad;
         tp.dbrows = cpl3 + w.cl3.off_rows; tp.hnorm = reinterpret_cast<const float*>(cpl3 + w.cl3.off_hnorm);
         tp.m = K; tp.m_pad = w.cl3.m_pad; tp.d_pad = w.cl3.d_pad; tp.d_used = 2 * w.d_pad + d;
-        tp.tau = tau; tp.status = status;
+        tp.status = status;
         rc = launch_assign_tc(tp, asg_sc, asg_id, l1_count, st);
         if (rc != FL_OK) return rc;
         assign_finalize_kernel<true><<<fin_grid, 128, 0, st>>>(
@@ -632,4 +731,154 @@ extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, c
     fp.k = 1; fp.rerank = 9; fp.row_offset = 0;
     fp.out_dist = reinterpret_cast<float*>(base + w.off_fbdist); fp.out_idx = labels; fp.verify = 0;
     return launch_knn_finalize(fp, w.fb_cap, st);
+}
+
+extern "C" int fl_kmeans_assign_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, const float* c,
+                                       int K, int64_t ldc, int d, int32_t* labels, void* ws, int64_t ws_bytes,
+                                       int32_t* status, void* stream) {
+    FL_CHECK_ARG(n >= 0 && K >= 1 && d >= 1 && ldx >= d && ldc >= d, "fl_kmeans_assign_tc_f32: bad shape");
+    if (!assign_tc_supported(n > 0 ? n : 1, K, d)) { set_error("fl_kmeans_assign_tc_f32: d=%d > 256 is not supported", d); return FL_EUNSUPPORTED; }
+    if (n == 0) return FL_OK;
+    FL_CHECK_ARG(x && c && labels && ws, "fl_kmeans_assign_tc_f32: null pointer");
+    FL_CHECK_ARG((reinterpret_cast<uintptr_t>(ws) & 255) == 0, "fl_kmeans_assign_tc_f32: workspace must be 256-byte aligned");
+    FL_CHECK_ARG(n < (1ll << 31), "fl_kmeans_assign_tc_f32: more than 2^31 rows");
+    const AssignTcWs w = assign_tc_plan(n, K, d, xplane != nullptr);
+    if (ws_bytes < w.bytes) { set_error("fl_kmeans_assign_tc_f32: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes); return FL_EWORKSPACE; }
+    cudaStream_t st = (cudaStream_t)stream;
+    char* base = static_cast<char*>(ws);
+    if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
+
+    // sample plane (query side), whose operand format the plain centroid plane shares
+    const char* xpl = static_cast<const char*>(xplane);
+    const float2* xsq;
+    const uint32_t* fmt;
+    int rc;
+    if (!xpl) {
+        float2* xs = reinterpret_cast<float2*>(base + w.off_xsq);
+        uint32_t* f = reinterpret_cast<uint32_t*>(base + w.off_xfmt);
+        rc = launch_operand_format(x, n, ldx, d, f, st);
+        if (rc == FL_OK) rc = launch_query_plane(x, n, ldx, d, base + w.off_xplane, w.n_pad, w.d_pad, st, DT_F32, xs, f);
+        if (rc != FL_OK) return rc;
+        xpl = base + w.off_xplane;
+        xsq = xs;
+        fmt = f;
+    } else {
+        xsq = reinterpret_cast<const float2*>(xpl + round_up(w.n_pad * w.pitch * 2, 1024));
+        fmt = reinterpret_cast<const uint32_t*>(xpl + xplane_fmt_offset(n, d));
+    }
+    return assign_tc_run(x, n, ldx, xpl, xsq, fmt, c, K, ldc, d, labels, base, w, LivePoints{}, nullptr, 0, status, st);
+}
+
+// ---------------------------------------------------------------------------------------
+// Whole Lloyd loops on the tensor cores.  An iteration scores only the points whose bounds no longer prove their label
+// (lloyd_bounds_kernel): all of them in the first few, a tenth later on -- and moves only the rows that change sides between
+// the sums.  1M x 128 in 1 024 clusters, 20 iterations: 9.4 ms with every point scored in every iteration, 6.4 so.
+struct LloydTcWs { AssignTcWs a; int64_t most, off_bounds, off_list, off_gather, off_count, off_prev, off_shift, bytes; };
+static LloydTcWs lloyd_tc_plan(int64_t n, int K, int d) {
+    LloydTcWs w{};
+    w.a = assign_tc_plan(n, K, d, 1);
+    // Up to this many listed points are gathered; beyond, scoring all in place is as cheap (a gathered row is read and
+    // written once more, 0.1 ns of the 0.2 that its scores take).
+    w.most = n / 2;
+    int64_t cur = w.a.bytes;
+    w.off_bounds = take(cur, n * 8);
+    w.off_list = take(cur, n * 4);
+    w.off_gather = take(cur, round_up(w.most > 0 ? w.most : 1, 128) * w.a.pitch * 2);
+    w.off_count = take(cur, 32);
+    w.off_prev = take(cur, n * 4);
+    w.off_shift = take(cur, (int64_t)K * 4);
+    w.bytes = cur;
+    return w;
+}
+
+extern "C" int fl_kmeans_lloyd_tc_supported(int64_t n, int K, int d) {
+    return n >= 1 && n < (1ll << 31) && K >= 1 && d >= 1 && assign_tc_split(d) ? 1 : 0;
+}
+extern "C" int64_t fl_kmeans_lloyd_tc_workspace_bytes(int64_t n, int K, int d) {
+    return fl_kmeans_lloyd_tc_supported(n, K, d) ? lloyd_tc_plan(n, K, d).bytes : 0;
+}
+
+extern "C" int fl_kmeans_lloyd_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, int d, int K, float* cents_a,
+                                      float* cents_b, float* sums, int32_t* cnts, int32_t* labels, int iters, float tol, int refresh,
+                                      int32_t* ctl, int32_t* host, int* n_iter, void* ws, int64_t ws_bytes, int32_t* status,
+                                      void* stream) {
+    FL_CHECK_ARG(n >= 1 && K >= 1 && d >= 1 && ldx >= d && iters >= 1 && refresh >= 1, "fl_kmeans_lloyd_tc_f32: bad shape");
+    FL_CHECK_ARG(x && xplane && cents_a && cents_b && sums && cnts && labels && ctl && n_iter && ws && (host || !(tol > 0.f)),
+                 "fl_kmeans_lloyd_tc_f32: null pointer");
+    FL_CHECK_ARG((reinterpret_cast<uintptr_t>(ws) & 255) == 0 && (reinterpret_cast<uintptr_t>(xplane) & 255) == 0,
+                 "fl_kmeans_lloyd_tc_f32: workspace and sample plane must be 256-byte aligned");
+    if (!fl_kmeans_lloyd_tc_supported(n, K, d)) { set_error("fl_kmeans_lloyd_tc_f32: n=%lld, d=%d not supported", (long long)n, d); return FL_EUNSUPPORTED; }
+    const LloydTcWs w = lloyd_tc_plan(n, K, d);
+    if (ws_bytes < w.bytes) { set_error("fl_kmeans_lloyd_tc_f32: workspace %lld < %lld bytes", (long long)ws_bytes, (long long)w.bytes); return FL_EWORKSPACE; }
+    cudaStream_t st = (cudaStream_t)stream;
+    const bool test = tol > 0.f;
+    if (test) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        FL_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+        FL_CHECK_ARG(cap == cudaStreamCaptureStatusNone, "fl_kmeans_lloyd_tc_f32: a loop that tests convergence cannot be captured");
+        *host = 0;
+    }
+    char* base = static_cast<char*>(ws);
+    const char* xpl = static_cast<const char*>(xplane);
+    const float2* xsq = reinterpret_cast<const float2*>(xpl + round_up(w.a.n_pad * w.a.pitch * 2, 1024));
+    const uint32_t* fmt = reinterpret_cast<const uint32_t*>(xpl + xplane_fmt_offset(n, d));
+    int* count = reinterpret_cast<int*>(base + w.off_count);
+    int* list = reinterpret_cast<int*>(base + w.off_list);
+    int32_t* prev = reinterpret_cast<int32_t*>(base + w.off_prev);
+    float* shift = reinterpret_cast<float*>(base + w.off_shift);
+    float2* bounds = reinterpret_cast<float2*>(base + w.off_bounds);
+    const int32_t* done = test ? ctl + LLOYD_DONE : nullptr;
+    if (status) FL_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t) * FL_STATUS_WORDS, st));
+    FL_CHECK_CUDA(cudaMemsetAsync(ctl, 0, sizeof(int32_t) * LLOYD_WORDS, st));
+    float* cur = cents_a;
+    float* nxt = cents_b;
+    auto step = [&](int it) -> int {
+        LivePoints live{};
+        live.bounds = bounds;
+        if (it > 0) {
+            FL_CHECK_CUDA(cudaMemsetAsync(count, 0, 32, st));
+            int64_t blocks = ceil_div(n, BOUNDS_THREADS * BOUNDS_PER);
+            if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+            lloyd_bounds_kernel<<<(unsigned)blocks, BOUNDS_THREADS, 0, st>>>(n, K, labels, bounds, shift, done, (int)w.most, list, count);
+            FL_CHECK_LAUNCH();
+            live.rows = list;
+            live.count = count;
+        }
+        int rc = assign_tc_run(x, n, ldx, xpl, xsq, fmt, cur, K, d, d, labels, base, w.a, live, base + w.off_gather,
+                               w.most > 0 ? w.most : 1, status, st);
+        if (rc != FL_OK) return rc;
+        if (it % refresh == 0) {
+            rc = fl_kmeans_update_f32(x, n, ldx, d, labels, K, sums, cnts, st);
+            if (rc != FL_OK) return rc;
+            FL_CHECK_CUDA(cudaMemcpyAsync(prev, labels, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
+        } else {
+            rc = fl_kmeans_update_delta_f32(x, n, ldx, d, labels, prev, K, sums, cnts, st);
+            if (rc != FL_OK) return rc;
+        }
+        return launch_kmeans_step(sums, cnts, cur, nxt, K, d, 0, tol, it, ctl, host, shift, st);
+    };
+    for (int it = 0; it < iters; ++it) {
+        // The host stays at most three iterations ahead: launches after the one that converges change nothing.
+        if (test && it >= 3) {
+            lloyd_wait(host, it - 2, st);
+            if (__atomic_load_n(host, __ATOMIC_ACQUIRE) < 0) break;
+        }
+        const int rc = step(it);
+        if (rc != FL_OK) {
+            if (test) cudaStreamSynchronize(st);           // launched steps still write to `host`
+            return rc;
+        }
+        float* t = cur; cur = nxt; nxt = t;
+    }
+    *n_iter = iters;
+    if (test) {
+        lloyd_wait(host, iters, st);
+        int v = __atomic_load_n(host, __ATOMIC_ACQUIRE);
+        if (v >= 0 && v < iters) {
+            FL_CHECK_CUDA(cudaStreamSynchronize(st));      // the stream stopped early: reports its error
+            v = __atomic_load_n(host, __ATOMIC_ACQUIRE);
+        }
+        *n_iter = v < 0 ? -v : v;
+    }
+    return FL_OK;
 }

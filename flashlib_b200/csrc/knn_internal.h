@@ -242,9 +242,11 @@ int64_t tc_query_rows_padded(int64_t nq);
 int launch_knn_tc(const TcKnnParams& p, cudaStream_t st);
 // k-means assignment on the same pipeline: asg_sc [nq_pad][2][2] (best, second-best score per
 // warpgroup half), asg_id [nq_pad][2] (best centroid per half).  Only qplane/nq_pad, dbrows/
-// m_pad/d_pad, tau (scratch) and status of `p` are used.
-// nq_dev (optional): device-resident count of live rows; query tiles beyond it are skipped.
-int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, const int* nq_dev, cudaStream_t st);
+// m_pad/d_pad/d_used, fmt and status of `p` are used.
+// nq_dev (optional): device-resident count of live rows; query tiles beyond it are skipped.  asg_rows (optional): the
+// row of the outputs that live row r writes.
+int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, const int* nq_dev, cudaStream_t st,
+                     const int* asg_rows = nullptr);
 
 // Split (hi/lo) operand planes of the second, more precise tensor-core stage (kmeans_tc.cu).
 // Database side: rows [m_pad][3 d_pad + 16] = [lo | hi | hi | norm terms] laid out by

@@ -129,6 +129,7 @@ struct TcKernelParams {
     void* lists;             // list modes: working lists of every CTA, tc_list_bytes()
     float2* gpool;           // global-pool modes: (score, row) pairs, [nq_pad][nsplit][TC_NWG][CAP]
     float* asg_sc; uint32_t* asg_id;   // assignment mode outputs: [rows][TC_NWG] x (best, second) / centroid
+    const int* asg_rows;     // optional, with nq_dev: output row of every (gathered) live query row
     int32_t* status;
     uint32_t wait_hint_ns;   // suspend-time hint of the barrier waits
     uint64_t wait_ns;        // limit of the MMA lane's barrier waits; a wait that runs out aborts the CTA
@@ -597,7 +598,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
             int t0, t1;
             tc_item_range(p, itp, split, t0, t1);
             const int64_t qrow = (int64_t)qt * TC_BM + quarter * 32 + lane;
-            float tau_in = __ldcg(p.tau + qrow);
+            float tau_in = MODE == TC_MODE_ASSIGN ? neg_inf() : __ldcg(p.tau + qrow);
             int qidx = -1;
             if (p.row_query != nullptr) {
                 // rows that belong to the same query (one per probed list) pass their thresholds on:
@@ -845,7 +846,8 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
             if (LIST) flush();
             if (!ok) break;
             if (MODE == TC_MODE_ASSIGN) {
-                const int64_t o = qrow * NWG + wg;
+                if (p.asg_rows != nullptr && qrow >= __ldcg(p.nq_dev)) continue;
+                const int64_t o = (p.asg_rows != nullptr ? (int64_t)__ldg(p.asg_rows + qrow) : qrow) * NWG + wg;
                 p.asg_sc[2 * o] = b1;
                 p.asg_sc[2 * o + 1] = b2;
                 p.asg_id[o] = (uint32_t)tbest * TC_BN + wg * (TC_BN / NWG) + (__float_as_uint(b1) & 0x7Fu);
@@ -1543,8 +1545,9 @@ int tc_prof_read(unsigned long long* host_out, int words) {
 
 // Assignment launch: queries = sample rows, database = centroids; writes per (row, warpgroup)
 // the best and second-best score and the best centroid.
-int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, const int* nq_dev, cudaStream_t st) {
-    FL_CHECK_ARG(p.qplane && p.dbrows && asg_sc && asg_id && p.tau, "tensor-core assignment launch with a null buffer");
+int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, const int* nq_dev, cudaStream_t st,
+                     const int* asg_rows) {
+    FL_CHECK_ARG(p.qplane && p.dbrows && asg_sc && asg_id && (nq_dev || !asg_rows), "tensor-core assignment launch with a null buffer");
     CUtensorMap map_q, map_q_aug, map_db, map_db_aug;
     const int pitch = p.d_pad + PLANE_AUG_COLS;
     int rc = make_map_bf16(&map_q, p.qplane, p.nq_pad, pitch, TC_BK, TC_BM);
@@ -1567,8 +1570,8 @@ int launch_assign_tc(const TcKnnParams& p, float* asg_sc, uint32_t* asg_id, cons
     kp.last_steps = tc_last_steps(p); kp.fmt = p.fmt;
     kp.nkc = sp.nkc; kp.nstage = sp.nstage;
     kp.off_b = sp.off_b; kp.off_pool_sc = sp.off_pool_sc; kp.off_pool_id = sp.off_pool_id; kp.off_bar = sp.off_bar;
-    kp.nq_pad = p.nq_pad; kp.tau = p.tau; kp.status = p.status;
-    kp.asg_sc = asg_sc; kp.asg_id = asg_id;
+    kp.nq_pad = p.nq_pad; kp.status = p.status;
+    kp.asg_rows = asg_rows; kp.asg_sc = asg_sc; kp.asg_id = asg_id;
     kp.nq_dev = nq_dev;
     kp.tile_stride = 1; kp.wait_hint_ns = tc_experiment().hint_ns;
     kp.wait_ns = tc_experiment().wait_ns;      // (a limit of zero gives up after a few microseconds of waiting)

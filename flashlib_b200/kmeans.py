@@ -258,6 +258,28 @@ def _lloyd_rows(x: torch.Tensor, K: int, cur, nxt, sums, cnts, labels, iters: in
     return n_iter.value
 
 
+def _lloyd_tc(x: torch.Tensor, K: int, cur, nxt, sums, cnts, labels, iters: int, tol: float, refresh: int) -> int:
+    """The whole Lloyd loop of one ``(N, D)`` problem on the tensor cores in one library call; returns the iterations run."""
+    lib = _lib.load()
+    _lib.require_device()
+    N, D = x.shape
+    ctl = torch.empty(lib.fl_kmeans_lloyd_words(), dtype=torch.int32, device=x.device)
+    status = torch.empty(_lib.FL_STATUS_WORDS, dtype=torch.int32, device=x.device)
+    host = torch.empty(1, dtype=torch.int32, pin_memory=True) if tol > 0.0 else None
+    n_iter = ctypes.c_int(0)
+    with torch.cuda.device(x.device):
+        xplane = _x_plane(x)
+        ws_bytes = lib.fl_kmeans_lloyd_tc_workspace_bytes(N, K, D)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
+        _lib.check(lib.fl_kmeans_lloyd_tc_f32(x.data_ptr(), N, x.stride(0), xplane.data_ptr(), D, K, cur.data_ptr(), nxt.data_ptr(),
+                                              sums.data_ptr(), cnts.data_ptr(), labels.data_ptr(), iters, max(tol, 0.0), refresh,
+                                              ctl.data_ptr(), host.data_ptr() if host is not None else None,
+                                              ctypes.addressof(n_iter), ws.data_ptr(), ws_bytes, status.data_ptr(),
+                                              _stream_ptr(x.device)))
+        _defer_status_check(status)
+    return n_iter.value
+
+
 def batch_kmeans_Euclid(x: torch.Tensor, n_clusters: int, max_iters: int = 100, tol: float = 0.0,
                         init_centroids: Optional[torch.Tensor] = None, verbose: bool = False, **_ignored):
     """Batched Lloyd k-means, ``x`` ``(B, N, D)`` on CUDA.
@@ -296,6 +318,10 @@ def batch_kmeans_Euclid(x: torch.Tensor, n_clusters: int, max_iters: int = 100, 
             x32 = x32.contiguous()
         n_iter = _lloyd_rows(x32, K, cur, nxt, sums_buf, cnts_buf, cluster_ids, max_iters, tol,
                              DELTA_REFRESH if incremental else 1)
+        return cluster_ids, (nxt if n_iter % 2 else cur).to(x.dtype), n_iter
+    if (max_iters >= 1 and N >= 1 and not verbose and incremental and _use_tensor_cores(N, K, D, assign_mode, B)
+            and _lib.load().fl_kmeans_lloyd_tc_supported(N, K, D)):
+        n_iter = _lloyd_tc(_as_f32_rows(x32[0]), K, cur, nxt, sums_buf, cnts_buf, cluster_ids, max_iters, tol, DELTA_REFRESH)
         return cluster_ids, (nxt if n_iter % 2 else cur).to(x.dtype), n_iter
     it = 0
     for it in range(max_iters):

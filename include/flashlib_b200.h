@@ -363,7 +363,17 @@ int     fl_kmeans_lloyd_words(void);
 int     fl_kmeans_lloyd_f32(const float* x, int batch, int64_t n, int64_t ldx, int64_t x_batch_stride, int d, int K,
                             float* cents_a, float* cents_b, float* sums, int32_t* cnts, int32_t* labels, int iters,
                             float tol, int refresh, int32_t* ctl, int32_t* host, int* n_iter, void* stream);
-/* 1 where that loop beats single steps with the tile kernel; 1 where an assignment is faster on the   */
+/* The same for one problem on the tensor cores (d <= 128: fl_kmeans_lloyd_tc_supported), with the      */
+/* sample plane of fl_kmeans_prepare_x_f32.  An iteration scores only the points whose distance bounds */
+/* no longer prove their label.  status: as fl_kmeans_assign_tc_f32, of the last iteration, an error   */
+/* of any.                                                                                             */
+int     fl_kmeans_lloyd_tc_supported(int64_t n, int K, int d);
+int64_t fl_kmeans_lloyd_tc_workspace_bytes(int64_t n, int K, int d);
+int     fl_kmeans_lloyd_tc_f32(const float* x, int64_t n, int64_t ldx, const void* xplane, int d, int K, float* cents_a,
+                               float* cents_b, float* sums, int32_t* cnts, int32_t* labels, int iters, float tol, int refresh,
+                               int32_t* ctl, int32_t* host, int* n_iter, void* ws, int64_t ws_bytes, int32_t* status,
+                               void* stream);
+/* 1 where fl_kmeans_lloyd_f32 beats single steps with the tile kernel; 1 where an assignment is faster on the   */
 /* CUDA cores than on the tensor cores (fl_kmeans_assign_tc_f32).                                      */
 int     fl_kmeans_lloyd_pick(int batch, int64_t n, int K, int d);
 int     fl_kmeans_assign_pick(int batch, int64_t n, int K, int d);
