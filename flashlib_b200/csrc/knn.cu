@@ -229,7 +229,7 @@ static KnnWs knn_ws_plan(int64_t nq, int64_t m, int d, int k, int mode, int stag
         const int64_t m_pad = round_up(m, 256);
         w.nq_pad = round_up(nq, 128);
         w.small = !shared_seed && (tc_small(w.nq_pad, m_pad) || d > 512);
-        if (!w.small) w.nq_pad = tc_query_rows_padded(nq);
+        if (!w.small || d > 512) w.nq_pad = tc_query_rows_padded(nq);      // (pairs of CTAs there too)
         if (w.small) {
             w.kg = k_real;                                 // (no pool in shared memory whatever d is)
             tc_small_split(w.nq_pad, m_pad, &w.nsplit, &w.rows_per_split);

@@ -60,7 +60,7 @@ constexpr int TC_B_STAGE = TC_B_CHUNK + TC_B_AUG;   // ring slot: a K-chunk, plu
                                                     // columns when it is the tile's last chunk
 // Streamed query tile (more than 512 features): a slot also holds the query tile's chunk and, for the
 // tile's last chunk, its norm columns.
-constexpr int TC_STREAM_STAGE = TC_B_STAGE + TC_A_CHUNK + TC_A_AUG;
+constexpr int TC_STREAM_A = TC_A_CHUNK + TC_A_AUG;
 constexpr int TC_MAX_STAGES = 6;
 constexpr uint64_t TC_WAIT_DEFAULT_NS = 2000000000ull;   // 2 s per wait unless the launch says otherwise
 
@@ -303,7 +303,7 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     constexpr int SLOT_CHUNK = B_ROWS * 128, SLOT_B_BYTES = B_ROWS * 128 + B_ROWS * 32;
     constexpr bool CAN_STREAM = MODE == TC_MODE_KNN_GPOOL || MODE == TC_MODE_KNN_GPOOL_BIG || MODE == TC_MODE_SEED;
     const bool stream_a = CAN_STREAM && p.stream_a != 0;
-    const uint32_t slot_bytes = stream_a ? (uint32_t)TC_STREAM_STAGE : (uint32_t)SLOT_B_BYTES;
+    const uint32_t slot_bytes = stream_a ? (uint32_t)(SLOT_B_BYTES + TC_STREAM_A) : (uint32_t)SLOT_B_BYTES;
     constexpr uint32_t OPERAND_CTAS = PAIR ? 2u : 1u;         // CTAs whose loads one operand barrier counts
 
     if (tid == 0) {
@@ -400,9 +400,9 @@ knn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                         const bool last = (kc == p.nkc - 1);
                         const uint32_t slot = b_addr + s * slot_bytes, full = BAR(B_FULL + s);
                         if (leader) {
-                            uint32_t bytes = (last ? SLOT_B_BYTES : SLOT_CHUNK) * OPERAND_CTAS;
+                            uint32_t bytes = last ? SLOT_B_BYTES : SLOT_CHUNK;
                             if (stream_a) bytes += TC_A_CHUNK + (last ? TC_A_AUG : 0);
-                            mbar_expect_tx(full, bytes);
+                            mbar_expect_tx(full, bytes * OPERAND_CTAS);
                         }
                         load(slot, &map_db, kc * TC_BK, row0, full);
                         if (last) load(slot + SLOT_CHUNK, &map_db_aug, d_pad, row0, full);
@@ -1318,7 +1318,7 @@ static int tc_prepare(const TcKnnParams& p, float* dbg, int64_t dbg_ld, TcLaunch
     const bool stream = p.d_pad > 512;
     FL_CHECK_ARG(!stream || p.pair_pools != nullptr, "tensor-core kNN launch: more than 512 features go with pair pools");
     L->sp = tc_smem_plan(p.d_pad, smem_optin_bytes(), L->mid ? TC_MID_CAP + 1 : 0,
-                         stream ? TC_STREAM_STAGE : TC_B_STAGE, stream ? 0 : 1);
+                         stream ? TC_B_STAGE + TC_STREAM_A : TC_B_STAGE, stream ? 0 : 1);
     if (L->sp.nstage < 2) { set_error("tensor-core kNN: feature dimension %d leaves no room for the TMA ring", p.d_pad); return FL_EUNSUPPORTED; }
     const TcExperiment& ex = tc_experiment();
     TcKernelParams& kp = L->kp;
@@ -1465,33 +1465,32 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
     const int pitch = p.d_pad + PLANE_AUG_COLS;
     const int items = kp.n_qtiles * kp.nsplit;
     const int grid = items < sm_count() ? items : sm_count();
-    // CTA pairs (cta_group::2): list modes over uniform ranges and an even number of query tiles.
-    const bool pair = !gp && !mid && dbg == nullptr && p.item_t0 == nullptr && p.nq_dev == nullptr &&
+    // CTA pairs (cta_group::2): list modes and streamed query tiles over uniform ranges, an even number of query tiles.  A
+    // streamed chunk of 64 features is 48 KB for 512 cycles of MMA; in a pair each CTA loads 32, which leaves room for
+    // five ring slots in place of three (2 000 x 200 000 x 768 in bf16: 996 -> 662 us, scoring 814 -> 493).
+    const bool stream = kp.stream_a != 0;
+    const bool pair = (!gp || stream) && !mid && dbg == nullptr && p.item_t0 == nullptr && p.nq_dev == nullptr &&
                       tc_pair_enabled(p.nq_pad);
-    if (L.gpb) {
-        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
-    } else if (gp) {
-        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
-        knn_tc_kernel<false, TC_MODE_KNN_GPOOL><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
-    } else if (pair) {
+    if (pair) {
         CUtensorMap map_db_h, map_db_aug_h;
         rc = cached_map_bf16(&map_db_h, p.dbrows, p.m_pad, pitch, TC_BK, TC_BN / 2);
         if (rc == FL_OK) rc = cached_map_bf16(&map_db_aug_h, p.dbrows, p.m_pad, pitch, PLANE_AUG_COLS, TC_BN / 2);
         if (rc != FL_OK) return rc;
-        const TcSmemPlan spp = tc_smem_plan(p.d_pad, smem_optin_bytes(), 0, TC_B_STAGE / 2);
+        const TcSmemPlan spp = tc_smem_plan(p.d_pad, smem_optin_bytes(), 0, TC_B_STAGE / 2 + (stream ? TC_STREAM_A : 0), stream ? 0 : 1);
         TcKernelParams kq = kp;
         kq.nstage = spp.nstage; kq.off_b = spp.off_b; kq.off_pool_sc = spp.off_pool_sc; kq.off_pool_id = spp.off_pool_id;
         kq.off_bar = spp.off_bar;
         const int pair_items = (kp.n_qtiles / 2) * kp.nsplit;
         int clusters = sm_count() / 2;
         if (clusters > pair_items) clusters = pair_items;
-        auto kern = big ? knn_tc_kernel<false, TC_MODE_KNN_BIG, true>
+        auto kern = L.gpb ? knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG, true>
+                  : gp  ? knn_tc_kernel<false, TC_MODE_KNN_GPOOL, true>
+                  : big ? knn_tc_kernel<false, TC_MODE_KNN_BIG, true>
                         : kp.dbg_flags != 0 ? knn_tc_kernel<true, TC_MODE_KNN, true> : knn_tc_kernel<false, TC_MODE_KNN, true>;
         FL_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, spp.bytes));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(2 * clusters));
-        cfg.blockDim = dim3(TC_LIST_THREADS);
+        cfg.blockDim = dim3(gp ? TC_THREADS : TC_LIST_THREADS);
         cfg.dynamicSmemBytes = (size_t)spp.bytes;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -1500,6 +1499,12 @@ static int launch_tc_main(const TcKnnParams& p, float* dbg, int64_t dbg_ld, cuda
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         FL_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, L.map_q, L.map_q_aug, map_db_h, map_db_aug_h, kq));
+    } else if (L.gpb) {
+        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
+        knn_tc_kernel<false, TC_MODE_KNN_GPOOL_BIG><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
+    } else if (gp) {
+        FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_GPOOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
+        knn_tc_kernel<false, TC_MODE_KNN_GPOOL><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
     } else if (mid) {
         FL_CHECK_CUDA(cudaFuncSetAttribute(knn_tc_kernel<false, TC_MODE_KNN_MID>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp.bytes));
         knn_tc_kernel<false, TC_MODE_KNN_MID><<<grid, TC_THREADS, sp.bytes, st>>>(L.map_q, L.map_q_aug, L.map_db, L.map_db_aug, kp);
