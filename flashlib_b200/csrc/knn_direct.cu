@@ -168,8 +168,12 @@ static __device__ __noinline__ float dir_first_threshold(const float* keys, int 
 // keys are looked at together before any is kept: a key that k of them reach is the threshold
 // from then on, so that the pools hardly ever fill -- without it every warp sorts its way
 // down from an empty pool, and four queries over 1M x 128 rows took 176 us in place of 133.
+//
+// Blocks an SM holds: four of one query and rows read four values at a time, whose eight loads a thread are then 128 KB in
+// flight (1M x 128: scan 124 us with two blocks and the next eight loads hoisted over the folding, 117 so; 4.4 TB/s).
+constexpr int dir_blocks(int nq, int npl, int vec) { return nq == 1 && npl == 1 && vec <= 4 ? 4 : 2; }
 template <int NQ, int NPL, bool F32, int VEC>
-__global__ void __launch_bounds__(DIR_THREADS, 2) direct_scan_kernel(const DirectParams p) {
+__global__ void __launch_bounds__(DIR_THREADS, dir_blocks(NQ, NPL, VEC)) direct_scan_kernel(const DirectParams p) {
     extern __shared__ __align__(16) float dir_smem[];
     constexpr int STEP = 8 * VEC;
     const int dq = (p.d + STEP - 1) / STEP * STEP;         // query pitch in shared memory, zero padded
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(DIR_THREADS, 2) direct_scan_kernel(const Direc
             for (int qi = 0; qi < NQ; ++qi) acc[j][qi] = 0.f;
         const char* row = db + (base + g) * p.ldb * ES;
         const int left = (int)(r1 - base < 32 ? r1 - base : 32);   // rows of this pass (none: <= 0)
-#pragma unroll (NQ <= 2 ? 2 : 1)
+#pragma unroll (NQ <= 2 && dir_blocks(NQ, NPL, VEC) == 2 ? 2 : 1)
         for (int f0 = 0; f0 < dq; f0 += STEP) {
             const int f = f0 + sl * VEC;
             const bool in = f < p.d;
@@ -499,7 +503,7 @@ static size_t dir_smem_bytes(int nq, int d, int step, int npl) {
 }
 
 // Queries per block and row ranges.  Four queries share a row read while that leaves a block for every SM and their rows
-// and pools take 100 KB at most, otherwise two or one; two ranges per SM, but no more than the database has passes of
+// and pools take 100 KB at most, otherwise two or one; two ranges per SM (four for one query), but no more than the database has passes of
 // a block (256 rows), dealt evenly (257 rows: 160 and 97).
 static void dir_geometry(int64_t nq, int64_t m, int d, int k, int* nqb, int* nchunk, int64_t* rows_per_chunk) {
     const int npl = dir_npl(k);
@@ -507,8 +511,9 @@ static void dir_geometry(int64_t nq, int64_t m, int d, int k, int* nqb, int* nch
     int n = DIR_MAX_QUERIES;
     while (n > 1 && (n / 2 >= nq || ceil_div(nq, n) * max_chunks < sm_count() || dir_smem_bytes(n, d, 64, npl) > 100 * 1024)) n >>= 1;
     const int64_t groups = ceil_div(nq, n);
-    int64_t c = ceil_div((int64_t)2 * sm_count(), groups);
-    if (groups < 2 * sm_count() && groups * c > 2 * sm_count() && c > 1 && groups * (c - 1) >= sm_count() * 3 / 2) --c;
+    const int64_t fit = (int64_t)dir_blocks(n, npl, 4) * sm_count();
+    int64_t c = ceil_div(fit, groups);
+    if (groups < fit && groups * c > fit && c > 1 && groups * (c - 1) >= fit * 3 / 4) --c;
     if (c > max_chunks) c = max_chunks;
     if (c < 1) c = 1;
     *rows_per_chunk = round_up(ceil_div(m, c), 32);
